@@ -175,9 +175,16 @@ struct LaunchShape {
   uint32_t park_pct = 50;       // an epoch parks its rays once at most this % of them remain
   uint32_t park_min = 4096;     // epochs of at most this many rays run to the end
   uint32_t wl_shade_min = 32;   // modes 1 and 2: rays a warp shades together once that many wait
+  uint32_t spread_warps = 16;   // resident warps per multiprocessor that a launch of few rays is spread over (the
+                                // batch sets 32 when a scene's tree is beyond an L1: kSpreadPrims)
   uint32_t loop_guard = 0;      // loop iterations of one warp of a persistent kernel before it stops
                                 // and flags error 8 (0: kDefaultLoopGuard); from omg_params.loop_guard
 };
+// A scene of more primitives than this (112 bytes each with its nodes) does not
+// stay in a multiprocessor's L1: its walks wait on L2, and twice the warps pay
+// (4096 rays on 49k primitives: 1 ray a warp 1.37 ms, 2 rays 1.45 ms; on 12
+// primitives 0.90 and 0.87 ms).
+constexpr uint32_t kSpreadPrims = 1024;
 constexpr uint32_t kDefaultLoopGuard = 1u << 22;
 
 // Wavefront state (wavefront.cu). One record per ray of the batch, indexed by

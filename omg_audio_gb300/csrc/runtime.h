@@ -120,6 +120,7 @@ struct BatchRec {
   DevBuf<WfCtl> d_wf_ctl;
   WfState wf{};
   bool coop_ok = false;           // near-tie rule and every mesh scene has a 4-wide tree (mode 2)
+  bool deep = false;              // a scene beyond kSpreadPrims primitives
   DevBuf<uint32_t> d_ep_q;        // epoch queues (2 x rays)
   DevBuf<EpochCtl> d_ep_ctl;      // kMaxEpochs + 1 records
   LaunchShape shape;

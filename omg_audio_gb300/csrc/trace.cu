@@ -15,6 +15,8 @@
 // as the reference's (and the f32 oracle's) does. The only transcendentals,
 // cos/sin of the sphere azimuth, come from the f32 sincos of
 // device_common.cuh, which the f32 oracle evaluates identically.
+#include <algorithm>
+
 #include "shade_common.cuh"
 #include "walk.cuh"
 
@@ -141,6 +143,10 @@ __device__ __noinline__ void epoch_tally(const EpochArgs& ea, bool ended, bool p
 // not a runtime flag, so that each variant carries only its own walk: the
 // loop body is then small enough for the instruction cache.
 //
+// lane_cap: lanes of a warp that take rays (launch_trace: fewer than 32 when
+// the launch has fewer rays than the chip has lanes); the other lanes take
+// part in the warp's leaf rounds.
+//
 // Registers: the launch bound (256, 4) caps a thread at 64. Across the loop a
 // lane keeps only what the walk reads (the ray, its job, the walk state); the
 // segment's hit is computed in the shading pass from the walk's result, and
@@ -156,7 +162,7 @@ __global__ void __launch_bounds__(256, 4) trace_kernel(const DJob* __restrict__ 
                                                        const DPanelGroup* __restrict__ groups, float* __restrict__ acc,
                                                     DLaunch* __restrict__ hdr, uint32_t* __restrict__ job_segments,
                                                     uint32_t refill_min, int walk_budget, uint32_t shade_min,
-                                                    EpochArgs ea) {
+                                                    uint32_t lane_cap, EpochArgs ea) {
   constexpr bool wide = TIE && WIDE;
   const unsigned FULL = 0xffffffffu;
   const uint32_t lane = threadIdx.x & 31u;
@@ -241,13 +247,13 @@ __global__ void __launch_bounds__(256, 4) trace_kernel(const DJob* __restrict__ 
       break;
     }
     // ---- refill idle lanes from the ray queue (warp-aggregated)
-    const unsigned idle = __ballot_sync(FULL, phase == IDLE);
-    if (!exhausted && idle != 0u && (__popc(idle) >= (int)refill_min || idle == FULL)) {
+    const unsigned idle = __ballot_sync(FULL, phase == IDLE && lane < lane_cap);
+    if (!exhausted && idle != 0u && (__popc(idle) >= (int)refill_min || __popc(idle) == (int)lane_cap)) {
       uint32_t base = 0;
       if (lane == 0) base = atomicAdd(fetch, (uint32_t)__popc(idle));
       base = __shfl_sync(FULL, base, 0);
       if (base >= n_rays) exhausted = true;
-      if (phase == IDLE) {
+      if (phase == IDLE && lane < lane_cap) {
         const uint32_t k = base + (uint32_t)__popc(idle & lt_mask);
         if (k < n_rays) {
           if (rq) {
@@ -618,6 +624,29 @@ cudaError_t launch_trace(const DJob* jobs, uint32_t n_jobs, uint32_t total_rays,
   const bool wl = shape.mode == 1 && ea.st.pos && threads <= 256;
   const uint32_t wl_shade = shape.wl_shade_min == 0 ? 32u : (shape.wl_shade_min > 32 ? 32u : shape.wl_shade_min);
   const bool wide = shape.wide != 0;
+  // Rays a warp holds at once. A launch with fewer rays than the chip has lanes
+  // is bound by one ray's chain of segments: its walk's dependent loads, and
+  // the other rays of its warp, whose divergent paths run one after another.
+  // So the rays are spread over as many warps as are worth keeping resident
+  // (spread_warps a multiprocessor), in blocks of 64 threads so that the
+  // multiprocessors get equal shares. Measured (rays: 32 a warp -> this rule):
+  // a 64-bounce call on the 40-room world, 4096 rays 3.90 -> 1.37 ms, 65,536
+  // rays 4.59 -> 4.28 ms; 200 bounces on the 12-triangle room, 4096 rays
+  // 1.37 -> 0.87 ms. At 65,536 rays on the small room 16 a warp is 1.60 ms
+  // against 1.53 ms, hence its lower spread_warps.
+  uint32_t lane_cap = 32;
+  if (!ep) {
+    const uint64_t warps = std::min<uint64_t>(want * threads / 32u, (uint64_t)n_sms * shape.spread_warps);
+    while (lane_cap > 1 && total_rays <= warps * (lane_cap / 2u)) lane_cap >>= 1;
+    if (lane_cap < 32u) {
+      const uint32_t spread_threads = threads < 64u ? threads : 64u;
+      want = want * threads / spread_threads;
+      threads = spread_threads;
+      need = ((uint64_t)total_rays * (32u / lane_cap) + threads - 1) / threads;
+      blocks = (uint32_t)(want < need ? want : need);
+      if (blocks == 0) blocks = 1;
+    }
+  }
 #define OMG_TRACE_LAUNCH(NB, TIE)                                                                         \
   if (wl)                                                                                                      \
     trace_wl_kernel<NB, TIE><<<blocks, threads, 0, s>>>(jobs, n_jobs, total_rays, scenes, job_mats, panels,    \
@@ -625,15 +654,15 @@ cudaError_t launch_trace(const DJob* jobs, uint32_t n_jobs, uint32_t total_rays,
   else if (TIE && wide)                                                                                        \
     trace_kernel<NB, TIE, true, false><<<blocks, threads, 0, s>>>(jobs, n_jobs, total_rays, scenes, job_mats,   \
                                                                   panels, groups, acc, hdr, job_segments, refill, \
-                                                                  steps, shade_min, ea);                          \
+                                                                  steps, shade_min, lane_cap, ea);                          \
   else if (TIE && wt)                                                                                          \
     trace_kernel<NB, TIE, false, true><<<blocks, threads, 0, s>>>(jobs, n_jobs, total_rays, scenes, job_mats,   \
                                                                   panels, groups, acc, hdr, job_segments, refill, \
-                                                                  steps, shade_min, ea);                          \
+                                                                  steps, shade_min, lane_cap, ea);                          \
   else                                                                                                         \
     trace_kernel<NB, TIE, false, false><<<blocks, threads, 0, s>>>(jobs, n_jobs, total_rays, scenes, job_mats,  \
                                                                    panels, groups, acc, hdr, job_segments, refill,\
-                                                                   steps, shade_min, ea)
+                                                                   steps, shade_min, lane_cap, ea)
   if (max_nb <= 3) {
     if (tie) OMG_TRACE_LAUNCH(3, true);
     else OMG_TRACE_LAUNCH(3, false);

@@ -277,17 +277,46 @@ int32_t alloc_batch(omg_ctx* ctx, BatchRec& B) {
   CK(B.d_job_mats.alloc(B.job_mats.size()));
   CK(B.d_panels.alloc(B.panels.size()));
   CK(B.d_groups.alloc(B.groups.size()));
-  CK(B.d_acc.alloc(B.n_acc));
-  CK(B.d_out.alloc(B.n_out));
-  CK(B.d_hdr.alloc(1));
-  CK(B.d_seg.alloc(B.n_jobs));
   CK(B.d_rjobs.alloc(B.n_jobs));
-  CK(B.d_reverb.alloc(B.n_jobs));
-  CK(B.h_out.alloc(B.n_out));
-  CK(B.h_reverb.alloc(B.n_jobs));
-  CK(B.h_hdr.alloc(1));
-  CK(B.h_seg.alloc(B.n_jobs));
   CK(B.h_jobs.alloc(B.n_jobs));
+  // the block of everything that a launch clears or returns (BatchRec::d_block)
+  size_t off = 0;
+  auto place = [&](size_t bytes) {
+    const size_t at = off;
+    off = (off + bytes + 15u) & ~(size_t)15u;
+    return at;
+  };
+  const size_t o_acc = place(B.n_acc * sizeof(float));
+  const size_t o_ep = place((kMaxEpochs + 1) * sizeof(EpochCtl));
+  const size_t o_hdr = place(sizeof(DLaunch));
+  const size_t o_seg = place(B.n_jobs * sizeof(uint32_t));
+  B.clear_bytes = off;
+  const size_t o_rev = place(B.n_jobs * sizeof(omg_reverb));
+  const size_t o_out = place(B.n_out * sizeof(float));
+  CK(B.d_block.alloc(off));
+  B.ret_off = o_hdr;
+  B.ret_bytes = o_out + B.n_out * sizeof(float) - o_hdr;
+  CK(B.h_block.alloc(B.ret_bytes));
+  unsigned char *d = B.d_block.p, *h = B.h_block.p;
+  B.d_acc = {reinterpret_cast<float*>(d + o_acc), B.n_acc};
+  B.d_ep_ctl = {reinterpret_cast<EpochCtl*>(d + o_ep), kMaxEpochs + 1};
+  B.d_hdr = {reinterpret_cast<DLaunch*>(d + o_hdr), 1};
+  B.d_seg = {reinterpret_cast<uint32_t*>(d + o_seg), B.n_jobs};
+  B.d_reverb = {reinterpret_cast<omg_reverb*>(d + o_rev), B.n_jobs};
+  B.d_out = {reinterpret_cast<float*>(d + o_out), B.n_out};
+  B.h_hdr = {reinterpret_cast<DLaunch*>(h), 1};
+  B.h_seg = {reinterpret_cast<uint32_t*>(h + (o_seg - o_hdr)), B.n_jobs};
+  B.h_reverb = {reinterpret_cast<omg_reverb*>(h + (o_rev - o_hdr)), B.n_jobs};
+  B.h_out = {reinterpret_cast<float*>(h + (o_out - o_hdr)), B.n_out};
+  if (!B.done) CK(cudaEventCreateWithFlags(&B.done, cudaEventDisableTiming));
+  return OMG_OK;
+}
+
+// The per-ray records and queues, once the batch's shape runs more than one
+// persistent mode-0 launch (not inside a capture: it allocates).
+int32_t ensure_staging(omg_ctx* ctx, BatchRec& B) {
+  const LaunchShape& sh = B.shape;
+  if (B.wf.ctl || (sh.mode == 0 && sh.epochs == 0 && sh.wf_iters == 0)) return OMG_OK;
   const size_t cap = B.total_rays;
   CK(B.d_wf_pos.alloc(cap));
   CK(B.d_wf_dir.alloc(cap));
@@ -295,12 +324,10 @@ int32_t alloc_batch(omg_ctx* ctx, BatchRec& B) {
   CK(B.d_wf_bounce.alloc(cap));
   CK(B.d_wf_queue.alloc(2 * cap));
   CK(B.d_wf_hit.alloc(cap));
-  CK(B.d_wf_ctl.alloc(1));
   CK(B.d_ep_q.alloc(2 * cap));
-  CK(B.d_ep_ctl.alloc(kMaxEpochs + 1));
+  CK(B.d_wf_ctl.alloc(1));
   B.wf = WfState{B.d_wf_pos.p, B.d_wf_dir.p, B.d_wf_e.p, B.d_wf_bounce.p, B.d_wf_hit.p, B.d_wf_queue.p,
                  B.d_wf_ctl.p, B.total_rays};
-  if (!B.done) CK(cudaEventCreateWithFlags(&B.done, cudaEventDisableTiming));
   return OMG_OK;
 }
 
@@ -327,10 +354,7 @@ int32_t upload_batch(omg_ctx* ctx, BatchRec& B) {
 // part 1: clear the scratch and trace; part 2: finalize and reverb.
 int32_t record_launch(omg_ctx* ctx, BatchRec& B, cudaStream_t s, int parts = 3) {
   if (parts & 1) {
-    CK(cudaMemsetAsync(B.d_hdr.p, 0, sizeof(DLaunch), s));
-    CK(cudaMemsetAsync(B.d_acc.p, 0, B.n_acc * sizeof(float), s));
-    CK(cudaMemsetAsync(B.d_seg.p, 0, B.n_jobs * sizeof(uint32_t), s));
-    CK(cudaMemsetAsync(B.d_ep_ctl.p, 0, (kMaxEpochs + 1) * sizeof(EpochCtl), s));
+    CK(cudaMemsetAsync(B.d_block.p, 0, B.clear_bytes, s));
     // cooperative walks need the near-tie rule and a 4-wide tree in every scene
     LaunchShape eff = B.shape;
     eff.loop_guard = ctx->prm.loop_guard;
@@ -350,19 +374,17 @@ int32_t record_launch(omg_ctx* ctx, BatchRec& B, cudaStream_t s, int parts = 3) 
 }
 
 int32_t record_readback(omg_ctx* ctx, BatchRec& B, cudaStream_t s) {
-  CK(cudaMemcpyAsync(B.h_out.p, B.d_out.p, B.n_out * sizeof(float), cudaMemcpyDeviceToHost, s));
-  CK(cudaMemcpyAsync(B.h_reverb.p, B.d_reverb.p, B.n_jobs * sizeof(omg_reverb), cudaMemcpyDeviceToHost, s));
-  CK(cudaMemcpyAsync(B.h_hdr.p, B.d_hdr.p, sizeof(DLaunch), cudaMemcpyDeviceToHost, s));
-  CK(cudaMemcpyAsync(B.h_seg.p, B.d_seg.p, B.n_jobs * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+  CK(cudaMemcpyAsync(B.h_block.p, B.d_block.p + B.ret_off, B.ret_bytes, cudaMemcpyDeviceToHost, s));
   return OMG_OK;
 }
 
 // Record the batch's work into one executable graph on capture stream cs.
 int32_t capture_graph(omg_ctx* ctx, BatchRec& B, cudaStream_t cs, bool io, int parts, cudaGraphExec_t* out) {
   cudaGraph_t g;
+  int32_t rc = ensure_staging(ctx, B);
+  if (rc) return rc;
   cudaError_t e = cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal);
   if (e != cudaSuccess) return fail(ctx, e, "cudaStreamBeginCapture");
-  int32_t rc = OMG_OK;
   if (io) {
     e = cudaMemcpyAsync(B.d_jobs.p, B.h_jobs.p, B.n_jobs * sizeof(DJob), cudaMemcpyHostToDevice, cs);
     if (e != cudaSuccess) rc = fail(ctx, e, "cudaMemcpyAsync jobs");
@@ -378,29 +400,38 @@ int32_t capture_graph(omg_ctx* ctx, BatchRec& B, cudaStream_t cs, bool io, int p
   return OMG_OK;
 }
 
-int32_t build_graphs(omg_ctx* ctx, BatchRec& B) {
+void drop_graphs(BatchRec& B) {
   for (cudaGraphExec_t* g : {&B.graph, &B.graph_io, &B.graph_a, &B.graph_b}) {
     if (*g) cudaGraphExecDestroy(*g);
     *g = nullptr;
   }
+}
+
+// One of the batch's graphs, recorded when first asked for (a batch is
+// launched through one or two of the four).
+int32_t need_graph(omg_ctx* ctx, BatchRec& B, bool io, int parts, cudaGraphExec_t* slot) {
+  if (*slot) return OMG_OK;
   cudaStream_t cs;
   CK(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
-  int32_t rc = capture_graph(ctx, B, cs, false, 3, &B.graph);
-  if (rc == OMG_OK) rc = capture_graph(ctx, B, cs, true, 3, &B.graph_io);
-  if (rc == OMG_OK) rc = capture_graph(ctx, B, cs, false, 1, &B.graph_a);
-  if (rc == OMG_OK) rc = capture_graph(ctx, B, cs, false, 2, &B.graph_b);
+  int32_t rc = capture_graph(ctx, B, cs, io, parts, slot);
   cudaStreamDestroy(cs);
   return rc;
 }
 
+// The graph a batch of this kind is launched through: with its copies (io), or the device work alone.
+int32_t build_graphs(omg_ctx* ctx, BatchRec& B, bool io) {
+  drop_graphs(B);
+  return need_graph(ctx, B, io, 3, io ? &B.graph_io : &B.graph);
+}
+
 int32_t prepare_batch(omg_ctx* ctx, BatchRec& B, const omg_job* jobs, uint32_t n_jobs, const omg_panel* panels,
-                      uint32_t n_panels) {
+                      uint32_t n_panels, bool io) {
   B.shape = ctx->shape;
   int32_t rc = fill_batch(ctx, B, jobs, n_jobs, panels, n_panels);
   if (rc) return rc;
   if ((rc = alloc_batch(ctx, B))) return rc;
   if ((rc = upload_batch(ctx, B))) return rc;
-  if ((rc = build_graphs(ctx, B))) return rc;
+  if ((rc = build_graphs(ctx, B, io))) return rc;
   B.signature = batch_signature(jobs, n_jobs, n_panels, ctx->prm);
   return OMG_OK;
 }
@@ -445,10 +476,12 @@ void copy_results(const BatchRec& B, float* bins, float* dirs, omg_reverb* rever
 int32_t run_io(omg_ctx* ctx, BatchRec& B, float* bins, float* dirs, omg_reverb* reverb) {
   std::memcpy(B.h_jobs.p, B.jobs.data(), B.n_jobs * sizeof(DJob));
   ctx->last_h2d += B.n_jobs * sizeof(DJob);
-  ctx->last_d2h = B.n_out * sizeof(float) + B.n_jobs * (sizeof(omg_reverb) + sizeof(uint32_t)) + sizeof(DLaunch);
+  ctx->last_d2h = B.ret_bytes;
+  int32_t rc = need_graph(ctx, B, true, 3, &B.graph_io);
+  if (rc) return rc;
   CK(cudaGraphLaunch(B.graph_io, ctx->stream));
   CK(cudaEventRecord(B.done, ctx->stream));
-  int32_t rc = wait_event(ctx, B.done, timeout_of(ctx));
+  rc = wait_event(ctx, B.done, timeout_of(ctx));
   if (rc) return rc;
   if ((rc = check_kernel_flags(ctx, B))) return rc;
   copy_results(B, bins, dirs, reverb);
@@ -483,7 +516,7 @@ int32_t refill_batch(omg_ctx* ctx, BatchRec& B, const omg_job* jobs, uint32_t n_
   // the context's launch shape changed since the graphs were recorded
   if (std::memcmp(&B.shape, &ctx->shape, sizeof(LaunchShape)) != 0) {
     B.shape = ctx->shape;
-    if ((rc = build_graphs(ctx, B))) return rc;
+    if ((rc = build_graphs(ctx, B, B.graph_io != nullptr))) return rc;
   }
   return OMG_OK;
 }
@@ -496,7 +529,7 @@ int32_t one_shot(omg_ctx* ctx, const omg_job* jobs, uint32_t n_jobs, const omg_p
   uint64_t sig = batch_signature(jobs, n_jobs, n_panels, ctx->prm);
   if (!ctx->cached || ctx->cached->signature != sig) {
     ctx->cached.reset(new BatchRec());
-    int32_t rc = prepare_batch(ctx, *ctx->cached, jobs, n_jobs, panels, n_panels);
+    int32_t rc = prepare_batch(ctx, *ctx->cached, jobs, n_jobs, panels, n_panels, true);
     if (rc) {
       ctx->cached.reset();
       return rc;
@@ -528,7 +561,7 @@ namespace omg {
 
 int32_t batch_prepare(omg_ctx* ctx, BatchRec& B, const omg_job* jobs, uint32_t n_jobs, const omg_panel* panels,
                       uint32_t n_panels) {
-  return prepare_batch(ctx, B, jobs, n_jobs, panels, n_panels);
+  return prepare_batch(ctx, B, jobs, n_jobs, panels, n_panels, false);
 }
 int32_t batch_refill(omg_ctx* ctx, BatchRec& B, const omg_job* jobs, uint32_t n_jobs, const omg_panel* panels,
                      uint32_t n_panels) {
@@ -538,6 +571,11 @@ uint64_t batch_layout(const omg_job* jobs, uint32_t n_jobs, uint32_t n_panels, c
   return batch_signature(jobs, n_jobs, n_panels, P);
 }
 int32_t batch_flags(omg_ctx* ctx, const BatchRec& B) { return check_kernel_flags(ctx, B); }
+int32_t batch_graph(omg_ctx* ctx, BatchRec& B, cudaGraphExec_t* g) {
+  int32_t rc = need_graph(ctx, B, false, 3, &B.graph);
+  *g = B.graph;
+  return rc;
+}
 
 }  // namespace omg
 
@@ -595,7 +633,7 @@ int32_t omg_set_limits(omg_ctx* ctx, uint32_t walk_budget, uint32_t loop_guard) 
   // the loop guard is a kernel argument recorded in each batch's graphs
   ctx->cached.reset();
   for (auto& kv : ctx->batches)
-    if ((rc = build_graphs(ctx, *kv.second))) return rc;
+    if ((rc = build_graphs(ctx, *kv.second, false))) return rc;
   return OMG_OK;
 }
 
@@ -661,7 +699,7 @@ int32_t omg_batch_create(omg_ctx* ctx, const omg_job* jobs, uint32_t n_jobs, con
                          uint32_t n_panels, uint32_t* batch_id) {
   if (!ctx || !jobs || !n_jobs || !batch_id || (n_panels && !panels)) return OMG_E_INVALID;
   std::unique_ptr<BatchRec> B(new BatchRec());
-  int32_t rc = prepare_batch(ctx, *B, jobs, n_jobs, panels, n_panels);
+  int32_t rc = prepare_batch(ctx, *B, jobs, n_jobs, panels, n_panels, false);
   if (rc) return rc;
   *batch_id = ctx->next_batch++;
   ctx->batches[*batch_id] = std::move(B);
@@ -675,7 +713,10 @@ int32_t omg_batch_launch_part(omg_ctx* ctx, uint32_t id, uint32_t part) {
   auto it = ctx->batches.find(id);
   if (it == ctx->batches.end()) return OMG_E_NOT_FOUND;
   BatchRec& B = *it->second;
-  CK(cudaGraphLaunch(part == 0 ? B.graph : (part == 1 ? B.graph_a : B.graph_b), ctx->stream));
+  cudaGraphExec_t* g = part == 0 ? &B.graph : (part == 1 ? &B.graph_a : &B.graph_b);
+  int32_t rc = need_graph(ctx, B, false, part == 0 ? 3 : (int)part, g);
+  if (rc) return rc;
+  CK(cudaGraphLaunch(*g, ctx->stream));
   return OMG_OK;
 }
 
@@ -785,7 +826,7 @@ int32_t omg_submit_world(omg_ctx* ctx, uint32_t scene_id, const omg_world_job* j
   job_from_world(j, scene_id, *job, n_panels);
   Ticket t;
   t.batch.reset(new BatchRec());
-  int32_t rc = prepare_batch(ctx, *t.batch, &j, 1, panels, n_panels);
+  int32_t rc = prepare_batch(ctx, *t.batch, &j, 1, panels, n_panels, true);
   if (rc) return rc;
   BatchRec& B = *t.batch;
   std::memcpy(B.h_jobs.p, B.jobs.data(), sizeof(DJob));
@@ -970,7 +1011,7 @@ int32_t omg_batch_autotune(omg_ctx* ctx, uint32_t id, uint32_t reps, omg_tune_re
   cudaEventDestroy(e1);
   B.shape = rc == OMG_OK ? best_shape : keep;
   if (rc) return rc;
-  if ((rc = build_graphs(ctx, B))) return rc;
+  if ((rc = build_graphs(ctx, B, false))) return rc;
   ctx->shape = best_shape;
   shape_to_result(best_shape, best_ms, best);
   return OMG_OK;
@@ -1002,7 +1043,7 @@ int32_t omg_batch_set_shape(omg_ctx* ctx, uint32_t id, const omg_tune_result* sh
   sh.wide = shape->wide ? 1u : 0u;
   sh.wl_shade_min = shape->wl_shade_min == 0 ? 32u : shape->wl_shade_min;
   B.shape = sh;
-  int32_t rc = build_graphs(ctx, B);
+  int32_t rc = build_graphs(ctx, B, false);
   if (rc) return rc;
   ctx->shape = sh;
   return OMG_OK;

@@ -157,7 +157,9 @@ int32_t omg_late_submit(omg_ctx* ctx, uint32_t field_id, const uint32_t* slots, 
     }
     std::memcpy(B->h_jobs.p, B->jobs.data(), n_jobs * sizeof(DJob));
     CK(cudaMemcpyAsync(B->d_jobs.p, B->h_jobs.p, n_jobs * sizeof(DJob), cudaMemcpyHostToDevice, ctx->stream));
-    CK(cudaGraphLaunch(B->graph, ctx->stream));
+    cudaGraphExec_t g = nullptr;
+    if ((rc = batch_graph(ctx, *B, &g))) return rc;
+    CK(cudaGraphLaunch(g, ctx->stream));
     CK(cudaMemcpyAsync(L.d_up.p, L.h_up.p, n_jobs * sizeof(DLateUpdate), cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaMemcpyAsync(L.d_rj.p, L.h_rj.p, n_jobs * sizeof(DReverbJob), cudaMemcpyHostToDevice, ctx->stream));
     CK(launch_late_update(L.d_up.p, n_jobs, B->d_out.p, L.avg.p, L.version.p, L.d_rj.p, L.d_rev.p, L.state.p,

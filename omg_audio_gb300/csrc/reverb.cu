@@ -1,9 +1,16 @@
-// estimate_reverb on the GPU (crates/omg-core/src/tracer.rs:204-257): one warp
-// per (echogram, band). FP64 is used only here, for the Schroeder backward
-// integral and the line fit. The late level is the reference's own f32 sum of
-// the bins from 80 ms on, in its order (tracer.rs:246-254), by one lane. The
-// warp first stages the band's bins in shared memory (coalesced loads), so the
-// sequential sums read shared memory instead of waiting on one load each.
+// estimate_reverb on the GPU (crates/omg-core/src/tracer.rs:204-257): one
+// block per (echogram, band). FP64 is used only here, for the Schroeder
+// backward integral and the line fit. The late level is the reference's own
+// f32 sum of the bins from 80 ms on, in its order (tracer.rs:246-254).
+//
+// What bounds it: serial chains. The FP64 unit takes a warp's add 16 cycles
+// and returns it some 40 later, so one warp per band (chunks of 63 bins of a
+// 2000-bin curve summed one after another, twice) took 49 us for one job and
+// 108 us for 64. Here kEdcThreads threads sum chunks a quarter as long, a
+// block-wide scan joins them, and one further warp runs the late level's
+// sequential f32 sum (4 cycles an add, its loads ahead of it) beside them.
+// Shared memory holds one 8-byte slot a bin: the bin, then its place on the
+// curve.
 #include <cfloat>
 
 #include "omg_internal.h"
@@ -12,21 +19,30 @@ namespace omg {
 
 namespace {
 
+constexpr uint32_t kEdcThreads = 128;
+constexpr uint32_t kEdcWarps = kEdcThreads / 32;
+constexpr uint32_t kReverbThreads = kEdcThreads + 32;   // the last warp: the late level
+
 __device__ __forceinline__ double db_of(double e, double total) {
   return 10.0 * log10(fmax(e / total, 1e-12));
 }
 
-__global__ void reverb_kernel(const DReverbJob* __restrict__ rj, uint32_t n_jobs, const float* __restrict__ bins,
-                              omg_reverb* __restrict__ out, const uint32_t* __restrict__ job_segments,
-                              uint32_t max_bins) {
-  extern __shared__ double edc[];           // max_bins doubles, then the band's bins (max_bins floats)
-  float* sb = reinterpret_cast<float*>(edc + max_bins);
+// the warps of the decay curve only (named barrier 1)
+__device__ __forceinline__ void edc_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kEdcThreads) : "memory"); }
+
+__global__ void __launch_bounds__(kReverbThreads)
+    reverb_kernel(const DReverbJob* __restrict__ rj, uint32_t n_jobs, const float* __restrict__ bins,
+                  omg_reverb* __restrict__ out, const uint32_t* __restrict__ job_segments) {
+  extern __shared__ double edc[];           // n bins: first as f32 in each slot's low word, then the FP64 curve
+  __shared__ double s_tot[kEdcWarps];
+  __shared__ uint32_t s_f5[kEdcWarps], s_f25[kEdcWarps], s_neg[kEdcWarps];
+  __shared__ double s_fit[4][kEdcWarps];
   const uint32_t j = blockIdx.x, b = blockIdx.y;
   const DReverbJob R = rj[j];
-  const uint32_t lane = threadIdx.x;
+  const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
   if (j >= n_jobs) return;
   if (b >= R.nb) {
-    if (b < OMG_MAX_BANDS && lane == 0) {
+    if (b < OMG_MAX_BANDS && tid == 0) {
       out[j].rt60[b] = 0.0f;
       out[j].level[b] = 0.0f;
       out[j].rt60_fit[b] = 0.0f;
@@ -35,34 +51,91 @@ __global__ void reverb_kernel(const DReverbJob* __restrict__ rj, uint32_t n_jobs
   }
   const uint32_t n = R.n_bins, nb = R.nb;
   const float* B = bins + R.bins_off;
-  for (uint32_t i = lane; i < n; i += 32) sb[i] = B[(uint64_t)i * nb + b];
-  __syncwarp();
-  // per-lane contiguous chunk, sequential backward sum, then a suffix scan of
-  // the chunk totals across the warp
-  const uint32_t chunk = (n + 31) / 32;
-  const uint32_t lo = lane * chunk, hi = min(n, lo + chunk);
+
+  if (warp == kEdcWarps) {
+    // tracer.rs:246: late_start = (0.080 / BIN_DT) as usize in f32. The warp
+    // loads kAhead groups of 32 bins while it adds the previous ones, bin after
+    // bin, every lane the same sum.
+    constexpr uint32_t kAhead = 4;
+    const float q = 0.080f / R.bin_dt;
+    const uint64_t ls = (q >= 0.0f) ? (uint64_t)q : 0;
+    float late = 0.0f;
+    if (ls < n) {
+      float cur[kAhead], nxt[kAhead];
+      auto load = [&](float (&v)[kAhead], uint32_t i0) {
+#pragma unroll
+        for (uint32_t g = 0; g < kAhead; g++) {
+          const uint32_t i = i0 + 32u * g + lane;
+          v[g] = i < n ? B[(uint64_t)i * nb + b] : 0.0f;
+        }
+      };
+      load(cur, (uint32_t)ls);
+      for (uint32_t i0 = (uint32_t)ls; i0 < n; i0 += 32u * kAhead) {
+        load(nxt, i0 + 32u * kAhead);
+#pragma unroll
+        for (uint32_t g = 0; g < kAhead; g++) {
+          const uint32_t left = n - min(n, i0 + 32u * g);
+          if (left >= 32u) {
+#pragma unroll
+            for (int k = 0; k < 32; k++) late += __shfl_sync(0xffffffffu, cur[g], k);
+          } else {
+            for (uint32_t k = 0; k < left; k++) late += __shfl_sync(0xffffffffu, cur[g], (int)k);
+          }
+          cur[g] = nxt[g];
+        }
+      }
+    }
+    if (lane == 0) {
+      out[j].level[b] = fminf(sqrtf(late), 0.7f);
+      if (b == 0) out[j].segments = job_segments ? job_segments[j] : 0;
+    }
+    return;
+  }
+
+  bool neg = false;
+  for (uint32_t i = tid; i < n; i += kEdcThreads) {
+    const float v = B[(uint64_t)i * nb + b];
+    neg |= v < 0.0f;
+    reinterpret_cast<float*>(edc)[2u * i] = v;
+  }
+  neg = __any_sync(0xffffffffu, neg);
+  if (lane == 0) s_neg[warp] = neg ? 1u : 0u;
+  edc_sync();
+  bool any_neg = false;
+  for (uint32_t w = 0; w < kEdcWarps; w++) any_neg |= s_neg[w] != 0u;
+
+  // per-thread contiguous chunk, sequential backward sum, then an exclusive
+  // suffix scan of the chunk totals over the block
+  const uint32_t chunk = (n + kEdcThreads - 1) / kEdcThreads;
+  const uint32_t lo = min(n, tid * chunk), hi = min(n, lo + chunk);
   double run = 0.0;
   for (int64_t i = (int64_t)hi - 1; i >= (int64_t)lo; i--) {
-    run += (double)sb[i];
+    run += (double)reinterpret_cast<const float*>(edc)[2 * i];
     edc[i] = run;
   }
-  // exclusive suffix of chunk totals: sum over lanes > lane
   double incl = run;
   for (int off = 1; off < 32; off <<= 1) {
-    double v = __shfl_down_sync(0xffffffffu, incl, off);
+    const double v = __shfl_down_sync(0xffffffffu, incl, off);
     if (lane + off < 32) incl += v;
   }
-  const double after = incl - run;
+  if (lane == 0) s_tot[warp] = incl;
+  double after = __shfl_down_sync(0xffffffffu, incl, 1);
+  if (lane == 31) after = 0.0;
+  edc_sync();
+  double later = 0.0;
+  for (uint32_t w = kEdcWarps - 1; w > warp; w--) later += s_tot[w];
+  after += later;
   for (uint32_t i = lo; i < hi; i++) edc[i] += after;
-  __syncwarp();
-  const double total = __shfl_sync(0xffffffffu, incl, 0);
+  edc_sync();
+  const double total = edc[0];
 
   float rt60 = 0.5f, fit = 0.5f;
   if (total > 0.0) {
-    // first bins at <= -5 dB and <= -25 dB. The EDC is non-increasing, so each
-    // lane stops at its first bin past both levels. The dB value is computed
-    // only for a bin within 1e-9 (relative) of a level's energy: elsewhere the
-    // energy ratio decides the same comparison, without a logarithm per bin.
+    // first bins at <= -5 dB and <= -25 dB. The curve of bins that are not
+    // negative does not rise, so a chunk whose last bin is above -5 dB holds
+    // neither. The dB value is computed only for a bin within 1e-9 (relative)
+    // of a level's energy: elsewhere the energy ratio decides the same
+    // comparison, without a logarithm per bin.
     const double r5 = sqrt(0.1);            // 10^(-5/10)
     const double e5 = total * r5, e25 = total * (r5 * 0.01);
     auto below = [&](double e, double level, double thr) {
@@ -71,14 +144,23 @@ __global__ void reverb_kernel(const DReverbJob* __restrict__ rj, uint32_t n_jobs
       return db_of(e, total) <= level;
     };
     uint32_t f5 = 0xFFFFFFFFu, f25 = 0xFFFFFFFFu;
-    for (uint32_t i = lane; i < n && f25 == 0xFFFFFFFFu; i += 32) {
-      const double e = edc[i];
-      if (f5 == 0xFFFFFFFFu && below(e, -5.0, e5)) f5 = i;
-      if (below(e, -25.0, e25)) f25 = i;
+    if (lo < hi && (any_neg || below(edc[hi - 1], -5.0, e5))) {
+      for (uint32_t i = lo; i < hi && f25 == 0xFFFFFFFFu; i++) {
+        const double e = edc[i];
+        if (f5 == 0xFFFFFFFFu && below(e, -5.0, e5)) f5 = i;
+        if (below(e, -25.0, e25)) f25 = i;
+      }
     }
-    for (int off = 16; off > 0; off >>= 1) {
-      f5 = min(f5, __shfl_xor_sync(0xffffffffu, f5, off));
-      f25 = min(f25, __shfl_xor_sync(0xffffffffu, f25, off));
+    f5 = __reduce_min_sync(0xffffffffu, f5);
+    f25 = __reduce_min_sync(0xffffffffu, f25);
+    if (lane == 0) {
+      s_f5[warp] = f5;
+      s_f25[warp] = f25;
+    }
+    edc_sync();
+    for (uint32_t w = 0; w < kEdcWarps; w++) {
+      f5 = min(f5, s_f5[w]);
+      f25 = min(f25, s_f25[w]);
     }
     // the reference stops scanning at t25, so t5 is only set when found first
     if (f25 != 0xFFFFFFFFu && f5 != 0xFFFFFFFFu && f5 <= f25 && f25 > f5) {
@@ -88,7 +170,7 @@ __global__ void reverb_kernel(const DReverbJob* __restrict__ rj, uint32_t n_jobs
       rt60 = fminf(fmaxf(-60.0f * dt / ddb, 0.1f), 5.0f);
       // least-squares T20 line of dB(EDC) over [t5, t25]
       double sx = 0, sy = 0, sxx = 0, sxy = 0;
-      for (uint32_t i = f5 + lane; i <= f25; i += 32) {
+      for (uint32_t i = f5 + tid; i <= f25; i += kEdcThreads) {
         const double x = (double)i * (double)R.bin_dt, y = db_of(edc[i], total);
         sx += x; sy += y; sxx += x * x; sxy += x * y;
       }
@@ -98,24 +180,33 @@ __global__ void reverb_kernel(const DReverbJob* __restrict__ rj, uint32_t n_jobs
         sxx += __shfl_xor_sync(0xffffffffu, sxx, off);
         sxy += __shfl_xor_sync(0xffffffffu, sxy, off);
       }
-      const double cnt = (double)(f25 - f5 + 1);
-      const double den = cnt * sxx - sx * sx;
-      if (den > 0) {
-        const double slope = (cnt * sxy - sx * sy) / den;
-        if (slope < 0) fit = (float)fmin(fmax(-60.0 / slope, 0.1), 5.0);
+      if (lane == 0) {
+        s_fit[0][warp] = sx;
+        s_fit[1][warp] = sy;
+        s_fit[2][warp] = sxx;
+        s_fit[3][warp] = sxy;
+      }
+      edc_sync();
+      if (tid == 0) {
+        sx = sy = sxx = sxy = 0.0;
+        for (uint32_t w = 0; w < kEdcWarps; w++) {
+          sx += s_fit[0][w];
+          sy += s_fit[1][w];
+          sxx += s_fit[2][w];
+          sxy += s_fit[3][w];
+        }
+        const double cnt = (double)(f25 - f5 + 1);
+        const double den = cnt * sxx - sx * sx;
+        if (den > 0) {
+          const double slope = (cnt * sxy - sx * sy) / den;
+          if (slope < 0) fit = (float)fmin(fmax(-60.0 / slope, 0.1), 5.0);
+        }
       }
     }
   }
-  if (lane == 0) {
+  if (tid == 0) {
     out[j].rt60[b] = rt60;
     out[j].rt60_fit[b] = fit;
-    // tracer.rs:246: late_start = (0.080 / BIN_DT) as usize in f32
-    const float q = 0.080f / R.bin_dt;
-    const uint64_t ls = (q >= 0.0f) ? (uint64_t)q : 0;
-    float late = 0.0f;
-    for (uint64_t i = ls; i < n; i++) late += sb[i];
-    out[j].level[b] = fminf(sqrtf(late), 0.7f);
-    if (b == 0) out[j].segments = job_segments ? job_segments[j] : 0;
   }
 }
 
@@ -124,14 +215,14 @@ __global__ void reverb_kernel(const DReverbJob* __restrict__ rj, uint32_t n_jobs
 cudaError_t launch_reverb(const DReverbJob* rj, uint32_t n_jobs, uint32_t max_bins, const float* bins,
                           omg_reverb* out, const uint32_t* job_segments, cudaStream_t s) {
   if (n_jobs == 0) return cudaSuccess;
-  size_t smem = (size_t)max_bins * (sizeof(double) + sizeof(float));
-  if (smem > 227 * 1024) return cudaErrorInvalidValue;   // more than 19,370 bins: beyond a block's shared memory
-  if (smem > 48 * 1024) {
+  if (max_bins > kMaxBins) return cudaErrorInvalidValue;
+  const size_t smem = (size_t)max_bins * sizeof(double);
+  if (smem > 40 * 1024) {   // beyond the default limit with the block's own few arrays
     cudaError_t e = cudaFuncSetAttribute(reverb_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
   }
   dim3 grid(n_jobs, OMG_MAX_BANDS);
-  reverb_kernel<<<grid, 32, smem, s>>>(rj, n_jobs, bins, out, job_segments, max_bins);
+  reverb_kernel<<<grid, kReverbThreads, smem, s>>>(rj, n_jobs, bins, out, job_segments);
   return cudaGetLastError();
 }
 

@@ -56,6 +56,13 @@ struct PinBuf {
   }
 };
 
+// A typed range inside a buffer that another member owns.
+template <class T>
+struct BufView {
+  T* p = nullptr;
+  size_t n = 0;
+};
+
 struct SceneRec {
   uint32_t n_tris = 0, n_prims = 0, n_nodes = 0, n_bands = 3;
   int32_t root = 0;
@@ -103,17 +110,23 @@ struct BatchRec {
   DevBuf<DMat> d_job_mats;
   DevBuf<DPanel> d_panels;
   DevBuf<DPanelGroup> d_groups;
-  DevBuf<float> d_acc, d_out;
-  DevBuf<DLaunch> d_hdr;
-  DevBuf<uint32_t> d_seg;
   DevBuf<DReverbJob> d_rjobs;
-  DevBuf<omg_reverb> d_reverb;
-  PinBuf<float> h_out;
-  PinBuf<omg_reverb> h_reverb;
-  PinBuf<DLaunch> h_hdr;
-  PinBuf<uint32_t> h_seg;
+  // One device block and its pinned image of the part that travels back, laid
+  // out [acc | epoch records | header | segments | reverb | echograms]: one
+  // memset clears the first clear_bytes (up to the segments), one copy returns
+  // everything from ret_off (the header) on.
+  DevBuf<unsigned char> d_block;
+  PinBuf<unsigned char> h_block;
+  size_t clear_bytes = 0, ret_off = 0, ret_bytes = 0;
+  BufView<float> d_acc, d_out, h_out;
+  BufView<EpochCtl> d_ep_ctl;     // kMaxEpochs + 1 records
+  BufView<DLaunch> d_hdr, h_hdr;
+  BufView<uint32_t> d_seg, h_seg;
+  BufView<omg_reverb> d_reverb, h_reverb;
   PinBuf<DJob> h_jobs;
-  // wavefront rounds: per-ray state, two ray-id queues, control block
+  // launch shapes beyond one persistent launch (wavefront rounds, epochs, modes
+  // 1 and 2): per-ray state, two ray-id queues, control block; allocated once
+  // a shape needs them
   DevBuf<float4> d_wf_pos, d_wf_dir, d_wf_e;
   DevBuf<uint32_t> d_wf_bounce, d_wf_queue;
   DevBuf<float2> d_wf_hit;
@@ -122,8 +135,8 @@ struct BatchRec {
   bool coop_ok = false;           // near-tie rule and every mesh scene has a 4-wide tree (mode 2)
   bool deep = false;              // a scene beyond kSpreadPrims primitives
   DevBuf<uint32_t> d_ep_q;        // epoch queues (2 x rays)
-  DevBuf<EpochCtl> d_ep_ctl;      // kMaxEpochs + 1 records
   LaunchShape shape;
+  // recorded when first needed (batch_graph)
   cudaGraphExec_t graph = nullptr;         // device-only launch
   cudaGraphExec_t graph_io = nullptr;      // H2D jobs + launch + D2H results
   cudaGraphExec_t graph_a = nullptr;       // clear + trace
@@ -204,6 +217,8 @@ int32_t batch_refill(omg_ctx* ctx, BatchRec& B, const omg_job* jobs, uint32_t n_
                      uint32_t n_panels);
 uint64_t batch_layout(const omg_job* jobs, uint32_t n_jobs, uint32_t n_panels, const omg_params& P);
 int32_t batch_flags(omg_ctx* ctx, const BatchRec& B);
+// The batch's device-only graph (clear, trace, finalize, reverb), recorded when first asked for.
+int32_t batch_graph(omg_ctx* ctx, BatchRec& B, cudaGraphExec_t* g);
 constexpr uint32_t kMaxScenes = 4096;     // scene ids 1 .. kMaxScenes-1
 bool valid_material(const omg_material& m, uint32_t nb);
 bool finite3(const float* v);

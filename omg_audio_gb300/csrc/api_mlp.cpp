@@ -9,70 +9,54 @@
 #include <numeric>
 #include <random>
 
+#include "mlp_net.h"
 #include "runtime.h"
 
 using namespace omg;
 
 namespace omg {
 
-struct MlpLayer {
-  uint32_t in = 0, out = 0;
-  DevBuf<float> W, b, mW, vW, mb, vb;
-  float* gW = nullptr;    // the gradients: views into the member's gradient block
-  float* gb = nullptr;
-  DevBuf<uint16_t> Wh;    // bf16 copy of W [out x in]
-  DevBuf<uint16_t> Wht;   // its transpose [in x out]: the K-major operand of dX = dZ . W
+// Scratch of one launch of `tiles` 128-row tiles of `members` members
+// (MlpRowsArgs): the images that the weight gradients read, GELU'(Z).
+struct MlpScratch {
+  uint64_t tiles = 0;              // members x tiles
+  DevBuf<uint16_t> xt, at, dzt;
+  DevBuf<float> gz;
 };
 
-// The work buffers of one batch of `cap` rows. Besides the row-major
-// activations and gradients, the backward pass keeps their bf16 transposes
-// (xht, At, dZht: [features x rows]), so that every GEMM of training reads
-// both operands K-major (the pipelined path of mlp.cu).
-struct MlpBufs {
+// One of the two chunks of rows in flight during inference.
+struct MlpChunk {
   uint32_t cap = 0;
-  DevBuf<uint16_t> xh, xht;               // batch input (bf16) and its transpose
-  DevBuf<float> t;                        // batch targets
-  std::vector<DevBuf<float>> Z;           // pre-activations per layer
-  std::vector<DevBuf<uint16_t>> A, At;    // bf16 activations per hidden layer, and transposes
-  DevBuf<float> out, dX, dZ;
-  DevBuf<uint16_t> dZh, dZht;
-};
-
-// One ensemble member's training lane: its buffers, stream, step graph,
-// epoch permutation and device step counter.
-struct MlpTrainer {
-  MlpBufs bufs;
-  cudaStream_t stream = nullptr;
-  cudaGraphExec_t graph = nullptr;
-  DevBuf<uint32_t> perm, step;
-  PinBuf<uint32_t> h_perm;
-  PinBuf<float> h_loss;
-  ~MlpTrainer() {
-    if (graph) cudaGraphExecDestroy(graph);
-    if (stream) cudaStreamDestroy(stream);
+  DevBuf<float> x, y, mean, std, spread;   // y: [member][row][out]
+  PinBuf<float> h_x, h_mean, h_std, h_spread;
+  cudaEvent_t done = nullptr;
+  ~MlpChunk() {
+    if (done) cudaEventDestroy(done);
   }
 };
 
 struct MlpRec {
   omg_mlp_config cfg{};
-  std::vector<std::vector<MlpLayer>> members;   // [member][layer]
-  // per member, one block: every layer's gW then gb, then the loss (one memset clears it)
-  std::vector<DevBuf<float>> grads;
-  uint64_t grad_floats = 0;
+  MlpNet net{};
+  // every member's parameters, AdamW moments and gradients (net.p_stride floats a member), the
+  // weights' bf16 images
+  DevBuf<float> P, M1, V1, G;
+  DevBuf<uint16_t> img;
+  DevBuf<float> loss;                           // per member
   // standardization (host and device)
   std::vector<float> x_mean, x_std, y_mean, y_std;
   DevBuf<float> d_x_mean, d_x_std, d_y_mean, d_y_std;
-  // inference buffers
-  uint32_t icap = 0;
-  DevBuf<float> xin, acc, acc2;
-  PinBuf<float> h_x, h_mean, h_std;
+  MlpChunk chunk[2];                            // inference
+  MlpScratch train_s, grad_s;
+  DevBuf<float> grad_x, grad_y;                 // omg_mlp_grad's batch
   // dataset (standardized, device)
   uint32_t n_data = 0;
   DevBuf<float> X, Y;
   uint64_t step = 0;
-  MlpBufs io;                                   // inference and omg_mlp_grad, on the context's stream
-  std::vector<std::unique_ptr<MlpTrainer>> trainers;   // training, one per member
   DevBuf<float> sched;                          // per step: learning rate, bias corrections 1 and 2
+  DevBuf<uint32_t> perm, counters;              // two epochs' permutations; step counter, ticket
+  PinBuf<uint32_t> h_perm;
+  DevBuf<float> epoch_loss;
   DevBuf<uint32_t> err;
   PinBuf<float> h_loss;
 };
@@ -83,134 +67,76 @@ namespace {
 
 uint32_t n_layers(const MlpRec& M) { return M.cfg.n_hidden + 1; }
 
-int32_t ensure_batch(omg_ctx* ctx, const MlpRec& M, MlpBufs& W, uint32_t rows, bool backward) {
-  if (rows <= W.cap) return OMG_OK;
-  const uint32_t L = n_layers(M), H = M.cfg.hidden;
-  CK(W.xh.alloc((size_t)rows * M.cfg.n_in));
-  CK(W.t.alloc((size_t)rows * M.cfg.n_out));
-  W.Z.resize(L);
-  W.A.resize(L);
-  W.At.resize(L);
-  for (uint32_t l = 0; l < L; l++) {
-    const uint32_t o = l + 1 == L ? M.cfg.n_out : H;
-    CK(W.Z[l].alloc((size_t)rows * o));
-    CK(W.A[l].alloc((size_t)rows * o));
-    if (backward) CK(W.At[l].alloc((size_t)rows * o));
+// The layout of one member (MlpLayerDesc).
+MlpNet make_net(const omg_mlp_config& c) {
+  MlpNet N{};
+  N.n_layers = c.n_hidden + 1;
+  N.members = c.members;
+  uint32_t in = c.n_in, p = 0, im = 0;
+  for (uint32_t l = 0; l < N.n_layers; l++) {
+    MlpLayerDesc& D = N.L[l];
+    D.in = in;
+    D.out = l + 1 == N.n_layers ? c.n_out : c.hidden;
+    D.ip = (D.in + 15u) & ~15u;
+    D.op = (D.out + 15u) & ~15u;
+    D.w_off = p;
+    p += (D.in * D.out + 3u) & ~3u;
+    D.b_off = p;
+    p += (D.out + 3u) & ~3u;
+    D.img_off = im;
+    im += D.ip * D.op;
+    in = D.out;
   }
-  const uint32_t wide = std::max(std::max(H, M.cfg.n_out), M.cfg.n_in);
-  CK(W.out.alloc((size_t)rows * M.cfg.n_out));
-  CK(W.dX.alloc((size_t)rows * wide));
-  CK(W.dZ.alloc((size_t)rows * wide));
-  CK(W.dZh.alloc((size_t)rows * wide));
-  if (backward) {
-    CK(W.xht.alloc((size_t)rows * M.cfg.n_in));
-    CK(W.dZht.alloc((size_t)rows * wide));
-  }
-  W.cap = rows;
+  N.p_stride = p;
+  N.img_stride = im;
+  return N;
+}
+
+int32_t ensure_scratch(omg_ctx* ctx, const MlpRec& M, MlpScratch& S, uint64_t tiles) {
+  if (tiles <= S.tiles) return OMG_OK;
+  const uint32_t L = n_layers(M);
+  S.tiles = 0;
+  CK(S.xt.alloc(tiles * 128u * M.net.L[0].ip));
+  CK(S.at.alloc(tiles * (L - 1) * 128u * M.cfg.hidden));
+  CK(S.dzt.alloc(tiles * L * 128u * kMlpWide));
+  CK(S.gz.alloc(tiles * (L - 1) * 128u * M.cfg.hidden));
+  S.tiles = tiles;
   return OMG_OK;
 }
 
-// columns per CTA of a GEMM with n output columns: 64 (more, smaller CTAs:
-// these GEMMs are short and latency-bound), or all of them when fewer
-uint32_t n_tile_of(uint32_t n) { return n > 64 ? 64u : ((n + 15) & ~15u); }
-
-// X0 (bf16, rows x n_in) -> out (f32, rows x n_out); keeps Z and A (and, for
-// training, the transposed activations At) for backward
-int32_t forward(omg_ctx* ctx, MlpRec& M, MlpBufs& W, uint32_t e, uint32_t rows, bool keep_t, cudaStream_t s) {
-  const uint32_t L = n_layers(M);
-  auto& net = M.members[e];
-  const uint16_t* x = W.xh.p;
-  uint32_t in = M.cfg.n_in;
-  for (uint32_t l = 0; l < L; l++) {
-    MlpLayer& Ly = net[l];
-    const bool last = l + 1 == L;
-    GemmArgs g{};
-    g.A = x;
-    g.a_rs = in;
-    g.a_ks = 1;
-    g.B = Ly.Wh.p;
-    g.b_rs = Ly.in;
-    g.b_ks = 1;
-    g.M = rows;
-    g.N = Ly.out;
-    g.K = in;
-    g.n_tile = n_tile_of(Ly.out);
-    g.bias = Ly.b.p;
-    g.err = M.err.p;
-    if (last) {
-      g.D = W.out.p;
-      g.ldd = Ly.out;
-    } else {
-      g.Z = W.Z[l].p;
-      g.ldz = Ly.out;
-      g.Y = W.A[l].p;
-      g.ldy = Ly.out;
-      if (keep_t) {
-        g.Yt = W.At[l].p;
-        g.ldyt = rows;
-      }
-      g.act = 1;
-    }
-    CK(launch_gemm(g, 1, s));
-    x = W.A[l].p;
-    in = Ly.out;
-  }
-  return OMG_OK;
+// The launch arguments of a training pass of `rows` rows from X, Y (standardized) through scratch S.
+MlpRowsArgs rows_args(const MlpRec& M, const MlpScratch& S, const float* X, const float* Y, uint32_t rows,
+                      uint32_t member0) {
+  MlpRowsArgs a{};
+  a.net = M.net;
+  a.rows = rows;
+  a.member0 = member0;
+  a.P = M.P.p;
+  a.img = M.img.p;
+  a.X = X;
+  a.Y = Y;
+  a.G = M.G.p;
+  a.loss = M.loss.p;
+  a.xt = S.xt.p;
+  a.at = S.at.p;
+  a.dzt = S.dzt.p;
+  a.gz = S.gz.p;
+  a.err = M.err.p;
+  return a;
 }
 
-// gradients of the MSE (targets in W.t) into the layers' gW, gb and the loss
-// into the member's gradient block (all zeroed here first, in one memset).
-// Every GEMM reads K-major operands: dW = dZ^T X from the transposes dZht and
-// xht / At, dX = dZ W from dZh and Wht.
-int32_t backward(omg_ctx* ctx, MlpRec& M, MlpBufs& W, uint32_t e, uint32_t rows, cudaStream_t s) {
-  const uint32_t L = n_layers(M);
-  auto& net = M.members[e];
-  float* loss = M.grads[e].p + M.grad_floats - 1;
-  CK(cudaMemsetAsync(M.grads[e].p, 0, M.grad_floats * 4, s));   // every gW, gb and the loss
-  MlpLayer& top = net[L - 1];
-  CK(launch_grad_tile(0, W.out.p, W.t.p, nullptr, rows, M.cfg.n_out, W.dZ.p, W.dZh.p, W.dZht.p, top.gb, loss, s));
-  for (int l = (int)L - 1; l >= 0; l--) {
-    MlpLayer& Ly = net[l];
-    const uint16_t* xt = l == 0 ? W.xht.p : W.At[l - 1].p;
-    // dW = dZ^T . X  (reduction over the batch, split over grid z; gW zeroed above)
-    GemmArgs g{};
-    g.A = W.dZht.p;
-    g.a_rs = rows;
-    g.a_ks = 1;
-    g.B = xt;
-    g.b_rs = rows;
-    g.b_ks = 1;
-    g.M = Ly.out;
-    g.N = Ly.in;
-    g.K = rows;
-    g.n_tile = n_tile_of(Ly.in);
-    g.D = Ly.gW;
-    g.ldd = Ly.in;
-    g.accumulate = 1;
-    g.err = M.err.p;
-    const uint32_t split = std::max(1u, std::min(8u, rows / 512u));
-    CK(launch_gemm(g, split, s));
-    if (l == 0) break;
-    // dX = dZ . W, then dZ of the layer below through GELU' (and its bias gradient)
-    GemmArgs h{};
-    h.A = W.dZh.p;
-    h.a_rs = Ly.out;
-    h.a_ks = 1;
-    h.B = Ly.Wht.p;
-    h.b_rs = Ly.out;
-    h.b_ks = 1;
-    h.M = rows;
-    h.N = Ly.in;
-    h.K = Ly.out;
-    h.n_tile = n_tile_of(Ly.in);
-    h.D = W.dX.p;
-    h.ldd = Ly.in;
-    h.err = M.err.p;
-    CK(launch_gemm(h, 1, s));
-    CK(launch_grad_tile(1, W.dX.p, W.Z[l - 1].p, nullptr, rows, Ly.in, W.dZ.p, W.dZh.p, W.dZht.p,
-                        net[l - 1].gb, nullptr, s));
-  }
-  return OMG_OK;
+MlpDwArgs dw_args(const MlpRec& M, const MlpScratch& S, uint32_t rows, uint32_t members, uint32_t member0) {
+  MlpDwArgs a{};
+  a.net = M.net;
+  a.tiles = rows / 128u;
+  a.members = members;
+  a.member0 = member0;
+  a.G = M.G.p;
+  a.xt = S.xt.p;
+  a.at = S.at.p;
+  a.dzt = S.dzt.p;
+  a.err = M.err.p;
+  return a;
 }
 
 int32_t check_err(omg_ctx* ctx, MlpRec& M) {
@@ -218,7 +144,7 @@ int32_t check_err(omg_ctx* ctx, MlpRec& M) {
   CK(cudaMemcpyAsync(&e, M.err.p, 4, cudaMemcpyDeviceToHost, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
   if (e) {
-    ctx->last_error = "surrogate GEMM: an mbarrier wait ran out";
+    ctx->last_error = "surrogate network: an mbarrier wait ran out";
     CK(cudaMemsetAsync(M.err.p, 0, 4, ctx->stream));
     return OMG_E_TIMEOUT;
   }
@@ -239,6 +165,26 @@ int32_t sync_norm(omg_ctx* ctx, MlpRec& M) {
   return OMG_OK;
 }
 
+// Copy between packed host arrays and a member's padded block: W then b per layer.
+template <class F>
+void each_param(const MlpNet& N, F&& f) {
+  for (uint32_t l = 0; l < N.n_layers; l++) {
+    f(N.L[l].w_off, N.L[l].in * N.L[l].out);
+    f(N.L[l].b_off, N.L[l].out);
+  }
+}
+
+void copy_big(float* dst, const float* src, uint64_t n) {
+  // one thread copies at about 17 GB/s into freshly mapped pages
+  const int threads = n * sizeof(float) >= (1u << 20) ? 4 : 1;
+  const uint64_t per = (n + threads - 1) / threads;
+#pragma omp parallel for num_threads(threads) schedule(static)
+  for (int t = 0; t < threads; t++) {
+    const uint64_t lo = std::min<uint64_t>(n, per * t), hi = std::min<uint64_t>(n, lo + per);
+    std::memcpy(dst + lo, src + lo, (hi - lo) * sizeof(float));
+  }
+}
+
 bool valid_cfg(const omg_mlp_config& c) {
   return c.n_in >= 1 && c.n_in <= 1024 && c.hidden >= 16 && c.hidden <= 256 && c.hidden % 16 == 0 &&
          c.n_hidden >= 1 && c.n_hidden <= 16 && c.n_out >= 1 && c.n_out <= 256 && c.members >= 1 &&
@@ -252,68 +198,43 @@ extern "C" {
 int32_t omg_mlp_create(omg_ctx* ctx, const omg_mlp_config* cfg, uint32_t* id) {
   if (!ctx || !cfg || !id || !valid_cfg(*cfg)) return OMG_E_INVALID;
   if (cudaSetDevice(ctx->device) != cudaSuccess) return fail(ctx, cudaGetLastError(), "cudaSetDevice");
-  CK(gemm_init());
+  CK(mlp_net_init());
   std::shared_ptr<MlpRec> M(new MlpRec());
   M->cfg = *cfg;
-  const uint32_t L = cfg->n_hidden + 1;
+  M->net = make_net(*cfg);
+  const MlpNet& N = M->net;
+  const uint32_t L = N.n_layers;
   std::mt19937_64 rng(cfg->seed ? cfg->seed : 1u);
-  M->members.resize(cfg->members);
+  const size_t np = (size_t)N.p_stride * cfg->members, ni = (size_t)N.img_stride * cfg->members;
+  std::vector<float> p0(np, 0.0f);
   for (uint32_t e = 0; e < cfg->members; e++) {
-    M->members[e].resize(L);
-    uint32_t in = cfg->n_in;
     for (uint32_t l = 0; l < L; l++) {
-      MlpLayer& Ly = M->members[e][l];
-      Ly.in = in;
-      Ly.out = l + 1 == L ? cfg->n_out : cfg->hidden;
-      const size_t nw = (size_t)Ly.out * Ly.in;
+      const MlpLayerDesc& D = N.L[l];
       // He-style normal init (std sqrt(2 / fan_in)), zero biases
-      std::normal_distribution<float> nd(0.0f, std::sqrt(2.0f / (float)Ly.in));
-      std::vector<float> w(nw);
-      for (auto& v : w) v = nd(rng);
+      std::normal_distribution<float> nd(0.0f, std::sqrt(2.0f / (float)D.in));
+      float* w = p0.data() + (size_t)e * N.p_stride + D.w_off;
+      const size_t nw = (size_t)D.out * D.in;
+      for (size_t i = 0; i < nw; i++) w[i] = nd(rng);
       if (l + 1 == L)
-        for (auto& v : w) v *= 0.5f;
-      CK(Ly.W.alloc(nw));
-      CK(Ly.Wh.alloc(nw));
-      CK(Ly.Wht.alloc(nw));
-      CK(Ly.mW.alloc(nw));
-      CK(Ly.vW.alloc(nw));
-
-      CK(Ly.b.alloc(Ly.out));
-      CK(Ly.mb.alloc(Ly.out));
-      CK(Ly.vb.alloc(Ly.out));
-
-      CK(cudaMemcpy(Ly.W.p, w.data(), nw * 4, cudaMemcpyHostToDevice));
-      CK(cudaMemset(Ly.mW.p, 0, nw * 4));
-      CK(cudaMemset(Ly.vW.p, 0, nw * 4));
-      CK(cudaMemset(Ly.b.p, 0, Ly.out * 4));
-      CK(cudaMemset(Ly.mb.p, 0, Ly.out * 4));
-      CK(cudaMemset(Ly.vb.p, 0, Ly.out * 4));
-      CK(launch_to_bf16_t(Ly.W.p, Ly.out, Ly.in, Ly.Wh.p, Ly.Wht.p, ctx->stream));
-      in = Ly.out;
+        for (size_t i = 0; i < nw; i++) w[i] *= 0.5f;
     }
   }
-  // the gradient blocks: per member every layer's gW then gb, then the loss
-  {
-    uint64_t n = 1;
-    for (auto& Ly : M->members[0]) n += (uint64_t)Ly.out * Ly.in + Ly.out;
-    M->grad_floats = n;
-    M->grads.resize(cfg->members);
-    for (uint32_t e = 0; e < cfg->members; e++) {
-      CK(M->grads[e].alloc(n));
-      uint64_t off = 0;
-      for (auto& Ly : M->members[e]) {
-        Ly.gW = M->grads[e].p + off;
-        off += (uint64_t)Ly.out * Ly.in;
-        Ly.gb = M->grads[e].p + off;
-        off += Ly.out;
-      }
-    }
-  }
+  CK(M->P.alloc(np));
+  CK(M->M1.alloc(np));
+  CK(M->V1.alloc(np));
+  CK(M->G.alloc(np));
+  CK(M->img.alloc(ni));
+  CK(M->loss.alloc(cfg->members));
+  CK(cudaMemcpy(M->P.p, p0.data(), np * 4, cudaMemcpyHostToDevice));
+  CK(cudaMemsetAsync(M->M1.p, 0, np * 4, ctx->stream));
+  CK(cudaMemsetAsync(M->V1.p, 0, np * 4, ctx->stream));
+  CK(cudaMemsetAsync(M->G.p, 0, np * 4, ctx->stream));
+  CK(cudaMemsetAsync(M->img.p, 0, ni * 2, ctx->stream));   // the images' padding stays zero
+  CK(launch_mlp_images(N, M->P.p, M->img.p, ctx->stream));
   M->x_mean.assign(cfg->n_in, 0.0f);
   M->x_std.assign(cfg->n_in, 1.0f);
   M->y_mean.assign(cfg->n_out, 0.0f);
   M->y_std.assign(cfg->n_out, 1.0f);
-  CK(M->h_loss.alloc(1));
   CK(M->err.alloc(1));
   CK(cudaMemsetAsync(M->err.p, 0, 4, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
@@ -374,21 +295,21 @@ int32_t omg_mlp_set_data(omg_ctx* ctx, uint32_t id, const float* x, const float*
   return OMG_OK;
 }
 
-// Training. Every member trains on its own stream, concurrently: one step
-// (gather the batch, forward, backward, AdamW of every layer, step counter) is
-// recorded once into a CUDA graph per member and launched steps-per-epoch
-// times per epoch; the step's batch rows (this epoch's permutation, uploaded
-// before the epoch) and its learning rate and bias corrections (a schedule
-// uploaded once) are read on the device at the step counter. The host waits
-// once per epoch, for the losses.
+// Training: three launches a step for all members together (the rows' forward
+// and backward pass, the weight gradients, AdamW), recorded into a CUDA graph
+// that is launched steps-per-epoch times per epoch. The step's batch rows (the
+// epoch's permutation) and its learning rate and bias corrections (a schedule
+// uploaded once) are read on the device at the step counter. Two epochs'
+// permutations are resident: the host shuffles the next epoch's, a thread a
+// member, while the device runs this one.
 int32_t omg_mlp_train(omg_ctx* ctx, uint32_t id, const omg_mlp_train_config* tc, float* epoch_loss) {
   if (!ctx || !tc || tc->epochs == 0 || tc->batch == 0 || tc->batch % 128 != 0) return OMG_E_INVALID;
   auto it = ctx->mlps.find(id);
   if (it == ctx->mlps.end()) return OMG_E_NOT_FOUND;
   MlpRec& M = *it->second;
   if (M.n_data < tc->batch) return OMG_E_INVALID;
-  const uint32_t L = n_layers(M), B = tc->batch, E = M.cfg.members;
-  const uint32_t spe = M.n_data / B;
+  const uint32_t B = tc->batch, E = M.cfg.members, n = M.n_data;
+  const uint32_t spe = n / B;
   const uint64_t total = (uint64_t)spe * tc->epochs;
   if (total >= (1ull << 31)) return OMG_E_INVALID;
   // the schedule: cosine decay from lr to lr_final, AdamW bias corrections
@@ -399,85 +320,99 @@ int32_t omg_mlp_train(omg_ctx* ctx, uint32_t id, const omg_mlp_train_config* tc,
     sched[3 * t + 1] = (float)(1.0 - std::pow((double)tc->beta1, (double)(t + 1)));
     sched[3 * t + 2] = (float)(1.0 - std::pow((double)tc->beta2, (double)(t + 1)));
   }
-  CK(gemm_init());   // outside the captures below
-  CK(M.sched.alloc(sched.size()));
-  CK(cudaMemcpy(M.sched.p, sched.data(), sched.size() * 4, cudaMemcpyHostToDevice));
-  CK(cudaStreamSynchronize(ctx->stream));
-  M.trainers.resize(E);
-  int32_t rc = OMG_OK;
-  for (uint32_t e = 0; e < E; e++) {
-    if (!M.trainers[e]) M.trainers[e].reset(new MlpTrainer());
-    MlpTrainer& T = *M.trainers[e];
-    if (!T.stream) CK(cudaStreamCreateWithFlags(&T.stream, cudaStreamNonBlocking));
-    if ((rc = ensure_batch(ctx, M, T.bufs, B, true))) return rc;
-    CK(T.perm.alloc(M.n_data));
-    CK(T.h_perm.alloc(M.n_data));
-    CK(T.step.alloc(1));
-    CK(T.h_loss.alloc(1));
-    CK(cudaMemsetAsync(T.step.p, 0, 4, T.stream));
-    // record one training step
-    if (T.graph) {
-      cudaGraphExecDestroy(T.graph);
-      T.graph = nullptr;
-    }
-    cudaStream_t s = T.stream;
-    MlpBufs& W = T.bufs;
-    CK(cudaStreamSynchronize(s));
-    CK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-    auto record = [&]() -> int32_t {
-      CK(launch_gather_pair(M.X.p, M.cfg.n_in, M.Y.p, M.cfg.n_out, T.perm.p, T.step.p, spe, B, W.xh.p, W.xht.p,
-                            W.t.p, s));
-      int32_t r;
-      if ((r = forward(ctx, M, W, e, B, true, s))) return r;
-      if ((r = backward(ctx, M, W, e, B, s))) return r;
-      AdamwTable tab{};
-      uint64_t off = 0;
-      for (uint32_t l = 0; l < L; l++) {
-        MlpLayer& Ly = M.members[e][l];
-        tab.L[l] = AdamwLayer{Ly.W.p, Ly.mW.p, Ly.vW.p, Ly.b.p, Ly.mb.p, Ly.vb.p, Ly.gW, Ly.gb, Ly.Wh.p, Ly.Wht.p,
-                              Ly.in, Ly.out, off};
-        off += (uint64_t)Ly.in * Ly.out + Ly.out;
-      }
-      tab.n = L;
-      tab.total = off;
-      CK(launch_adamw_all(tab, M.sched.p, T.step.p, tc->beta1, tc->beta2, tc->eps, tc->weight_decay, s));
-      CK(launch_step(T.step.p, s));
-      return OMG_OK;
-    };
-    rc = record();
+  CK(mlp_net_init());   // outside the capture below
+  cudaStream_t s = ctx->stream;
+  const uint64_t half = (uint64_t)E * n, n_loss = (uint64_t)E * tc->epochs;
+  CK(cudaStreamSynchronize(s));
+  if (M.sched.n < sched.size()) CK(M.sched.alloc(sched.size()));
+  if (M.perm.n < 2 * half) {
+    CK(M.perm.alloc(2 * half));
+    CK(M.h_perm.alloc(2 * half));
+  }
+  if (!M.counters.p) CK(M.counters.alloc(2));
+  if (M.epoch_loss.n < n_loss) CK(M.epoch_loss.alloc(n_loss));
+  int32_t rc = ensure_scratch(ctx, M, M.train_s, (uint64_t)E * (B / 128u));
+  if (rc) return rc;
+  CK(cudaMemcpyAsync(M.sched.p, sched.data(), sched.size() * 4, cudaMemcpyHostToDevice, s));
+  CK(cudaMemsetAsync(M.counters.p, 0, 8, s));
+  CK(cudaMemsetAsync(M.G.p, 0, M.G.n * 4, s));          // each step leaves them zero again
+  CK(cudaMemsetAsync(M.loss.p, 0, M.loss.n * 4, s));
+  MlpRowsArgs ra = rows_args(M, M.train_s, M.X.p, M.Y.p, B, 0);
+  ra.perm = M.perm.p;
+  ra.perm_half = half;
+  ra.perm_member = n;
+  ra.step = M.counters.p;
+  ra.spe = spe;
+  MlpAdamwArgs aa{};
+  aa.net = M.net;
+  aa.P = M.P.p;
+  aa.M1 = M.M1.p;
+  aa.V1 = M.V1.p;
+  aa.G = M.G.p;
+  aa.img = M.img.p;
+  aa.sched = M.sched.p;
+  aa.step = M.counters.p;
+  aa.ticket = M.counters.p + 1;
+  aa.loss = M.loss.p;
+  aa.epoch_loss = M.epoch_loss.p;
+  aa.spe = spe;
+  aa.epochs = tc->epochs;
+  aa.b1 = tc->beta1;
+  aa.b2 = tc->beta2;
+  aa.eps = tc->eps;
+  aa.wd = tc->weight_decay;
+  cudaGraphExec_t graph = nullptr;
+  {
+    cudaStream_t cs;
+    CK(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
+    cudaError_t ce = cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal);
     cudaGraph_t g = nullptr;
-    cudaError_t ce = cudaStreamEndCapture(s, &g);
-    if (rc) {
+    if (ce == cudaSuccess) {
+      ce = launch_mlp_rows(ra, E, true, cs);
+      if (ce == cudaSuccess) ce = launch_mlp_dw(dw_args(M, M.train_s, B, E, 0), ctx->n_sms, cs);
+      if (ce == cudaSuccess) ce = launch_mlp_adamw(aa, ctx->n_sms, cs);
+      const cudaError_t ee = cudaStreamEndCapture(cs, &g);
+      if (ce == cudaSuccess) ce = ee;
+      if (ce == cudaSuccess) ce = cudaGraphInstantiate(&graph, g, 0);
       if (g) cudaGraphDestroy(g);
-      return rc;
     }
-    if (ce != cudaSuccess) return fail(ctx, ce, "cudaStreamEndCapture");
-    ce = cudaGraphInstantiate(&T.graph, g, 0);
-    cudaGraphDestroy(g);
-    if (ce != cudaSuccess) return fail(ctx, ce, "cudaGraphInstantiate");
+    cudaStreamDestroy(cs);
+    if (ce != cudaSuccess) return fail(ctx, ce, "training step capture");
   }
   std::vector<std::mt19937_64> rngs;
   for (uint32_t e = 0; e < E; e++) rngs.emplace_back((tc->seed ? tc->seed : 7u) + 0x9E3779B97F4A7C15ull * e);
-  for (uint32_t ep = 0; ep < tc->epochs; ep++) {
-    for (uint32_t e = 0; e < E; e++) {
-      MlpTrainer& T = *M.trainers[e];
-      std::iota(T.h_perm.p, T.h_perm.p + M.n_data, 0u);
-      std::shuffle(T.h_perm.p, T.h_perm.p + M.n_data, rngs[e]);
-      CK(cudaMemcpyAsync(T.perm.p, T.h_perm.p, (size_t)M.n_data * 4, cudaMemcpyHostToDevice, T.stream));
+  auto shuffle_epoch = [&](uint32_t ep) {
+    const int threads = (uint64_t)E * n >= 4096u ? (int)E : 1;
+#pragma omp parallel for num_threads(threads) schedule(static)
+    for (int e = 0; e < (int)E; e++) {
+      uint32_t* p = M.h_perm.p + (ep & 1u) * half + (uint64_t)e * n;
+      std::iota(p, p + n, 0u);
+      std::shuffle(p, p + n, rngs[e]);
     }
-    for (uint32_t st = 0; st < spe; st++)
-      for (uint32_t e = 0; e < E; e++) CK(cudaGraphLaunch(M.trainers[e]->graph, M.trainers[e]->stream));
-    for (uint32_t e = 0; e < E; e++) {
-      MlpTrainer& T = *M.trainers[e];
-      CK(cudaMemcpyAsync(T.h_loss.p, M.grads[e].p + M.grad_floats - 1, 4, cudaMemcpyDeviceToHost, T.stream));
-    }
-    // the permutation buffers are refilled next epoch: wait for this one
-    for (uint32_t e = 0; e < E; e++) {
-      MlpTrainer& T = *M.trainers[e];
-      CK(cudaStreamSynchronize(T.stream));
-      if (epoch_loss) epoch_loss[(size_t)e * tc->epochs + ep] = T.h_loss.p[0];
-    }
+  };
+  // from here on every exit waits for what was enqueued: it reads sched and the permutations
+  cudaError_t ce = cudaSuccess;
+  cudaEvent_t ev[2] = {nullptr, nullptr};
+  for (int k = 0; k < 2 && ce == cudaSuccess; k++) ce = cudaEventCreateWithFlags(&ev[k], cudaEventDisableTiming);
+  for (uint32_t ep = 0; ep < tc->epochs && ce == cudaSuccess; ep++) {
+    // this half's previous epoch (two before) is done with its permutations
+    if (ep >= 2) ce = cudaEventSynchronize(ev[ep & 1u]);
+    if (ce != cudaSuccess) break;
+    shuffle_epoch(ep);
+    const uint64_t at = (ep & 1u) * half;
+    ce = cudaMemcpyAsync(M.perm.p + at, M.h_perm.p + at, half * 4, cudaMemcpyHostToDevice, s);
+    for (uint32_t st = 0; st < spe && ce == cudaSuccess; st++) ce = cudaGraphLaunch(graph, s);
+    if (ce == cudaSuccess) ce = cudaEventRecord(ev[ep & 1u], s);
   }
+  std::vector<float> losses(n_loss);
+  if (ce == cudaSuccess) ce = cudaMemcpyAsync(losses.data(), M.epoch_loss.p, n_loss * 4, cudaMemcpyDeviceToHost, s);
+  const cudaError_t se = cudaStreamSynchronize(s);
+  for (int k = 0; k < 2; k++)
+    if (ev[k]) cudaEventDestroy(ev[k]);
+  cudaGraphExecDestroy(graph);
+  if (ce != cudaSuccess) return fail(ctx, ce, "training");
+  if (se != cudaSuccess) return fail(ctx, se, "training");
+  if (epoch_loss) std::copy(losses.begin(), losses.end(), epoch_loss);
   M.step += total;
   return check_err(ctx, M);
 }
@@ -496,43 +431,62 @@ int32_t surrogate_run(omg_ctx* ctx, uint32_t id, const float* x, uint32_t n, flo
   if (it == ctx->mlps.end()) return OMG_E_NOT_FOUND;
   MlpRec& M = *it->second;
   const uint32_t ni = M.cfg.n_in, no = M.cfg.n_out, E = M.cfg.members;
-  const uint32_t chunk = 32768;
-  const uint32_t rows_max = std::min(n, chunk);
-  int32_t rc = ensure_batch(ctx, M, M.io, rows_max, false);
-  if (rc) return rc;
-  if (M.icap < rows_max) {
-    CK(M.xin.alloc((size_t)rows_max * ni));
-    CK(M.acc.alloc((size_t)rows_max * no));
-    CK(M.acc2.alloc((size_t)rows_max * no));
-    CK(M.h_x.alloc((size_t)rows_max * ni));
-    CK(M.h_mean.alloc((size_t)rows_max * no));
-    CK(M.h_std.alloc((size_t)rows_max * no));
-    M.icap = rows_max;
+  // Rows a launch: the row tiles of all members fill the chip once (one CTA a
+  // multiprocessor); two chunks in flight, so that the copies and the host's
+  // part of one run under the other's kernels.
+  const uint32_t wave = 128u * std::max(1u, (uint32_t)ctx->n_sms / E);
+  const uint32_t parts = (n + wave - 1) / wave;
+  const uint32_t chunk = std::min(n, ((n + parts - 1) / parts + 127u) / 128u * 128u);
+  for (MlpChunk& C : M.chunk) {
+    if (C.cap >= chunk || (&C != M.chunk && n <= chunk)) continue;
+    C.cap = 0;
+    CK(C.x.alloc((size_t)chunk * ni));
+    CK(C.y.alloc((size_t)chunk * no * E));
+    CK(C.mean.alloc((size_t)chunk * no));
+    CK(C.std.alloc((size_t)chunk * no));
+    CK(C.spread.alloc(chunk));
+    CK(C.h_x.alloc((size_t)chunk * ni));
+    CK(C.h_mean.alloc((size_t)chunk * no));
+    CK(C.h_std.alloc((size_t)chunk * no));
+    CK(C.h_spread.alloc(chunk));
+    if (!C.done) CK(cudaEventCreateWithFlags(&C.done, cudaEventDisableTiming));
+    C.cap = chunk;
   }
   cudaStream_t s = ctx->stream;
-  // everything on the device: standardize, every member's forward, the
-  // ensemble's mean and spread in the targets' units
-  for (uint32_t r0 = 0; r0 < n; r0 += chunk) {
+  auto submit = [&](MlpChunk& C, uint32_t r0) -> int32_t {
     const uint32_t rows = std::min(chunk, n - r0);
     const uint64_t nx = (uint64_t)rows * ni, ny = (uint64_t)rows * no;
-    std::memcpy(M.h_x.p, x + (uint64_t)r0 * ni, nx * 4);
-    CK(cudaMemcpyAsync(M.xin.p, M.h_x.p, nx * 4, cudaMemcpyHostToDevice, s));
-    CK(launch_standardize(M.xin.p, M.d_x_mean.p, M.d_x_std.p, ni, nx, M.io.xh.p, s));
-    for (uint32_t e = 0; e < E; e++) {
-      if ((rc = forward(ctx, M, M.io, e, rows, false, s))) return rc;
-      CK(launch_ensemble(M.io.out.p, M.d_y_mean.p, M.d_y_std.p, no, ny, M.acc.p, M.acc2.p, e == 0, e + 1 == E,
-                         1.0f / (float)E, s));
-    }
-    CK(cudaMemcpyAsync(M.h_mean.p, M.acc.p, ny * 4, cudaMemcpyDeviceToHost, s));
-    if (y_std) CK(cudaMemcpyAsync(M.h_std.p, M.acc2.p, ny * 4, cudaMemcpyDeviceToHost, s));
-    if (row_spread) {
-      // the per-row spread reuses the bf16 input buffer's space as f32 scratch
-      CK(launch_row_spread(M.acc.p, M.acc2.p, no, rows, level, M.xin.p, s));
-      CK(cudaMemcpyAsync(row_spread + r0, M.xin.p, (size_t)rows * 4, cudaMemcpyDeviceToHost, s));
-    }
-    CK(cudaStreamSynchronize(s));
-    std::memcpy(y_mean + (uint64_t)r0 * no, M.h_mean.p, ny * 4);
-    if (y_std) std::memcpy(y_std + (uint64_t)r0 * no, M.h_std.p, ny * 4);
+    std::memcpy(C.h_x.p, x + (uint64_t)r0 * ni, nx * 4);
+    CK(cudaMemcpyAsync(C.x.p, C.h_x.p, nx * 4, cudaMemcpyHostToDevice, s));
+    MlpRowsArgs a{};
+    a.net = M.net;
+    a.rows = rows;
+    a.P = M.P.p;
+    a.img = M.img.p;
+    a.X = C.x.p;
+    a.x_mean = M.d_x_mean.p;
+    a.x_sd = M.d_x_std.p;
+    a.out = C.y.p;
+    a.err = M.err.p;
+    CK(launch_mlp_rows(a, E, false, s));
+    CK(launch_mlp_ensemble(C.y.p, E, rows, no, M.d_y_mean.p, M.d_y_std.p, level, C.mean.p, y_std ? C.std.p : nullptr,
+                           row_spread ? C.spread.p : nullptr, s));
+    CK(cudaMemcpyAsync(C.h_mean.p, C.mean.p, ny * 4, cudaMemcpyDeviceToHost, s));
+    if (y_std) CK(cudaMemcpyAsync(C.h_std.p, C.std.p, ny * 4, cudaMemcpyDeviceToHost, s));
+    if (row_spread) CK(cudaMemcpyAsync(C.h_spread.p, C.spread.p, (size_t)rows * 4, cudaMemcpyDeviceToHost, s));
+    CK(cudaEventRecord(C.done, s));
+    return OMG_OK;
+  };
+  int32_t rc = OMG_OK;
+  if ((rc = submit(M.chunk[0], 0))) return rc;
+  for (uint32_t r0 = 0, k = 0; r0 < n; r0 += chunk, k ^= 1u) {
+    if (n - r0 > chunk && (rc = submit(M.chunk[k ^ 1u], r0 + chunk))) return rc;
+    MlpChunk& C = M.chunk[k];
+    const uint32_t rows = std::min(chunk, n - r0);
+    if ((rc = wait_event(ctx, C.done, timeout_of(ctx)))) return rc;
+    copy_big(y_mean + (uint64_t)r0 * no, C.h_mean.p, (uint64_t)rows * no);
+    if (y_std) copy_big(y_std + (uint64_t)r0 * no, C.h_std.p, (uint64_t)rows * no);
+    if (row_spread) std::memcpy(row_spread + r0, C.h_spread.p, (size_t)rows * 4);
   }
   return check_err(ctx, M);
 }
@@ -560,33 +514,31 @@ int32_t omg_mlp_grad(omg_ctx* ctx, uint32_t id, uint32_t member, const float* x,
   if (it == ctx->mlps.end()) return OMG_E_NOT_FOUND;
   MlpRec& M = *it->second;
   if (member >= M.cfg.members) return OMG_E_INVALID;
-  // the inference buffers may have been sized without the transposes
-  if (M.io.cap && !M.io.xht.p) M.io.cap = 0;
-  int32_t rc = ensure_batch(ctx, M, M.io, n, true);
+  int32_t rc = ensure_scratch(ctx, M, M.grad_s, n / 128u);
   if (rc) return rc;
   cudaStream_t s = ctx->stream;
-  MlpBufs& W = M.io;
-  DevBuf<float> xd;
-  CK(xd.alloc((size_t)n * M.cfg.n_in));
-  CK(cudaMemcpyAsync(xd.p, x, (size_t)n * M.cfg.n_in * 4, cudaMemcpyHostToDevice, s));
-  CK(cudaMemcpyAsync(W.t.p, y, (size_t)n * M.cfg.n_out * 4, cudaMemcpyHostToDevice, s));
-  CK(launch_to_bf16_t(xd.p, n, M.cfg.n_in, W.xh.p, W.xht.p, s));
-  if ((rc = forward(ctx, M, W, member, n, true, s))) return rc;
-  if ((rc = backward(ctx, M, W, member, n, s))) return rc;
-  CK(cudaMemcpyAsync(M.h_loss.p, M.grads[member].p + M.grad_floats - 1, 4, cudaMemcpyDeviceToHost, s));
-  size_t off = 0;
-  for (auto& Ly : M.members[member]) {
-    if (grads) {
-      CK(cudaMemcpyAsync(grads + off, Ly.gW, (size_t)Ly.out * Ly.in * 4, cudaMemcpyDeviceToHost, s));
-      off += (size_t)Ly.out * Ly.in;
-      CK(cudaMemcpyAsync(grads + off, Ly.gb, (size_t)Ly.out * 4, cudaMemcpyDeviceToHost, s));
-      off += Ly.out;
-    }
-  }
+  const MlpNet& N = M.net;
+  if (M.grad_x.n < (size_t)n * M.cfg.n_in) CK(M.grad_x.alloc((size_t)n * M.cfg.n_in));
+  if (M.grad_y.n < (size_t)n * M.cfg.n_out) CK(M.grad_y.alloc((size_t)n * M.cfg.n_out));
+  CK(cudaMemcpyAsync(M.grad_x.p, x, (size_t)n * M.cfg.n_in * 4, cudaMemcpyHostToDevice, s));
+  CK(cudaMemcpyAsync(M.grad_y.p, y, (size_t)n * M.cfg.n_out * 4, cudaMemcpyHostToDevice, s));
+  float* G = M.G.p + (uint64_t)member * N.p_stride;
+  CK(cudaMemsetAsync(G, 0, (size_t)N.p_stride * 4, s));
+  CK(cudaMemsetAsync(M.loss.p + member, 0, 4, s));
+  CK(launch_mlp_rows(rows_args(M, M.grad_s, M.grad_x.p, M.grad_y.p, n, member), 1, true, s));
+  CK(launch_mlp_dw(dw_args(M, M.grad_s, n, 1, member), ctx->n_sms, s));
+  if (M.h_loss.n < N.p_stride + 1u) CK(M.h_loss.alloc(N.p_stride + 1u));
+  CK(cudaMemcpyAsync(M.h_loss.p, M.loss.p + member, 4, cudaMemcpyDeviceToHost, s));
+  if (grads) CK(cudaMemcpyAsync(M.h_loss.p + 1, G, (size_t)N.p_stride * 4, cudaMemcpyDeviceToHost, s));
   CK(cudaStreamSynchronize(s));
-  if (loss) {
-    *loss = M.h_loss.p[0];
+  if (grads) {
+    size_t off = 0;
+    each_param(N, [&](uint32_t at, uint32_t k) {
+      std::memcpy(grads + off, M.h_loss.p + 1 + at, (size_t)k * 4);
+      off += k;
+    });
   }
+  if (loss) *loss = M.h_loss.p[0];
   return check_err(ctx, M);
 }
 
@@ -603,32 +555,36 @@ int32_t omg_mlp_params(omg_ctx* ctx, uint32_t id, uint32_t what, float* out, uin
     if (out) std::copy(v.begin(), v.end(), out + n);
     n += v.size();
   };
-  auto put_dev = [&](const float* p, size_t k) -> cudaError_t {
-    if (out) {
-      cudaError_t e = cudaMemcpy(out + n, p, k * 4, cudaMemcpyDeviceToHost);
-      if (e != cudaSuccess) return e;
-    }
-    n += k;
-    return cudaSuccess;
-  };
   CK(cudaStreamSynchronize(ctx->stream));
+  const MlpNet& N = M.net;
+  const size_t np = (size_t)N.p_stride * N.members;
+  std::vector<float> w, v;
+  if (out) {
+    w.resize(np);
+    CK(cudaMemcpy(w.data(), what == 1 ? M.P.p : M.M1.p, np * 4, cudaMemcpyDeviceToHost));
+    if (what == 2) {
+      v.resize(np);
+      CK(cudaMemcpy(v.data(), M.V1.p, np * 4, cudaMemcpyDeviceToHost));
+    }
+  }
+  auto put = [&](const std::vector<float>& src, uint32_t e, uint32_t at, uint32_t k) {
+    if (out) std::memcpy(out + n, src.data() + (size_t)e * N.p_stride + at, (size_t)k * 4);
+    n += k;
+  };
   if (what == 1) {
     put_host(M.x_mean);
     put_host(M.x_std);
     put_host(M.y_mean);
     put_host(M.y_std);
-    for (auto& net : M.members)
-      for (auto& Ly : net) {
-        CK(put_dev(Ly.W.p, (size_t)Ly.out * Ly.in));
-        CK(put_dev(Ly.b.p, Ly.out));
-      }
+    for (uint32_t e = 0; e < N.members; e++) each_param(N, [&](uint32_t at, uint32_t k) { put(w, e, at, k); });
   } else {
-    for (auto& net : M.members)
-      for (auto& Ly : net) {
-        CK(put_dev(Ly.mW.p, (size_t)Ly.out * Ly.in));
-        CK(put_dev(Ly.vW.p, (size_t)Ly.out * Ly.in));
-        CK(put_dev(Ly.mb.p, Ly.out));
-        CK(put_dev(Ly.vb.p, Ly.out));
+    for (uint32_t e = 0; e < N.members; e++)
+      for (uint32_t l = 0; l < N.n_layers; l++) {
+        const MlpLayerDesc& D = N.L[l];
+        put(w, e, D.w_off, D.in * D.out);
+        put(v, e, D.w_off, D.in * D.out);
+        put(w, e, D.b_off, D.out);
+        put(v, e, D.b_off, D.out);
       }
     if (out) out[n] = (float)M.step;
     n += 1;
@@ -651,32 +607,35 @@ int32_t omg_mlp_set_params(omg_ctx* ctx, uint32_t id, uint32_t what, const float
     std::copy(in + n, in + n + v.size(), v.begin());
     n += v.size();
   };
-  auto get_dev = [&](float* p, size_t k) -> cudaError_t {
-    cudaError_t e = cudaMemcpy(p, in + n, k * 4, cudaMemcpyHostToDevice);
+  const MlpNet& N = M.net;
+  const size_t np = (size_t)N.p_stride * N.members;
+  std::vector<float> w(np, 0.0f), v;
+  auto get = [&](std::vector<float>& dst, uint32_t e, uint32_t at, uint32_t k) {
+    std::memcpy(dst.data() + (size_t)e * N.p_stride + at, in + n, (size_t)k * 4);
     n += k;
-    return e;
   };
   if (what == 1) {
     get_host(M.x_mean);
     get_host(M.x_std);
     get_host(M.y_mean);
     get_host(M.y_std);
-    for (auto& net : M.members)
-      for (auto& Ly : net) {
-        CK(get_dev(Ly.W.p, (size_t)Ly.out * Ly.in));
-        CK(get_dev(Ly.b.p, Ly.out));
-        CK(launch_to_bf16_t(Ly.W.p, Ly.out, Ly.in, Ly.Wh.p, Ly.Wht.p, ctx->stream));
-      }
+    for (uint32_t e = 0; e < N.members; e++) each_param(N, [&](uint32_t at, uint32_t k) { get(w, e, at, k); });
+    CK(cudaMemcpy(M.P.p, w.data(), np * 4, cudaMemcpyHostToDevice));
+    CK(launch_mlp_images(N, M.P.p, M.img.p, ctx->stream));
     int32_t rc2 = sync_norm(ctx, M);
     if (rc2) return rc2;
   } else {
-    for (auto& net : M.members)
-      for (auto& Ly : net) {
-        CK(get_dev(Ly.mW.p, (size_t)Ly.out * Ly.in));
-        CK(get_dev(Ly.vW.p, (size_t)Ly.out * Ly.in));
-        CK(get_dev(Ly.mb.p, Ly.out));
-        CK(get_dev(Ly.vb.p, Ly.out));
+    v.assign(np, 0.0f);
+    for (uint32_t e = 0; e < N.members; e++)
+      for (uint32_t l = 0; l < N.n_layers; l++) {
+        const MlpLayerDesc& D = N.L[l];
+        get(w, e, D.w_off, D.in * D.out);
+        get(v, e, D.w_off, D.in * D.out);
+        get(w, e, D.b_off, D.out);
+        get(v, e, D.b_off, D.out);
       }
+    CK(cudaMemcpy(M.M1.p, w.data(), np * 4, cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(M.V1.p, v.data(), np * 4, cudaMemcpyHostToDevice));
     M.step = (uint64_t)in[n];
   }
   CK(cudaStreamSynchronize(ctx->stream));

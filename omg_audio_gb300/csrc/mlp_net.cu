@@ -1,0 +1,645 @@
+// The surrogate's network on the tensor cores, whole passes a launch:
+//   rows_kernel    one CTA takes 128 rows of one member through every layer:
+//                  inference, or the forward pass, the loss and the backward
+//                  chain of a training step
+//   dw_kernel      the weight gradients of every layer and member
+//   adamw_kernel   the optimizer over every parameter
+//   ensemble_kernel  the members' mean and spread
+//
+// What bounds it, and why whole passes. A layer is 0.5 GFLOP for the training
+// batch (0.3 us of the chip), so a launch per layer spends its time in launch
+// gaps, prologues and trips of the activations through L2: 22 dependent launches
+// of 6 to 34 us made a training step of the 38-256x4-192 ensemble at 4096 rows
+// 583 us. Rows do not meet before the weight gradients, so a CTA keeps its rows'
+// activations in shared memory from the first layer to the last and back, and
+// only the weights stream in, one 128 KB layer ahead, while the previous
+// layer's epilogue runs. The epilogues (bias, GELU and its derivative from one
+// tanh, per element) are then the largest part: 16 warps share them.
+//
+// Operand images. An activation tile (128 rows) and a layer's weights are kept,
+// in shared and in global memory alike, as 8 x 8 core matrices (128 B: 8 rows of
+// 8 consecutive features), the row groups of one feature block contiguous:
+//   element (row, k): (k / 8) * 16 R + 16 row + 2 (k % 8) bytes, R rows
+// One bulk copy moves a whole tile or layer. Read K-major the image is the
+// operand of the forward product (and dZ of the input gradient); read MN-major
+// it is the transposed operand of the weight gradient (both sides) and of the
+// input gradient (the weights), so nothing is transposed in memory.
+#include <algorithm>
+
+#include <cuda_bf16.h>
+
+#include "mlp_net.h"
+#include "tc_gemm.cuh"
+
+namespace omg {
+
+namespace {
+
+constexpr uint32_t kRows = 128;               // rows a CTA owns (the MMA's M)
+constexpr uint32_t kWide = kMlpWide;          // widest layer, and the first layer's K a step
+constexpr uint32_t kRowThreads = 512;
+constexpr uint32_t kTileBytes = kRows * kWide * 2;
+constexpr uint32_t kWBytes = kWide * kWide * 2;
+constexpr uint32_t kRowsSmem = kTileBytes + kWBytes;
+constexpr uint32_t kPolls = 1u << 22;         // mbarrier poll limit (error 16 in the error word)
+
+__device__ __forceinline__ float gelu_f(float z, float t) { return 0.5f * z * (1.0f + t); }
+
+// tanh form of GELU: the inner tanh, shared by the value and the derivative
+__device__ __forceinline__ float gelu_tanh(float z) {
+  const float k0 = 0.7978845608028654f, k1 = 0.044715f;
+  const float u = k0 * (z + k1 * z * z * z);
+  return tanhf(u);
+}
+
+__device__ __forceinline__ float gelu_grad(float z, float t) {
+  const float k0 = 0.7978845608028654f, k1 = 0.044715f;
+  const float du = k0 * (1.0f + 3.0f * k1 * z * z);
+  return 0.5f * (1.0f + t) + 0.5f * z * (1.0f - t * t) * du;
+}
+
+__device__ __forceinline__ uint32_t pack2(float a, float b) {
+  return (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(a)) |
+         ((uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(b)) << 16);
+}
+
+// 16 consecutive features of one row into the tile image (two 16-byte stores;
+// a warp's lanes are consecutive rows: contiguous, no bank conflict)
+__device__ __forceinline__ void put16(uint8_t* tile, uint32_t row, uint32_t c, const float (&v)[16]) {
+  uint8_t* p = tile + (c >> 3) * (16u * kRows) + 16u * row;
+  *reinterpret_cast<uint4*>(p) =
+      make_uint4(pack2(v[0], v[1]), pack2(v[2], v[3]), pack2(v[4], v[5]), pack2(v[6], v[7]));
+  *reinterpret_cast<uint4*>(p + 16u * kRows) =
+      make_uint4(pack2(v[8], v[9]), pack2(v[10], v[11]), pack2(v[12], v[13]), pack2(v[14], v[15]));
+}
+
+// Sums of 16 columns over the warp's 32 rows, halving the columns a lane holds
+// at each step: 16 shuffles. Lane l (even) returns the sum of column
+// ((l >> 4) & 1) * 8 + ((l >> 3) & 1) * 4 + ((l >> 2) & 1) * 2 + ((l >> 1) & 1).
+__device__ __forceinline__ float column_sum16(float (&v)[16], uint32_t lane) {
+#pragma unroll
+  for (int h = 8; h >= 1; h >>= 1) {
+    const bool up = (lane & (2u * h)) != 0u;
+#pragma unroll
+    for (int j = 0; j < h; j++) {
+      const float keep = up ? v[j + h] : v[j], send = up ? v[j] : v[j + h];
+      v[j] = keep + __shfl_xor_sync(0xffffffffu, send, 2 * h);
+    }
+  }
+  return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
+}
+__device__ __forceinline__ uint32_t column_of(uint32_t lane) {
+  return ((lane >> 4) & 1u) * 8u + ((lane >> 3) & 1u) * 4u + ((lane >> 2) & 1u) * 2u + ((lane >> 1) & 1u);
+}
+
+template <bool TRAIN>
+__global__ void __launch_bounds__(kRowThreads, 1) rows_kernel(const __grid_constant__ MlpRowsArgs g) {
+  extern __shared__ __align__(1024) uint8_t smem[];
+  uint8_t* tile = smem;                        // the rows' activations (or gradients) of the current layer
+  uint8_t* wbuf = smem + kTileBytes;           // the current layer's weights
+  __shared__ __align__(8) uint64_t bar_w, bar_mma;
+  __shared__ uint32_t taddr_s;
+  __shared__ float s_bias[kWide];
+  const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+  const uint32_t row = (warp & 3u) * 32u + lane, cg = warp >> 2;   // TMEM lane, column group (4 of them)
+  const uint32_t t0 = blockIdx.x, member = g.member0 + blockIdx.y;
+  const MlpNet& N = g.net;
+  const uint32_t L = N.n_layers;
+  const float* P = g.P + (uint64_t)member * N.p_stride;
+  const uint16_t* img = g.img + (uint64_t)member * N.img_stride;
+  const uint32_t grow = t0 * kRows + row;      // this thread's row of the batch
+  const bool live = t0 * kRows + (warp & 3u) * 32u < g.rows;       // (warp-uniform) any row of the warp
+  if (tid == 0) {
+    tc::mbar_init(&bar_w, 1);
+    tc::mbar_init(&bar_mma, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 0) tc::tmem_alloc(&taddr_s, 256);
+  tc::fence_before_sync();
+  __syncthreads();
+  tc::fence_after_sync();
+  const uint32_t taddr = taddr_s;
+  const uint32_t my_lanes = taddr + (((warp & 3u) * 32u) << 16);
+  uint32_t par_w = 0, par_mma = 0;             // thread 0's and every thread's next phase
+  bool loading = false;                        // thread 0: a weight load is in flight
+  bool ok = true;
+
+  // weights of layer l, K chunk c of kWide features (thread 0)
+  auto load_w = [&](uint32_t l, uint32_t c) {
+    const MlpLayerDesc& D = N.L[l];
+    const uint32_t k0 = c * kWide, kn = min(kWide, D.ip - k0), bytes = kn * D.op * 2u;
+    tc::mbar_expect_tx(&bar_w, bytes);
+    const uint8_t* src = reinterpret_cast<const uint8_t*>(img + D.img_off) + (uint64_t)k0 * D.op * 2u;
+    for (uint32_t o = 0; o < bytes; o += 32768u) tc::bulk_load(wbuf + o, src + o, min(32768u, bytes - o), &bar_w);
+    loading = true;
+  };
+  auto wait_w = [&]() {
+    if (loading) {
+      ok = tc::mbar_wait(&bar_w, par_w, kPolls) && ok;
+      par_w ^= 1u;
+      loading = false;
+    }
+  };
+  // the tile (K features) times the weights read K-major (bwd = false: N = op)
+  // or MN-major (bwd: N = ip), accumulated over K; the commit arrives on bar_mma
+  auto issue = [&](const MlpLayerDesc& D, bool bwd, uint32_t kn, bool acc0) {
+    tc::fence_after_sync();
+    const uint32_t a0 = tc::smem_u32(tile), b0 = tc::smem_u32(wbuf);
+    const uint32_t lead = 16u * D.op;          // bytes between the image's feature blocks
+    const uint32_t idesc = tc::idesc_bf16_f32(bwd ? D.ip : D.op, kRows) | (bwd ? tc::kTransB : 0u);
+    for (uint32_t s = 0; s < kn / 16u; s++) {
+      const uint64_t ad = tc::smem_desc(a0 + s * (32u * kRows), 16u * kRows, 128u);
+      const uint64_t bd = bwd ? tc::smem_desc(b0 + 256u * s, 128u, lead) : tc::smem_desc(b0 + s * 2u * lead, lead, 128u);
+      tc::mma_bf16(taddr, ad, bd, idesc, acc0 || s > 0);
+    }
+    tc::mma_commit(&bar_mma);
+  };
+  auto wait_mma = [&]() {
+    ok = tc::mbar_wait(&bar_mma, par_mma, kPolls) && ok;
+    par_mma ^= 1u;
+  };
+  // the columns of a layer of width w that this thread's warp handles
+  auto col_lo = [&](uint32_t w) { return min(w, cg * (((w >> 4) + 3u) / 4u) * 16u); };
+  auto col_hi = [&](uint32_t w) { return min(w, (cg + 1u) * (((w >> 4) + 3u) / 4u) * 16u); };
+
+  const uint64_t mt = (uint64_t)blockIdx.y * gridDim.x + t0;       // this CTA's slot of the scratch arrays
+  const uint32_t* idx = nullptr;
+  uint64_t src_row = grow;
+  if (TRAIN && g.perm) {
+    const uint32_t step = *g.step;
+    idx = g.perm + (uint64_t)((step / g.spe) & 1u) * g.perm_half + (uint64_t)member * g.perm_member +
+          (uint64_t)(step % g.spe) * g.rows;
+    src_row = idx[grow];
+  }
+  if (tid == 0) load_w(0, 0);
+
+  // ---------------------------------------------------------------- forward
+  for (uint32_t l = 0; l < L; l++) {
+    const MlpLayerDesc& D = N.L[l];
+    const uint32_t chunks = (D.ip + kWide - 1) / kWide;            // 1 beyond the first layer
+    for (uint32_t c = 0; c < chunks; c++) {
+      const uint32_t k0 = c * kWide, kn = min(kWide, D.ip - k0);
+      if (l == 0 && live) {
+        // inputs (standardized here for inference) to bf16, eight features a store
+        for (uint32_t f = 8u * cg; f < kn; f += 32u) {
+          float v[8];
+#pragma unroll
+          for (uint32_t j = 0; j < 8; j++) {
+            const uint32_t k = k0 + f + j;
+            v[j] = 0.0f;
+            if (k < D.in && grow < g.rows) {
+              v[j] = g.X[src_row * D.in + k];
+              if (!TRAIN) v[j] = (v[j] - g.x_mean[k]) / g.x_sd[k];
+            }
+          }
+          *reinterpret_cast<uint4*>(tile + (f >> 3) * (16u * kRows) + 16u * row) =
+              make_uint4(pack2(v[0], v[1]), pack2(v[2], v[3]), pack2(v[4], v[5]), pack2(v[6], v[7]));
+        }
+      }
+      tc::fence_proxy_async();
+      tc::fence_before_sync();
+      __syncthreads();
+      if (tid == 0) {
+        wait_w();
+        if (ok) issue(D, false, kn, c > 0);
+        if (TRAIN) {
+          // the layer's input, an operand of its weight gradient
+          uint8_t* dst = reinterpret_cast<uint8_t*>(l == 0 ? g.xt + mt * (kRows * D.ip) + (uint64_t)k0 * kRows
+                                                           : g.at + (mt * (L - 1u) + (l - 1u)) * (kRows * D.ip));
+          tc::bulk_store(dst, tile, kn * kRows * 2u);
+        }
+      }
+      if (ok) wait_mma();
+      if (tid == 0) {
+        // the weight buffer is free: the next chunk or layer under this epilogue
+        if (c + 1 < chunks) load_w(l, c + 1);
+        else if (l + 1 < L) load_w(l + 1, 0);
+        if (TRAIN) tc::bulk_store_wait_read();
+      }
+      if (c + 1 == chunks)
+        for (uint32_t i = tid; i < D.op; i += kRowThreads) s_bias[i] = i < D.out ? P[D.b_off + i] : 0.0f;
+      if (__syncthreads_or(!ok)) goto bail;
+      tc::fence_after_sync();
+    }
+    if (l + 1 < L) {
+      if (live) {
+        for (uint32_t c = col_lo(D.op); c < col_hi(D.op); c += 16u) {
+          float v[16];
+          tc::tmem_ld16(my_lanes + c, v);
+          float gp[16];
+#pragma unroll
+          for (int j = 0; j < 16; j++) {
+            const float z = v[j] + s_bias[c + j];
+            const float t = gelu_tanh(z);
+            v[j] = gelu_f(z, t);
+            if (TRAIN) gp[j] = gelu_grad(z, t);
+          }
+          put16(tile, row, c, v);
+          if (TRAIN) {
+            // GELU'(z) in f32 for the way back, read again by this thread alone
+            float4* gd = reinterpret_cast<float4*>(g.gz) + ((mt * (L - 1u) + l) * (D.op / 4u) + c / 4u) * kRows + row;
+#pragma unroll
+            for (int q = 0; q < 4; q++)
+              gd[q * kRows] = make_float4(gp[4 * q], gp[4 * q + 1], gp[4 * q + 2], gp[4 * q + 3]);
+          }
+        }
+      }
+    } else if (!TRAIN) {
+      float* o = g.out + ((uint64_t)blockIdx.y * g.rows + grow) * D.out;
+      if (live) {
+        for (uint32_t c = col_lo(D.op); c < col_hi(D.op); c += 16u) {
+          float v[16];
+          tc::tmem_ld16(my_lanes + c, v);
+          if (grow < g.rows) {
+#pragma unroll
+            for (int j = 0; j < 16; j++) v[j] += s_bias[c + j];
+            if (D.out % 4u == 0u && c + 16u <= D.out) {
+#pragma unroll
+              for (int q = 0; q < 4; q++)
+                reinterpret_cast<float4*>(o + c)[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+            } else {
+#pragma unroll
+              for (int j = 0; j < 16; j++)
+                if (c + j < D.out) o[c + j] = v[j];
+            }
+          }
+        }
+      }
+    } else {
+      // the mean squared error and its gradient
+      const float inv_n = 1.0f / ((float)g.rows * (float)D.out);
+      const float* y = g.Y + src_row * D.out;
+      float lsum = 0.0f;
+      for (uint32_t c = col_lo(D.op); c < col_hi(D.op); c += 16u) {
+        float v[16];
+        tc::tmem_ld16(my_lanes + c, v);
+#pragma unroll
+        for (int j = 0; j < 16; j++) {
+          const bool in = c + j < D.out;
+          const float e = in ? v[j] + s_bias[c + j] - y[c + j] : 0.0f;
+          lsum += e * e;
+          v[j] = 2.0f * e * inv_n;
+        }
+        put16(tile, row, c, v);
+        const float s = column_sum16(v, lane);
+        const uint32_t col = c + column_of(lane);
+        if ((lane & 1u) == 0u && col < D.out) atomicAdd(g.G + (uint64_t)member * N.p_stride + D.b_off + col, s);
+      }
+      for (int o = 16; o > 0; o >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
+      if (lane == 0) atomicAdd(g.loss + member, lsum * inv_n);
+    }
+  }
+  // --------------------------------------------------------------- backward
+  if (TRAIN) {
+    for (uint32_t l = L - 1;; l--) {
+      const MlpLayerDesc& D = N.L[l];
+      tc::fence_proxy_async();
+      tc::fence_before_sync();
+      __syncthreads();
+      if (tid == 0) {
+        // dZ of this layer: the input gradient's operand here, the weight gradient's later
+        tc::bulk_store(reinterpret_cast<uint8_t*>(g.dzt + (mt * L + l) * (kRows * kWide)), tile, D.op * kRows * 2u);
+        if (l > 0) {
+          wait_w();
+          if (ok) issue(D, true, D.op, false);
+        }
+      }
+      if (l == 0) break;
+      if (ok) wait_mma();
+      if (tid == 0) {
+        if (l > 1) load_w(l - 1, 0);
+        tc::bulk_store_wait_read();
+      }
+      if (__syncthreads_or(!ok)) goto bail;
+      tc::fence_after_sync();
+      const MlpLayerDesc& Dl = N.L[l - 1];     // dZ of the layer below = dX * GELU'(Z)
+      for (uint32_t c = col_lo(D.ip); c < col_hi(D.ip); c += 16u) {
+        float v[16];
+        const float4* gd =
+            reinterpret_cast<const float4*>(g.gz) + ((mt * (L - 1u) + (l - 1u)) * (D.ip / 4u) + c / 4u) * kRows + row;
+        float4 gp[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) gp[q] = gd[q * kRows];
+        tc::tmem_ld16(my_lanes + c, v);
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+          v[4 * q] *= gp[q].x;
+          v[4 * q + 1] *= gp[q].y;
+          v[4 * q + 2] *= gp[q].z;
+          v[4 * q + 3] *= gp[q].w;
+        }
+        put16(tile, row, c, v);
+        const float s = column_sum16(v, lane);
+        if ((lane & 1u) == 0u) atomicAdd(g.G + (uint64_t)member * N.p_stride + Dl.b_off + c + column_of(lane), s);
+      }
+    }
+    if (tid == 0) tc::bulk_store_wait();
+  }
+bail:
+  if (!ok && g.err) atomicOr(g.err, 16u);
+  if (tid == 0) {
+    // what is still in flight (only after a wait ran out) ends before the block does
+    if (loading) tc::mbar_wait(&bar_w, par_w, kPolls);
+    if (!ok) tc::mbar_wait(&bar_mma, par_mma ^ 1u, kPolls);
+    if (TRAIN) tc::bulk_store_wait();
+  }
+  tc::fence_before_sync();
+  __syncthreads();
+  if (warp == 0) tc::tmem_dealloc(taddr, 256);
+}
+
+// The weight gradients: dW[out x in] = dZ^T A over the batch's row tiles, both
+// read MN-major from the tile images that rows_kernel left. A CTA takes 128
+// output features x up to 256 input features of one layer of one member over
+// one share of the row tiles, two tiles in flight (96 KB each), and adds its
+// share to the gradient. Bound by those loads: 96 KB a tile for 1024 cycles of
+// MMA. The row tiles are split so that the wide layers' CTAs of all members
+// fill the chip once (launch_mlp_dw).
+constexpr uint32_t kDwThreads = 256;
+constexpr uint32_t kDwA = 16u * 16u * kRows;          // dZ: 16 feature blocks
+constexpr uint32_t kDwStage = kDwA + kTileBytes;
+constexpr uint32_t kDwSmem = 2u * kDwStage;
+
+__global__ void __launch_bounds__(kDwThreads, 1) dw_kernel(const __grid_constant__ MlpDwArgs g) {
+  extern __shared__ __align__(1024) uint8_t smem[];
+  __shared__ __align__(8) uint64_t full[2], done[2];
+  __shared__ uint32_t taddr_s;
+  const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+  const MlpNet& N = g.net;
+  const uint32_t L = N.n_layers;
+  // this CTA's layer (widest first), member, feature block, input block, share
+  uint32_t u = blockIdx.x, l = 0, mh = 1, nh = 1;
+  for (uint32_t k = 0; k < L; k++) {
+    l = k + 1 < L ? k + 1 : 0;
+    mh = (N.L[l].op + 127u) / 128u;
+    nh = (N.L[l].ip + kWide - 1) / kWide;
+    const uint32_t units = mh * nh * g.members * g.splits;
+    if (u < units) break;
+    u -= units;
+  }
+  const MlpLayerDesc& D = N.L[l];
+  const uint32_t share = u % g.splits, h = (u / g.splits) % mh, nb = (u / g.splits / mh) % nh;
+  const uint32_t mi = u / (g.splits * mh * nh);                       // member of this launch
+  const uint32_t per = (g.tiles + g.splits - 1) / g.splits, tb = share * per, te = min(g.tiles, tb + per);
+  if (tb >= te) return;
+  const uint32_t n0 = nb * kWide, nn = min(kWide, D.ip - n0);
+  const uint32_t mo = min(128u, D.op - 128u * h);                     // output features here (the rest of M is unused)
+  if (tid == 0) {
+    for (int i = 0; i < 2; i++) {
+      tc::mbar_init(&full[i], 1);
+      tc::mbar_init(&done[i], 1);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 0) tc::tmem_alloc(&taddr_s, 256);
+  tc::fence_before_sync();
+  __syncthreads();
+  tc::fence_after_sync();
+  const uint32_t taddr = taddr_s;
+  const uint32_t bz = mo * kRows * 2u, ba = nn * kRows * 2u;
+  bool ok = true;
+  const uint32_t n = te - tb;
+  if (tid == 0) {
+    auto load = [&](uint32_t i) {
+      const uint64_t mt = (uint64_t)mi * g.tiles + tb + i;
+      uint8_t* s = smem + (i & 1u) * kDwStage;
+      const uint8_t* z = reinterpret_cast<const uint8_t*>(g.dzt + (mt * L + l) * (kRows * kWide)) + h * kDwA;
+      const uint8_t* a = reinterpret_cast<const uint8_t*>(l == 0 ? g.xt + mt * (kRows * D.ip) + (uint64_t)n0 * kRows
+                                                                 : g.at + (mt * (L - 1u) + (l - 1u)) * (kRows * D.ip));
+      tc::mbar_expect_tx(&full[i & 1u], bz + ba);
+      tc::bulk_load(s, z, bz, &full[i & 1u]);
+      for (uint32_t o = 0; o < ba; o += 32768u)
+        tc::bulk_load(s + kDwA + o, a + o, min(32768u, ba - o), &full[i & 1u]);
+    };
+    load(0);
+    if (n > 1) load(1);
+    const uint32_t idesc = tc::idesc_bf16_f32(nn, 128u) | tc::kTransA | tc::kTransB;
+    for (uint32_t i = 0; i < n && ok; i++) {
+      const uint32_t b = i & 1u, ph = (i >> 1) & 1u;
+      ok = tc::mbar_wait(&full[b], ph, kPolls);
+      if (!ok) break;
+      const uint32_t a0 = tc::smem_u32(smem + b * kDwStage), b0 = a0 + kDwA;
+      for (uint32_t s = 0; s < kRows / 16u; s++)
+        tc::mma_bf16(taddr, tc::smem_desc(a0 + 256u * s, 128u, 16u * kRows), tc::smem_desc(b0 + 256u * s, 128u, 16u * kRows),
+                     idesc, i > 0 || s > 0);
+      tc::mma_commit(&done[b]);
+      // the stage is refilled once its MMAs are done, while the other stage's run
+      if (i >= 1 && i + 1 < n) {
+        ok = tc::mbar_wait(&done[b ^ 1u], ((i - 1) >> 1) & 1u, kPolls);
+        if (ok) load(i + 1);
+      }
+    }
+    // the last MMAs (and with them every earlier one)
+    if (ok) ok = tc::mbar_wait(&done[(n - 1) & 1u], ((n - 1) >> 1) & 1u, kPolls);
+    if (!ok) {
+      if (g.err) atomicOr(g.err, 16u);
+      // one more bounded wait for what may be in flight
+      for (uint32_t b = 0; b < 2; b++) {
+        tc::mbar_wait(&full[b], 0, 1u << 16);
+        tc::mbar_wait(&done[b], 0, 1u << 16);
+      }
+    }
+  }
+  if (!__syncthreads_or(!ok)) {
+    tc::fence_after_sync();
+    const uint32_t o = 128u * h + (warp & 3u) * 32u + lane;
+    float* W = g.G + (uint64_t)(g.member0 + mi) * N.p_stride + D.w_off + (uint64_t)o * D.in + n0;
+    const bool v4 = D.in % 4u == 0u;            // (w_off and n0 are multiples of 4)
+    const uint32_t nv = min(nn, D.in - n0);     // columns that exist
+    for (uint32_t c = 16u * (warp >> 2); c < nn; c += 32u) {
+      float v[16];
+      tc::tmem_ld16(taddr + (((warp & 3u) * 32u) << 16) + c, v);
+      if (o < D.out) {
+#pragma unroll
+        for (uint32_t q = 0; q < 16; q += 4) {
+          if (v4 && c + q < nv) {
+            asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(W + c + q), "f"(v[q]), "f"(v[q + 1]),
+                         "f"(v[q + 2]), "f"(v[q + 3])
+                         : "memory");
+          } else {
+#pragma unroll
+            for (uint32_t j = 0; j < 4; j++)
+              if (c + q + j < nv) atomicAdd(W + c + q + j, v[q + j]);
+          }
+        }
+      }
+    }
+  }
+  tc::fence_before_sync();
+  __syncthreads();
+  if (warp == 0) tc::tmem_dealloc(taddr, 256);
+}
+
+// bf16 copy of one parameter into its layer's image
+__device__ __forceinline__ void put_image(uint16_t* img, const MlpLayerDesc& D, uint32_t o, uint32_t k, float x) {
+  img[D.img_off + (uint64_t)(k >> 3) * (8u * D.op) + 8u * o + (k & 7u)] = __bfloat16_as_ushort(__float2bfloat16_rn(x));
+}
+
+// AdamW over every member's parameters, four a thread; the weights' bf16 images
+// follow, and the gradients are left zero for the next step. The block that
+// ends last closes the step: the counter, and at an epoch's end its losses.
+__global__ void __launch_bounds__(256) adamw_kernel(const __grid_constant__ MlpAdamwArgs g) {
+  const MlpNet& N = g.net;
+  const uint32_t t = *g.step;
+  const float lr = g.sched[3u * t], bc1 = g.sched[3u * t + 1u], bc2 = g.sched[3u * t + 2u];
+  const uint32_t quads = N.p_stride / 4u;
+  const uint64_t total = (uint64_t)quads * N.members;
+  for (uint64_t q = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; q < total; q += (uint64_t)gridDim.x * blockDim.x) {
+    const uint32_t e = (uint32_t)(q / quads), p = 4u * (uint32_t)(q % quads);
+    const uint64_t at = (uint64_t)e * N.p_stride + p;
+    uint32_t l = 0;
+    while (l + 1 < N.n_layers && p >= N.L[l + 1].w_off) l++;
+    const MlpLayerDesc& D = N.L[l];
+    const bool isw = p < D.b_off;               // (b_off is a multiple of 4: a quad is all weights or none)
+    float4 W = reinterpret_cast<const float4*>(g.P)[at / 4];
+    float4 M = reinterpret_cast<const float4*>(g.M1)[at / 4];
+    float4 V = reinterpret_cast<const float4*>(g.V1)[at / 4];
+    const float4 G = reinterpret_cast<const float4*>(g.G)[at / 4];
+    float x[4] = {W.x, W.y, W.z, W.w}, m[4] = {M.x, M.y, M.z, M.w}, v[4] = {V.x, V.y, V.z, V.w};
+    const float gr[4] = {G.x, G.y, G.z, G.w};
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      m[j] = g.b1 * m[j] + (1.0f - g.b1) * gr[j];
+      v[j] = g.b2 * v[j] + (1.0f - g.b2) * gr[j] * gr[j];
+      const float mh = m[j] / bc1, vh = v[j] / bc2;
+      x[j] = x[j] - lr * (mh / (sqrtf(vh) + g.eps) + (isw ? g.wd : 0.0f) * x[j]);
+    }
+    reinterpret_cast<float4*>(g.P)[at / 4] = make_float4(x[0], x[1], x[2], x[3]);
+    reinterpret_cast<float4*>(g.M1)[at / 4] = make_float4(m[0], m[1], m[2], m[3]);
+    reinterpret_cast<float4*>(g.V1)[at / 4] = make_float4(v[0], v[1], v[2], v[3]);
+    reinterpret_cast<float4*>(g.G)[at / 4] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (isw) {
+      uint16_t* im = g.img + (uint64_t)e * N.img_stride;
+      uint32_t i = p - D.w_off, o = i / D.in, k = i - o * D.in;
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        if (o < D.out) put_image(im, D, o, k, x[j]);
+        if (++k == D.in) {
+          k = 0;
+          o++;
+        }
+      }
+    }
+  }
+  __shared__ bool last;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last = atomicAdd(g.ticket, 1u) + 1u == gridDim.x;
+  }
+  __syncthreads();
+  if (last) {
+    const bool ends = (t + 1u) % g.spe == 0u;
+    if (threadIdx.x < N.members) {
+      if (ends) g.epoch_loss[(uint64_t)threadIdx.x * g.epochs + t / g.spe] = g.loss[threadIdx.x];
+      g.loss[threadIdx.x] = 0.0f;
+    }
+    if (threadIdx.x == 0) {
+      *g.ticket = 0;
+      *g.step = t + 1u;
+    }
+  }
+}
+
+// Every member's images from its f32 parameters
+__global__ void image_kernel(const __grid_constant__ MlpNet N, const float* __restrict__ P, uint16_t* __restrict__ img) {
+  const uint32_t e = blockIdx.y;
+  for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < N.p_stride; p += gridDim.x * blockDim.x) {
+    uint32_t l = 0;
+    while (l + 1 < N.n_layers && p >= N.L[l + 1].w_off) l++;
+    const MlpLayerDesc& D = N.L[l];
+    const uint32_t i = p - D.w_off;
+    if (i < D.in * D.out)
+      put_image(img + (uint64_t)e * N.img_stride, D, i / D.in, i % D.in, P[(uint64_t)e * N.p_stride + p]);
+  }
+}
+
+// One warp per row: the members' outputs in the targets' units, their mean and
+// spread (sums in member order), and per row the largest spread among outputs
+// whose mean is >= level.
+__global__ void __launch_bounds__(256) ensemble_kernel(const float* __restrict__ y, uint32_t members, uint32_t rows, uint32_t cols,
+                                const float* __restrict__ mean, const float* __restrict__ sd, float inv_e,
+                                float level, float* __restrict__ out_mean, float* __restrict__ out_std,
+                                float* __restrict__ out_spread) {
+  const uint32_t row = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31u;
+  if (row >= rows) return;
+  float most = 0.0f;
+  for (uint32_t c = lane; c < cols; c += 32) {
+    const float s = sd[c], b = mean[c];
+    float a = 0.0f, a2 = 0.0f;
+    for (uint32_t e = 0; e < members; e++) {
+      const float v = y[((uint64_t)e * rows + row) * cols + c] * s + b;
+      a = e == 0 ? v : a + v;
+      a2 = e == 0 ? v * v : a2 + v * v;
+    }
+    const float m = a * inv_e;
+    const float d = sqrtf(fmaxf(a2 * inv_e - m * m, 0.0f));
+    const uint64_t i = (uint64_t)row * cols + c;
+    out_mean[i] = m;
+    if (out_std) out_std[i] = d;
+    if (m >= level) most = fmaxf(most, d);
+  }
+  for (int o = 16; o > 0; o >>= 1) most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, o));
+  if (lane == 0 && out_spread) out_spread[row] = most;
+}
+
+}  // namespace
+
+// The kernels' shared-memory limits (call it outside any stream capture,
+// before the first launch on a device; repeating it is harmless).
+cudaError_t mlp_net_init() {
+  cudaError_t e = cudaFuncSetAttribute(rows_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRowsSmem);
+  if (e != cudaSuccess) return e;
+  e = cudaFuncSetAttribute(rows_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRowsSmem);
+  if (e != cudaSuccess) return e;
+  return cudaFuncSetAttribute(dw_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDwSmem);
+}
+
+cudaError_t launch_mlp_rows(const MlpRowsArgs& a, uint32_t members, bool train, cudaStream_t s) {
+  if (a.rows == 0 || members == 0) return cudaSuccess;
+  const dim3 grid((a.rows + kRows - 1) / kRows, members);
+  if (train) rows_kernel<true><<<grid, kRowThreads, kRowsSmem, s>>>(a);
+  else rows_kernel<false><<<grid, kRowThreads, kRowsSmem, s>>>(a);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_mlp_dw(MlpDwArgs a, int n_sms, cudaStream_t s) {
+  const uint32_t L = a.net.n_layers;
+  auto units = [&](uint32_t l) {
+    return ((a.net.L[l].op + 127u) / 128u) * ((a.net.L[l].ip + kWide - 1) / kWide) * a.members;
+  };
+  uint32_t wide = 0, all = 0;
+  for (uint32_t l = 0; l < L; l++) {
+    all += units(l);
+    if (l > 0) wide += units(l);
+  }
+  // shares of the row tiles: the layers beyond the first fill the chip once
+  // (the first, narrow one's CTAs are short and fill the gaps)
+  a.splits = std::max(1u, std::min(a.tiles, (uint32_t)n_sms / std::max(1u, wide)));
+  dw_kernel<<<all * a.splits, kDwThreads, kDwSmem, s>>>(a);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_mlp_adamw(const MlpAdamwArgs& a, int n_sms, cudaStream_t s) {
+  const uint64_t quads = (uint64_t)a.net.p_stride / 4u * a.net.members;
+  const uint32_t blocks = (uint32_t)std::min<uint64_t>((quads + 255) / 256, (uint64_t)n_sms * 8u);
+  adamw_kernel<<<blocks, 256, 0, s>>>(a);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_mlp_images(const MlpNet& net, const float* P, uint16_t* img, cudaStream_t s) {
+  const dim3 grid(std::min(1024u, (net.p_stride + 255u) / 256u), net.members);
+  image_kernel<<<grid, 256, 0, s>>>(net, P, img);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_mlp_ensemble(const float* y, uint32_t members, uint32_t rows, uint32_t cols, const float* mean,
+                                const float* sd, float level, float* out_mean, float* out_std, float* out_spread,
+                                cudaStream_t s) {
+  if (rows == 0) return cudaSuccess;
+  ensemble_kernel<<<(rows + 7) / 8, 256, 0, s>>>(y, members, rows, cols, mean, sd, 1.0f / (float)members, level,
+                                                 out_mean, out_std, out_spread);
+  return cudaGetLastError();
+}
+
+}  // namespace omg

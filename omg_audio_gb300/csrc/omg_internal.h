@@ -335,7 +335,7 @@ struct DDomeLaunch {
 cudaError_t launch_dome(const DDomeLaunch& L, cudaStream_t s);
 
 // mlp.cu: tensor-core GEMM D[M x N] = A[M x K] . B[N x K]^T (bf16 in, f32
-// accumulate) with strided operands and a fused epilogue.
+// accumulate) with strided operands.
 struct GemmArgs {
   const void* A;            // __nv_bfloat16; element (m, k) at A[m a_rs + k a_ks]
   int64_t a_rs, a_ks;
@@ -343,56 +343,14 @@ struct GemmArgs {
   int64_t b_rs, b_ks;
   uint32_t M, N, K;
   uint32_t n_tile;          // columns per CTA: multiple of 16, <= 256
-  const float* bias;        // [N] or null
-  float* D;                 // f32 [M x ldd] or null
+  float* D;                 // f32 [M x ldd]
   int64_t ldd;
   uint32_t accumulate;      // 1: D += (atomically; K split over grid z)
-  float* Z;                 // pre-activation f32 or null
-  int64_t ldz;
-  void* Y;                  // __nv_bfloat16 activation out or null
-  int64_t ldy;
-  void* Yt;                 // the same activation transposed (element (m, n) at Yt[n ldyt + m]) or null
-  int64_t ldyt;
-  uint32_t act;             // 0 none, 1 GELU (tanh form)
   uint32_t* err;            // error word: 16 = an mbarrier wait ran out
 };
 size_t gemm_smem_bytes();
 cudaError_t gemm_init();
 cudaError_t launch_gemm(const GemmArgs& g, uint32_t k_split, cudaStream_t s);
-// backward elementwise on 32 x 32 tiles: mode 0 the MSE loss gradient of
-// P = outputs against Q = targets (weights w per column, nullable; loss +=),
-// mode 1 dZ = P (dA) * GELU'(Q (Z)); writes dZ, its bf16 copy and transpose,
-// and adds the column sums into gb (zeroed by the caller)
-cudaError_t launch_grad_tile(uint32_t mode, const float* P, const float* Q, const float* w, uint32_t rows,
-                             uint32_t cols, float* dZ, void* dZh, void* dZht, float* gb, float* loss, cudaStream_t s);
-// AdamW of every layer of one ensemble member in one launch
-struct AdamwLayer {
-  float *W, *mW, *vW, *b, *mb, *vb;
-  const float *gW, *gb;
-  void *Wh, *Wht;
-  uint32_t in, out;
-  uint64_t off;             // first element of this layer in the launch's index space (W then b)
-};
-constexpr int kMaxAdamwLayers = 17;
-struct AdamwTable {
-  AdamwLayer L[kMaxAdamwLayers];
-  uint32_t n;
-  uint64_t total;
-};
-cudaError_t launch_adamw_all(const AdamwTable& tab, const float* sched, const uint32_t* step, float b1, float b2,
-                             float eps, float wd, cudaStream_t s);
-// inputs (bf16 copy + transpose) and targets (f32) of this step's batch rows
-cudaError_t launch_gather_pair(const float* X, uint32_t xcols, const float* Y, uint32_t ycols, const uint32_t* perm,
-                               const uint32_t* step, uint32_t spe, uint32_t rows, void* xh, void* xht, float* t,
-                               cudaStream_t s);
-cudaError_t launch_step(uint32_t* step, cudaStream_t s);
-cudaError_t launch_to_bf16_t(const float* x, uint32_t rows, uint32_t cols, void* xh, void* xht, cudaStream_t s);
-cudaError_t launch_standardize(const float* x, const float* mean, const float* sd, uint32_t cols, uint64_t n,
-                               void* out, cudaStream_t s);
-cudaError_t launch_ensemble(const float* y, const float* mean, const float* sd, uint32_t cols, uint64_t n,
-                            float* acc, float* acc2, bool first, bool last, float inv_e, cudaStream_t s);
-cudaError_t launch_row_spread(const float* mean, const float* sd, uint32_t cols, uint32_t rows, float level,
-                              float* out, cudaStream_t s);
 cudaError_t build_dome_fan(float4* fan, uint32_t n_fan, cudaStream_t s);
 
 // early.cu: world early reflections (pt_mesh.rs). One surface of the table

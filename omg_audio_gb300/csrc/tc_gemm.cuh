@@ -35,6 +35,22 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t saddr) {
   return d;
 }
 
+// The same with the caller's strides, for operand images without a chunked K:
+// K-major, `lbo` bytes between core matrices along K and `sbo` between 8-row
+// groups; MN-major (the image read transposed: a core matrix is then 8 K rows
+// of 8 consecutive M or N elements), `lbo` bytes between core matrices along K
+// and `sbo` between them along M or N.
+__device__ __forceinline__ uint64_t smem_desc(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
+  uint64_t d = 0;
+  d |= (uint64_t)((saddr & 0x3FFFFu) >> 4);
+  d |= (uint64_t)((lbo >> 4) & 0x3FFFu) << 16;
+  d |= (uint64_t)((sbo >> 4) & 0x3FFFu) << 32;
+  d |= (uint64_t)1 << 46;
+  return d;
+}
+// idesc_bf16_f32 bits that make A or B MN-major
+constexpr uint32_t kTransA = 1u << 15, kTransB = 1u << 16;
+
 // Instruction descriptor of tcgen05.mma kind::f16: f32 accumulator, bf16 A
 // and B, both K-major, N = n (multiple of 16, <= 256), M = 128.
 __host__ __device__ constexpr uint32_t idesc_bf16_f32(uint32_t n, uint32_t m) {
@@ -109,6 +125,26 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* mbar, uint32_t parity, uint3
   }
   return false;
 }
+
+// Bulk copies (multiples of 16 bytes, 16-byte aligned). A load completes on an
+// mbarrier that was told to expect its bytes; a store completes with its group.
+__device__ __forceinline__ void mbar_expect_tx(uint64_t* mbar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(mbar)), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void bulk_load(void* smem_dst, const void* gsrc, uint32_t bytes, uint64_t* mbar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                   smem_u32(smem_dst)),
+               "l"(gsrc), "r"(bytes), "r"(smem_u32(mbar))
+               : "memory");
+}
+__device__ __forceinline__ void bulk_store(void* gdst, const void* smem_src, uint32_t bytes) {
+  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;\n\tcp.async.bulk.commit_group;" ::"l"(gdst),
+               "r"(smem_u32(smem_src)), "r"(bytes)
+               : "memory");
+}
+// this thread's bulk stores have read their shared memory / are complete
+__device__ __forceinline__ void bulk_store_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+__device__ __forceinline__ void bulk_store_wait() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
 // Asynchronous 16-byte global -> shared copies (cp.async, L2 only): `bytes`
 // (0 or 16) are read, the rest of the 16 bytes is filled with zeros.

@@ -27,8 +27,7 @@ struct MlpScratch {
 // One of the two chunks of rows in flight during inference.
 struct MlpChunk {
   uint32_t cap = 0;
-  DevBuf<float> x, y, mean, std, spread;   // y: [member][row][out]
-  PinBuf<float> h_x, h_mean, h_std, h_spread;
+  DevBuf<float> y, mean, std, spread;      // y: [member][row][out]
   cudaEvent_t done = nullptr;
   ~MlpChunk() {
     if (done) cudaEventDestroy(done);
@@ -46,7 +45,10 @@ struct MlpRec {
   // standardization (host and device)
   std::vector<float> x_mean, x_std, y_mean, y_std;
   DevBuf<float> d_x_mean, d_x_std, d_y_mean, d_y_std;
-  MlpChunk chunk[2];                            // inference
+  // inference: a group's inputs, two chunks' outputs, the stream of the copies back
+  DevBuf<float> xin;
+  MlpChunk chunk[2];
+  cudaStream_t back = nullptr;
   MlpScratch train_s, grad_s;
   DevBuf<float> grad_x, grad_y;                 // omg_mlp_grad's batch
   // dataset (standardized, device)
@@ -58,12 +60,18 @@ struct MlpRec {
   PinBuf<uint32_t> h_perm;
   DevBuf<float> epoch_loss;
   DevBuf<uint32_t> err;
+  PinBuf<uint32_t> h_err;
+  ~MlpRec() {
+    if (back) cudaStreamDestroy(back);
+  }
   PinBuf<float> h_loss;
 };
 
 }  // namespace omg
 
 namespace {
+
+constexpr uint32_t kGraphSteps = 8;   // training steps recorded in one graph
 
 uint32_t n_layers(const MlpRec& M) { return M.cfg.n_hidden + 1; }
 
@@ -139,11 +147,12 @@ MlpDwArgs dw_args(const MlpRec& M, const MlpScratch& S, uint32_t rows, uint32_t 
   return a;
 }
 
+// The kernels' error word, brought to M.h_err behind the work on stream s; then, once that is done, its meaning.
+cudaError_t fetch_err(MlpRec& M, cudaStream_t s) {
+  return cudaMemcpyAsync(M.h_err.p, M.err.p, 4, cudaMemcpyDeviceToHost, s);
+}
 int32_t check_err(omg_ctx* ctx, MlpRec& M) {
-  uint32_t e = 0;
-  CK(cudaMemcpyAsync(&e, M.err.p, 4, cudaMemcpyDeviceToHost, ctx->stream));
-  CK(cudaStreamSynchronize(ctx->stream));
-  if (e) {
+  if (*M.h_err.p) {
     ctx->last_error = "surrogate network: an mbarrier wait ran out";
     CK(cudaMemsetAsync(M.err.p, 0, 4, ctx->stream));
     return OMG_E_TIMEOUT;
@@ -171,17 +180,6 @@ void each_param(const MlpNet& N, F&& f) {
   for (uint32_t l = 0; l < N.n_layers; l++) {
     f(N.L[l].w_off, N.L[l].in * N.L[l].out);
     f(N.L[l].b_off, N.L[l].out);
-  }
-}
-
-void copy_big(float* dst, const float* src, uint64_t n) {
-  // one thread copies at about 17 GB/s into freshly mapped pages
-  const int threads = n * sizeof(float) >= (1u << 20) ? 4 : 1;
-  const uint64_t per = (n + threads - 1) / threads;
-#pragma omp parallel for num_threads(threads) schedule(static)
-  for (int t = 0; t < threads; t++) {
-    const uint64_t lo = std::min<uint64_t>(n, per * t), hi = std::min<uint64_t>(n, lo + per);
-    std::memcpy(dst + lo, src + lo, (hi - lo) * sizeof(float));
   }
 }
 
@@ -236,6 +234,8 @@ int32_t omg_mlp_create(omg_ctx* ctx, const omg_mlp_config* cfg, uint32_t* id) {
   M->y_mean.assign(cfg->n_out, 0.0f);
   M->y_std.assign(cfg->n_out, 1.0f);
   CK(M->err.alloc(1));
+  CK(M->h_err.alloc(1));
+  CK(M->h_loss.alloc(1));
   CK(cudaMemsetAsync(M->err.p, 0, 4, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
   int32_t rc = sync_norm(ctx, *M);
@@ -361,23 +361,34 @@ int32_t omg_mlp_train(omg_ctx* ctx, uint32_t id, const omg_mlp_train_config* tc,
   aa.b2 = tc->beta2;
   aa.eps = tc->eps;
   aa.wd = tc->weight_decay;
-  cudaGraphExec_t graph = nullptr;
+  // two graphs: kGraphSteps steps (the gap between two graphs is some us), and one step for the rest of an epoch
+  const uint32_t per_graph[2] = {std::min(spe, kGraphSteps), 1u};
+  cudaGraphExec_t graph[2] = {nullptr, nullptr};
   {
     cudaStream_t cs;
     CK(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
-    cudaError_t ce = cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal);
-    cudaGraph_t g = nullptr;
-    if (ce == cudaSuccess) {
-      ce = launch_mlp_rows(ra, E, true, cs);
-      if (ce == cudaSuccess) ce = launch_mlp_dw(dw_args(M, M.train_s, B, E, 0), ctx->n_sms, cs);
-      if (ce == cudaSuccess) ce = launch_mlp_adamw(aa, ctx->n_sms, cs);
+    cudaError_t ce = cudaSuccess;
+    for (int k = 0; k < 2 && ce == cudaSuccess; k++) {
+      if (k == 1 && spe % per_graph[0] == 0) break;
+      ce = cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal);
+      if (ce != cudaSuccess) break;
+      for (uint32_t i = 0; i < per_graph[k] && ce == cudaSuccess; i++) {
+        ce = launch_mlp_rows(ra, E, true, cs);
+        if (ce == cudaSuccess) ce = launch_mlp_dw(dw_args(M, M.train_s, B, E, 0), ctx->n_sms, cs);
+        if (ce == cudaSuccess) ce = launch_mlp_adamw(aa, ctx->n_sms, cs);
+      }
+      cudaGraph_t g = nullptr;
       const cudaError_t ee = cudaStreamEndCapture(cs, &g);
       if (ce == cudaSuccess) ce = ee;
-      if (ce == cudaSuccess) ce = cudaGraphInstantiate(&graph, g, 0);
+      if (ce == cudaSuccess) ce = cudaGraphInstantiate(&graph[k], g, 0);
       if (g) cudaGraphDestroy(g);
     }
     cudaStreamDestroy(cs);
-    if (ce != cudaSuccess) return fail(ctx, ce, "training step capture");
+    if (ce != cudaSuccess) {
+      for (cudaGraphExec_t g : graph)
+        if (g) cudaGraphExecDestroy(g);
+      return fail(ctx, ce, "training step capture");
+    }
   }
   std::vector<std::mt19937_64> rngs;
   for (uint32_t e = 0; e < E; e++) rngs.emplace_back((tc->seed ? tc->seed : 7u) + 0x9E3779B97F4A7C15ull * e);
@@ -401,15 +412,21 @@ int32_t omg_mlp_train(omg_ctx* ctx, uint32_t id, const omg_mlp_train_config* tc,
     shuffle_epoch(ep);
     const uint64_t at = (ep & 1u) * half;
     ce = cudaMemcpyAsync(M.perm.p + at, M.h_perm.p + at, half * 4, cudaMemcpyHostToDevice, s);
-    for (uint32_t st = 0; st < spe && ce == cudaSuccess; st++) ce = cudaGraphLaunch(graph, s);
+    for (uint32_t st = 0; st < spe && ce == cudaSuccess;) {
+      const int k = spe - st >= per_graph[0] ? 0 : 1;
+      ce = cudaGraphLaunch(graph[k], s);
+      st += per_graph[k];
+    }
     if (ce == cudaSuccess) ce = cudaEventRecord(ev[ep & 1u], s);
   }
   std::vector<float> losses(n_loss);
   if (ce == cudaSuccess) ce = cudaMemcpyAsync(losses.data(), M.epoch_loss.p, n_loss * 4, cudaMemcpyDeviceToHost, s);
+  if (ce == cudaSuccess) ce = fetch_err(M, s);
   const cudaError_t se = cudaStreamSynchronize(s);
   for (int k = 0; k < 2; k++)
     if (ev[k]) cudaEventDestroy(ev[k]);
-  cudaGraphExecDestroy(graph);
+  for (cudaGraphExec_t g : graph)
+    if (g) cudaGraphExecDestroy(g);
   if (ce != cudaSuccess) return fail(ctx, ce, "training");
   if (se != cudaSuccess) return fail(ctx, se, "training");
   if (epoch_loss) std::copy(losses.begin(), losses.end(), epoch_loss);
@@ -431,39 +448,42 @@ int32_t surrogate_run(omg_ctx* ctx, uint32_t id, const float* x, uint32_t n, flo
   if (it == ctx->mlps.end()) return OMG_E_NOT_FOUND;
   MlpRec& M = *it->second;
   const uint32_t ni = M.cfg.n_in, no = M.cfg.n_out, E = M.cfg.members;
-  // Rows a launch: the row tiles of all members fill the chip once (one CTA a
-  // multiprocessor); two chunks in flight, so that the copies and the host's
-  // part of one run under the other's kernels.
+  // Rows a launch (chunk): the row tiles of all members fill the chip once (one
+  // CTA a multiprocessor). Two chunks are in flight: one's results are copied
+  // straight into the caller's arrays while the other's kernels run (8 MB from
+  // the device into pageable memory take 60 us on the GB300's host, a copy
+  // through pinned memory 53 us and 170 us more for the host's part). The
+  // inputs go up for up to kGroup chunks at a time.
+  constexpr uint32_t kGroup = 8;
   const uint32_t wave = 128u * std::max(1u, (uint32_t)ctx->n_sms / E);
   const uint32_t parts = (n + wave - 1) / wave;
   const uint32_t chunk = std::min(n, ((n + parts - 1) / parts + 127u) / 128u * 128u);
-  for (MlpChunk& C : M.chunk) {
-    if (C.cap >= chunk || (&C != M.chunk && n <= chunk)) continue;
+  const uint64_t group = (uint64_t)chunk * kGroup;
+  cudaStream_t s = ctx->stream;
+  if (!M.back) CK(cudaStreamCreateWithFlags(&M.back, cudaStreamNonBlocking));
+  if (M.xin.n < std::min<uint64_t>(n, group) * ni) CK(M.xin.alloc(std::min<uint64_t>(n, group) * ni));
+  for (int k = 0; k < (n > chunk ? 2 : 1); k++) {
+    MlpChunk& C = M.chunk[k];
+    if (!C.done) CK(cudaEventCreateWithFlags(&C.done, cudaEventDisableTiming));
+    if (C.cap >= chunk && (!y_std || C.std.p)) continue;
     C.cap = 0;
-    CK(C.x.alloc((size_t)chunk * ni));
     CK(C.y.alloc((size_t)chunk * no * E));
     CK(C.mean.alloc((size_t)chunk * no));
-    CK(C.std.alloc((size_t)chunk * no));
+    if (y_std) CK(C.std.alloc((size_t)chunk * no));
     CK(C.spread.alloc(chunk));
-    CK(C.h_x.alloc((size_t)chunk * ni));
-    CK(C.h_mean.alloc((size_t)chunk * no));
-    CK(C.h_std.alloc((size_t)chunk * no));
-    CK(C.h_spread.alloc(chunk));
-    if (!C.done) CK(cudaEventCreateWithFlags(&C.done, cudaEventDisableTiming));
     C.cap = chunk;
   }
-  cudaStream_t s = ctx->stream;
-  auto submit = [&](MlpChunk& C, uint32_t r0) -> int32_t {
-    const uint32_t rows = std::min(chunk, n - r0);
-    const uint64_t nx = (uint64_t)rows * ni, ny = (uint64_t)rows * no;
-    std::memcpy(C.h_x.p, x + (uint64_t)r0 * ni, nx * 4);
-    CK(cudaMemcpyAsync(C.x.p, C.h_x.p, nx * 4, cudaMemcpyHostToDevice, s));
+  auto submit = [&](uint64_t r0) -> int32_t {
+    MlpChunk& C = M.chunk[(r0 / chunk) & 1u];
+    const uint32_t rows = (uint32_t)std::min<uint64_t>(chunk, n - r0);
+    if (r0 % group == 0)
+      CK(cudaMemcpyAsync(M.xin.p, x + r0 * ni, std::min<uint64_t>(n - r0, group) * ni * 4, cudaMemcpyHostToDevice, s));
     MlpRowsArgs a{};
     a.net = M.net;
     a.rows = rows;
     a.P = M.P.p;
     a.img = M.img.p;
-    a.X = C.x.p;
+    a.X = M.xin.p + (r0 % group) * ni;
     a.x_mean = M.d_x_mean.p;
     a.x_sd = M.d_x_std.p;
     a.out = C.y.p;
@@ -471,22 +491,21 @@ int32_t surrogate_run(omg_ctx* ctx, uint32_t id, const float* x, uint32_t n, flo
     CK(launch_mlp_rows(a, E, false, s));
     CK(launch_mlp_ensemble(C.y.p, E, rows, no, M.d_y_mean.p, M.d_y_std.p, level, C.mean.p, y_std ? C.std.p : nullptr,
                            row_spread ? C.spread.p : nullptr, s));
-    CK(cudaMemcpyAsync(C.h_mean.p, C.mean.p, ny * 4, cudaMemcpyDeviceToHost, s));
-    if (y_std) CK(cudaMemcpyAsync(C.h_std.p, C.std.p, ny * 4, cudaMemcpyDeviceToHost, s));
-    if (row_spread) CK(cudaMemcpyAsync(C.h_spread.p, C.spread.p, (size_t)rows * 4, cudaMemcpyDeviceToHost, s));
+    if (r0 + rows == n) CK(fetch_err(M, s));
     CK(cudaEventRecord(C.done, s));
     return OMG_OK;
   };
   int32_t rc = OMG_OK;
-  if ((rc = submit(M.chunk[0], 0))) return rc;
-  for (uint32_t r0 = 0, k = 0; r0 < n; r0 += chunk, k ^= 1u) {
-    if (n - r0 > chunk && (rc = submit(M.chunk[k ^ 1u], r0 + chunk))) return rc;
-    MlpChunk& C = M.chunk[k];
-    const uint32_t rows = std::min(chunk, n - r0);
+  if ((rc = submit(0))) return rc;
+  for (uint64_t r0 = 0; r0 < n; r0 += chunk) {
+    if (n - r0 > chunk && (rc = submit(r0 + chunk))) return rc;
+    MlpChunk& C = M.chunk[(r0 / chunk) & 1u];
+    const uint64_t rows = std::min<uint64_t>(chunk, n - r0);
     if ((rc = wait_event(ctx, C.done, timeout_of(ctx)))) return rc;
-    copy_big(y_mean + (uint64_t)r0 * no, C.h_mean.p, (uint64_t)rows * no);
-    if (y_std) copy_big(y_std + (uint64_t)r0 * no, C.h_std.p, (uint64_t)rows * no);
-    if (row_spread) std::memcpy(row_spread + r0, C.h_spread.p, (size_t)rows * 4);
+    CK(cudaMemcpyAsync(y_mean + r0 * no, C.mean.p, rows * no * 4, cudaMemcpyDeviceToHost, M.back));
+    if (y_std) CK(cudaMemcpyAsync(y_std + r0 * no, C.std.p, rows * no * 4, cudaMemcpyDeviceToHost, M.back));
+    if (row_spread) CK(cudaMemcpyAsync(row_spread + r0, C.spread.p, rows * 4, cudaMemcpyDeviceToHost, M.back));
+    CK(cudaStreamSynchronize(M.back));   // the chunk's buffers are free for the one after next
   }
   return check_err(ctx, M);
 }
@@ -527,17 +546,22 @@ int32_t omg_mlp_grad(omg_ctx* ctx, uint32_t id, uint32_t member, const float* x,
   CK(cudaMemsetAsync(M.loss.p + member, 0, 4, s));
   CK(launch_mlp_rows(rows_args(M, M.grad_s, M.grad_x.p, M.grad_y.p, n, member), 1, true, s));
   CK(launch_mlp_dw(dw_args(M, M.grad_s, n, 1, member), ctx->n_sms, s));
-  if (M.h_loss.n < N.p_stride + 1u) CK(M.h_loss.alloc(N.p_stride + 1u));
   CK(cudaMemcpyAsync(M.h_loss.p, M.loss.p + member, 4, cudaMemcpyDeviceToHost, s));
-  if (grads) CK(cudaMemcpyAsync(M.h_loss.p + 1, G, (size_t)N.p_stride * 4, cudaMemcpyDeviceToHost, s));
-  CK(cudaStreamSynchronize(s));
-  if (grads) {
-    size_t off = 0;
+  CK(fetch_err(M, s));
+  uint64_t packed = 0;
+  each_param(N, [&](uint32_t, uint32_t k) { packed += k; });
+  if (grads && packed == N.p_stride) {
+    CK(cudaMemcpyAsync(grads, G, packed * 4, cudaMemcpyDeviceToHost, s));   // the block has no padding
+  } else if (grads) {
+    cudaError_t e = cudaSuccess;
+    uint64_t off = 0;
     each_param(N, [&](uint32_t at, uint32_t k) {
-      std::memcpy(grads + off, M.h_loss.p + 1 + at, (size_t)k * 4);
+      if (e == cudaSuccess) e = cudaMemcpyAsync(grads + off, G + at, (size_t)k * 4, cudaMemcpyDeviceToHost, s);
       off += k;
     });
+    CK(e);
   }
+  CK(cudaStreamSynchronize(s));
   if (loss) *loss = M.h_loss.p[0];
   return check_err(ctx, M);
 }

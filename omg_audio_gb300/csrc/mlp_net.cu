@@ -59,8 +59,8 @@ __device__ __forceinline__ float gelu_grad(float z, float t) {
 }
 
 __device__ __forceinline__ uint32_t pack2(float a, float b) {
-  return (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(a)) |
-         ((uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(b)) << 16);
+  const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);   // one conversion, a in the low half
+  return *reinterpret_cast<const uint32_t*>(&h);
 }
 
 // 16 consecutive features of one row into the tile image (two 16-byte stores;
@@ -90,6 +90,27 @@ __device__ __forceinline__ float column_sum16(float (&v)[16], uint32_t lane) {
 }
 __device__ __forceinline__ uint32_t column_of(uint32_t lane) {
   return ((lane >> 4) & 1u) * 8u + ((lane >> 3) & 1u) * 4u + ((lane >> 2) & 1u) * 2u + ((lane >> 1) & 1u);
+}
+
+// The accumulator's columns [lo, hi) in chunks of 16 through f(column, values):
+// the next chunk is on its way out of TMEM while this one is worked on.
+template <class F>
+__device__ __forceinline__ void for_columns(uint32_t lanes, uint32_t lo, uint32_t hi, F&& f) {
+  if (lo >= hi) return;
+  float a[16], b[16];
+  tc::tmem_ld16_async(lanes + lo, a);
+  for (uint32_t c = lo;;) {
+    tc::tmem_wait(a);
+    if (c + 16u < hi) tc::tmem_ld16_async(lanes + c + 16u, b);
+    f(c, a);
+    c += 16u;
+    if (c >= hi) break;
+    tc::tmem_wait(b);
+    if (c + 16u < hi) tc::tmem_ld16_async(lanes + c + 16u, a);
+    f(c, b);
+    c += 16u;
+    if (c >= hi) break;
+  }
 }
 
 template <bool TRAIN>
@@ -223,9 +244,7 @@ __global__ void __launch_bounds__(kRowThreads, 1) rows_kernel(const __grid_const
     }
     if (l + 1 < L) {
       if (live) {
-        for (uint32_t c = col_lo(D.op); c < col_hi(D.op); c += 16u) {
-          float v[16];
-          tc::tmem_ld16(my_lanes + c, v);
+        for_columns(my_lanes, col_lo(D.op), col_hi(D.op), [&](uint32_t c, float (&v)[16]) {
           float gp[16];
 #pragma unroll
           for (int j = 0; j < 16; j++) {
@@ -242,14 +261,12 @@ __global__ void __launch_bounds__(kRowThreads, 1) rows_kernel(const __grid_const
             for (int q = 0; q < 4; q++)
               gd[q * kRows] = make_float4(gp[4 * q], gp[4 * q + 1], gp[4 * q + 2], gp[4 * q + 3]);
           }
-        }
+        });
       }
     } else if (!TRAIN) {
       float* o = g.out + ((uint64_t)blockIdx.y * g.rows + grow) * D.out;
       if (live) {
-        for (uint32_t c = col_lo(D.op); c < col_hi(D.op); c += 16u) {
-          float v[16];
-          tc::tmem_ld16(my_lanes + c, v);
+        for_columns(my_lanes, col_lo(D.op), col_hi(D.op), [&](uint32_t c, float (&v)[16]) {
           if (grow < g.rows) {
 #pragma unroll
             for (int j = 0; j < 16; j++) v[j] += s_bias[c + j];
@@ -263,28 +280,45 @@ __global__ void __launch_bounds__(kRowThreads, 1) rows_kernel(const __grid_const
                 if (c + j < D.out) o[c + j] = v[j];
             }
           }
-        }
+        });
       }
     } else {
       // the mean squared error and its gradient
       const float inv_n = 1.0f / ((float)g.rows * (float)D.out);
-      const float* y = g.Y + src_row * D.out;
+      const uint32_t lo = col_lo(D.op), hi = col_hi(D.op);
       float lsum = 0.0f;
-      for (uint32_t c = col_lo(D.op); c < col_hi(D.op); c += 16u) {
-        float v[16];
-        tc::tmem_ld16(my_lanes + c, v);
+      float y[16];
+      const float* yr = g.Y + src_row * D.out;
+      auto load_y = [&](uint32_t c) {
+        if (D.out % 4u == 0u) {
+          const float4* y4 = reinterpret_cast<const float4*>(yr + c);
+#pragma unroll
+          for (uint32_t q = 0; q < 4; q++) {
+            const float4 w = c + 4u * q < D.out ? __ldg(y4 + q) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            y[4 * q] = w.x;
+            y[4 * q + 1] = w.y;
+            y[4 * q + 2] = w.z;
+            y[4 * q + 3] = w.w;
+          }
+        } else {
+#pragma unroll
+          for (uint32_t j = 0; j < 16; j++) y[j] = c + j < D.out ? __ldg(yr + c + j) : 0.0f;
+        }
+      };
+      if (lo < hi) load_y(lo);
+      for_columns(my_lanes, lo, hi, [&](uint32_t c, float (&v)[16]) {
 #pragma unroll
         for (int j = 0; j < 16; j++) {
-          const bool in = c + j < D.out;
-          const float e = in ? v[j] + s_bias[c + j] - y[c + j] : 0.0f;
+          const float e = c + j < D.out ? v[j] + s_bias[c + j] - y[j] : 0.0f;
           lsum += e * e;
           v[j] = 2.0f * e * inv_n;
         }
+        if (c + 16u < hi) load_y(c + 16u);
         put16(tile, row, c, v);
         const float s = column_sum16(v, lane);
         const uint32_t col = c + column_of(lane);
         if ((lane & 1u) == 0u && col < D.out) atomicAdd(g.G + (uint64_t)member * N.p_stride + D.b_off + col, s);
-      }
+      });
       for (int o = 16; o > 0; o >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
       if (lane == 0) atomicAdd(g.loss + member, lsum * inv_n);
     }
@@ -305,6 +339,16 @@ __global__ void __launch_bounds__(kRowThreads, 1) rows_kernel(const __grid_const
         }
       }
       if (l == 0) break;
+      const MlpLayerDesc& Dl = N.L[l - 1];     // dZ of the layer below = dX * GELU'(Z)
+      const uint32_t lo = col_lo(D.ip), hi = col_hi(D.ip);
+      const float4* gd = reinterpret_cast<const float4*>(g.gz) + (mt * (L - 1u) + (l - 1u)) * (D.ip / 4u) * kRows + row;
+      // GELU'(z) of the next columns is loaded ahead: the first ones while the product runs
+      float4 gp[4];
+      auto load_g = [&](uint32_t c) {
+#pragma unroll
+        for (uint32_t q = 0; q < 4; q++) gp[q] = gd[(c / 4u + q) * kRows];
+      };
+      if (lo < hi) load_g(lo);
       if (ok) wait_mma();
       if (tid == 0) {
         if (l > 1) load_w(l - 1, 0);
@@ -312,15 +356,7 @@ __global__ void __launch_bounds__(kRowThreads, 1) rows_kernel(const __grid_const
       }
       if (__syncthreads_or(!ok)) goto bail;
       tc::fence_after_sync();
-      const MlpLayerDesc& Dl = N.L[l - 1];     // dZ of the layer below = dX * GELU'(Z)
-      for (uint32_t c = col_lo(D.ip); c < col_hi(D.ip); c += 16u) {
-        float v[16];
-        const float4* gd =
-            reinterpret_cast<const float4*>(g.gz) + ((mt * (L - 1u) + (l - 1u)) * (D.ip / 4u) + c / 4u) * kRows + row;
-        float4 gp[4];
-#pragma unroll
-        for (int q = 0; q < 4; q++) gp[q] = gd[q * kRows];
-        tc::tmem_ld16(my_lanes + c, v);
+      for_columns(my_lanes, lo, hi, [&](uint32_t c, float (&v)[16]) {
 #pragma unroll
         for (int q = 0; q < 4; q++) {
           v[4 * q] *= gp[q].x;
@@ -328,10 +364,11 @@ __global__ void __launch_bounds__(kRowThreads, 1) rows_kernel(const __grid_const
           v[4 * q + 2] *= gp[q].z;
           v[4 * q + 3] *= gp[q].w;
         }
+        if (c + 16u < hi) load_g(c + 16u);
         put16(tile, row, c, v);
         const float s = column_sum16(v, lane);
         if ((lane & 1u) == 0u) atomicAdd(g.G + (uint64_t)member * N.p_stride + Dl.b_off + c + column_of(lane), s);
-      }
+      });
     }
     if (tid == 0) tc::bulk_store_wait();
   }

@@ -178,7 +178,8 @@ int32_t fill_batch(omg_ctx* ctx, BatchRec& B, const omg_job* jobs, uint32_t n_jo
   B.max_bins = 0;
   B.n_bin_floats = 0;
   B.n_dir_floats = 0;
-  bool coop_ok = P.tie_mode != 0, deep = false;
+  bool coop_ok = P.tie_mode != 0, deep = false, box_only = true;
+  float last_time = 0.0f;
   // per-job panel materials are placed after all box wall materials
   for (uint32_t i = 0; i < n_jobs; i++) {
     const omg_job& j = jobs[i];
@@ -206,10 +207,16 @@ int32_t fill_batch(omg_ctx* ctx, BatchRec& B, const omg_job* jobs, uint32_t n_jo
     d.max_bounces = P.max_bounces;
     d.dir_band = P.dir_band;
     d.bin_dt = P.bin_dt;
-    d.max_time = max_time;
-    d.rr = P.receiver_radius;
     d.wall_eps = P.wall_eps;
     d.c = P.speed_of_sound;
+    // (a bisection: once for neighbouring jobs of the same length)
+    if (i > 0 && max_time == last_time) {
+      d.rr2 = B.jobs[i - 1].rr2;
+      d.dist_max = B.jobs[i - 1].dist_max;
+    } else {
+      set_thresholds(d, P.receiver_radius, max_time);
+    }
+    last_time = max_time;
     if (j.geom == OMG_GEOM_BOX) {
       if (!finite3(j.box_size)) return OMG_E_INVALID;
       for (int k = 0; k < 3; k++) d.box[k] = j.box_size[k];
@@ -223,6 +230,7 @@ int32_t fill_batch(omg_ctx* ctx, BatchRec& B, const omg_job* jobs, uint32_t n_jo
       if (it == ctx->scenes.end()) return OMG_E_NOT_FOUND;
       if (it->second->n_bands != nb) return OMG_E_INVALID;
       d.scene = j.scene_id;
+      box_only = false;
       if (it->second->n_nodes4 == 0) coop_ok = false;
       if (it->second->n_prims > kSpreadPrims) deep = true;
     } else {
@@ -267,6 +275,7 @@ int32_t fill_batch(omg_ctx* ctx, BatchRec& B, const omg_job* jobs, uint32_t n_jo
   B.total_rays = (uint32_t)rays;
   B.coop_ok = coop_ok;
   B.deep = deep;
+  B.box_only = box_only;
   B.n_acc = acc;
   B.n_out = out;
   return OMG_OK;
@@ -359,6 +368,7 @@ int32_t record_launch(omg_ctx* ctx, BatchRec& B, cudaStream_t s, int parts = 3) 
     LaunchShape eff = B.shape;
     eff.loop_guard = ctx->prm.loop_guard;
     if (B.deep) eff.spread_warps = 32;
+    eff.box_only = B.box_only;
     if (eff.mode == 2 && !B.coop_ok) eff.mode = 0;
     if (eff.tail_mode == 2 && !B.coop_ok) eff.tail_mode = 0;
     CK(launch_wavefront(B.d_jobs.p, B.n_jobs, B.total_rays, B.max_nb, ctx->d_scenes.p, B.d_job_mats.p,

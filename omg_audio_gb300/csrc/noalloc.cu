@@ -164,10 +164,9 @@ extern "C" int32_t omg_trace_box_noalloc(const omg_box_job* job, const omg_param
   d.max_bounces = prm->max_bounces;
   d.dir_band = prm->dir_band;
   d.bin_dt = prm->bin_dt;
-  d.max_time = prm->max_time;
-  d.rr = prm->receiver_radius;
   d.wall_eps = prm->wall_eps;
   d.c = prm->speed_of_sound;
+  set_thresholds(d, prm->receiver_radius, prm->max_time);
   d.box_mat = 0;
   d.ray_base = 0;
   d.acc_off = 0;
@@ -180,6 +179,7 @@ extern "C" int32_t omg_trace_box_noalloc(const omg_box_job* job, const omg_param
   noalloc_setup_kernel<<<64, 256, 0, s>>>(scratch, d, walls, acc);
   LaunchShape shape;
   shape.loop_guard = prm->loop_guard;
+  shape.box_only = true;
   cudaError_t e = launch_trace(reinterpret_cast<const DJob*>(scratch + kJobOff), 1, job->n_rays, nb, nullptr,
                                reinterpret_cast<const DMat*>(scratch + kMatOff), nullptr, nullptr, scratch,
                                reinterpret_cast<DLaunch*>(scratch + kHdrOff),

@@ -16,7 +16,10 @@
 //   mats    : 80 B per material, with the branch weights precomputed (bit-identical
 //             to computing them per bounce: same f32 operations, same order)
 #pragma once
+#include <cmath>
 #include <cstdint>
+#include <cstring>
+#include <limits>
 #include <vector>
 #include <cuda_runtime.h>
 
@@ -124,8 +127,8 @@ struct alignas(16) DJob {
   uint32_t max_bounces;
   uint32_t dir_band;
   float bin_dt;
-  float max_time;
-  float rr;               // receiver radius
+  float rr2;              // the least f32 whose square root is not below the receiver radius: sqrt(s) < rr iff s < rr2
+  float dist_max;         // the largest f32 with dist / c not above max_time: dist / c > max_time iff dist > dist_max
   float wall_eps;
   float c;                // speed of sound
   uint32_t panel_off;
@@ -136,6 +139,37 @@ struct alignas(16) DJob {
   uint64_t acc_off;       // float offset of this job's accumulators
   uint64_t out_off;       // float offset of this job's output (bins then dirs)
 };
+
+// DJob's two thresholds. The correctly rounded square root and quotient do not
+// fall as their argument grows, so a comparison of their result is one of the
+// argument with the f32 at which it changes, found by bisection over the bit
+// patterns of 0 .. infinity.
+template <class Pred>
+inline float least_f32(Pred&& holds) {   // the least f32 in [0, inf] with holds(x) (false below, true from there on)
+  uint32_t lo = 0, hi = 0x7F800000u;     // holds(hi), or nothing up to infinity does
+  auto at = [](uint32_t b) {
+    float f;
+    std::memcpy(&f, &b, 4);
+    return f;
+  };
+  while (lo < hi) {
+    const uint32_t mid = lo + (hi - lo) / 2;
+    if (holds(at(mid))) hi = mid;
+    else lo = mid + 1;
+  }
+  return at(lo);
+}
+inline void set_thresholds(DJob& d, float radius, float max_time) {   // (d.c is set)
+  d.rr2 = radius > 0.0f ? least_f32([&](float s) { return !(std::sqrt(s) < radius); }) : 0.0f;
+  const float c = d.c;
+  if (!(std::numeric_limits<float>::infinity() / c > max_time)) {
+    d.dist_max = std::numeric_limits<float>::infinity();   // no distance passes
+  } else {
+    const float first = least_f32([&](float x) { return x / c > max_time; });
+    // the f32 below it; nothing is below 0 (every distance passes)
+    d.dist_max = first > 0.0f ? std::nextafter(first, 0.0f) : -1.0f;
+  }
+}
 
 // Per-launch header in device memory (scratch: cleared before every launch).
 struct alignas(16) DLaunch {
@@ -177,6 +211,7 @@ struct LaunchShape {
   uint32_t wl_shade_min = 32;   // modes 1 and 2: rays a warp shades together once that many wait
   uint32_t spread_warps = 16;   // resident warps per multiprocessor that a launch of few rays is spread over (the
                                 // batch sets 32 when a scene's tree is beyond an L1: kSpreadPrims)
+  bool box_only = false;        // every job of the launch is a shoebox (set by the batch)
   uint32_t loop_guard = 0;      // loop iterations of one warp of a persistent kernel before it stops
                                 // and flags error 8 (0: kDefaultLoopGuard); from omg_params.loop_guard
 };
@@ -240,9 +275,8 @@ cudaError_t launch_trace(const DJob* jobs, uint32_t n_jobs, uint32_t total_rays,
                          const DPanelGroup* groups, float* acc,
                          DLaunch* hdr, uint32_t* job_segments, const LaunchShape& shape, int n_sms, bool tie,
                          cudaStream_t s, const EpochArgs* ep = nullptr, bool wt = false);
-// trace.cu: load the per-lane trace kernel variants launch_trace may pick for a
-// single launch (3 and 8 bands, with and without the near-tie rule) now, so
-// that a later launch does not wait for the driver's lazy module loading.
+// trace.cu: load the shoebox trace kernels (3 and 8 bands) now, so that a later
+// launch does not wait for the driver's lazy module loading.
 cudaError_t preload_trace_kernels();
 // coop.cu: the mode-2 persistent kernel (same arguments as launch_trace).
 cudaError_t launch_trace_coop(const DJob* jobs, uint32_t n_jobs, uint32_t total_rays, uint32_t max_nb,

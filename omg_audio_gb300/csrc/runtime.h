@@ -134,6 +134,7 @@ struct BatchRec {
   WfState wf{};
   bool coop_ok = false;           // near-tie rule and every mesh scene has a 4-wide tree (mode 2)
   bool deep = false;              // a scene beyond kSpreadPrims primitives
+  bool box_only = false;          // every job is a shoebox
   DevBuf<uint32_t> d_ep_q;        // epoch queues (2 x rays)
   LaunchShape shape;
   // recorded when first needed (batch_graph)

@@ -28,23 +28,22 @@ struct Hit {
   const DMat* m;
 };
 
-// scene.rs:39-88 — analytic shoebox. (Out of line: only shoebox jobs take it,
-// and the persistent kernels' loop stays small for the instruction cache.)
-static __device__ __noinline__ bool box_hit(const DJob& J, const DMat* __restrict__ job_mats, float px, float py,
-                                        float pz, float dx, float dy, float dz, Hit& h) {
+// scene.rs:39-88 — analytic shoebox.
+static __device__ __forceinline__ bool box_hit_body(const DJob& J, const DMat* __restrict__ job_mats, float px,
+                                                    float py, float pz, float dx, float dy, float dz, Hit& h) {
   if (!(px > 0.0f && px < J.box[0] && py > 0.0f && py < J.box[1] && pz > 0.0f && pz < J.box[2])) return false;
   float bt = FLT_MAX;
   int bw = 0;
   const float p[3] = {px, py, pz}, d[3] = {dx, dy, dz};
 #pragma unroll
   for (int axis = 0; axis < 3; axis++) {
-    float di = d[axis];
-    if (di > 1e-9f) {
-      float t = (J.box[axis] - p[axis]) / di;
-      if (t < bt) { bt = t; bw = 2 * axis + 1; }
-    } else if (di < -1e-9f) {
-      float t = -p[axis] / di;
-      if (t < bt) { bt = t; bw = 2 * axis; }
+    // the wall ahead: (size - p) / d or -p / d, one division for both signs
+    const float di = d[axis];
+    const bool up = di > 1e-9f;
+    const float num = up ? J.box[axis] - p[axis] : -p[axis];
+    if (up || di < -1e-9f) {
+      const float t = num / di;
+      if (t < bt) { bt = t; bw = 2 * axis + (up ? 1 : 0); }
     }
   }
   if (!isfinite(bt) || bt <= 0.0f) return false;
@@ -56,64 +55,99 @@ static __device__ __noinline__ bool box_hit(const DJob& J, const DMat* __restric
   h.m = job_mats + J.box_mat + bw;
   return true;
 }
+// Out of line for kernels whose jobs are mostly meshes: their loop stays small
+// for the instruction cache.
+static __device__ __noinline__ bool box_hit(const DJob& J, const DMat* __restrict__ job_mats, float px, float py,
+                                            float pz, float dx, float dy, float dz, Hit& h) {
+  return box_hit_body(J, job_mats, px, py, pz, dx, dy, dz, h);
+}
 
 // scene.rs:94-137 — panel slab ENTRY test, nearest of base and panels.
-// Panels are tested group by group: a group (and then a panel) is skipped when
-// its box cannot meet the segment's bounding box grown by 1 cm. An entry point
-// at t0 in (1e-4, best t) lies on the panel's box and on the segment, so both
-// boxes contain it (to within rounding, far below 1 cm at room coordinates).
-// Without a base hit the segment is unbounded and every panel is tested. The
-// reference scans panels in order with a strict `<`, so among equal entry
-// distances the first panel wins: here, the lowest original index.
+//
+// A group of up to 4 panels is skipped when its union box cannot meet the
+// segment's bounding box grown by 1 cm: an entry point at t0 in (1e-4, best t)
+// lies on the panel's box and on the segment, so both boxes contain it (to
+// within rounding, far below 1 cm at room coordinates). Without a base hit the
+// segment is unbounded and every group is tested. A group's panels then go
+// through a slab test with products by 1/d in place of the reference's six
+// divisions; its interval is widened by 4e-6, more than the products differ
+// from the quotients (2 ulp), so it passes every panel that the exact test
+// passes, and few others. Only those take the exact test, all lanes of the
+// warp together whichever of the group's panels theirs is (lanes meet
+// different panels, and the divisions of one panel after another were 45 % of
+// a trace of shoebox rooms with four apertures each). Going through the groups
+// the same way (a bit a group, then each lane its own next one) costs the mesh
+// kernels 200 bytes of spills more: 31.0 against 28.4 ms for 96 uneven rooms.
+//
+// The reference scans panels in order with a strict `<`, so among equal entry
+// distances the first panel wins: here, the lowest original index. The result
+// does not depend on the order of the tests.
 __device__ __forceinline__ bool panels_hit(const DJob& J, const DPanel* __restrict__ panels,
                                            const DPanelGroup* __restrict__ groups,
                                            const DMat* __restrict__ job_mats, float px, float py, float pz, float dx,
                                            float dy, float dz, bool have, Hit& h) {
   const float p[3] = {px, py, pz}, d[3] = {dx, dy, dz};
-  float slo[3], shi[3];
+  float slo[3], shi[3], inv[3];
   const bool bounded = have;
   uint32_t best_orig = 0xFFFFFFFFu;  // the current best is the base hit
-  if (bounded) {
 #pragma unroll
-    for (int a = 0; a < 3; a++) {
-      const float q = p[a] + d[a] * h.t;
-      slo[a] = fminf(p[a], q) - 0.01f;
-      shi[a] = fmaxf(p[a], q) + 0.01f;
-    }
+  for (int a = 0; a < 3; a++) {
+    const float q = p[a] + d[a] * h.t;
+    slo[a] = fminf(p[a], q) - 0.01f;
+    shi[a] = fmaxf(p[a], q) + 0.01f;
+    inv[a] = __frcp_rn(d[a]);
   }
   for (uint32_t g = 0; g < J.n_groups; g++) {
     const DPanelGroup& G = groups[J.group_off + g];
     if (bounded && (G.mx[0] < slo[0] || G.mn[0] > shi[0] || G.mx[1] < slo[1] || G.mn[1] > shi[1] ||
                     G.mx[2] < slo[2] || G.mn[2] > shi[2]))
       continue;
-    for (uint32_t i = G.first; i < G.first + G.count; i++) {
-      const DPanel& pn = panels[i];
-      if (bounded && (pn.mx[0] < slo[0] || pn.mn[0] > shi[0] || pn.mx[1] < slo[1] || pn.mn[1] > shi[1] ||
-                      pn.mx[2] < slo[2] || pn.mn[2] > shi[2]))
-        continue;
+    const uint32_t first = G.first, count = G.count;
+    uint32_t cand = 0;
+    const float reach = have ? h.t * (1.0f + 1e-5f) : FLT_MAX;
+    for (uint32_t k = 0; k < count; k++) {
+      const float4 lo4 = __ldg(reinterpret_cast<const float4*>(panels + first + k));
+      const float4 hi4 = __ldg(reinterpret_cast<const float4*>(panels + first + k) + 1);
+      const float lo[3] = {lo4.x, lo4.y, lo4.z}, hi[3] = {hi4.x, hi4.y, hi4.z};
+      float n0 = 0.0f, f0 = FLT_MAX;
+#pragma unroll
+      for (int a = 0; a < 3; a++) {
+        // |d| < 1e-9 (the exact test's own case) bounds nothing here
+        const bool flat = fabsf(d[a]) < 1e-9f;
+        const float ta = (lo[a] - p[a]) * inv[a], tb = (hi[a] - p[a]) * inv[a];
+        n0 = fmaxf(n0, flat ? 0.0f : fminf(ta, tb));
+        f0 = fminf(f0, flat ? FLT_MAX : fmaxf(ta, tb));
+      }
+      // n0 >= 0; a negative f0 is a panel behind the ray
+      if (n0 <= f0 * (1.0f + 4e-6f) && n0 > 0.9999e-4f && n0 <= reach) cand |= 1u << k;
+    }
+    while (cand) {
+      const uint32_t k = (uint32_t)__ffs((int)cand) - 1u;
+      cand &= cand - 1u;
+      const DPanel& pn = panels[first + k];
       float t0 = 0.0f, t1 = FLT_MAX;
       int axis = 3;
       bool miss = false;
 #pragma unroll
       for (int a = 0; a < 3; a++) {
-        if (miss) break;
-        float da = d[a], pa = p[a], lo = pn.mn[a], hi = pn.mx[a];
+        const float da = d[a], pa = p[a], lo = pn.mn[a], hi = pn.mx[a];
         if (fabsf(da) < 1e-9f) {
-          if (pa < lo || pa > hi) { t0 = FLT_MAX; miss = true; }
+          if (pa < lo || pa > hi) miss = true;
         } else {
           float ta = (lo - pa) / da, tb = (hi - pa) / da;
           if (ta > tb) { float tmp = ta; ta = tb; tb = tmp; }
           if (ta > t0) { t0 = ta; axis = a; }
           t1 = fminf(t1, tb);
-          if (t0 > t1) { t0 = FLT_MAX; miss = true; }
+          if (t0 > t1) miss = true;
         }
       }
       const bool closer = !have || t0 < h.t || (t0 == h.t && best_orig != 0xFFFFFFFFu && pn.orig < best_orig);
-      if (t0 > 1e-4f && t0 < FLT_MAX && axis < 3 && closer) {
+      if (!miss && t0 > 1e-4f && t0 < FLT_MAX && axis < 3 && closer) {
         h.t = t0;
-        h.nx = h.ny = h.nz = 0.0f;
-        float s = d[axis] > 0.0f ? -1.0f : 1.0f;
-        if (axis == 0) h.nx = s; else if (axis == 1) h.ny = s; else h.nz = s;
+        const float s = (axis == 0 ? dx : (axis == 1 ? dy : dz)) > 0.0f ? -1.0f : 1.0f;
+        h.nx = axis == 0 ? s : 0.0f;
+        h.ny = axis == 1 ? s : 0.0f;
+        h.nz = axis == 2 ? s : 0.0f;
         h.m = job_mats + pn.mat;
         have = true;
         best_orig = pn.orig;
@@ -184,7 +218,7 @@ __device__ __forceinline__ bool shade_segment(const DJob& J, float* __restrict__
     if (s > 0.0f && s < t_hit) {
       const float cx = px + dx * s, cy = py + dy * s, cz = pz + dz * s;
       const float ddx = cx - J.lis[0], ddy = cy - J.lis[1], ddz = cz - J.lis[2];
-      if (sqrtf(ddx * ddx + ddy * ddy + ddz * ddz) < J.rr) {
+      if (ddx * ddx + ddy * ddy + ddz * ddz < J.rr2) {     // sqrt(..) < rr (DJob::rr2)
         const float arrival = (dist + s) / J.c;
         const float q = arrival / J.bin_dt;
         if (q < (float)J.n_bins) {          // (q as usize) < NBINS, q >= 0
@@ -203,7 +237,7 @@ __device__ __forceinline__ bool shade_segment(const DJob& J, float* __restrict__
     py = py + dy * t_hit;
     pz = pz + dz * t_hit;
     dist = dist + t_hit;
-    if (dist / J.c > J.max_time) done = true;
+    if (dist > J.dist_max) done = true;                    // dist / c > max_time (DJob::dist_max)
   }
   if (!done) {
     const DMat& M = *h.m;

@@ -154,7 +154,10 @@ __device__ __noinline__ void epoch_tally(const EpochArgs& ea, bool ended, bool p
 // distance, stream, segment count, ray id) lives, for up to 4 bands, in shared
 // memory, a column per thread. The 3-band near-tie kernel then has 16 bytes of
 // spill stores, against 184 with that state in registers.
-template <int NB, bool TIE, bool WIDE, bool WT>
+//
+// BOX: every job of the launch is a shoebox: no walk, every segment is one
+// shading pass.
+template <int NB, bool TIE, bool WIDE, bool WT, bool BOX>
 __global__ void __launch_bounds__(256, 4) trace_kernel(const DJob* __restrict__ jobs, uint32_t n_jobs,
                                                        uint32_t total_rays, const DScene* __restrict__ scenes,
                                                        const DMat* __restrict__ job_mats,
@@ -233,7 +236,7 @@ __global__ void __launch_bounds__(256, 4) trace_kernel(const DJob* __restrict__ 
   // begin one segment from (p, d): a mesh walk, or (a shoebox) the shading
   // pass at once, which computes the box hit
   auto begin_segment = [&](const DJob& J) {
-    if (J.geom == OMG_GEOM_BOX) {
+    if (BOX || J.geom == OMG_GEOM_BOX) {
       phase = SHADE;
     } else {
       walk_begin<TIE>(w, scenes[J.scene], px, py, pz, dx, dy, dz, wide);
@@ -292,13 +295,14 @@ __global__ void __launch_bounds__(256, 4) trace_kernel(const DJob* __restrict__ 
     // ---- this iteration either shades or walks, for the whole warp: lanes
     // whose walk is done wait until at least shade_min of them are ready (or
     // no lane is walking), so that the shading code runs with full lanes
-    const unsigned walking = __ballot_sync(FULL, phase == WALK);
+    const unsigned walking = BOX ? 0u : __ballot_sync(FULL, phase == WALK);
     const unsigned ready = __ballot_sync(FULL, phase == SHADE);
     const bool shade_now = ready != 0u && (walking == 0u || __popc(ready) >= (int)shade_min);
 
     // ---- closest-hit walk, at most walk_budget steps this iteration; a lane
     // whose walk is over waits to shade, its result kept in w until then
-    if (TIE && !wide) {
+    if (BOX) {
+    } else if (TIE && !wide) {
       // near-tie walks on the binary tree: the node phase lane by lane, then
       // the pending leaves tested by the whole warp together
       if (!shade_now) {
@@ -337,7 +341,9 @@ __global__ void __launch_bounds__(256, 4) trace_kernel(const DJob* __restrict__ 
       h.t = FLT_MAX;
       h.m = nullptr;
       bool have;
-      if (J.geom == OMG_GEOM_BOX) {
+      if (BOX) {
+        have = box_hit_body(J, job_mats, px, py, pz, dx, dy, dz, h);
+      } else if (J.geom == OMG_GEOM_BOX) {
         have = box_hit(J, job_mats, px, py, pz, dx, dy, dz, h);
       } else {
         const DScene& S = scenes[J.scene];
@@ -647,29 +653,30 @@ cudaError_t launch_trace(const DJob* jobs, uint32_t n_jobs, uint32_t total_rays,
       if (blocks == 0) blocks = 1;
     }
   }
-#define OMG_TRACE_LAUNCH(NB, TIE)                                                                         \
-  if (wl)                                                                                                      \
-    trace_wl_kernel<NB, TIE><<<blocks, threads, 0, s>>>(jobs, n_jobs, total_rays, scenes, job_mats, panels,    \
-                                                        groups, acc, hdr, job_segments, steps, wl_shade, wide, ea);  \
-  else if (TIE && wide)                                                                                        \
-    trace_kernel<NB, TIE, true, false><<<blocks, threads, 0, s>>>(jobs, n_jobs, total_rays, scenes, job_mats,   \
-                                                                  panels, groups, acc, hdr, job_segments, refill, \
-                                                                  steps, shade_min, lane_cap, ea);                          \
-  else if (TIE && wt)                                                                                          \
-    trace_kernel<NB, TIE, false, true><<<blocks, threads, 0, s>>>(jobs, n_jobs, total_rays, scenes, job_mats,   \
-                                                                  panels, groups, acc, hdr, job_segments, refill, \
-                                                                  steps, shade_min, lane_cap, ea);                          \
-  else                                                                                                         \
-    trace_kernel<NB, TIE, false, false><<<blocks, threads, 0, s>>>(jobs, n_jobs, total_rays, scenes, job_mats,  \
-                                                                   panels, groups, acc, hdr, job_segments, refill,\
-                                                                   steps, shade_min, lane_cap, ea)
+#define OMG_TRACE_LAUNCH(NB, TIE, WIDE, WT, BOX)                                                              \
+  trace_kernel<NB, TIE, WIDE, WT, BOX><<<blocks, threads, 0, s>>>(jobs, n_jobs, total_rays, scenes, job_mats, \
+                                                                  panels, groups, acc, hdr, job_segments,     \
+                                                                  refill, steps, shade_min, lane_cap, ea)
+#define OMG_TRACE_PICK(NB)                                                                                    \
+  if (wl && tie)                                                                                              \
+    trace_wl_kernel<NB, true><<<blocks, threads, 0, s>>>(jobs, n_jobs, total_rays, scenes, job_mats, panels,  \
+                                                         groups, acc, hdr, job_segments, steps, wl_shade,     \
+                                                         wide, ea);                                           \
+  else if (wl)                                                                                                \
+    trace_wl_kernel<NB, false><<<blocks, threads, 0, s>>>(jobs, n_jobs, total_rays, scenes, job_mats, panels, \
+                                                          groups, acc, hdr, job_segments, steps, wl_shade,    \
+                                                          wide, ea);                                          \
+  else if (shape.box_only) OMG_TRACE_LAUNCH(NB, false, false, false, true);                                   \
+  else if (!tie) OMG_TRACE_LAUNCH(NB, false, false, false, false);                                            \
+  else if (wide) OMG_TRACE_LAUNCH(NB, true, true, false, false);                                              \
+  else if (wt) OMG_TRACE_LAUNCH(NB, true, false, true, false);                                                \
+  else OMG_TRACE_LAUNCH(NB, true, false, false, false)
   if (max_nb <= 3) {
-    if (tie) OMG_TRACE_LAUNCH(3, true);
-    else OMG_TRACE_LAUNCH(3, false);
+    OMG_TRACE_PICK(3);
   } else {
-    if (tie) OMG_TRACE_LAUNCH(8, true);
-    else OMG_TRACE_LAUNCH(8, false);
+    OMG_TRACE_PICK(8);
   }
+#undef OMG_TRACE_PICK
 #undef OMG_TRACE_LAUNCH
   return cudaGetLastError();
 }
@@ -677,10 +684,8 @@ cudaError_t launch_trace(const DJob* jobs, uint32_t n_jobs, uint32_t total_rays,
 cudaError_t preload_trace_kernels() {
   cudaFuncAttributes fa;
   cudaError_t e;
-  if ((e = cudaFuncGetAttributes(&fa, trace_kernel<3, false, false, false>)) != cudaSuccess) return e;
-  if ((e = cudaFuncGetAttributes(&fa, trace_kernel<3, true, false, false>)) != cudaSuccess) return e;
-  if ((e = cudaFuncGetAttributes(&fa, trace_kernel<8, false, false, false>)) != cudaSuccess) return e;
-  return cudaFuncGetAttributes(&fa, trace_kernel<8, true, false, false>);
+  if ((e = cudaFuncGetAttributes(&fa, trace_kernel<3, false, false, false, true>)) != cudaSuccess) return e;
+  return cudaFuncGetAttributes(&fa, trace_kernel<8, false, false, false, true>);
 }
 
 cudaError_t launch_finalize(const DJob* jobs, uint32_t n_jobs, const float* acc, float* out, uint64_t total_out,

@@ -107,6 +107,21 @@ __device__ __forceinline__ bool ray_aabb(float lx, float ly, float lz, float hx,
   return t0 <= t1;
 }
 
+// ray_aabb by minima and maxima, for rays whose products cannot be a NaN (no
+// direction component near 0, finite origin): there `ta > tb ? tb : ta` is the
+// minimum, so the result is ray_aabb's.
+__device__ __forceinline__ bool ray_aabb_minmax(float lx, float ly, float lz, float hx, float hy, float hz, float ox,
+                                                float oy, float oz, float ix, float iy, float iz, float tmax,
+                                                float& tout) {
+  const float ax = (lx - ox) * ix, bx = (hx - ox) * ix;
+  const float ay = (ly - oy) * iy, by = (hy - oy) * iy;
+  const float az = (lz - oz) * iz, bz = (hz - oz) * iz;
+  const float t0 = fmaxf(fmaxf(fminf(ax, bx), fminf(ay, by)), fmaxf(fminf(az, bz), 0.0f));
+  const float t1 = fminf(fminf(fmaxf(ax, bx), fmaxf(ay, by)), fminf(fmaxf(az, bz), tmax));
+  tout = t0;
+  return t0 <= t1;
+}
+
 // Slab test with t = fma(l, inv, -o inv) (oi = o inv) and min/max
 // instructions, on boxes grown by DScene::nodes_f's margin. For an origin
 // with |o_a| <= 7 M_a it accepts every box ray_aabb accepts on the ungrown

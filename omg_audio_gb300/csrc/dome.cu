@@ -123,7 +123,7 @@ __device__ bool trace_escape(const DScene& S, const DDomeLaunch& L, float px, fl
 
 // The specular escape of every (listener, fan ray) under the near-tie rule,
 // one lane each, with the persistent tracer's walk: the node phase lane by
-// lane (walk_spec_nodes, the grown binary boxes), then the pending leaves
+// lane (walk_nodes, the grown binary boxes), then the pending leaves
 // tested by the whole warp (coop_leaf_rounds). The closest hit under this
 // rule does not depend on the walk, so each event sees the hit
 // any other near-tie walk finds; the events follow in trace_escape's f32 operations. Lanes
@@ -171,10 +171,10 @@ __global__ void __launch_bounds__(kEscThreads) dome_escape_walk_kernel(DDomeLaun
     bool over = false;
     if (active) {
       int st = 1 << 30;   // the node phase runs until the warp's lanes hold leaves (bounded by the walk budget)
-      over = walk_spec_nodes(w, S, r.px, r.py, r.pz, r.dx, r.dy, r.dz, st, err);
+      over = walk_nodes<true>(w, S, r.px, r.py, r.pz, st, err);
     }
-    coop_leaf_rounds<WT>(w, active && !over, WT ? S.prims_wt : S.prims, WT, r.px, r.py, r.pz, r.dx, r.dy, r.dz,
-                         s_slots[threadIdx.x >> 5], kCoopRounds, err);
+    coop_leaf_rounds<true, WT>(w, active && !over, WT ? S.prims_wt : S.prims, r.px, r.py, r.pz, r.dx, r.dy, r.dz,
+                               s_slots[threadIdx.x >> 5], kCoopRounds, err);
     if (active) {
       if (!over && w.cur == kDone && w.leaf == 0) over = !walk_restart_fixed(w, S.root, S.walk_budget);
       if (over) {

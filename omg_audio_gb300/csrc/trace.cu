@@ -24,63 +24,14 @@ namespace omg {
 
 namespace {
 
-// Up to `steps` node visits / leaf tests; returns true when the walk is done.
+// Up to `steps` node visits and leaf tests of a lane on its own; returns true
+// when the walk is done.
 template <bool TIE>
 __device__ __forceinline__ bool walk_steps(Walk& w, const DScene& S, float ox, float oy, float oz, float dx,
                                            float dy, float dz, int steps, bool wide, uint32_t* err) {
   if (TIE && wide && S.nodes4) return walk4_steps(w, S, ox, oy, oz, dx, dy, dz, steps, err);
-  const float4* __restrict__ nodes = S.nodes;
-  const float4* __restrict__ prims = S.prims;   // the first-found rule: the reference's test (no watertight context)
-  if (!TIE) {
-    // the reference's order: each node or leaf as it is reached
-    while (steps-- > 0 && w.cur != kDone) {
-      if (w.budget-- == 0u) {
-        atomicOr(err, 4u);
-        w.cur = kDone;
-        break;
-      }
-      if (w.cur >= 0) {
-        const float4 n0 = __ldg(nodes + 4 * w.cur + 0);
-        const float4 n1 = __ldg(nodes + 4 * w.cur + 1);
-        const float4 n2 = __ldg(nodes + 4 * w.cur + 2);
-        const float4 n3 = __ldg(nodes + 4 * w.cur + 3);
-        const float tmax = walk_cull<false>(w);
-        float ta, tb;
-        const bool h0 = ray_aabb(n0.x, n0.y, n0.z, n0.w, n1.x, n1.y, ox, oy, oz, w.ix, w.iy, w.iz, tmax, ta);
-        const bool h1 = ray_aabb(n1.z, n1.w, n2.x, n2.y, n2.z, n2.w, ox, oy, oz, w.ix, w.iy, w.iz, tmax, tb);
-        const int c0 = __float_as_int(n3.x), c1 = __float_as_int(n3.y);
-        if (h0 && h1) {
-          int nr, fr;
-          float nt, ft;
-          if (ta <= tb) { nr = c0; nt = ta; fr = c1; ft = tb; }
-          else { nr = c1; nt = tb; fr = c0; ft = ta; }
-          if (w.sp < STACK_DEPTH) {
-            w.stack_ref[w.sp] = fr;
-            w.stack_t[w.sp] = ft;
-            w.sp++;
-          } else {
-            atomicOr(err, 1u);
-          }
-          w.cur = (walk_have(w) && nt >= w.t_best) ? walk_pop<TIE>(w) : nr;
-        } else if (h0) {
-          w.cur = (walk_have(w) && ta >= w.t_best) ? walk_pop<TIE>(w) : c0;
-        } else if (h1) {
-          w.cur = (walk_have(w) && tb >= w.t_best) ? walk_pop<TIE>(w) : c1;
-        } else {
-          w.cur = walk_pop<TIE>(w);
-        }
-      } else {
-        bool have = walk_have(w);
-        float t_cull = walk_cull<false>(w);
-        uint32_t sb = 0, tb = 0;
-        TieState ts = tie_begin();
-        leaf_test<false>(prims, w.cur, ox, oy, oz, dx, dy, dz, have, w.t_best, t_cull, w.prim_best, sb, tb, ts);
-        w.cur = walk_pop<TIE>(w);
-      }
-    }
-    return w.cur == kDone;
-  }
-  return walk_spec(w, S, ox, oy, oz, dx, dy, dz, steps, err);
+  if (TIE) return walk_spec(w, S, ox, oy, oz, dx, dy, dz, steps, err);
+  return walk_first(w, S, ox, oy, oz, dx, dy, dz, steps, err);
 }
 
 // A ray parked between two segments: its state into the per-ray records, for
@@ -122,14 +73,14 @@ __device__ __noinline__ void epoch_tally(const EpochArgs& ea, bool ended, bool p
   }
 }
 
-// The tracer. Each lane runs a small state machine so that a lane whose
-// closest-hit walk ends shades its segment and starts the next one at once,
-// while the other lanes of its warp keep walking: per loop iteration a lane
-// takes at most `walk_steps` traversal steps, then shades if its walk is done.
-// Idle lanes refill from the global ray queue. Walking and shading alternate
-// per warp: lanes whose walk is done wait until `shade_min` of them can shade
-// together (or nothing else is walking), so the shading code, which is long,
-// does not run once per lane.
+// The tracer. A lane owns a ray; per loop iteration the warp refills its idle
+// lanes from the global ray queue, walks every lane's segment to its closest
+// hit, and shades them all together. Walks of a warp differ in length, but the
+// shading code is long, and running it for the lanes whose walk is over while
+// the others go on walking costs more than the wait (64 pairs on the 40-room
+// world: 15 % at groups of 16 lanes), except where walks differ most; and with
+// the walk over, none of its state is carried through the shading (64 pairs
+// 7.98 -> 8.07 ms, 96 uneven rooms 27.9 -> 27.3 ms, the city 21.6 -> 20.8 ms).
 //
 // In an epoch chain (ea.cur set) the queue is this epoch's: fresh rays, or
 // parked rays whose state is restored from the per-ray records. Once at most
@@ -164,8 +115,8 @@ __global__ void __launch_bounds__(256, 4) trace_kernel(const DJob* __restrict__ 
                                                        const DPanel* __restrict__ panels,
                                                        const DPanelGroup* __restrict__ groups, float* __restrict__ acc,
                                                     DLaunch* __restrict__ hdr, uint32_t* __restrict__ job_segments,
-                                                    uint32_t refill_min, int walk_budget, uint32_t shade_min,
-                                                    uint32_t lane_cap, EpochArgs ea) {
+                                                    uint32_t refill_min, int walk_budget, uint32_t lane_cap,
+                                                    EpochArgs ea) {
   constexpr bool wide = TIE && WIDE;
   const unsigned FULL = 0xffffffffu;
   const uint32_t lane = threadIdx.x & 31u;
@@ -219,9 +170,6 @@ __global__ void __launch_bounds__(256, 4) trace_kernel(const DJob* __restrict__ 
   auto cold_rid = [&]() { return kColdShared ? s_rid[me] : r_rid; };
   int walk_stack_ref[STACK_DEPTH];
   float walk_stack_t[STACK_DEPTH];
-  Walk w;
-  w.stack_ref = walk_stack_ref;
-  w.stack_t = walk_stack_t;
   uint32_t* err = &hdr->error;
   const WfState& rs = ea.st;
   const uint32_t* rq = ea.in_q;
@@ -233,16 +181,9 @@ __global__ void __launch_bounds__(256, 4) trace_kernel(const DJob* __restrict__ 
   uint32_t iters = 0;   // loop guard (warp-uniform: every lane runs every iteration)
   __shared__ uint8_t s_slots[kMaxWarps][256];   // coop_leaf_rounds' slot lists, one per warp
 
-  // begin one segment from (p, d): a mesh walk, or (a shoebox) the shading
-  // pass at once, which computes the box hit
-  auto begin_segment = [&](const DJob& J) {
-    if (BOX || J.geom == OMG_GEOM_BOX) {
-      phase = SHADE;
-    } else {
-      walk_begin<TIE>(w, scenes[J.scene], px, py, pz, dx, dy, dz, wide);
-      phase = WALK;
-    }
-  };
+  // one segment from (p, d): a mesh walk, or (a shoebox) the shading pass
+  // alone, which computes the box hit
+  auto begin_segment = [&](const DJob& J) { phase = BOX || J.geom == OMG_GEOM_BOX ? SHADE : WALK; };
 
   while (true) {
     if (++iters > ea.max_loop) {
@@ -292,48 +233,57 @@ __global__ void __launch_bounds__(256, 4) trace_kernel(const DJob* __restrict__ 
     // the epoch's park signal (sticky; raised only once its queue is drained)
     if (may_park && !parking) parking = *((volatile const uint32_t*)&ea.cur->park) != 0u;
 
-    // ---- this iteration either shades or walks, for the whole warp: lanes
-    // whose walk is done wait until at least shade_min of them are ready (or
-    // no lane is walking), so that the shading code runs with full lanes
-    const unsigned walking = BOX ? 0u : __ballot_sync(FULL, phase == WALK);
-    const unsigned ready = __ballot_sync(FULL, phase == SHADE);
-    const bool shade_now = ready != 0u && (walking == 0u || __popc(ready) >= (int)shade_min);
-
-    // ---- closest-hit walk, at most walk_budget steps this iteration; a lane
-    // whose walk is over waits to shade, its result kept in w until then
-    if (BOX) {
-    } else if (TIE && !wide) {
-      // near-tie walks on the binary tree: the node phase lane by lane, then
-      // the pending leaves tested by the whole warp together
-      if (!shade_now) {
-        const bool wk = phase == WALK;
-        const float4* lp = nullptr;
-        bool over = false, lwt = false;
-        if (wk) {
-          const DScene& S = scenes[jobs[ji].scene];
-          lwt = WT && S.prims_wt != nullptr;
-          lp = lwt ? S.prims_wt : S.prims;
-          int st = walk_budget;
-          over = walk_spec_nodes(w, S, px, py, pz, dx, dy, dz, st, err);
+    // ---- the closest-hit walks of every lane's segment, to their end: the
+    // node phase lane by lane, then the pending leaves tested by the whole
+    // warp together
+    int hit_prim = -1;
+    float hit_t = FLT_MAX;
+    if (!BOX) {
+      Walk w;
+      w.stack_ref = walk_stack_ref;
+      w.stack_t = walk_stack_t;
+      w.cur = kDone;
+      w.leaf = 0;
+      bool walking = phase == WALK;
+      if (walking) walk_begin<TIE>(w, scenes[jobs[ji].scene], px, py, pz, dx, dy, dz, wide);
+      while (__any_sync(FULL, walking)) {
+        if (++iters > ea.max_loop) break;
+        bool over = false;
+        if (wide) {
+          if (walking)
+            over = walk_steps<TIE>(w, scenes[jobs[ji].scene], px, py, pz, dx, dy, dz, walk_budget, wide, err);
+        } else {
+          const float4* lp = nullptr;
+          if (walking) {
+            const DScene& S = scenes[jobs[ji].scene];
+            lp = WT ? S.prims_wt : S.prims;
+            int st = walk_budget;
+            over = walk_nodes<TIE>(w, S, px, py, pz, st, err);
+          }
+          coop_leaf_rounds<TIE, WT>(w, walking && !over, lp, px, py, pz, dx, dy, dz, s_slots[threadIdx.x >> 5],
+                                    kCoopRounds, err);
+          if (walking && !over && w.cur == kDone && w.leaf == 0) {
+            over = true;
+            if (TIE) {
+              // an ambiguous near-tie window: the walk starts over in fixed mode
+              const DScene& S = scenes[jobs[ji].scene];
+              over = !walk_restart_fixed(w, S.root, S.walk_budget);
+            }
+          }
         }
-        coop_leaf_rounds<WT>(w, wk && !over, lp, lwt, px, py, pz, dx, dy, dz, s_slots[threadIdx.x >> 5],
-                             kCoopRounds, err);
-        if (wk) {
-          const DScene& S = scenes[jobs[ji].scene];
-          // an ambiguous near-tie window: the walk starts over in fixed mode
-          if (!over && w.cur == kDone && w.leaf == 0) over = !walk_restart_fixed(w, S.root, S.walk_budget);
-          if (over) phase = SHADE;
-        }
+        if (over) walking = false;
       }
-    } else if (!shade_now && phase == WALK) {
-      const DJob& J = jobs[ji];
-      const DScene& S = scenes[J.scene];
-      if (walk_steps<TIE>(w, S, px, py, pz, dx, dy, dz, walk_budget, wide, err)) phase = SHADE;
+      if (iters > ea.max_loop) {
+        atomicOr(err, 8u);
+        break;
+      }
+      hit_prim = w.prim_best;
+      hit_t = w.t_best;
     }
 
     // ---- one segment of the bounce loop (tracer.rs:103-200)
     bool ended = false, parked = false;
-    if (shade_now && phase == SHADE) {
+    if (phase != IDLE) {
       const DJob& J = jobs[ji];
       // the segment's closest hit: the shoebox's, or the walk's (normal of
       // the original triangle, against d)
@@ -347,14 +297,14 @@ __global__ void __launch_bounds__(256, 4) trace_kernel(const DJob* __restrict__ 
         have = box_hit(J, job_mats, px, py, pz, dx, dy, dz, h);
       } else {
         const DScene& S = scenes[J.scene];
-        have = walk_have(w);
+        have = hit_prim >= 0;
         if (have) {
-          const float4 p0 = __ldg(S.prims + 3 * w.prim_best + 0);
-          const float4 p1 = __ldg(S.prims + 3 * w.prim_best + 1);
+          const float4 p0 = __ldg(S.prims + 3 * hit_prim + 0);
+          const float4 p1 = __ldg(S.prims + 3 * hit_prim + 1);
           const float4 nn = __ldg(S.normals + __float_as_uint(p1.w));
           float nx = nn.x, ny = nn.y, nz = nn.z;
           if (nx * dx + ny * dy + nz * dz > 0.0f) { nx = nx * -1.0f; ny = ny * -1.0f; nz = nz * -1.0f; }
-          h.t = w.t_best;
+          h.t = hit_t;
           h.nx = nx; h.ny = ny; h.nz = nz;
           h.m = S.mats + __float_as_uint(p0.w);
         }
@@ -625,7 +575,6 @@ cudaError_t launch_trace(const DJob* jobs, uint32_t n_jobs, uint32_t total_rays,
   if (blocks == 0) blocks = 1;
   uint32_t refill = shape.refill_min == 0 ? 1 : (shape.refill_min > 32 ? 32 : shape.refill_min);
   const int steps = shape.walk_steps == 0 ? 1000000 : (int)shape.walk_steps;
-  const uint32_t shade_min = shape.shade_min == 0 ? 1u : (shape.shade_min > 32 ? 32u : shape.shade_min);
   // the warp-local wavefront needs the per-ray records and at most 8 warps a block
   const bool wl = shape.mode == 1 && ea.st.pos && threads <= 256;
   const uint32_t wl_shade = shape.wl_shade_min == 0 ? 32u : (shape.wl_shade_min > 32 ? 32u : shape.wl_shade_min);
@@ -656,7 +605,7 @@ cudaError_t launch_trace(const DJob* jobs, uint32_t n_jobs, uint32_t total_rays,
 #define OMG_TRACE_LAUNCH(NB, TIE, WIDE, WT, BOX)                                                              \
   trace_kernel<NB, TIE, WIDE, WT, BOX><<<blocks, threads, 0, s>>>(jobs, n_jobs, total_rays, scenes, job_mats, \
                                                                   panels, groups, acc, hdr, job_segments,     \
-                                                                  refill, steps, shade_min, lane_cap, ea)
+                                                                  refill, steps, lane_cap, ea)
 #define OMG_TRACE_PICK(NB)                                                                                    \
   if (wl && tie)                                                                                              \
     trace_wl_kernel<NB, true><<<blocks, threads, 0, s>>>(jobs, n_jobs, total_rays, scenes, job_mats, panels,  \

@@ -1,7 +1,7 @@
 // The per-lane closest-hit walk of the persistent tracer (trace.cu) and of the
 // dome's escape walk (dome.cu): a walk that stops after a step budget and
-// resumes, the near-tie rule on a compact state, the speculative node phase
-// on the grown boxes, and the pending leaves tested by the whole warp.
+// resumes, the near-tie rule on a compact state, the speculative node phase,
+// and the pending leaves tested by the whole warp.
 #pragma once
 #include "device_common.cuh"
 
@@ -15,7 +15,8 @@ namespace {
 // split into registers once inlined); the two stacks live beside it.
 struct Walk {
   int cur;
-  int leaf;          // postponed leaf (TIE), or 0
+  int leaf;          // postponed leaf, or 0
+  float cur_t, leaf_t;   // first-found rule: their boxes' entry distances
   int sp;
   int prim_best;     // the winner so far (-1: no hit yet)
   float t_best;
@@ -47,15 +48,29 @@ constexpr int kDone = 0x7FFFFFFF;  // never a node index (< 2^28)
 constexpr int kMaxWarps = 8;       // warps of a trace_kernel block (at most 256 threads)
 constexpr int kCoopRounds = 8;     // cooperative leaf rounds per loop iteration
 
+// The next stacked entry that is not culled (its entry distance in w.cur_t), or kDone.
 template <bool TIE>
 __device__ __forceinline__ int walk_pop(Walk& w) {
   const float cull = walk_cull<TIE>(w);
   while (w.sp > 0) {
     w.sp--;
-    if (TIE ? w.stack_t[w.sp] > cull : (walk_have(w) && w.stack_t[w.sp] >= w.t_best)) continue;
+    const float t = w.stack_t[w.sp];
+    if (TIE ? t > cull : (walk_have(w) && t >= w.t_best)) continue;
+    if (!TIE) w.cur_t = t;
     return w.stack_ref[w.sp];
   }
   return kDone;
+}
+
+// A leaf that the walk has reached is postponed (one at a time; a second one
+// stays in cur and ends the descent).
+template <bool TIE>
+__device__ __forceinline__ void walk_postpone(Walk& w) {
+  if (w.cur < 0 && w.leaf == 0) {
+    w.leaf = w.cur;
+    if (!TIE) w.leaf_t = w.cur_t;
+    w.cur = walk_pop<TIE>(w);
+  }
 }
 
 template <bool TIE>
@@ -65,6 +80,7 @@ __device__ __forceinline__ void walk_begin(Walk& w, const DScene& S, float ox, f
   // near-tie rule lets the visit order differ
   w.cur = S.n_prims ? ((TIE && wide && S.nodes4) ? S.root4 : S.root) : kDone;
   w.leaf = 0;
+  if (!TIE) w.cur_t = 0.0f;
   w.sp = 0;
   w.prim_best = -1;
   w.t_best = FLT_MAX;
@@ -95,41 +111,38 @@ __device__ __forceinline__ bool walk_restart_fixed(Walk& w, int root, uint32_t b
   return true;
 }
 
-// One hit of a near-tie walk, primitive i at t with authored surface s and
-// original triangle tr (the rule of tie_take, device_common.cuh, on the
-// compact state).
-__device__ __forceinline__ void walk_take_tie(Walk& w, const float4* __restrict__ prims, uint32_t i, float t,
-                                              uint32_t s, uint32_t tr) {
-  {
-    const bool have = w.prim_best >= 0;
-    // the winner's key, read back from its primitive
-    auto less_than_best = [&]() {
-      const uint32_t bs = __float_as_uint(__ldg(prims + 3 * w.prim_best + 2).w);
-      const uint32_t btr = __float_as_uint(__ldg(prims + 3 * w.prim_best + 1).w);
-      return tie_key_less(s, tr, t, bs, btr, w.t_best);
-    };
-    bool take;
-    if (w.flags & kWalkFixed) {
-      take = t <= w.t_min * (1.0f + kTieRel) && (!have || less_than_best());
-    } else if (!have) {
-      take = true;
-      w.t_min = t;
-    } else if (t < w.t_min) {
-      const float win = t * (1.0f + kTieRel);
-      if (w.t_best <= win) {
-        take = less_than_best();
-      } else {
-        if (w.t_min <= win) w.flags |= kWalkAmb;
-        take = true;
-      }
-      w.t_min = t;
+// One hit of a near-tie walk, primitive i at t (the rule of tie_take,
+// device_common.cuh, on the compact state; the ids of the hit and of the
+// winner so far are read only when their keys are compared).
+__device__ __forceinline__ void walk_take_tie(Walk& w, const float4* __restrict__ prims, uint32_t i, float t) {
+  const bool have = w.prim_best >= 0;
+  auto less_than_best = [&]() {
+    const uint32_t s = __float_as_uint(__ldg(&prims[3 * i + 2].w)), tr = __float_as_uint(__ldg(&prims[3 * i + 1].w));
+    const uint32_t bs = __float_as_uint(__ldg(&prims[3 * w.prim_best + 2].w));
+    const uint32_t btr = __float_as_uint(__ldg(&prims[3 * w.prim_best + 1].w));
+    return tie_key_less(s, tr, t, bs, btr, w.t_best);
+  };
+  bool take;
+  if (w.flags & kWalkFixed) {
+    take = t <= w.t_min * (1.0f + kTieRel) && (!have || less_than_best());
+  } else if (!have) {
+    take = true;
+    w.t_min = t;
+  } else if (t < w.t_min) {
+    const float win = t * (1.0f + kTieRel);
+    if (w.t_best <= win) {
+      take = less_than_best();
     } else {
-      take = t <= w.t_min * (1.0f + kTieRel) && less_than_best();
+      if (w.t_min <= win) w.flags |= kWalkAmb;
+      take = true;
     }
-    if (take) {
-      w.prim_best = (int)i;
-      w.t_best = t;
-    }
+    w.t_min = t;
+  } else {
+    take = t <= w.t_min * (1.0f + kTieRel) && less_than_best();
+  }
+  if (take) {
+    w.prim_best = (int)i;
+    w.t_best = t;
   }
 }
 
@@ -145,7 +158,7 @@ __device__ __forceinline__ void walk_leaf_tie(Walk& w, const float4* __restrict_
     const float4 p2 = __ldg(prims + 3 * i + 2);
     float t;
     if (!tri_hit(wt, p0, p1, p2, ox, oy, oz, dx, dy, dz, t)) continue;
-    walk_take_tie(w, prims, i, t, __float_as_uint(p2.w), __float_as_uint(p1.w));
+    walk_take_tie(w, prims, i, t);
   }
 }
 
@@ -187,82 +200,93 @@ __device__ __forceinline__ bool walk4_steps(Walk& w, const DScene& S, float ox, 
   return w.cur == kDone;
 }
 
-// The node phase of the near-tie walk (TIE = true): speculative while-while
-// descent over the grown boxes with the fused multiply-add slab test,
+// Up to `steps` steps of the node phase: speculative while-while descent,
 // postponing one leaf, until every lane of the warp holds a leaf (or has none
-// left to reach). A ray whose origin lies beyond the boxes' margin (|o_a| >
-// 7 M_a: never in a trace that starts inside the scene) or that runs along a
-// coordinate plane (a direction component of 0) uses the plain slab test on
-// the same grown boxes. Returns true when the walk ran out of its budget (it
-// is then over, flag 4 raised).
-__device__ __forceinline__ bool walk_spec_nodes(Walk& w, const DScene& S, float ox, float oy, float oz, float dx,
-                                                float dy, float dz, int& steps, uint32_t* err) {
-  const float4* __restrict__ tnodes = S.nodes_f;
-  while (steps > 0 && w.cur >= 0 && w.cur != kDone) {
-    steps--;
-    if (w.budget-- == 0u) {
-      atomicOr(err, 4u);
-      w.cur = kDone;
-      w.leaf = 0;
-      return true;
-    }
-    const float4 n0 = __ldg(tnodes + 4 * w.cur + 0);
-    const float4 n1 = __ldg(tnodes + 4 * w.cur + 1);
-    const float4 n2 = __ldg(tnodes + 4 * w.cur + 2);
-    const float4 n3 = __ldg(tnodes + 4 * w.cur + 3);
-    const float tmax = walk_cull<true>(w);   // infinite before the first hit; the final window in fixed mode
+// left to reach). Returns true when the walk ran out of its budget (it is then
+// over, flag 4 raised).
+//
+// Near-tie rule: over the grown boxes with the fused multiply-add slab test. A
+// ray whose origin lies beyond the boxes' margin (|o_a| > 7 M_a: never in a
+// trace that starts inside the scene) or that runs along a coordinate plane (a
+// direction component of 0) uses the plain slab test on the same grown boxes.
+//
+// First-found rule: the reference's boxes and its slab test (by minima and
+// maxima where no product can be a NaN). The descent may pass nodes that the
+// reference would have culled with the hits of a leaf postponed here, so a
+// leaf is tested only if its entry distance is still below the best hit when
+// its turn comes. That is the reference's own condition: a box lies inside its
+// parent's, so its rounded entry distance is no less than any ancestor's, the
+// best hit only falls, and so a leaf that passes it was reached through
+// ancestors that passed it too; and the order in which leaves are reached does
+// not depend on the hits.
+template <bool TIE>
+__device__ __forceinline__ bool walk_nodes(Walk& w, const DScene& S, float ox, float oy, float oz, int& steps,
+                                           uint32_t* err) {
+  const float4* __restrict__ tnodes = TIE ? S.nodes_f : S.nodes;
+  // steps left, by the caller's allowance and by the walk's budget
+  uint32_t left = min((uint32_t)steps, w.budget);
+  const uint32_t allowed = left;
+  while (w.cur >= 0 && w.cur != kDone && left != 0u) {
+    left--;
+    const float4* __restrict__ nd = tnodes + 4 * (size_t)(uint32_t)w.cur;
+    const float4 n0 = __ldg(nd + 0), n1 = __ldg(nd + 1), n2 = __ldg(nd + 2), n3 = __ldg(nd + 3);
+    const float tmax = walk_cull<TIE>(w);   // infinite before the first hit; the final window in fixed mode
     float ta, tb;
     bool h0, h1;
     if (w.flags & kWalkFast) {
-      const float oix = ox * w.ix, oiy = oy * w.iy, oiz = oz * w.iz;
-      h0 = ray_aabb_fma(n0.x, n0.y, n0.z, n0.w, n1.x, n1.y, oix, oiy, oiz, w.ix, w.iy, w.iz, tmax, ta);
-      h1 = ray_aabb_fma(n1.z, n1.w, n2.x, n2.y, n2.z, n2.w, oix, oiy, oiz, w.ix, w.iy, w.iz, tmax, tb);
+      if (TIE) {
+        const float oix = ox * w.ix, oiy = oy * w.iy, oiz = oz * w.iz;
+        h0 = ray_aabb_fma(n0.x, n0.y, n0.z, n0.w, n1.x, n1.y, oix, oiy, oiz, w.ix, w.iy, w.iz, tmax, ta);
+        h1 = ray_aabb_fma(n1.z, n1.w, n2.x, n2.y, n2.z, n2.w, oix, oiy, oiz, w.ix, w.iy, w.iz, tmax, tb);
+      } else {
+        h0 = ray_aabb_minmax(n0.x, n0.y, n0.z, n0.w, n1.x, n1.y, ox, oy, oz, w.ix, w.iy, w.iz, tmax, ta);
+        h1 = ray_aabb_minmax(n1.z, n1.w, n2.x, n2.y, n2.z, n2.w, ox, oy, oz, w.ix, w.iy, w.iz, tmax, tb);
+      }
     } else {
       h0 = ray_aabb(n0.x, n0.y, n0.z, n0.w, n1.x, n1.y, ox, oy, oz, w.ix, w.iy, w.iz, tmax, ta);
       h1 = ray_aabb(n1.z, n1.w, n2.x, n2.y, n2.z, n2.w, ox, oy, oz, w.ix, w.iy, w.iz, tmax, tb);
     }
     const int c0 = __float_as_int(n3.x), c1 = __float_as_int(n3.y);
-    if (h0 && h1) {
-      int nr, fr;
-      float ft;
-      if (ta <= tb) { nr = c0; fr = c1; ft = tb; }
-      else { nr = c1; fr = c0; ft = ta; }
-      if (w.sp < STACK_DEPTH) {
-        w.stack_ref[w.sp] = fr;
-        w.stack_t[w.sp] = ft;
-        w.sp++;
-      } else {
-        atomicOr(err, 1u);
+    if (h0 || h1) {
+      const bool first0 = h0 && (!h1 || ta <= tb);      // c0 is the one to enter
+      if (h0 && h1) {
+        if (w.sp < STACK_DEPTH) {
+          w.stack_ref[w.sp] = first0 ? c1 : c0;
+          w.stack_t[w.sp] = first0 ? tb : ta;
+          w.sp++;
+        } else {
+          atomicOr(err, 1u);
+        }
       }
-      w.cur = nr;   // the nearer entry t <= tmax = t_cull: never culled here
-    } else if (h0) {
-      w.cur = c0;
-    } else if (h1) {
-      w.cur = c1;
+      w.cur = first0 ? c0 : c1;   // its entry t <= tmax: not culled here
+      if (!TIE) w.cur_t = first0 ? ta : tb;
     } else {
-      w.cur = walk_pop<true>(w);
+      w.cur = walk_pop<TIE>(w);
     }
-    if (w.cur < 0 && w.leaf == 0) {
-      w.leaf = w.cur;
-      w.cur = walk_pop<true>(w);
-    }
+    walk_postpone<TIE>(w);
     if (__all_sync(__activemask(), w.leaf < 0 || w.cur == kDone)) break;
   }
-  if (w.leaf == 0 && w.cur < 0) {
-    w.leaf = w.cur;
-    w.cur = walk_pop<true>(w);
+  walk_postpone<TIE>(w);
+  const uint32_t used = allowed - left;
+  steps -= (int)used;
+  w.budget -= used;
+  if (w.budget == 0u && w.cur >= 0 && w.cur != kDone) {
+    atomicOr(err, 4u);
+    w.cur = kDone;
+    w.leaf = 0;
+    return true;
   }
   return false;
 }
 
 // The near-tie walk (TIE = true): speculative while-while over the grown
-// boxes with the fused multiply-add slab test (walk_spec_nodes), then the
+// boxes with the fused multiply-add slab test (walk_nodes), then the
 // postponed leaves one after another.
 __device__ __forceinline__ bool walk_spec(Walk& w, const DScene& S, float ox, float oy, float oz, float dx,
                                           float dy, float dz, int steps, uint32_t* err) {
   const bool wt = S.prims_wt != nullptr;
   const float4* __restrict__ prims = wt ? S.prims_wt : S.prims;
-  if (walk_spec_nodes(w, S, ox, oy, oz, dx, dy, dz, steps, err)) return true;
+  if (walk_nodes<true>(w, S, ox, oy, oz, steps, err)) return true;
   while (w.leaf < 0 && steps > 0) {
     steps--;
     if (w.budget-- == 0u) {
@@ -285,26 +309,67 @@ __device__ __forceinline__ bool walk_spec(Walk& w, const DScene& S, float ox, fl
   return false;
 }
 
-// Leaves of near-tie walks tested by the whole warp (every lane calls this,
-// warp-uniformly; `own`: this lane is walking). A leaf holds 1 to 8
-// primitives, and one lane testing its own leaf's primitives one after
-// another leaves most of the warp idle; here the primitives of every lane's
-// pending leaf are laid out in a per-warp slot list (shared memory, `slots`:
-// 256 bytes), each lane tests one slot's primitive against the slot owner's
-// ray (fetched by shuffles), and each owner then takes its hits in leaf order,
-// so the near-tie state sees the sequence walk_leaf_tie would give it. After a
-// round, a walk whose next node is a leaf postpones it, and rounds repeat
-// while any lane holds a leaf (at most `rounds`).
-// WT: the warp may hold walks of watertight scenes (the owner's flag is then
-// read); false compiles the reference's test alone.
-template <bool WT>
-__device__ __forceinline__ void coop_leaf_rounds(Walk& w, bool own_walk, const float4* lane_prims, bool wt,
-                                                 float ox, float oy, float oz, float dx, float dy, float dz,
-                                                 uint8_t* __restrict__ slots, int rounds, uint32_t* err) {
+// The first-found walk of a lane on its own: the node phase, then its
+// postponed leaf, skipped if culled by now.
+__device__ __forceinline__ bool walk_first(Walk& w, const DScene& S, float ox, float oy, float oz, float dx, float dy,
+                                           float dz, int steps, uint32_t* err) {
+  if (walk_nodes<false>(w, S, ox, oy, oz, steps, err)) return true;
+  while (w.leaf < 0 && steps > 0) {
+    steps--;
+    if (w.budget-- == 0u) {
+      atomicOr(err, 4u);
+      w.cur = kDone;
+      w.leaf = 0;
+      return true;
+    }
+    if (!walk_have(w) || w.leaf_t < w.t_best) {
+      const uint32_t code = ~(uint32_t)w.leaf;
+      const uint32_t start = code >> 3, end = start + (code & 7u) + 1u;
+      for (uint32_t i = start; i < end; i++) {
+        float t;
+        if (ray_tri(__ldg(S.prims + 3 * i), __ldg(S.prims + 3 * i + 1), __ldg(S.prims + 3 * i + 2), ox, oy, oz, dx, dy,
+                    dz, t) &&
+            (!walk_have(w) || t < w.t_best)) {
+          w.t_best = t;
+          w.prim_best = (int)i;
+        }
+      }
+    }
+    w.leaf = 0;
+    walk_postpone<false>(w);
+  }
+  return w.cur == kDone && w.leaf == 0;
+}
+
+// Leaves tested by the whole warp (every lane calls this, warp-uniformly;
+// own_walk: this lane is walking). A leaf holds 1 to 8 primitives, and one lane
+// testing its own leaf's primitives one after another leaves most of the warp
+// idle; here the primitives of every lane's pending leaf are laid out in a
+// per-warp slot list (shared memory, `slots`: 256 bytes), each lane tests one
+// slot's primitive against the slot owner's ray (fetched by shuffles), and each
+// owner then takes its hits in leaf order, so its state sees the sequence that
+// testing them one by one would give it. After a round, a walk whose next node
+// is a leaf postpones it, and rounds repeat while any lane holds a leaf (at
+// most `rounds`).
+//
+// First-found rule: a leaf whose entry distance is no longer below the best
+// hit when its turn comes is skipped (walk_nodes).
+//
+// WT: the warp may hold walks of watertight scenes; false compiles the
+// reference's test alone.
+//
+// (Exchanging the rays through shared memory and both pending leaves in one
+// round, with the hits back through a ballot, was slower: 5.37 against 4.93 G
+// warp instructions for 64 pairs on the 40-room world, 8.7 against 8.0 ms. The
+// owners' loops over their own hits run with two or three lanes; the loop over
+// the slot ranks here runs with all.)
+template <bool TIE, bool WT>
+__device__ __forceinline__ void coop_leaf_rounds(Walk& w, bool own_walk, const float4* lane_prims, float ox, float oy,
+                                                 float oz, float dx, float dy, float dz, uint8_t* __restrict__ slots,
+                                                 int rounds, uint32_t* err) {
   const unsigned FULL = 0xffffffffu;
   const uint32_t lane = threadIdx.x & 31u;
-  // the owner's primitives, its watertight flag in bit 0 (the arrays are 16-byte aligned)
-  const unsigned long long my_prims = reinterpret_cast<unsigned long long>(lane_prims) | ((WT && wt) ? 1ull : 0ull);
+  const unsigned long long my_prims = reinterpret_cast<unsigned long long>(lane_prims);
   while (rounds-- > 0) {
     bool own = own_walk && w.leaf < 0;
     if (__ballot_sync(FULL, own) == 0u) break;
@@ -321,6 +386,7 @@ __device__ __forceinline__ void coop_leaf_rounds(Walk& w, bool own_walk, const f
         const uint32_t code = ~(uint32_t)w.leaf;
         start = code >> 3;
         cnt = (code & 7u) + 1u;
+        if (!TIE && walk_have(w) && w.leaf_t >= w.t_best) cnt = 0;
         w.leaf = 0;
       }
     }
@@ -344,7 +410,7 @@ __device__ __forceinline__ void coop_leaf_rounds(Walk& w, bool own_walk, const f
       const float rx = __shfl_sync(FULL, ox, o), ry = __shfl_sync(FULL, oy, o), rz = __shfl_sync(FULL, oz, o);
       const float sx = __shfl_sync(FULL, dx, o), sy = __shfl_sync(FULL, dy, o), sz = __shfl_sync(FULL, dz, o);
       const unsigned long long op = __shfl_sync(FULL, my_prims, o);
-      const float4* P = reinterpret_cast<const float4*>(WT ? (op & ~1ull) : op);
+      const float4* P = reinterpret_cast<const float4*>(op);
       const uint32_t i = o_start + (p - o_excl);
       // the slot's hit distance, infinity for a miss
       float t = __int_as_float(0x7f800000);
@@ -359,25 +425,24 @@ __device__ __forceinline__ void coop_leaf_rounds(Walk& w, bool own_walk, const f
         if (hit) t = th;
       }
       // each owner takes its slots of this chunk in leaf order: the distance
-      // from the slot's lane; its primitive (the owner's start + k) and that
-      // primitive's surface and triangle ids the owner reads itself, for hits
+      // from the slot's lane; its primitive is the owner's start + k
       for (uint32_t k = 0; k < kmax; k++) {
         const uint32_t q = excl + k;
         const bool mine = own && k < cnt && q >= base && q < base + 32u;
         const uint32_t src = mine ? q - base : lane;
         const float tk = __shfl_sync(FULL, t, src);
         if (mine && tk < __int_as_float(0x7f800000)) {
-          const uint32_t ik = start + k;
-          const float* pw = reinterpret_cast<const float*>(lane_prims + 3 * ik);
-          walk_take_tie(w, lane_prims, ik, tk, __float_as_uint(__ldg(pw + 11)), __float_as_uint(__ldg(pw + 7)));
+          if (TIE) {
+            walk_take_tie(w, lane_prims, start + k, tk);
+          } else if (!walk_have(w) || tk < w.t_best) {
+            w.t_best = tk;
+            w.prim_best = (int)(start + k);
+          }
         }
       }
     }
     __syncwarp();
-    if (own && w.cur < 0) {
-      w.leaf = w.cur;
-      w.cur = walk_pop<true>(w);
-    }
+    if (own) walk_postpone<TIE>(w);
   }
 }
 

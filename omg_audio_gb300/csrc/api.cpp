@@ -178,7 +178,7 @@ int32_t fill_batch(omg_ctx* ctx, BatchRec& B, const omg_job* jobs, uint32_t n_jo
   B.max_bins = 0;
   B.n_bin_floats = 0;
   B.n_dir_floats = 0;
-  bool coop_ok = P.tie_mode != 0, deep = false, box_only = true;
+  bool coop_ok = P.tie_mode != 0, deep = false, box_only = true, solo_ok = true;
   float last_time = 0.0f;
   // per-job panel materials are placed after all box wall materials
   for (uint32_t i = 0; i < n_jobs; i++) {
@@ -231,6 +231,7 @@ int32_t fill_batch(omg_ctx* ctx, BatchRec& B, const omg_job* jobs, uint32_t n_jo
       if (it->second->n_bands != nb) return OMG_E_INVALID;
       d.scene = j.scene_id;
       box_only = false;
+      if (it->second->n_nodes4 == 0 && it->second->root >= 0) solo_ok = false;
       if (it->second->n_nodes4 == 0) coop_ok = false;
       if (it->second->n_prims > kSpreadPrims) deep = true;
     } else {
@@ -276,6 +277,7 @@ int32_t fill_batch(omg_ctx* ctx, BatchRec& B, const omg_job* jobs, uint32_t n_jo
   B.coop_ok = coop_ok;
   B.deep = deep;
   B.box_only = box_only;
+  B.solo_ok = solo_ok;
   B.n_acc = acc;
   B.n_out = out;
   return OMG_OK;
@@ -369,6 +371,7 @@ int32_t record_launch(omg_ctx* ctx, BatchRec& B, cudaStream_t s, int parts = 3) 
     eff.loop_guard = ctx->prm.loop_guard;
     if (B.deep) eff.spread_warps = 32;
     eff.box_only = B.box_only;
+    eff.solo_ok = B.solo_ok;
     if (eff.mode == 2 && !B.coop_ok) eff.mode = 0;
     if (eff.tail_mode == 2 && !B.coop_ok) eff.tail_mode = 0;
     CK(launch_wavefront(B.d_jobs.p, B.n_jobs, B.total_rays, B.max_nb, ctx->d_scenes.p, B.d_job_mats.p,

@@ -189,9 +189,10 @@ int32_t scene_upload_impl(omg_ctx* ctx, const float* pos, uint32_t nv, const uin
       CK(S->nodes_f.alloc(S->n_nodes * 4));
       CK(cudaMemcpy(S->nodes_f.p, grown.data(), grown.size() * 4, cudaMemcpyHostToDevice));
     }
-    // the 4-wide tree serves near-tie walks only: its boxes are grown likewise
+    // the 4-wide tree: its boxes are grown likewise for near-tie walks; a
+    // first-found context walks it with the reference's own boxes (solo.cu)
     std::vector<float> grown_ref = S->ref_boxes;
-    grow_ref_boxes(grown_ref, S->fast_m, pad);
+    if (ctx->prm.tie_mode != 0) grow_ref_boxes(grown_ref, S->fast_m, pad);
     std::vector<float> dev_nodes4;
     uint32_t need = 0;
     S->root4 = flatten_bvh4(grown_ref, S->ref_ab, dev_nodes4, &need);

@@ -7,7 +7,8 @@
 //             n0 = (c0.lo.x, c0.lo.y, c0.lo.z, c0.hi.x)
 //             n1 = (c0.hi.y, c0.hi.z, c1.lo.x, c1.lo.y)
 //             n2 = (c1.lo.z, c1.hi.x, c1.hi.y, c1.hi.z)
-//             n3 = (c0 ref, c1 ref, -, -) as int bits
+//             n3 = (c0 ref, c1 ref, split, -) as int bits; split (host-numbered trees): c0's
+//             primitives lie below this leaf-order index, c1's from it on
 //             ref >= 0: internal node index; ref < 0: leaf ~((start << 3) | (count - 1))
 //   prims   : 48 B per tessellated primitive, in leaf order
 //             p0 = (a.xyz, material id)  p1 = (e1.xyz, original tri id)  p2 = (e2.xyz, surface id)
@@ -211,6 +212,7 @@ struct LaunchShape {
   uint32_t wl_shade_min = 32;   // modes 1 and 2: rays a warp shades together once that many wait
   uint32_t spread_warps = 16;   // resident warps per multiprocessor that a launch of few rays is spread over (the
                                 // batch sets 32 when a scene's tree is beyond an L1: kSpreadPrims)
+  bool solo_ok = false;         // every mesh scene can be walked by whole warps (solo.cu; set by the batch)
   bool box_only = false;        // every job of the launch is a shoebox (set by the batch)
   uint32_t loop_guard = 0;      // loop iterations of one warp of a persistent kernel before it stops
                                 // and flags error 8 (0: kDefaultLoopGuard); from omg_params.loop_guard
@@ -278,6 +280,12 @@ cudaError_t launch_trace(const DJob* jobs, uint32_t n_jobs, uint32_t total_rays,
 // trace.cu: load the shoebox trace kernels (3 and 8 bands) now, so that a later
 // launch does not wait for the driver's lazy module loading.
 cudaError_t preload_trace_kernels();
+// solo.cu: the tracer for launches of few rays, one warp per ray (every mesh
+// scene has a 4-wide tree or is one leaf); max_loop as in EpochArgs.
+cudaError_t launch_trace_solo(const DJob* jobs, uint32_t n_jobs, uint32_t total_rays, uint32_t max_nb,
+                              const DScene* scenes, const DMat* job_mats, const DPanel* panels, float* acc,
+                              DLaunch* hdr, uint32_t* job_segments, uint32_t max_loop, int n_sms, bool tie, bool wt,
+                              cudaStream_t s);
 // coop.cu: the mode-2 persistent kernel (same arguments as launch_trace).
 cudaError_t launch_trace_coop(const DJob* jobs, uint32_t n_jobs, uint32_t total_rays, uint32_t max_nb,
                               const DScene* scenes, const DMat* job_mats, const DPanel* panels,

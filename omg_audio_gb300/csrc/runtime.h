@@ -135,6 +135,7 @@ struct BatchRec {
   bool coop_ok = false;           // near-tie rule and every mesh scene has a 4-wide tree (mode 2)
   bool deep = false;              // a scene beyond kSpreadPrims primitives
   bool box_only = false;          // every job is a shoebox
+  bool solo_ok = false;           // every mesh scene has a 4-wide tree or is one leaf (solo.cu)
   DevBuf<uint32_t> d_ep_q;        // epoch queues (2 x rays)
   LaunchShape shape;
   // recorded when first needed (batch_graph)

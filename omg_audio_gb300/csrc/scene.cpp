@@ -532,6 +532,21 @@ int32_t flatten_bvh2(const std::vector<float>& ref_boxes, const std::vector<uint
     std::memcpy(&o[12], &r0, 4);
     std::memcpy(&o[13], &r1, 4);
   }
+  // where each node's primitives part: child 0's lie below this leaf-order
+  // index, child 1's from it on (-1 if a tree's leaves are not in that order)
+  std::vector<uint32_t> lo(nref), hi(nref);
+  for (uint32_t i = 0; i < nref; i++)
+    if (ref_ab[2 * i] & kLeafBit) {
+      lo[i] = ref_ab[2 * i] & ~kLeafBit;
+      hi[i] = lo[i] + ref_ab[2 * i + 1];
+    }
+  for (size_t k = order.size(); k-- > 0;) {   // children before parents
+    const uint32_t i = order[k], c0 = ref_ab[2 * i], c1 = ref_ab[2 * i + 1];
+    lo[i] = lo[c0];
+    hi[i] = hi[c1];
+    const int32_t split = hi[c0] == lo[c1] ? (int32_t)lo[c1] : -1;
+    std::memcpy(&dev_nodes[(size_t)dev_of[i] * 16 + 14], &split, 4);
+  }
   return 0;
 }
 

@@ -205,11 +205,12 @@ static __device__ __noinline__ void record_arrival(const DJob& J, float* __restr
 
 // One segment after its closest hit (tracer.rs:110-200): the receiver test with
 // compensated histogram adds, then advance, absorb, transmit or scatter.
-// Returns true when the ray ends here.
+// Returns true when the ray ends here. lead: this lane records arrivals (false:
+// another lane of the warp runs the same segment and does).
 template <int NB>
 __device__ __forceinline__ bool shade_segment(const DJob& J, float* __restrict__ acc, const Hit& h, bool have,
                                               float t_hit, float& px, float& py, float& pz, float& dx, float& dy,
-                                              float& dz, float& dist, float (&e)[NB], Pcg& rng) {
+                                              float& dz, float& dist, float (&e)[NB], Pcg& rng, bool lead = true) {
   const uint32_t nb = J.nb;
   // receiver sphere crossing along this segment (tracer.rs:110-128)
   {
@@ -221,7 +222,7 @@ __device__ __forceinline__ bool shade_segment(const DJob& J, float* __restrict__
       if (ddx * ddx + ddy * ddy + ddz * ddz < J.rr2) {     // sqrt(..) < rr (DJob::rr2)
         const float arrival = (dist + s) / J.c;
         const float q = arrival / J.bin_dt;
-        if (q < (float)J.n_bins) {          // (q as usize) < NBINS, q >= 0
+        if (lead && q < (float)J.n_bins) {  // (q as usize) < NBINS, q >= 0
           Bands<NB> eb;
 #pragma unroll
           for (int b = 0; b < NB; b++) eb.v[b] = e[b];

@@ -565,6 +565,17 @@ cudaError_t launch_trace(const DJob* jobs, uint32_t n_jobs, uint32_t total_rays,
   // flags error 8: by default far above any legitimate count (each iteration
   // advances a walk, a shading pass or the ray queue)
   ea.max_loop = shape.loop_guard ? shape.loop_guard : kDefaultLoopGuard;
+  // Few rays on meshes: a warp per ray (solo.cu). Its work per ray is larger, so
+  // the lanes win again from about two rays per resident warp: 4096, 8192 and
+  // 16,384 rays on the 40-room world 0.72, 1.16 and 1.92 ms against 1.20, 1.51
+  // and 1.81 ms (near-tie rule), 0.82, 1.36, 2.18 against 1.51, 1.96, 2.38 ms
+  // (first-found rule); on the 12-triangle room 0.46, 0.80, 1.40 against 0.79,
+  // 0.89, 1.00 ms. Shoeboxes have no walk to share (a 4096-ray call 0.15
+  // against 0.14 ms).
+  if (!ep && shape.mode == 0 && !shape.wide && shape.solo_ok && !shape.box_only &&
+      total_rays <= 2u * 28u * (uint32_t)n_sms)
+    return launch_trace_solo(jobs, n_jobs, total_rays, max_nb, scenes, job_mats, panels, acc, hdr, job_segments,
+                             ea.max_loop, n_sms, tie, wt, s);
   if (shape.mode == 2 && tie && ea.st.pos)
     return launch_trace_coop(jobs, n_jobs, total_rays, max_nb, scenes, job_mats, panels, groups, acc, hdr,
                              job_segments, shape, n_sms, ea, s);

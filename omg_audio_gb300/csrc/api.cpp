@@ -260,7 +260,8 @@ int32_t fill_batch(omg_ctx* ctx, BatchRec& B, const omg_job* jobs, uint32_t n_jo
     rays += j.n_rays;
     if (rays > 0xFFFFFFFFull) return OMG_E_INVALID;
     d.acc_off = acc;
-    d.out_off = out;
+    d.out_off = B.n_bin_floats;
+    d.dir_off = B.n_dir_floats;   // behind every job's bins: below
     acc += acc_floats(n_bins, nb);
     out += out_floats(n_bins, nb);
     B.max_nb = std::max(B.max_nb, nb);
@@ -273,6 +274,7 @@ int32_t fill_batch(omg_ctx* ctx, BatchRec& B, const omg_job* jobs, uint32_t n_jo
     r.nb = nb;
     r.bin_dt = P.bin_dt;
   }
+  for (DJob& d : B.jobs) d.dir_off += B.n_bin_floats;
   B.total_rays = (uint32_t)rays;
   B.coop_ok = coop_ok;
   B.deep = deep;
@@ -283,7 +285,15 @@ int32_t fill_batch(omg_ctx* ctx, BatchRec& B, const omg_job* jobs, uint32_t n_jo
   return OMG_OK;
 }
 
-int32_t alloc_batch(omg_ctx* ctx, BatchRec& B) {
+// Echograms of this size and more are copied straight into the caller's
+// arrays: on the GB300's host a device copy into pageable memory runs at the
+// link's rate (3 MB in 31 us, 12 MB in 85 us), while the host's copy out of
+// pinned memory took 140 us for 3 MB. Below it the copy is one node of the
+// batch's graph (11 us against 17).
+constexpr size_t kDirectBytes = 512u << 10;
+
+// stage: the results wait in pinned memory whatever their size (tickets).
+int32_t alloc_batch(omg_ctx* ctx, BatchRec& B, bool stage) {
   CK(B.d_jobs.alloc(B.n_jobs));
   CK(B.d_job_mats.alloc(B.job_mats.size()));
   CK(B.d_panels.alloc(B.panels.size()));
@@ -307,7 +317,9 @@ int32_t alloc_batch(omg_ctx* ctx, BatchRec& B) {
   CK(B.d_block.alloc(off));
   B.ret_off = o_hdr;
   B.ret_bytes = o_out + B.n_out * sizeof(float) - o_hdr;
-  CK(B.h_block.alloc(B.ret_bytes));
+  B.direct = !stage && B.n_out * sizeof(float) >= kDirectBytes;
+  B.staged_bytes = B.direct ? o_out - o_hdr : B.ret_bytes;
+  CK(B.h_block.alloc(B.staged_bytes));
   unsigned char *d = B.d_block.p, *h = B.h_block.p;
   B.d_acc = {reinterpret_cast<float*>(d + o_acc), B.n_acc};
   B.d_ep_ctl = {reinterpret_cast<EpochCtl*>(d + o_ep), kMaxEpochs + 1};
@@ -318,7 +330,7 @@ int32_t alloc_batch(omg_ctx* ctx, BatchRec& B) {
   B.h_hdr = {reinterpret_cast<DLaunch*>(h), 1};
   B.h_seg = {reinterpret_cast<uint32_t*>(h + (o_seg - o_hdr)), B.n_jobs};
   B.h_reverb = {reinterpret_cast<omg_reverb*>(h + (o_rev - o_hdr)), B.n_jobs};
-  B.h_out = {reinterpret_cast<float*>(h + (o_out - o_hdr)), B.n_out};
+  if (!B.direct) B.h_out = {reinterpret_cast<float*>(h + (o_out - o_hdr)), B.n_out};
   if (!B.done) CK(cudaEventCreateWithFlags(&B.done, cudaEventDisableTiming));
   return OMG_OK;
 }
@@ -387,7 +399,7 @@ int32_t record_launch(omg_ctx* ctx, BatchRec& B, cudaStream_t s, int parts = 3) 
 }
 
 int32_t record_readback(omg_ctx* ctx, BatchRec& B, cudaStream_t s) {
-  CK(cudaMemcpyAsync(B.h_block.p, B.d_block.p + B.ret_off, B.ret_bytes, cudaMemcpyDeviceToHost, s));
+  CK(cudaMemcpyAsync(B.h_block.p, B.d_block.p + B.ret_off, B.staged_bytes, cudaMemcpyDeviceToHost, s));
   return OMG_OK;
 }
 
@@ -438,11 +450,11 @@ int32_t build_graphs(omg_ctx* ctx, BatchRec& B, bool io) {
 }
 
 int32_t prepare_batch(omg_ctx* ctx, BatchRec& B, const omg_job* jobs, uint32_t n_jobs, const omg_panel* panels,
-                      uint32_t n_panels, bool io) {
+                      uint32_t n_panels, bool io, bool stage) {
   B.shape = ctx->shape;
   int32_t rc = fill_batch(ctx, B, jobs, n_jobs, panels, n_panels);
   if (rc) return rc;
-  if ((rc = alloc_batch(ctx, B))) return rc;
+  if ((rc = alloc_batch(ctx, B, stage))) return rc;
   if ((rc = upload_batch(ctx, B))) return rc;
   if ((rc = build_graphs(ctx, B, io))) return rc;
   B.signature = batch_signature(jobs, n_jobs, n_panels, ctx->prm);
@@ -459,30 +471,23 @@ int32_t check_kernel_flags(omg_ctx* ctx, const BatchRec& B) {
   return OMG_OK;
 }
 
-// The jobs' echograms from the pinned staging arrays into the caller's
-// buffers. Large results are copied by a few threads, job by job (one thread
-// copies at about 17 GB/s into freshly mapped pages).
-void copy_results(const BatchRec& B, float* bins, float* dirs, omg_reverb* reverb) {
-  std::vector<uint64_t> bo(B.n_jobs), dof(B.n_jobs);
-  uint64_t b = 0, d = 0;
-  for (uint32_t i = 0; i < B.n_jobs; i++) {
-    bo[i] = b;
-    dof[i] = d;
-    b += (uint64_t)B.jobs[i].n_bins * B.jobs[i].nb;
-    d += (uint64_t)B.jobs[i].n_bins * 3;
-  }
-  const int threads = (b + d) * sizeof(float) >= (1u << 20) ? 4 : 1;
-#pragma omp parallel for num_threads(threads) schedule(static)
-  for (int64_t i = 0; i < (int64_t)B.n_jobs; i++) {
-    const DJob& j = B.jobs[i];
-    const uint64_t nbb = (uint64_t)j.n_bins * j.nb, nd = (uint64_t)j.n_bins * 3;
-    if (bins) std::memcpy(bins + bo[i], B.h_out.p + j.out_off, nbb * sizeof(float));
-    if (dirs) std::memcpy(dirs + dof[i], B.h_out.p + j.out_off + nbb, nd * sizeof(float));
+// The results of a finished batch into the caller's arrays: out of the pinned
+// image, or (direct) off the device on the context's stream.
+int32_t copy_results(omg_ctx* ctx, const BatchRec& B, float* bins, float* dirs, omg_reverb* reverb) {
+  const size_t nb = B.n_bin_floats * sizeof(float), nd = B.n_dir_floats * sizeof(float);
+  if (B.direct) {
+    if (bins) CK(cudaMemcpyAsync(bins, B.d_out.p, nb, cudaMemcpyDeviceToHost, ctx->stream));
+    if (dirs) CK(cudaMemcpyAsync(dirs, B.d_out.p + B.n_bin_floats, nd, cudaMemcpyDeviceToHost, ctx->stream));
+    CK(cudaStreamSynchronize(ctx->stream));
+  } else {
+    if (bins) std::memcpy(bins, B.h_out.p, nb);
+    if (dirs) std::memcpy(dirs, B.h_out.p + B.n_bin_floats, nd);
   }
   if (reverb) {
     std::memcpy(reverb, B.h_reverb.p, B.n_jobs * sizeof(omg_reverb));
     for (uint32_t i = 0; i < B.n_jobs; i++) reverb[i].segments = B.h_seg.p[i];
   }
+  return OMG_OK;
 }
 
 // One synchronous pass through the io graph: H2D jobs, launch, D2H, bounded wait.
@@ -497,8 +502,7 @@ int32_t run_io(omg_ctx* ctx, BatchRec& B, float* bins, float* dirs, omg_reverb* 
   rc = wait_event(ctx, B.done, timeout_of(ctx));
   if (rc) return rc;
   if ((rc = check_kernel_flags(ctx, B))) return rc;
-  copy_results(B, bins, dirs, reverb);
-  return OMG_OK;
+  return copy_results(ctx, B, bins, dirs, reverb);
 }
 
 // New per-job values into a batch whose job layout is unchanged: the job
@@ -542,7 +546,7 @@ int32_t one_shot(omg_ctx* ctx, const omg_job* jobs, uint32_t n_jobs, const omg_p
   uint64_t sig = batch_signature(jobs, n_jobs, n_panels, ctx->prm);
   if (!ctx->cached || ctx->cached->signature != sig) {
     ctx->cached.reset(new BatchRec());
-    int32_t rc = prepare_batch(ctx, *ctx->cached, jobs, n_jobs, panels, n_panels, true);
+    int32_t rc = prepare_batch(ctx, *ctx->cached, jobs, n_jobs, panels, n_panels, true, false);
     if (rc) {
       ctx->cached.reset();
       return rc;
@@ -574,7 +578,7 @@ namespace omg {
 
 int32_t batch_prepare(omg_ctx* ctx, BatchRec& B, const omg_job* jobs, uint32_t n_jobs, const omg_panel* panels,
                       uint32_t n_panels) {
-  return prepare_batch(ctx, B, jobs, n_jobs, panels, n_panels, false);
+  return prepare_batch(ctx, B, jobs, n_jobs, panels, n_panels, false, false);
 }
 int32_t batch_refill(omg_ctx* ctx, BatchRec& B, const omg_job* jobs, uint32_t n_jobs, const omg_panel* panels,
                      uint32_t n_panels) {
@@ -712,7 +716,7 @@ int32_t omg_batch_create(omg_ctx* ctx, const omg_job* jobs, uint32_t n_jobs, con
                          uint32_t n_panels, uint32_t* batch_id) {
   if (!ctx || !jobs || !n_jobs || !batch_id || (n_panels && !panels)) return OMG_E_INVALID;
   std::unique_ptr<BatchRec> B(new BatchRec());
-  int32_t rc = prepare_batch(ctx, *B, jobs, n_jobs, panels, n_panels, false);
+  int32_t rc = prepare_batch(ctx, *B, jobs, n_jobs, panels, n_panels, false, false);
   if (rc) return rc;
   *batch_id = ctx->next_batch++;
   ctx->batches[*batch_id] = std::move(B);
@@ -750,8 +754,7 @@ int32_t omg_batch_read(omg_ctx* ctx, uint32_t id, float* bins, float* dirs, omg_
   CK(cudaEventRecord(B.done, ctx->stream));
   if ((rc = wait_event(ctx, B.done, timeout_of(ctx)))) return rc;
   if ((rc = check_kernel_flags(ctx, B))) return rc;
-  copy_results(B, bins, dirs, reverb);
-  return OMG_OK;
+  return copy_results(ctx, B, bins, dirs, reverb);
 }
 
 int32_t omg_batch_sizes(omg_ctx* ctx, uint32_t id, uint64_t* nb, uint64_t* nd) {
@@ -839,7 +842,7 @@ int32_t omg_submit_world(omg_ctx* ctx, uint32_t scene_id, const omg_world_job* j
   job_from_world(j, scene_id, *job, n_panels);
   Ticket t;
   t.batch.reset(new BatchRec());
-  int32_t rc = prepare_batch(ctx, *t.batch, &j, 1, panels, n_panels, true);
+  int32_t rc = prepare_batch(ctx, *t.batch, &j, 1, panels, n_panels, true, true);
   if (rc) return rc;
   BatchRec& B = *t.batch;
   std::memcpy(B.h_jobs.p, B.jobs.data(), sizeof(DJob));
@@ -859,7 +862,7 @@ int32_t omg_poll(omg_ctx* ctx, uint32_t ticket, float* bins, float* dirs, omg_re
   if (q == cudaErrorNotReady) return OMG_PENDING;
   if (q != cudaSuccess) return fail(ctx, q, "cudaEventQuery");
   int32_t rc = check_kernel_flags(ctx, B);
-  if (rc == OMG_OK) copy_results(B, bins, dirs, reverb);
+  if (rc == OMG_OK) rc = copy_results(ctx, B, bins, dirs, reverb);
   ctx->tickets.erase(it);
   return rc;
 }

@@ -152,7 +152,7 @@ int32_t omg_late_submit(omg_ctx* ctx, uint32_t field_id, const uint32_t* slots, 
     for (uint32_t i = 0; i < n_jobs; i++) {
       const float a = alpha ? alpha[i] : (L.updates[slots[i]] == 0 ? 1.0f : 0.3f);
       L.updates[slots[i]]++;
-      L.h_up.p[i] = DLateUpdate{slots[i], L.tick + 1, B->jobs[i].out_off, a, 0};
+      L.h_up.p[i] = DLateUpdate{slots[i], L.tick + 1, B->jobs[i].out_off, B->jobs[i].dir_off, a, 0};
       L.h_rj.p[i] = DReverbJob{(uint64_t)slots[i] * per, L.n_bins, L.nb, L.bin_dt, 0};
     }
     std::memcpy(B->h_jobs.p, B->jobs.data(), n_jobs * sizeof(DJob));

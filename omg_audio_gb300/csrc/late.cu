@@ -24,12 +24,13 @@ __global__ void late_ema_kernel(const DLateUpdate* __restrict__ up, uint32_t n_u
   if (u >= n_up) return;
   const DLateUpdate U = up[u];
   const float alpha = U.alpha;
-  const uint64_t n = (uint64_t)n_bins * (nb + 3);   // bins then dirs, as the batch lays out one job
-  const float* o = fresh + U.fresh_off;
+  const uint64_t nbb = (uint64_t)n_bins * nb, n = nbb + (uint64_t)n_bins * 3;   // bins then dirs
+  const float *o = fresh + U.fresh_off, *od = fresh + U.fresh_dir_off;
   float* a = avg + (uint64_t)U.slot * n;
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
     const float ai = a[i];
-    a[i] = ai + alpha * (o[i] - ai);
+    const float oi = i < nbb ? o[i] : od[i - nbb];
+    a[i] = ai + alpha * (oi - ai);
   }
 }
 

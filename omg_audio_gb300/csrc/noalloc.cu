@@ -170,7 +170,7 @@ extern "C" int32_t omg_trace_box_noalloc(const omg_box_job* job, const omg_param
   d.box_mat = 0;
   d.ray_base = 0;
   d.acc_off = 0;
-  d.out_off = 0;
+  d.out_off = d.dir_off = 0;
   WallMats walls;
   for (int w = 0; w < 6; w++) walls.m[w] = make_dmat(job->walls[w], nb);
 

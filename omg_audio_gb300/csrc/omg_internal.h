@@ -138,7 +138,8 @@ struct alignas(16) DJob {
   uint32_t n_groups;
   uint32_t ray_base;      // first global ray id of this job
   uint64_t acc_off;       // float offset of this job's accumulators
-  uint64_t out_off;       // float offset of this job's output (bins then dirs)
+  uint64_t out_off;       // float offsets of this job's bins and directions in the batch's
+  uint64_t dir_off;       // output (every job's bins, then every job's directions)
 };
 
 // DJob's two thresholds. The correctly rounded square root and quotient do not
@@ -319,7 +320,7 @@ cudaError_t launch_reverb(const DReverbJob* rj, uint32_t n_jobs, uint32_t max_bi
 struct DLateUpdate {
   uint32_t slot;
   uint32_t tick;
-  uint64_t fresh_off;
+  uint64_t fresh_off, fresh_dir_off;
   float alpha;          // EMA weight of the fresh echogram
   uint32_t pad;
 };

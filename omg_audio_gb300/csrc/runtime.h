@@ -117,7 +117,11 @@ struct BatchRec {
   // everything from ret_off (the header) on.
   DevBuf<unsigned char> d_block;
   PinBuf<unsigned char> h_block;
-  size_t clear_bytes = 0, ret_off = 0, ret_bytes = 0;
+  // Results of kDirectBytes or more do not pass through pinned memory: the
+  // header, segments and reverb do (staged_bytes), the echograms are copied
+  // straight into the caller's arrays once the batch is done.
+  size_t clear_bytes = 0, ret_off = 0, ret_bytes = 0, staged_bytes = 0;
+  bool direct = false;
   BufView<float> d_acc, d_out, h_out;
   BufView<EpochCtl> d_ep_ctl;     // kMaxEpochs + 1 records
   BufView<DLaunch> d_hdr, h_hdr;

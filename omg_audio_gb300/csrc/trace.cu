@@ -512,7 +512,7 @@ __global__ void __launch_bounds__(256, 4) trace_wl_kernel(const DJob* __restrict
   }
 }
 
-// out = (sum + comp) * 2^-64 per float, bins then dirs, per job.
+// out = (sum + comp) * 2^-64 per float: every job's bins, then every job's dirs.
 __global__ void finalize_kernel(const DJob* __restrict__ jobs, uint32_t n_jobs, const float* __restrict__ acc,
                                 float* __restrict__ out) {
   const uint32_t j = blockIdx.y;
@@ -520,12 +520,12 @@ __global__ void finalize_kernel(const DJob* __restrict__ jobs, uint32_t n_jobs, 
   const DJob& J = jobs[j];
   const uint32_t nbb = J.n_bins * J.nb, nd = J.n_bins * 3;
   const float* A = acc + J.acc_off;
-  float* O = out + J.out_off;
+  float *O = out + J.out_off, *D = out + J.dir_off;
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nbb + nd; i += gridDim.x * blockDim.x) {
     float v;
     if (i < nbb) v = A[i] + A[nbb + i];
     else v = A[2 * nbb + (i - nbb)] + A[2 * nbb + nd + (i - nbb)];
-    O[i] = v * kAccUnscale;
+    (i < nbb ? O[i] : D[i - nbb]) = v * kAccUnscale;
   }
 }
 

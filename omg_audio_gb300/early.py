@@ -27,12 +27,15 @@ def _f3(v):
     return np.ascontiguousarray(np.asarray(v, np.float32).reshape(3))
 
 
+_RECORD = np.dtype(_lib.omg_mesh_record)
+
+
 def chains_to_c(chains: Sequence[Chain]):
+    """omg_chain records (three u16 surfaces and the u16 order each)."""
     arr = (_lib.omg_chain * max(1, len(chains)))()
-    for i, (c, o) in enumerate(chains):
-        for k in range(3):
-            arr[i].surf[k] = c[k]
-        arr[i].order = o
+    if len(chains):
+        flat = np.array([v for c, o in chains for v in (c[0], c[1], c[2], o)], np.int64).astype(np.uint16)
+        C.memmove(arr, _p(flat), C.sizeof(_lib.omg_chain) * len(chains))
     return arr
 
 
@@ -64,11 +67,11 @@ class WorldEarly:
     def discover(self, listener, n_rays: int = 768, rot: int = 0, use_boxes: bool = True) -> List[Chain]:
         """mesh_chains: unique chains in the reference's first-found order."""
         cap = 3 * max(n_rays, 1)
-        out = (_lib.omg_chain * cap)()
+        out = np.empty((cap, 4), np.uint16)
         n = C.c_uint32()
         self.ctx._check(lib().omg_early_discover(self.ctx.h, self.id, _p(_f3(listener)), n_rays, rot,
-                                                 int(use_boxes), out, cap, C.byref(n)), "omg_early_discover")
-        return [(tuple(int(v) for v in out[i].surf), int(out[i].order)) for i in range(min(n.value, cap))]
+                                                 int(use_boxes), _p(out), cap, C.byref(n)), "omg_early_discover")
+        return [((a, b, c), o) for a, b, c, o in out[:min(n.value, cap)].tolist()]
 
     def solve(self, sources: Sequence[Tuple[int, Sequence[float]]], chains: Sequence[Chain], listener,
               extras: Sequence = ()):
@@ -78,11 +81,9 @@ class WorldEarly:
         ns, nc = len(sources), len(chains)
         ids = np.array([s[0] for s in sources], np.uint16)
         pos = np.ascontiguousarray(np.array([s[1] for s in sources], np.float32).reshape(-1, 3))
-        ex = (_lib.omg_aabb * max(1, len(extras)))()
-        for i, (mn, mx, tr) in enumerate(extras):
-            for k in range(3):
-                ex[i].mn[k], ex[i].mx[k], ex[i].transmission[k] = mn[k], mx[k], tr[k]
-        out = (_lib.omg_mesh_record * max(1, ns * nc))()
+        ex = np.array([(mn[0], mn[1], mn[2], mx[0], mx[1], mx[2], tr[0], tr[1], tr[2]) for mn, mx, tr in extras]
+                      or [(0.0,) * 9], np.float32)                # omg_aabb records
+        out = np.empty(max(1, ns * nc), _RECORD)   # every record is written by the call
         self.ctx._check(lib().omg_early_solve(self.ctx.h, self.id, _p(ids), _p(pos), ns, chains_to_c(chains), nc,
-                                              _p(_f3(listener)), ex, len(extras), out), "omg_early_solve")
-        return np.ctypeslib.as_array(out)[:ns * nc].copy().reshape(ns, nc)
+                                              _p(_f3(listener)), _p(ex), len(extras), _p(out)), "omg_early_solve")
+        return out[:ns * nc].reshape(ns, nc)

@@ -6,6 +6,8 @@ Every call goes to libomg_cuda.so; nothing here computes a trace on the CPU.
 from __future__ import annotations
 
 import ctypes as C
+import functools
+import struct
 from dataclasses import dataclass
 from typing import Iterable, Optional, Sequence
 
@@ -58,7 +60,48 @@ class TraceConfig:
 Panel = tuple  # (mn[3], mx[3], Material): late.rs:88
 
 
+# Job and panel records are packed a record at a time (struct) instead of a field
+# at a time (ctypes): a material's 17 fields cost some 3 us one by one, most of
+# a large batch's host time. Values that struct refuses but a field assignment
+# takes (an integer out of range, a float beyond f32) go the field way.
+_PACK_ERRORS = (struct.error, OverflowError, TypeError, IndexError, ValueError)
+
+
+def _mat_format(na: int, nt: int) -> str:
+    """omg_material of na absorptions and nt transmissions (the rest zero)."""
+    if na > _lib.MAX_BANDS or nt > _lib.MAX_BANDS:
+        raise IndexError("more bands than omg_material holds")
+    return f"{na}f{4 * (_lib.MAX_BANDS - na)}xf{nt}f{4 * (_lib.MAX_BANDS - nt)}x"
+
+
+@functools.lru_cache(maxsize=64)
+def _panel_struct(na: int, nt: int) -> struct.Struct:
+    return struct.Struct("<6f" + _mat_format(na, nt))
+
+
+@functools.lru_cache(maxsize=64)
+def _job_struct(walls, ne: int) -> struct.Struct:
+    """omg_job; walls: the (na, nt) of the six wall materials, or None for a mesh."""
+    shape = "".join(_mat_format(*w) for w in walls) if walls else f"{6 * C.sizeof(_lib.omg_material)}x"
+    return struct.Struct("<2I3f" + shape + f"6fI{ne}f{4 * (_lib.MAX_BANDS - ne)}x3IfII")
+
+
 def panels_to_c(panels: Sequence[Panel]):
+    n = len(panels)
+    try:
+        buf = bytearray(C.sizeof(_lib.omg_panel) * max(1, n))
+        off, size = 0, C.sizeof(_lib.omg_panel)
+        for mn, mx, m in panels:
+            a, t = m.absorption, m.transmission
+            _panel_struct(len(a), len(t)).pack_into(buf, off, mn[0], mn[1], mn[2], mx[0], mx[1], mx[2], *a, m.scattering,
+                                                    *t)
+            off += size
+        return (_lib.omg_panel * max(1, n)).from_buffer(buf)
+    except _PACK_ERRORS:
+        return _panels_by_field(panels)
+
+
+def _panels_by_field(panels: Sequence[Panel]):
     arr = (_lib.omg_panel * max(1, len(panels)))()
     for i, (mn, mx, m) in enumerate(panels):
         for k in range(3):
@@ -82,6 +125,36 @@ def _reverbs_of(rv, n: int):
     """All n omg_reverb records of a ctypes array as (rt60, level, rt60_fit, segments) arrays, one copy."""
     rec = np.frombuffer(rv, _REVERB_DTYPE, count=n).copy()
     return rec["rt60"], rec["level"], rec["rt60_fit"], rec["segments"].tolist()
+
+
+@functools.lru_cache(maxsize=64)
+def _box_struct(walls, ne: int) -> struct.Struct:
+    return struct.Struct("<3f" + "".join(_mat_format(*w) for w in walls) + f"6fI{ne}f{4 * (_lib.MAX_BANDS - ne)}xI")
+
+
+def _box_job(size, walls, src, lis, n_rays, energy, seed, nb) -> _lib.omg_box_job:
+    j = _lib.omg_box_job()
+    try:
+        six = (walls[0], walls[1], walls[2], walls[3], walls[4], walls[5])
+        e = (1.0,) * nb if energy is None else [energy[b] for b in range(nb)]
+        st = _box_struct(tuple([(len(m.absorption), len(m.transmission)) for m in six]), nb)
+        st.pack_into(j, 0, size[0], size[1], size[2],
+                     *[v for m in six for v in (*m.absorption, m.scattering, *m.transmission)], src[0], src[1], src[2],
+                     lis[0], lis[1], lis[2], n_rays, *e, seed & 0xFFFFFFFF)
+        return j
+    except _PACK_ERRORS:
+        j = _lib.omg_box_job()
+    for k in range(3):
+        j.size[k] = size[k]
+        j.src[k] = src[k]
+        j.lis[k] = lis[k]
+    for w in range(6):
+        j.walls[w] = walls[w].to_c()
+    j.n_rays = n_rays
+    for b in range(nb):
+        j.energy[b] = 1.0 if energy is None else energy[b]
+    j.seed = seed & 0xFFFFFFFF
+    return j
 
 
 class Context:
@@ -159,17 +232,7 @@ class Context:
     def trace_box(self, size, walls: Sequence[Material], src, lis, n_rays: int, energy=None, seed: int = 1):
         """LateBackend::trace (late.rs:28-40): returns (Echogram, ReverbParams)."""
         nb = self.cfg.n_bands
-        j = _lib.omg_box_job()
-        for k in range(3):
-            j.size[k] = size[k]
-            j.src[k] = src[k]
-            j.lis[k] = lis[k]
-        for w in range(6):
-            j.walls[w] = walls[w].to_c()
-        j.n_rays = n_rays
-        for b in range(nb):
-            j.energy[b] = 1.0 if energy is None else energy[b]
-        j.seed = seed & 0xFFFFFFFF
+        j = _box_job(size, walls, src, lis, n_rays, energy, seed, nb)
         e = Echogram(self.cfg.n_bins, nb, self.cfg.bin_dt)
         rv = _lib.omg_reverb()
         self._check(lib().omg_trace_box(self.h, C.byref(j), _p(e.bins), _p(e.dirs), C.byref(rv)), "omg_trace_box")
@@ -312,8 +375,34 @@ class Job:
 
 
 def jobs_to_c(jobs: Sequence[Job], cfg: TraceConfig):
+    """omg_job records of the jobs, and how many floats of bins and directions they return."""
+    nbf = sum(j.bins_len(cfg) * j.bands(cfg) for j in jobs)
+    ndf = sum(j.bins_len(cfg) * 3 for j in jobs)
+    try:
+        size = C.sizeof(_lib.omg_job)
+        buf = bytearray(size * len(jobs))
+        for i, j in enumerate(jobs):
+            nb, s, l = j.bands(cfg), j.src, j.lis
+            e = (1.0,) * nb if j.energy is None else [j.energy[b] for b in range(nb)]
+            if j.scene is not None:
+                shape, head = None, (_lib.GEOM_MESH, j.scene.id, 0.0, 0.0, 0.0)
+                walls = ()
+            else:
+                w, z = j.box_walls, j.box_size
+                six = (w[0], w[1], w[2], w[3], w[4], w[5])
+                shape = tuple([(len(m.absorption), len(m.transmission)) for m in six])
+                head = (_lib.GEOM_BOX, 0, z[0], z[1], z[2])
+                walls = [v for m in six for v in (*m.absorption, m.scattering, *m.transmission)]
+            _job_struct(shape, nb).pack_into(buf, i * size, *head, *walls, s[0], s[1], s[2], l[0], l[1], l[2], j.n_rays,
+                                             *e, j.seed & 0xFFFFFFFF, nb, j.bins_len(cfg), j.max_time, j.panel_offset,
+                                             j.n_panels)
+        return (_lib.omg_job * len(jobs)).from_buffer(buf) if jobs else (_lib.omg_job * 0)(), nbf, ndf
+    except _PACK_ERRORS:
+        return _jobs_by_field(jobs, cfg), nbf, ndf
+
+
+def _jobs_by_field(jobs: Sequence[Job], cfg: TraceConfig):
     arr = (_lib.omg_job * len(jobs))()
-    nbf = ndf = 0
     for i, j in enumerate(jobs):
         c = arr[i]
         nb = j.bands(cfg)
@@ -338,9 +427,7 @@ def jobs_to_c(jobs: Sequence[Job], cfg: TraceConfig):
         c.max_time = j.max_time
         c.panel_offset = j.panel_offset
         c.n_panels = j.n_panels
-        nbf += c.n_bins * nb
-        ndf += c.n_bins * 3
-    return arr, nbf, ndf
+    return arr
 
 
 def split_outputs(jobs, cfg, bins, dirs, rv):

@@ -14,20 +14,17 @@ struct DomeRec {
   uint32_t eye_cap = 0;
   DevBuf<float> ema;          // eye_cap x 9 x nb
   DevBuf<uint32_t> primed;    // eye_cap
-  // per-call scratch
-  DevBuf<float> eyes, tp, raw, dir, energy;
-  DevBuf<uint8_t> esc;
-  DevBuf<DDomePanel> panels;
-  DevBuf<DLaunch> hdr;
-  DevBuf<uint32_t> events;
+  // A sample's inputs (listeners, panels) and its results, one block each on
+  // the device and pinned, one copy each way: [header | events | energies |
+  // directions | raw | escape flags | per-ray throughput], of which the leading
+  // part that the caller wants comes back.
+  DevBuf<unsigned char> d_in, d_out;
+  PinBuf<unsigned char> h_in, h_out;
+  struct Layout {
+    size_t events, energy, dir, raw, esc, tp, end;
+  } at{};
   cudaEvent_t done = nullptr;
   uint64_t last_events[2] = {0, 0};
-  // pinned staging of a submitted sample (inputs up, results down)
-  PinBuf<float> h_eyes, h_energy, h_dir, h_raw, h_tp;
-  PinBuf<uint8_t> h_esc;
-  PinBuf<DDomePanel> h_panels;
-  PinBuf<DLaunch> h_hdr;
-  PinBuf<uint32_t> h_events;
   bool pending = false;
   uint32_t p_eyes = 0, p_rays = 0, p_flags = 0;
   ~DomeRec() {
@@ -83,8 +80,6 @@ int32_t omg_dome_create(omg_ctx* ctx, uint32_t scene_id, const omg_dome_panel* g
   }
   CK(D->fan.alloc(n_fan));
   CK(build_dome_fan(D->fan.p, n_fan, ctx->stream));
-  CK(D->hdr.alloc(1));
-  CK(D->events.alloc(2));
   CK(cudaEventCreateWithFlags(&D->done, cudaEventDisableTiming));
   CK(cudaStreamSynchronize(ctx->stream));
   *probe_id = ctx->next_probe++;
@@ -153,38 +148,29 @@ int32_t dome_submit(omg_ctx* ctx, DomeRec& D, const float* eyes, uint32_t n_eyes
     D.eye_cap = cap;
   }
   const uint64_t nr = (uint64_t)n_eyes * n_rays;
-  if (D.eyes.n < 3ull * n_eyes) {
-    CK(D.eyes.alloc(3ull * n_eyes));
-    CK(D.h_eyes.alloc(3ull * n_eyes));
+  auto pad = [](size_t bytes) { return (bytes + 15u) & ~(size_t)15u; };
+  const size_t o_pan = pad(12ull * n_eyes), in_bytes = o_pan + pans.size() * sizeof(DDomePanel);
+  if (D.d_in.n < in_bytes) {
+    CK(D.d_in.alloc(in_bytes));
+    CK(D.h_in.alloc(in_bytes));
   }
-  if (D.tp.n < nr * nb) CK(D.tp.alloc(nr * nb));
-  if (D.esc.n < nr) CK(D.esc.alloc(nr));
-  if (D.raw.n < 9ull * nb * n_eyes) {
-    CK(D.raw.alloc(9ull * nb * n_eyes));
-    CK(D.energy.alloc(9ull * nb * n_eyes));
-    CK(D.dir.alloc(27ull * n_eyes));
-    CK(D.h_raw.alloc(9ull * nb * n_eyes));
-    CK(D.h_energy.alloc(9ull * nb * n_eyes));
-    CK(D.h_dir.alloc(27ull * n_eyes));
-  }
-  if ((flags & kWantEscape) && D.h_esc.n < nr) CK(D.h_esc.alloc(nr));
-  if ((flags & kWantTp) && D.h_tp.n < nr * nb) CK(D.h_tp.alloc(nr * nb));
-  if (D.panels.n < pans.size()) {
-    CK(D.panels.alloc(pans.size()));
-    CK(D.h_panels.alloc(pans.size()));
-  }
-  if (!D.h_hdr.p) {
-    CK(D.h_hdr.alloc(1));
-    CK(D.h_events.alloc(2));
-  }
-  std::memcpy(D.h_eyes.p, eyes, 12ull * n_eyes);
-  CK(cudaMemcpyAsync(D.eyes.p, D.h_eyes.p, 12ull * n_eyes, cudaMemcpyHostToDevice, s));
-  if (!pans.empty()) {
-    std::memcpy(D.h_panels.p, pans.data(), pans.size() * sizeof(DDomePanel));
-    CK(cudaMemcpyAsync(D.panels.p, D.h_panels.p, pans.size() * sizeof(DDomePanel), cudaMemcpyHostToDevice, s));
-  }
-  CK(cudaMemsetAsync(D.hdr.p, 0, sizeof(DLaunch), s));
-  CK(cudaMemsetAsync(D.events.p, 0, 8, s));
+  DomeRec::Layout at;
+  at.events = pad(sizeof(DLaunch));
+  at.energy = at.events + pad(2 * sizeof(uint32_t));
+  at.dir = at.energy + pad(9ull * nb * n_eyes * 4);
+  at.raw = at.dir + pad(27ull * n_eyes * 4);
+  at.esc = at.raw + pad(9ull * nb * n_eyes * 4);
+  at.tp = at.esc + pad(nr);
+  at.end = at.tp + nr * nb * 4;
+  const size_t back = (flags & kWantTp) ? at.end : (flags & kWantEscape) ? at.tp : (flags & kWantRaw) ? at.esc : at.raw;
+  if (D.d_out.n < at.end) CK(D.d_out.alloc(at.end));
+  if (D.h_out.n < back) CK(D.h_out.alloc(back));
+  D.at = at;
+  std::memcpy(D.h_in.p, eyes, 12ull * n_eyes);
+  if (!pans.empty()) std::memcpy(D.h_in.p + o_pan, pans.data(), pans.size() * sizeof(DDomePanel));
+  CK(cudaMemcpyAsync(D.d_in.p, D.h_in.p, in_bytes, cudaMemcpyHostToDevice, s));
+  CK(cudaMemsetAsync(D.d_out.p, 0, at.energy, s));   // the header and the event counters
+  unsigned char* out = D.d_out.p;
   DDomeLaunch L;
   std::memset(&L, 0, sizeof(L));
   L.scene = ctx->d_scenes.p + D.scene_id;
@@ -193,30 +179,25 @@ int32_t dome_submit(omg_ctx* ctx, DomeRec& D, const float* eyes, uint32_t n_eyes
   L.n_rays = n_rays;
   L.max_events = max_events;
   L.nb = nb;
-  L.panels = D.panels.p;
+  L.panels = reinterpret_cast<const DDomePanel*>(D.d_in.p + o_pan);
   L.n_glass = (uint32_t)D.glass.size();
   L.n_panels = (uint32_t)pans.size();
-  L.eyes = D.eyes.p;
+  L.eyes = reinterpret_cast<const float*>(D.d_in.p);
   L.n_eyes = n_eyes;
-  L.ray_tp = D.tp.p;
-  L.ray_escape = D.esc.p;
+  L.ray_tp = reinterpret_cast<float*>(out + at.tp);
+  L.ray_escape = out + at.esc;
   L.ema = D.ema.p;
   L.primed = D.primed.p;
-  L.raw = D.raw.p;
-  L.out_dir = D.dir.p;
-  L.out_energy = D.energy.p;
-  L.hdr = D.hdr.p;
-  L.events = D.events.p;
+  L.raw = reinterpret_cast<float*>(out + at.raw);
+  L.out_dir = reinterpret_cast<float*>(out + at.dir);
+  L.out_energy = reinterpret_cast<float*>(out + at.energy);
+  L.hdr = reinterpret_cast<DLaunch*>(out);
+  L.events = reinterpret_cast<uint32_t*>(out + at.events);
   L.tie = ctx->prm.tie_mode;
   L.wt = ctx->prm.tri_test == OMG_TRI_WATERTIGHT ? 1u : 0u;
+  L.n_sms = (uint32_t)ctx->n_sms;
   CK(launch_dome(L, s));
-  CK(cudaMemcpyAsync(D.h_energy.p, D.energy.p, 9ull * nb * n_eyes * 4, cudaMemcpyDeviceToHost, s));
-  CK(cudaMemcpyAsync(D.h_dir.p, D.dir.p, 27ull * n_eyes * 4, cudaMemcpyDeviceToHost, s));
-  if (flags & kWantRaw) CK(cudaMemcpyAsync(D.h_raw.p, D.raw.p, 9ull * nb * n_eyes * 4, cudaMemcpyDeviceToHost, s));
-  if (flags & kWantEscape) CK(cudaMemcpyAsync(D.h_esc.p, D.esc.p, nr, cudaMemcpyDeviceToHost, s));
-  if (flags & kWantTp) CK(cudaMemcpyAsync(D.h_tp.p, D.tp.p, nr * nb * 4, cudaMemcpyDeviceToHost, s));
-  CK(cudaMemcpyAsync(D.h_hdr.p, D.hdr.p, sizeof(DLaunch), cudaMemcpyDeviceToHost, s));
-  CK(cudaMemcpyAsync(D.h_events.p, D.events.p, 8, cudaMemcpyDeviceToHost, s));
+  CK(cudaMemcpyAsync(D.h_out.p, out, back, cudaMemcpyDeviceToHost, s));
   CK(cudaEventRecord(D.done, s));
   D.pending = true;
   D.p_eyes = n_eyes;
@@ -237,25 +218,29 @@ int32_t dome_collect(omg_ctx* ctx, DomeRec& D, omg_dome_bin* out, float* raw_ene
   D.pending = false;
   const uint32_t nb = D.nb, n_eyes = D.p_eyes;
   const uint64_t nr = (uint64_t)n_eyes * D.p_rays;
-  ctx->last_flags = D.h_hdr.p->error;
-  if (D.h_hdr.p->error) {
-    ctx->last_error = (D.h_hdr.p->error & 2u) ? "dome: too many crossings on one straight-through segment"
-                                              : "dome: traversal stack overflow";
+  const unsigned char* res = D.h_out.p;
+  const DomeRec::Layout& at = D.at;
+  const uint32_t error = reinterpret_cast<const DLaunch*>(res)->error;
+  ctx->last_flags = error;
+  if (error) {
+    ctx->last_error = (error & 2u) ? "dome: too many crossings on one straight-through segment"
+                                   : "dome: traversal stack overflow";
     return OMG_E_OVERFLOW;
   }
-  D.last_events[0] = D.h_events.p[0];
-  D.last_events[1] = D.h_events.p[1];
+  D.last_events[0] = reinterpret_cast<const uint32_t*>(res + at.events)[0];
+  D.last_events[1] = reinterpret_cast<const uint32_t*>(res + at.events)[1];
+  const float *dir = reinterpret_cast<const float*>(res + at.dir), *energy = reinterpret_cast<const float*>(res + at.energy);
   if (out)
     for (uint32_t e = 0; e < n_eyes; e++)
       for (uint32_t k = 0; k < 9; k++) {
         omg_dome_bin& o = out[e * 9 + k];
         std::memset(&o, 0, sizeof(o));
-        for (int c = 0; c < 3; c++) o.dir[c] = D.h_dir.p[(e * 9 + k) * 3 + c];
-        for (uint32_t b = 0; b < nb; b++) o.energy[b] = D.h_energy.p[(e * 9 + k) * nb + b];
+        for (int c = 0; c < 3; c++) o.dir[c] = dir[(e * 9 + k) * 3 + c];
+        for (uint32_t b = 0; b < nb; b++) o.energy[b] = energy[(e * 9 + k) * nb + b];
       }
-  if (raw_energy && (D.p_flags & kWantRaw)) std::memcpy(raw_energy, D.h_raw.p, 9ull * nb * n_eyes * 4);
-  if (escape && (D.p_flags & kWantEscape)) std::memcpy(escape, D.h_esc.p, nr);
-  if (ray_tp && (D.p_flags & kWantTp)) std::memcpy(ray_tp, D.h_tp.p, nr * nb * 4);
+  if (raw_energy && (D.p_flags & kWantRaw)) std::memcpy(raw_energy, res + at.raw, 9ull * nb * n_eyes * 4);
+  if (escape && (D.p_flags & kWantEscape)) std::memcpy(escape, res + at.esc, nr);
+  if (ray_tp && (D.p_flags & kWantTp)) std::memcpy(ray_tp, res + at.tp, nr * nb * 4);
   return OMG_OK;
 }
 

@@ -16,6 +16,7 @@ namespace omg {
 namespace {
 
 constexpr float PI_F = 3.14159265358979323846f;
+constexpr uint32_t kEscBlocks = 7;   // escape blocks a multiprocessor (28 warps, 72 registers)
 constexpr uint32_t kMaxCross = 64;   // crossings kept per straight-through segment
 
 // dome.rs:56-68
@@ -43,23 +44,36 @@ struct EscapeRay {
   uint32_t ev;
 };
 
-// One event of trace_escape (dome.rs:336-381) after its closest-hit walk:
-// mesh hit (mh, tm, prim) or none. Returns 0 when the ray goes on (the next
+// The nearest pane or leaf that a ray crosses before t_max (the first one of
+// equal distances; -1: none), one panel a lane (every lane calls this with the
+// same ray).
+__device__ __forceinline__ int warp_panels(const DDomeLaunch& L, float ox, float oy, float oz, float dx, float dy,
+                                           float dz, float t_max, float& tout) {
+  constexpr unsigned FULL = 0xffffffffu;
+  float bt = t_max;
+  int bi = 0x7FFFFFFF;
+  for (uint32_t k = threadIdx.x & 31u; k < L.n_panels; k += 32u) {
+    float t;
+    if (panel_hit(L.panels[k], ox, oy, oz, dx, dy, dz, bt, t)) {
+      bt = t;
+      bi = (int)k;
+    }
+  }
+  __syncwarp();
+  const uint32_t tb = __reduce_min_sync(FULL, bi != 0x7FFFFFFF ? __float_as_uint(bt) : 0x7f800000u);
+  const int i = __reduce_min_sync(FULL, bi != 0x7FFFFFFF && __float_as_uint(bt) == tb ? bi : 0x7FFFFFFF);
+  tout = __uint_as_float(tb);
+  return i == 0x7FFFFFFF ? -1 : i;
+}
+
+// One event of trace_escape (dome.rs:336-381) after its closest-hit walk: mesh
+// hit (mh, tm, prim) or none, and the nearest panel before it (pan at t_pan, or
+// -1). Returns 0 when the ray goes on (the next
 // walk starts from its new position), 1 when it escaped, 2 when it ends
 // without escaping. The same f32 operations as trace_escape.
 __device__ __forceinline__ int escape_event(const DScene& S, const DDomeLaunch& L, EscapeRay& r, bool mh, float tm,
-                                            int prim) {
+                                            int prim, int pan, float t_pan) {
   const uint32_t nb = L.nb;
-  const float t_mesh = mh ? tm : FLT_MAX;
-  float t_pan = t_mesh;
-  int pan = -1;
-  for (uint32_t k = 0; k < L.n_panels; k++) {
-    float t;
-    if (panel_hit(L.panels[k], r.px, r.py, r.pz, r.dx, r.dy, r.dz, t_pan, t)) {
-      t_pan = t;
-      pan = (int)k;
-    }
-  }
   if (pan >= 0) {
     const DDomePanel& P = L.panels[pan];
     if (!P.glass) return 2;  // a door leaf blocks
@@ -99,44 +113,28 @@ __device__ __forceinline__ int escape_event(const DScene& S, const DDomeLaunch& 
   return 0;
 }
 
-// dome.rs:328-382 under the reference's first-found rule (tie_mode 0): each
-// event's closest hit by the reference's ordered walk. Returns true (escaped)
-// with the throughput in tp.
-__device__ bool trace_escape(const DScene& S, const DDomeLaunch& L, float px, float py, float pz, float dx, float dy,
-                             float dz, float tp[MAXB], uint32_t& events) {
-  EscapeRay r{px, py, pz, dx, dy, dz, {}, 0u};
-#pragma unroll
-  for (int b = 0; b < MAXB; b++) r.tp[b] = 1.0f;
-  int e = 2;
-  for (uint32_t ev = 0; ev < L.max_events; ev++) {
-    events++;
-    float tm = FLT_MAX;
-    int prim = 0;
-    const bool mh = mesh_closest<false>(S, r.px, r.py, r.pz, r.dx, r.dy, r.dz, tm, prim, &L.hdr->error);
-    e = escape_event(S, L, r, mh, tm, prim);
-    if (e != 0) break;
-  }
-#pragma unroll
-  for (int b = 0; b < MAXB; b++) tp[b] = r.tp[b];
-  return e == 1;
-}
-
-// The specular escape of every (listener, fan ray) under the near-tie rule,
-// one lane each, with the persistent tracer's walk: the node phase lane by
-// lane (walk_nodes, the grown binary boxes), then the pending leaves
-// tested by the whole warp (coop_leaf_rounds). The closest hit under this
-// rule does not depend on the walk, so each event sees the hit
-// any other near-tie walk finds; the events follow in trace_escape's f32 operations. Lanes
-// past the last ray take part in the warp's leaf rounds only.
+// The specular escape of every (listener, fan ray), one lane each, with the
+// persistent tracer's walk: the node phase lane by lane (walk_nodes), then the
+// pending leaves tested by the whole warp (coop_leaf_rounds); each event's hit
+// is the one any other walk under the context's rule finds, and the events
+// follow in the reference's f32 operations (dome.rs:328-382). Lanes from
+// rays_per_warp on, and past the last ray, take part in the warp's leaf rounds
+// only. A fan of 64 listeners has 32,768 rays, 1024 full warps on 152
+// multiprocessors, each waiting on its own loads and on its lanes' divergent
+// paths one after another; launch_dome therefore spreads the rays over the
+// warps that the chip holds.
 constexpr uint32_t kEscThreads = 128;
-template <bool WT>
-__global__ void __launch_bounds__(kEscThreads) dome_escape_walk_kernel(DDomeLaunch L, uint32_t loop_guard) {
+template <bool TIE, bool WT>
+__global__ void __launch_bounds__(kEscThreads, kEscBlocks) dome_escape_walk_kernel(DDomeLaunch L, uint32_t loop_guard,
+                                                                                   uint32_t rays_per_warp) {
   __shared__ uint8_t s_slots[kEscThreads / 32][256];
-  const uint32_t gid = blockIdx.x * blockDim.x + threadIdx.x;
-  const uint32_t total = L.n_eyes * L.n_rays;
+  const uint32_t total = L.n_eyes * L.n_rays, lane = threadIdx.x & 31u;
+  const uint32_t gid = lane < rays_per_warp
+                           ? ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * rays_per_warp + lane
+                           : 0xFFFFFFFFu;
   const DScene& S = *L.scene;
   uint32_t* err = &L.hdr->error;
-  EscapeRay r;
+  EscapeRay r{};
   int walk_stack_ref[STACK_DEPTH];
   float walk_stack_t[STACK_DEPTH];
   Walk w;
@@ -144,6 +142,8 @@ __global__ void __launch_bounds__(kEscThreads) dome_escape_walk_kernel(DDomeLaun
   w.stack_t = walk_stack_t;
   w.cur = kDone;
   w.leaf = 0;
+  w.prim_best = -1;
+  w.t_best = FLT_MAX;
   bool active = gid < total && L.max_events > 0;
   int status = 2;
   uint32_t events = 0;
@@ -156,40 +156,66 @@ __global__ void __launch_bounds__(kEscThreads) dome_escape_walk_kernel(DDomeLaun
 #pragma unroll
     for (int b = 0; b < MAXB; b++) r.tp[b] = 1.0f;
     r.ev = 0;
-    if (active) {
-      walk_begin<true>(w, S, r.px, r.py, r.pz, r.dx, r.dy, r.dz, false);
+  }
+  constexpr unsigned FULL = 0xffffffffu;
+  uint32_t iters = 0;
+  while (__any_sync(FULL, active)) {
+    // the closest hits of every lane's event, then the events together
+    bool walking = active;
+    if (walking) {
+      walk_begin<TIE>(w, S, r.px, r.py, r.pz, r.dx, r.dy, r.dz, false);
       events++;
     }
-  }
-  uint32_t iters = 0;
-  while (__any_sync(0xffffffffu, active)) {
-    if (++iters > loop_guard) {
+    while (__any_sync(FULL, walking) && ++iters <= loop_guard) {
+      bool over = false;
+      if (walking) {
+        int st = 1 << 30;   // the node phase runs until the warp's lanes hold leaves (bounded by the walk budget)
+        over = walk_nodes<TIE>(w, S, r.px, r.py, r.pz, st, err);
+      }
+      coop_leaf_rounds<TIE, WT>(w, walking && !over, WT ? S.prims_wt : S.prims, r.px, r.py, r.pz, r.dx, r.dy, r.dz,
+                                s_slots[threadIdx.x >> 5], kCoopRounds, err);
+      if (walking && !over && w.cur == kDone && w.leaf == 0)
+        over = !TIE || !walk_restart_fixed(w, S.root, S.walk_budget);
+      if (over) walking = false;
+    }
+    if (iters > loop_guard) {
       atomicOr(err, 8u);
-      active = false;
       break;
     }
-    bool over = false;
-    if (active) {
-      int st = 1 << 30;   // the node phase runs until the warp's lanes hold leaves (bounded by the walk budget)
-      over = walk_nodes<true>(w, S, r.px, r.py, r.pz, st, err);
-    }
-    coop_leaf_rounds<true, WT>(w, active && !over, WT ? S.prims_wt : S.prims, r.px, r.py, r.pz, r.dx, r.dy, r.dz,
-                               s_slots[threadIdx.x >> 5], kCoopRounds, err);
-    if (active) {
-      if (!over && w.cur == kDone && w.leaf == 0) over = !walk_restart_fixed(w, S.root, S.walk_budget);
-      if (over) {
-        const int e = escape_event(S, L, r, walk_have(w), w.t_best, w.prim_best);
-        r.ev++;
-        if (e != 0) {
-          status = e;
-          active = false;
-        } else if (r.ev >= L.max_events) {
-          status = 2;
-          active = false;
-        } else {
-          walk_begin<true>(w, S, r.px, r.py, r.pz, r.dx, r.dy, r.dz, false);
-          events++;
+    // the panels: each lane its own ray against all of them, or, for few rays,
+    // the whole warp on one ray at a time (80 instructions a ray against 25 a panel)
+    int pan = -1;
+    const float t_mesh = w.prim_best >= 0 ? w.t_best : FLT_MAX;
+    float t_pan = t_mesh;
+    unsigned rays = __ballot_sync(FULL, active);
+    if (3u * (uint32_t)__popc(rays) <= L.n_panels) {
+      while (rays) {
+        const int o = __ffs((int)rays) - 1;
+        rays &= rays - 1u;
+        float t;
+        const int k = warp_panels(L, __shfl_sync(FULL, r.px, o), __shfl_sync(FULL, r.py, o),
+                                  __shfl_sync(FULL, r.pz, o), __shfl_sync(FULL, r.dx, o), __shfl_sync(FULL, r.dy, o),
+                                  __shfl_sync(FULL, r.dz, o), __shfl_sync(FULL, t_mesh, o), t);
+        if ((int)lane == o) {
+          pan = k;
+          t_pan = t;
         }
+      }
+    } else if (active) {
+      for (uint32_t k = 0; k < L.n_panels; k++) {
+        float t;
+        if (panel_hit(L.panels[k], r.px, r.py, r.pz, r.dx, r.dy, r.dz, t_pan, t)) {
+          t_pan = t;
+          pan = (int)k;
+        }
+      }
+    }
+    if (active) {
+      const int e = escape_event(S, L, r, walk_have(w), w.t_best, w.prim_best, pan, t_pan);
+      r.ev++;
+      if (e != 0 || r.ev >= L.max_events) {
+        status = e != 0 ? e : 2;
+        active = false;
       }
     }
   }
@@ -401,35 +427,20 @@ __device__ void through_warp(const DScene& S, const DDomeLaunch& L, ThroughSmem&
     for (int b = 0; b < MAXB; b++) tp[b] = 0.0f;
     return;
   }
-  for (uint32_t k = 0; k < L.n_panels; k++) {
+  // the panels one a lane, then the crossed ones' transmissions in order
+  for (uint32_t k0 = 0; k0 < L.n_panels; k0 += 32u) {
+    const uint32_t k = k0 + lane;
     float t;
-    if (panel_hit(L.panels[k], ex, ey, ez, dx, dy, dz, 80.0f, t)) {
+    unsigned crossed =
+        __ballot_sync(FULL, k < L.n_panels && panel_hit(L.panels[k], ex, ey, ez, dx, dy, dz, 80.0f, t));
+    while (crossed) {
+      const DDomePanel& P = L.panels[k0 + (uint32_t)__ffs((int)crossed) - 1u];
+      crossed &= crossed - 1u;
 #pragma unroll
       for (int b = 0; b < MAXB; b++)
-        if ((uint32_t)b < nb) tp[b] = tp[b] * L.panels[k].t2[b];
+        if ((uint32_t)b < nb) tp[b] = tp[b] * P.t2[b];
     }
   }
-}
-
-// The specular escape of every (listener, fan ray) under the first-found
-// rule, one thread each: its transmission goes to ray_tp and its escape flag
-// to ray_escape; the straight-through kernel then completes the rays that
-// need it.
-__global__ void dome_escape_kernel(DDomeLaunch L) {
-  const uint32_t gid = blockIdx.x * blockDim.x + threadIdx.x;
-  if (gid >= L.n_eyes * L.n_rays) return;
-  const uint32_t eye = gid / L.n_rays, j = gid % L.n_rays;
-  const DScene S = *L.scene;
-  const uint32_t i = (uint32_t)((uint64_t)j * L.n_fan / L.n_rays);  // dome.rs:434
-  const float4 f = L.fan[i];
-  const float ex = L.eyes[3 * eye], ey = L.eyes[3 * eye + 1], ez = L.eyes[3 * eye + 2];
-  float bp[MAXB];
-  uint32_t events = 0;
-  const bool esc = trace_escape(S, L, ex, ey, ez, f.x, f.y, f.z, bp, events);
-  float* o = L.ray_tp + (uint64_t)gid * L.nb;
-  for (uint32_t b = 0; b < L.nb; b++) o[b] = bp[b];
-  L.ray_escape[gid] = esc ? 1 : 0;
-  atomicAdd(&L.events[0], events);
 }
 
 // dome.rs:432-446 per ray: a near-full escape stands; otherwise the
@@ -589,14 +600,20 @@ cudaError_t build_dome_fan(float4* fan, uint32_t n, cudaStream_t s) {
 cudaError_t launch_dome(const DDomeLaunch& L, cudaStream_t s) {
   const uint64_t total = (uint64_t)L.n_eyes * L.n_rays;
   if (total == 0) return cudaSuccess;
+  // rays a warp: as few as fill half of the warps that the chip holds. 64
+  // listeners (32,768 rays, 16 a warp): 427 us a call, against 439 at 8 and 453
+  // at 32; 16 listeners 251 us against 376 with full warps
+  const uint64_t warps = (uint64_t)L.n_sms * kEscBlocks * (kEscThreads / 32) / 2u;
+  uint32_t rpw = 32;
+  while (rpw > 1 && total <= warps * (rpw / 2u)) rpw >>= 1;
+  const uint32_t per_block = rpw * (kEscThreads / 32);
+  const uint32_t blocks = (uint32_t)((total + per_block - 1) / per_block);
   if (L.tie && L.wt)
-    dome_escape_walk_kernel<true><<<(uint32_t)((total + kEscThreads - 1) / kEscThreads), kEscThreads, 0, s>>>(
-        L, kDefaultLoopGuard);
+    dome_escape_walk_kernel<true, true><<<blocks, kEscThreads, 0, s>>>(L, kDefaultLoopGuard, rpw);
   else if (L.tie)
-    dome_escape_walk_kernel<false><<<(uint32_t)((total + kEscThreads - 1) / kEscThreads), kEscThreads, 0, s>>>(
-        L, kDefaultLoopGuard);
+    dome_escape_walk_kernel<true, false><<<blocks, kEscThreads, 0, s>>>(L, kDefaultLoopGuard, rpw);
   else
-    dome_escape_kernel<<<(uint32_t)((total + 127) / 128), 128, 0, s>>>(L);
+    dome_escape_walk_kernel<false, false><<<blocks, kEscThreads, 0, s>>>(L, kDefaultLoopGuard, rpw);
   dome_through_kernel<<<(uint32_t)((total + kThroughWarps - 1) / kThroughWarps), 32 * kThroughWarps, 0, s>>>(L);
   dome_bins_kernel<<<L.n_eyes, kDomeBinThreads, 0, s>>>(L, 0.35f);
   return cudaGetLastError();

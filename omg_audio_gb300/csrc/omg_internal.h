@@ -374,6 +374,7 @@ struct DDomeLaunch {
   uint32_t* events;           // escape events + through calls (2 counters)
   uint32_t tie;               // near-tie rule of the escape raycasts (omg_params.tie_mode)
   uint32_t wt;                // the scene carries exact vertices (watertight test)
+  uint32_t n_sms;
 };
 cudaError_t launch_dome(const DDomeLaunch& L, cudaStream_t s);
 

@@ -580,9 +580,9 @@ class DomeProbe:
         n_rays = n_rays or self.n_fan
         nb = self.nb
         out = (_lib.omg_dome_bin * (9 * n_eyes))()
-        raw = np.zeros((n_eyes, 9, nb), np.float32)
-        esc = np.zeros((n_eyes, n_rays), np.uint8)
-        tp = np.zeros((n_eyes, n_rays, nb), np.float32)
+        raw = np.empty((n_eyes, 9, nb), np.float32)       # every value is written by the call
+        esc = np.empty((n_eyes, n_rays), np.uint8)
+        tp = np.empty((n_eyes, n_rays, nb), np.float32)
         arr = dome_panels_to_c(leaves, nb)
         rc = lib().omg_dome_sample(self.ctx.h, self.id, _p(eyes), n_eyes, arr, len(leaves), n_rays, max_events, out,
                                    _p(raw), _p(esc), _p(tp))

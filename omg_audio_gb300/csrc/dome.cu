@@ -1,6 +1,6 @@
 // Ambient-dome fan on the GPU (crates/omg-scene/src/dome.rs:293-478).
 //
-// One thread per (listener, fan ray) traces the specular escape
+// One lane per (listener, fan ray) traces the specular escape
 // (trace_escape, dome.rs:330-382: <= max_events mesh hits or pane crossings,
 // 80 m horizon); one warp per ray then adds, when the escape is not
 // near-full, the straight-through mass-law seep (trace_through,
@@ -38,9 +38,10 @@ __device__ __forceinline__ bool panel_hit(const DDomePanel& p, float ox, float o
 // The escape of one fan ray as a state machine around its closest-hit walks
 // (trace_escape, one event at a time): the ray's position, direction and
 // throughput, and how many events it has taken.
+template <int NB>
 struct EscapeRay {
   float px, py, pz, dx, dy, dz;
-  float tp[MAXB];
+  float tp[NB];
   uint32_t ev;
 };
 
@@ -71,14 +72,15 @@ __device__ __forceinline__ int warp_panels(const DDomeLaunch& L, float ox, float
 // -1). Returns 0 when the ray goes on (the next
 // walk starts from its new position), 1 when it escaped, 2 when it ends
 // without escaping. The same f32 operations as trace_escape.
-__device__ __forceinline__ int escape_event(const DScene& S, const DDomeLaunch& L, EscapeRay& r, bool mh, float tm,
+template <int NB>
+__device__ __forceinline__ int escape_event(const DScene& S, const DDomeLaunch& L, EscapeRay<NB>& r, bool mh, float tm,
                                             int prim, int pan, float t_pan) {
   const uint32_t nb = L.nb;
   if (pan >= 0) {
     const DDomePanel& P = L.panels[pan];
     if (!P.glass) return 2;  // a door leaf blocks
 #pragma unroll
-    for (int b = 0; b < MAXB; b++)
+    for (int b = 0; b < NB; b++)
       if ((uint32_t)b < nb) r.tp[b] = r.tp[b] * P.t2[b];
     const float adv = t_pan + 1e-3f;
     r.px = r.px + r.dx * adv;
@@ -93,7 +95,7 @@ __device__ __forceinline__ int escape_event(const DScene& S, const DDomeLaunch& 
   const float4 p1 = __ldg(S.prims + 3 * prim + 1);
   const DMat& M = S.mats[__float_as_uint(p0.w)];
 #pragma unroll
-  for (int b = 0; b < MAXB; b++)
+  for (int b = 0; b < NB; b++)
     if ((uint32_t)b < nb) r.tp[b] = r.tp[b] * (1.0f - M.absorption[b]);
   if (r.tp[1] < 2e-3f) return 2;
   const float4 nn = __ldg(S.normals + __float_as_uint(p1.w));
@@ -124,7 +126,7 @@ __device__ __forceinline__ int escape_event(const DScene& S, const DDomeLaunch& 
 // paths one after another; launch_dome therefore spreads the rays over the
 // warps that the chip holds.
 constexpr uint32_t kEscThreads = 128;
-template <bool TIE, bool WT>
+template <int NB, bool TIE, bool WT>
 __global__ void __launch_bounds__(kEscThreads, kEscBlocks) dome_escape_walk_kernel(DDomeLaunch L, uint32_t loop_guard,
                                                                                    uint32_t rays_per_warp) {
   __shared__ uint8_t s_slots[kEscThreads / 32][256];
@@ -134,7 +136,7 @@ __global__ void __launch_bounds__(kEscThreads, kEscBlocks) dome_escape_walk_kern
                            : 0xFFFFFFFFu;
   const DScene& S = *L.scene;
   uint32_t* err = &L.hdr->error;
-  EscapeRay r{};
+  EscapeRay<NB> r{};
   int walk_stack_ref[STACK_DEPTH];
   float walk_stack_t[STACK_DEPTH];
   Walk w;
@@ -154,7 +156,7 @@ __global__ void __launch_bounds__(kEscThreads, kEscBlocks) dome_escape_walk_kern
     r.px = L.eyes[3 * eye]; r.py = L.eyes[3 * eye + 1]; r.pz = L.eyes[3 * eye + 2];
     r.dx = f.x; r.dy = f.y; r.dz = f.z;
 #pragma unroll
-    for (int b = 0; b < MAXB; b++) r.tp[b] = 1.0f;
+    for (int b = 0; b < NB; b++) r.tp[b] = 1.0f;
     r.ev = 0;
   }
   constexpr unsigned FULL = 0xffffffffu;
@@ -221,7 +223,9 @@ __global__ void __launch_bounds__(kEscThreads, kEscBlocks) dome_escape_walk_kern
   }
   if (gid < total) {
     float* o = L.ray_tp + (uint64_t)gid * L.nb;
-    for (uint32_t b = 0; b < L.nb; b++) o[b] = r.tp[b];
+#pragma unroll
+    for (int b = 0; b < NB; b++)
+      if ((uint32_t)b < L.nb) o[b] = r.tp[b];
     L.ray_escape[gid] = status == 1 ? 1 : 0;
     atomicAdd(&L.events[0], events);
   }
@@ -229,11 +233,14 @@ __global__ void __launch_bounds__(kEscThreads, kEscBlocks) dome_escape_walk_kern
 
 // One warp's shared memory for the straight-through segment of one fan ray.
 constexpr uint32_t kThroughWarps = 4;        // rays (warps) per block
-constexpr uint32_t kWarpStack = 512;         // pending node refs of one warp's walk
+constexpr uint32_t kWarpStack = 512;         // pending nodes of one warp's walk
+constexpr uint32_t kWarpLeaves = 72;         // pending leaves (fewer than 8, and a round's 64 children)
 constexpr uint32_t kMaxThroughRounds = 1u << 20;
 struct ThroughSmem {
   int ref[kWarpStack];
+  int lref[kWarpLeaves];
   unsigned long long key[kWarpStack];        // the ref's depth-first position (below)
+  unsigned long long lkey[kWarpLeaves];
   float t[kMaxCross];                        // crossings as found
   uint32_t prim[kMaxCross];
   unsigned long long ckey[kMaxCross];
@@ -245,9 +252,11 @@ struct ThroughSmem {
 // Straight-through seep of one fan ray (trace_through, dome.rs:390-422) by a
 // whole warp. The crossings of the 50 m segment (segment_hits,
 // mesh.rs:546-604) are collected by a walk in which every lane takes one
-// pending ref per round (children whose box the segment meets are pushed
-// warp-aggregated, leaves test their primitives), so the any-hit walk, which
-// visits every node the segment meets, runs 32 nodes wide instead of one.
+// pending node per round (children whose box the segment meets are pushed
+// warp-aggregated), so the any-hit walk, which visits every node the segment
+// meets, runs 32 nodes wide instead of one. Leaves wait in a list of their own
+// and are tested eight at a time, four lanes each: a lane that met a leaf among
+// the nodes tested its primitives alone, in nearly every round.
 //
 // The reference sorts the crossings by t with a stable sort over its
 // depth-first visiting order (child b before child a) and then merges
@@ -282,18 +291,50 @@ __device__ void through_warp(const DScene& S, const DDomeLaunch& L, ThroughSmem&
       sy = sy * il;
       sz = sz * il;
       const float ix = __frcp_rn(sx), iy = __frcp_rn(sy), iz = __frcp_rn(sz);
+      const float kTiny = 8.673617379884035e-19f;   // 2^-60: no product of the slab test is a NaN
+      const bool fast = fabsf(sx) >= kTiny && fabsf(sy) >= kTiny && fabsf(sz) >= kTiny;
+      uint32_t sp = S.root >= 0 ? 1u : 0u, nl = 1u - sp, rounds = 0;
       if (lane == 0) {
-        W.ref[0] = S.root;
-        W.key[0] = 0ull;
+        (sp ? W.ref : W.lref)[0] = S.root;
+        (sp ? W.key : W.lkey)[0] = 0ull;
         W.n = 0u;
       }
       __syncwarp();
-      uint32_t sp = 1, rounds = 0;
-      while (sp > 0) {
+      while ((sp | nl) != 0u) {
         if (++rounds > kMaxThroughRounds) {
           fail |= 1u;
           break;
         }
+        if (nl >= 8u || sp == 0u) {
+          // ---- up to 8 leaves, four lanes each
+          const uint32_t take = nl < 8u ? nl : 8u, g = lane >> 2;
+          nl -= take;
+          const bool act = g < take;
+          const uint32_t code = act ? ~(uint32_t)W.lref[nl + g] : 0u;
+          const uint32_t start = code >> 3, cnt = act ? (code & 7u) + 1u : 0u;
+          for (uint32_t k = lane & 3u; __any_sync(FULL, k < cnt); k += 4u) {
+            if (k >= cnt) continue;
+            const uint32_t i = start + k;
+            const float4 p0 = __ldg(S.prims + 3 * i + 0);
+            const float4 p1 = __ldg(S.prims + 3 * i + 1);
+            const float4 p2 = __ldg(S.prims + 3 * i + 2);
+            float t;
+            if (ray_tri(p0, p1, p2, ex, ey, ez, sx, sy, sz, t)) {
+              const float tt = t / len;
+              if (tt > 1e-4f && tt < 1.0f - 1e-4f) {
+                const uint32_t q = atomicAdd(&W.n, 1u);
+                if (q < kMaxCross) {
+                  W.t[q] = tt;
+                  W.prim[q] = i;
+                  W.ckey[q] = W.lkey[nl + g];
+                }
+              }
+            }
+          }
+          __syncwarp();
+          continue;
+        }
+        // ---- up to 32 nodes, one a lane
         const uint32_t take = sp < 32u ? sp : 32u;
         const uint32_t base = sp - take;
         const bool act = lane < take;
@@ -307,18 +348,24 @@ __device__ void through_warp(const DScene& S, const DDomeLaunch& L, ThroughSmem&
         sp = base;
         bool h0 = false, h1 = false;
         int c0 = 0, c1 = 0;
-        if (act && cur >= 0) {
+        if (act) {
           const float4 n0 = __ldg(S.nodes + 4 * cur + 0);
           const float4 n1 = __ldg(S.nodes + 4 * cur + 1);
           const float4 n2 = __ldg(S.nodes + 4 * cur + 2);
           const float4 n3 = __ldg(S.nodes + 4 * cur + 3);
           float ta, tb;
-          h0 = ray_aabb(n0.x, n0.y, n0.z, n0.w, n1.x, n1.y, ex, ey, ez, ix, iy, iz, len, ta);
-          h1 = ray_aabb(n1.z, n1.w, n2.x, n2.y, n2.z, n2.w, ex, ey, ez, ix, iy, iz, len, tb);
+          if (fast) {
+            h0 = ray_aabb_minmax(n0.x, n0.y, n0.z, n0.w, n1.x, n1.y, ex, ey, ez, ix, iy, iz, len, ta);
+            h1 = ray_aabb_minmax(n1.z, n1.w, n2.x, n2.y, n2.z, n2.w, ex, ey, ez, ix, iy, iz, len, tb);
+          } else {
+            h0 = ray_aabb(n0.x, n0.y, n0.z, n0.w, n1.x, n1.y, ex, ey, ez, ix, iy, iz, len, ta);
+            h1 = ray_aabb(n1.z, n1.w, n2.x, n2.y, n2.z, n2.w, ex, ey, ez, ix, iy, iz, len, tb);
+          }
           c0 = __float_as_int(n3.x);
           c1 = __float_as_int(n3.y);
         }
-        const unsigned m0 = __ballot_sync(FULL, h0), m1 = __ballot_sync(FULL, h1);
+        const unsigned m0 = __ballot_sync(FULL, h0 && c0 >= 0), m1 = __ballot_sync(FULL, h1 && c1 >= 0);
+        const unsigned l0 = __ballot_sync(FULL, h0 && c0 < 0), l1 = __ballot_sync(FULL, h1 && c1 < 0);
         const uint32_t tot = (uint32_t)(__popc(m0) + __popc(m1));
         if (sp + tot > kWarpStack) {
           fail |= 1u;
@@ -327,37 +374,19 @@ __device__ void through_warp(const DScene& S, const DDomeLaunch& L, ThroughSmem&
         const uint32_t d = (uint32_t)(key & 63ull);
         const unsigned long long child = (key & ~63ull) | (unsigned long long)(d < 63u ? d + 1u : 63u);
         const unsigned long long abit = d < 58u ? (1ull << (63u - d)) : 0ull;
-        const uint32_t pos = sp + (uint32_t)(__popc(m0 & lt) + __popc(m1 & lt));
         if (h0) {
-          W.ref[pos] = c0;
-          W.key[pos] = child | abit;
+          const uint32_t at = c0 < 0 ? nl + (uint32_t)__popc(l0 & lt) : sp + (uint32_t)__popc(m0 & lt);
+          (c0 < 0 ? W.lref : W.ref)[at] = c0;
+          (c0 < 0 ? W.lkey : W.key)[at] = child | abit;
         }
         if (h1) {
-          W.ref[pos + (h0 ? 1u : 0u)] = c1;
-          W.key[pos + (h0 ? 1u : 0u)] = child;
+          const uint32_t at = c1 < 0 ? nl + (uint32_t)(__popc(l0) + __popc(l1 & lt))
+                                     : sp + (uint32_t)(__popc(m0) + __popc(m1 & lt));
+          (c1 < 0 ? W.lref : W.ref)[at] = c1;
+          (c1 < 0 ? W.lkey : W.key)[at] = child;
         }
         sp += tot;
-        if (act && cur < 0) {
-          const uint32_t code = ~(uint32_t)cur;
-          const uint32_t start = code >> 3, end = start + (code & 7u) + 1u;
-          for (uint32_t i = start; i < end; i++) {
-            const float4 p0 = __ldg(S.prims + 3 * i + 0);
-            const float4 p1 = __ldg(S.prims + 3 * i + 1);
-            const float4 p2 = __ldg(S.prims + 3 * i + 2);
-            float t;
-            if (ray_tri(p0, p1, p2, ex, ey, ez, sx, sy, sz, t)) {
-              const float tt = t / len;
-              if (tt > 1e-4f && tt < 1.0f - 1e-4f) {
-                const uint32_t k = atomicAdd(&W.n, 1u);
-                if (k < kMaxCross) {
-                  W.t[k] = tt;
-                  W.prim[k] = i;
-                  W.ckey[k] = key;
-                }
-              }
-            }
-          }
-        }
+        nl += (uint32_t)(__popc(l0) + __popc(l1));
         __syncwarp();
       }
       __syncwarp();
@@ -608,12 +637,18 @@ cudaError_t launch_dome(const DDomeLaunch& L, cudaStream_t s) {
   while (rpw > 1 && total <= warps * (rpw / 2u)) rpw >>= 1;
   const uint32_t per_block = rpw * (kEscThreads / 32);
   const uint32_t blocks = (uint32_t)((total + per_block - 1) / per_block);
-  if (L.tie && L.wt)
-    dome_escape_walk_kernel<true, true><<<blocks, kEscThreads, 0, s>>>(L, kDefaultLoopGuard, rpw);
-  else if (L.tie)
-    dome_escape_walk_kernel<true, false><<<blocks, kEscThreads, 0, s>>>(L, kDefaultLoopGuard, rpw);
-  else
-    dome_escape_walk_kernel<false, false><<<blocks, kEscThreads, 0, s>>>(L, kDefaultLoopGuard, rpw);
+#define OMG_ESCAPE(NB, TIE, WT) \
+  dome_escape_walk_kernel<NB, TIE, WT><<<blocks, kEscThreads, 0, s>>>(L, kDefaultLoopGuard, rpw)
+  if (L.nb <= 3) {
+    if (!L.tie) OMG_ESCAPE(3, false, false);
+    else if (L.wt) OMG_ESCAPE(3, true, true);
+    else OMG_ESCAPE(3, true, false);
+  } else {
+    if (!L.tie) OMG_ESCAPE(MAXB, false, false);
+    else if (L.wt) OMG_ESCAPE(MAXB, true, true);
+    else OMG_ESCAPE(MAXB, true, false);
+  }
+#undef OMG_ESCAPE
   dome_through_kernel<<<(uint32_t)((total + kThroughWarps - 1) / kThroughWarps), 32 * kThroughWarps, 0, s>>>(L);
   dome_bins_kernel<<<L.n_eyes, kDomeBinThreads, 0, s>>>(L, 0.35f);
   return cudaGetLastError();

@@ -18,20 +18,20 @@ struct EarlyRec {
   float root_lo[3] = {0, 0, 0}, root_hi[3] = {0, 0, 0};
   DevBuf<DSurf> surf;
   DevBuf<float4> mtrans, boxes;
-  DevBuf<uint32_t> err;
+  DevBuf<uint32_t> words;          // error bits, discovered chains
   // discovery scratch (grown on demand)
   uint32_t disc_rays = 0, tcap = 0;
   DevBuf<float> jitter;
-  DevBuf<unsigned long long> cand_key, tkey;
+  DevBuf<unsigned long long> cand_key;
+  DevBuf<unsigned long long> table;  // tcap keys, then their tcap words of index, cleared together
   DevBuf<omg_chain> cand_chain, d_out;
-  DevBuf<uint32_t> cand_slot, tidx, n_out;
+  DevBuf<uint32_t> cand_slot;
   // solve scratch
-  size_t src_cap = 0, chain_cap = 0, extra_cap = 0, rec_cap = 0;
-  DevBuf<uint16_t> d_ids;
-  DevBuf<float> d_pos;
-  DevBuf<omg_chain> d_chains;
-  DevBuf<omg_aabb> d_extras;
+  size_t in_cap = 0, rec_cap = 0;
+  DevBuf<uint8_t> d_in;            // one call's inputs: positions, blockers, chains, source ids
+  std::vector<uint8_t> h_in;
   DevBuf<omg_mesh_record> d_rec;
+  DevBuf<uint32_t> d_live;         // the solve's list of pairs that need walks (a count, then their numbers)
   PinBuf<uint32_t> h_word;         // [0] error bits, [1] discovered chains
   cudaEvent_t done = nullptr;
   ~EarlyRec() {
@@ -71,7 +71,8 @@ int32_t early_view(omg_ctx* ctx, const EarlyRec& R, DEarly& E) {
     E.root_lo[a] = R.root_lo[a];
     E.root_hi[a] = R.root_hi[a];
   }
-  E.err = R.err.p;
+  E.err = R.words.p;
+  E.n_sms = (uint32_t)ctx->n_sms;
   return OMG_OK;
 }
 
@@ -79,14 +80,13 @@ int32_t early_view(omg_ctx* ctx, const EarlyRec& R, DEarly& E) {
 // the context's bound, then clear the word; a set bit is a kernel-side
 // overflow.
 int32_t early_finish(omg_ctx* ctx, EarlyRec& R) {
-  CK(cudaMemcpyAsync(R.h_word.p, R.err.p, 4, cudaMemcpyDeviceToHost, ctx->stream));
-  CK(cudaMemcpyAsync(R.h_word.p + 1, R.n_out.p, 4, cudaMemcpyDeviceToHost, ctx->stream));
+  CK(cudaMemcpyAsync(R.h_word.p, R.words.p, 8, cudaMemcpyDeviceToHost, ctx->stream));
   CK(cudaEventRecord(R.done, ctx->stream));
   int32_t rc = wait_event(ctx, R.done, timeout_of(ctx));
   if (rc) return rc;
   const uint32_t e = R.h_word.p[0];
   if (e) {
-    CK(cudaMemset(R.err.p, 0, 4));
+    CK(cudaMemset(R.words.p, 0, 4));
     ctx->last_error = "early reflections: kernel error bits " + std::to_string(e) +
                       " (1 stack, 2 crossing list, 4 walk budget, 8 chain table)";
     return OMG_E_OVERFLOW;
@@ -180,10 +180,8 @@ int32_t omg_early_create(omg_ctx* ctx, uint32_t scene_id, const omg_panel* furni
   if (!mt.empty()) CK(cudaMemcpy(R->mtrans.p, mt.data(), mt.size() * sizeof(float4), cudaMemcpyHostToDevice));
   CK(R->boxes.alloc(bx.size()));
   if (!bx.empty()) CK(cudaMemcpy(R->boxes.p, bx.data(), bx.size() * sizeof(float4), cudaMemcpyHostToDevice));
-  CK(R->err.alloc(1));
-  CK(cudaMemset(R->err.p, 0, 4));
-  CK(R->n_out.alloc(1));
-  CK(cudaMemset(R->n_out.p, 0, 4));
+  CK(R->words.alloc(2));
+  CK(cudaMemset(R->words.p, 0, 8));
   CK(R->h_word.alloc(2));
   CK(cudaEventCreateWithFlags(&R->done, cudaEventDisableTiming));
   const uint32_t id = ctx->next_early++;
@@ -227,8 +225,7 @@ int32_t omg_early_discover(omg_ctx* ctx, uint32_t early_id, const float listener
     CK(R->cand_chain.alloc(3ull * nr));
     CK(R->cand_slot.alloc(3ull * nr));
     R->tcap = pow2_at_least(2ull * 3ull * nr);
-    CK(R->tkey.alloc(R->tcap));
-    CK(R->tidx.alloc(R->tcap));
+    CK(R->table.alloc(R->tcap + R->tcap / 2u));
     CK(R->d_out.alloc(3ull * nr));
     R->disc_rays = nr;
   }
@@ -245,11 +242,10 @@ int32_t omg_early_discover(omg_ctx* ctx, uint32_t early_id, const float listener
   }
   if (n_rays)
     CK(cudaMemcpyAsync(R->jitter.p, jit.data(), n_rays * sizeof(float), cudaMemcpyHostToDevice, ctx->stream));
-  CK(cudaMemsetAsync(R->tkey.p, 0, (size_t)R->tcap * 8, ctx->stream));
-  CK(cudaMemsetAsync(R->tidx.p, 0xFF, (size_t)R->tcap * 4, ctx->stream));
+  CK(cudaMemsetAsync(R->table.p, 0, (size_t)R->tcap * 12, ctx->stream));
   CK(launch_early_discover(E, listener, n_rays, rot, use_boxes != 0, R->jitter.p, R->cand_key.p, R->cand_chain.p,
-                           R->cand_slot.p, R->tkey.p, R->tidx.p, R->tcap, R->d_out.p, (uint32_t)n_cand, R->n_out.p,
-                           ctx->stream));
+                           R->cand_slot.p, R->table.p, (uint32_t*)(R->table.p + R->tcap), R->tcap, R->d_out.p,
+                           (uint32_t)n_cand, R->words.p + 1, ctx->stream));
   if ((rc = early_finish(ctx, *R))) return rc;
   const uint32_t n = R->h_word.p[1];
   const uint32_t w = n < cap ? n : cap;
@@ -275,30 +271,29 @@ int32_t omg_early_solve(omg_ctx* ctx, uint32_t early_id, const uint16_t* source_
   if (rc) return rc;
   const uint64_t n = (uint64_t)n_sources * n_chains;
   if (n == 0) return OMG_OK;
-  if (R->src_cap < n_sources) {
-    CK(R->d_ids.alloc(n_sources));
-    CK(R->d_pos.alloc(3ull * n_sources));
-    R->src_cap = n_sources;
-  }
-  if (R->chain_cap < n_chains) {
-    CK(R->d_chains.alloc(n_chains));
-    R->chain_cap = n_chains;
-  }
-  if (R->extra_cap < n_extras || R->extra_cap == 0) {
-    CK(R->d_extras.alloc(n_extras ? n_extras : 1));
-    R->extra_cap = n_extras ? n_extras : 1;
+  const size_t ex_off = 12ull * n_sources, ch_off = ex_off + n_extras * sizeof(omg_aabb),
+               id_off = ch_off + n_chains * sizeof(omg_chain), bytes = id_off + 2ull * n_sources;
+  static_assert(sizeof(omg_aabb) % 4 == 0 && sizeof(omg_chain) % 4 == 0 && alignof(omg_chain) <= 4, "packed inputs");
+  if (R->in_cap < bytes) {
+    CK(R->d_in.alloc(bytes));
+    R->in_cap = bytes;
   }
   if (R->rec_cap < n) {
     CK(R->d_rec.alloc(n));
+    CK(R->d_live.alloc(1 + (n < kEarlySlice ? n : kEarlySlice)));
     R->rec_cap = n;
   }
-  CK(cudaMemcpyAsync(R->d_ids.p, source_ids, n_sources * sizeof(uint16_t), cudaMemcpyHostToDevice, ctx->stream));
-  CK(cudaMemcpyAsync(R->d_pos.p, source_pos, 3ull * n_sources * sizeof(float), cudaMemcpyHostToDevice, ctx->stream));
-  CK(cudaMemcpyAsync(R->d_chains.p, chains, n_chains * sizeof(omg_chain), cudaMemcpyHostToDevice, ctx->stream));
-  if (n_extras)
-    CK(cudaMemcpyAsync(R->d_extras.p, extras, n_extras * sizeof(omg_aabb), cudaMemcpyHostToDevice, ctx->stream));
-  CK(launch_early_solve(E, R->d_ids.p, R->d_pos.p, n_sources, R->d_chains.p, n_chains, listener, R->d_extras.p,
-                        n_extras, R->d_rec.p, ctx->stream));
+  R->h_in.resize(bytes);
+  uint8_t* h = R->h_in.data();
+  std::memcpy(h, source_pos, ex_off);
+  if (n_extras) std::memcpy(h + ex_off, extras, ch_off - ex_off);
+  std::memcpy(h + ch_off, chains, id_off - ch_off);
+  std::memcpy(h + id_off, source_ids, bytes - id_off);
+  CK(cudaMemcpyAsync(R->d_in.p, h, bytes, cudaMemcpyHostToDevice, ctx->stream));
+  uint8_t* d = R->d_in.p;
+  CK(launch_early_solve(E, (const uint16_t*)(d + id_off), (const float*)d, n_sources, (const omg_chain*)(d + ch_off),
+                        n_chains, listener, (const omg_aabb*)(d + ex_off), n_extras, R->d_live.p, R->d_rec.p,
+                        ctx->stream));
   if ((rc = early_finish(ctx, *R))) return rc;
   CK(cudaMemcpy(out, R->d_rec.p, n * sizeof(omg_mesh_record), cudaMemcpyDeviceToHost));
   return OMG_OK;

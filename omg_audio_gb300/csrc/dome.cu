@@ -8,6 +8,7 @@
 // the rays of each listener in fan order (dome.rs:452-458,
 // the same f32 sums in the same order), applies the per-listener EMA and
 // writes the 9 bins. The fan is deterministic, so the result is too.
+#include "cross_walk.cuh"
 #include "device_common.cuh"
 #include "walk.cuh"
 
@@ -17,7 +18,6 @@ namespace {
 
 constexpr float PI_F = 3.14159265358979323846f;
 constexpr uint32_t kEscBlocks = 7;   // escape blocks a multiprocessor (28 warps, 72 registers)
-constexpr uint32_t kMaxCross = 64;   // crossings kept per straight-through segment
 
 // dome.rs:56-68
 __device__ __forceinline__ bool panel_hit(const DDomePanel& p, float ox, float oy, float oz, float dx, float dy,
@@ -233,44 +233,20 @@ __global__ void __launch_bounds__(kEscThreads, kEscBlocks) dome_escape_walk_kern
 
 // One warp's shared memory for the straight-through segment of one fan ray.
 constexpr uint32_t kThroughWarps = 4;        // rays (warps) per block
-constexpr uint32_t kWarpStack = 512;         // pending nodes of one warp's walk
-constexpr uint32_t kWarpLeaves = 72;         // pending leaves (fewer than 8, and a round's 64 children)
-constexpr uint32_t kMaxThroughRounds = 1u << 20;
 struct ThroughSmem {
-  int ref[kWarpStack];
-  int lref[kWarpLeaves];
-  unsigned long long key[kWarpStack];        // the ref's depth-first position (below)
-  unsigned long long lkey[kWarpLeaves];
-  float t[kMaxCross];                        // crossings as found
-  uint32_t prim[kMaxCross];
-  unsigned long long ckey[kMaxCross];
+  CrossShare x;
   float st[kMaxCross];                       // crossings sorted
   uint32_t sprim[kMaxCross];
-  uint32_t n;
 };
 
 // Straight-through seep of one fan ray (trace_through, dome.rs:390-422) by a
-// whole warp. The crossings of the 50 m segment (segment_hits,
-// mesh.rs:546-604) are collected by a walk in which every lane takes one
-// pending node per round (children whose box the segment meets are pushed
-// warp-aggregated), so the any-hit walk, which visits every node the segment
-// meets, runs 32 nodes wide instead of one. Leaves wait in a list of their own
-// and are tested eight at a time, four lanes each: a lane that met a leaf among
-// the nodes tested its primitives alone, in nearly every round.
-//
-// The reference sorts the crossings by t with a stable sort over its
-// depth-first visiting order (child b before child a) and then merges
-// clusters within 1e-4 / max(len, 1) keeping the lowest surface id (the
-// first one on equal ids). Each ref therefore carries its depth-first
-// position: bit 63 - d set for the a child at depth d (d < 58) above a
-// 6-bit depth, so that ordering crossings by (t, key, primitive) reproduces
-// the reference's order, and the merge and the transmission product then run
-// in that order, uniformly across the warp.
+// whole warp: the crossings of the 50 m segment (cross_walk.cuh), the
+// reference's merge and the transmission product in their order, uniformly
+// across the warp.
 __device__ void through_warp(const DScene& S, const DDomeLaunch& L, ThroughSmem& W, uint32_t lane, float ex,
                              float ey, float ez, float dx, float dy, float dz, float tp[MAXB]) {
   constexpr unsigned FULL = 0xffffffffu;
   const uint32_t nb = L.nb;
-  const uint32_t lt = (1u << lane) - 1u;
 #pragma unroll
   for (int b = 0; b < MAXB; b++) tp[b] = 1.0f;
   const float bx = ex + dx * 50.0f, by = ey + dy * 50.0f, bz = ez + dz * 50.0f;
@@ -291,107 +267,7 @@ __device__ void through_warp(const DScene& S, const DDomeLaunch& L, ThroughSmem&
       sy = sy * il;
       sz = sz * il;
       const float ix = __frcp_rn(sx), iy = __frcp_rn(sy), iz = __frcp_rn(sz);
-      const float kTiny = 8.673617379884035e-19f;   // 2^-60: no product of the slab test is a NaN
-      const bool fast = fabsf(sx) >= kTiny && fabsf(sy) >= kTiny && fabsf(sz) >= kTiny;
-      uint32_t sp = S.root >= 0 ? 1u : 0u, nl = 1u - sp, rounds = 0;
-      if (lane == 0) {
-        (sp ? W.ref : W.lref)[0] = S.root;
-        (sp ? W.key : W.lkey)[0] = 0ull;
-        W.n = 0u;
-      }
-      __syncwarp();
-      while ((sp | nl) != 0u) {
-        if (++rounds > kMaxThroughRounds) {
-          fail |= 1u;
-          break;
-        }
-        if (nl >= 8u || sp == 0u) {
-          // ---- up to 8 leaves, four lanes each
-          const uint32_t take = nl < 8u ? nl : 8u, g = lane >> 2;
-          nl -= take;
-          const bool act = g < take;
-          const uint32_t code = act ? ~(uint32_t)W.lref[nl + g] : 0u;
-          const uint32_t start = code >> 3, cnt = act ? (code & 7u) + 1u : 0u;
-          for (uint32_t k = lane & 3u; __any_sync(FULL, k < cnt); k += 4u) {
-            if (k >= cnt) continue;
-            const uint32_t i = start + k;
-            const float4 p0 = __ldg(S.prims + 3 * i + 0);
-            const float4 p1 = __ldg(S.prims + 3 * i + 1);
-            const float4 p2 = __ldg(S.prims + 3 * i + 2);
-            float t;
-            if (ray_tri(p0, p1, p2, ex, ey, ez, sx, sy, sz, t)) {
-              const float tt = t / len;
-              if (tt > 1e-4f && tt < 1.0f - 1e-4f) {
-                const uint32_t q = atomicAdd(&W.n, 1u);
-                if (q < kMaxCross) {
-                  W.t[q] = tt;
-                  W.prim[q] = i;
-                  W.ckey[q] = W.lkey[nl + g];
-                }
-              }
-            }
-          }
-          __syncwarp();
-          continue;
-        }
-        // ---- up to 32 nodes, one a lane
-        const uint32_t take = sp < 32u ? sp : 32u;
-        const uint32_t base = sp - take;
-        const bool act = lane < take;
-        int cur = 0;
-        unsigned long long key = 0ull;
-        if (act) {
-          cur = W.ref[base + lane];
-          key = W.key[base + lane];
-        }
-        __syncwarp();
-        sp = base;
-        bool h0 = false, h1 = false;
-        int c0 = 0, c1 = 0;
-        if (act) {
-          const float4 n0 = __ldg(S.nodes + 4 * cur + 0);
-          const float4 n1 = __ldg(S.nodes + 4 * cur + 1);
-          const float4 n2 = __ldg(S.nodes + 4 * cur + 2);
-          const float4 n3 = __ldg(S.nodes + 4 * cur + 3);
-          float ta, tb;
-          if (fast) {
-            h0 = ray_aabb_minmax(n0.x, n0.y, n0.z, n0.w, n1.x, n1.y, ex, ey, ez, ix, iy, iz, len, ta);
-            h1 = ray_aabb_minmax(n1.z, n1.w, n2.x, n2.y, n2.z, n2.w, ex, ey, ez, ix, iy, iz, len, tb);
-          } else {
-            h0 = ray_aabb(n0.x, n0.y, n0.z, n0.w, n1.x, n1.y, ex, ey, ez, ix, iy, iz, len, ta);
-            h1 = ray_aabb(n1.z, n1.w, n2.x, n2.y, n2.z, n2.w, ex, ey, ez, ix, iy, iz, len, tb);
-          }
-          c0 = __float_as_int(n3.x);
-          c1 = __float_as_int(n3.y);
-        }
-        const unsigned m0 = __ballot_sync(FULL, h0 && c0 >= 0), m1 = __ballot_sync(FULL, h1 && c1 >= 0);
-        const unsigned l0 = __ballot_sync(FULL, h0 && c0 < 0), l1 = __ballot_sync(FULL, h1 && c1 < 0);
-        const uint32_t tot = (uint32_t)(__popc(m0) + __popc(m1));
-        if (sp + tot > kWarpStack) {
-          fail |= 1u;
-          break;
-        }
-        const uint32_t d = (uint32_t)(key & 63ull);
-        const unsigned long long child = (key & ~63ull) | (unsigned long long)(d < 63u ? d + 1u : 63u);
-        const unsigned long long abit = d < 58u ? (1ull << (63u - d)) : 0ull;
-        if (h0) {
-          const uint32_t at = c0 < 0 ? nl + (uint32_t)__popc(l0 & lt) : sp + (uint32_t)__popc(m0 & lt);
-          (c0 < 0 ? W.lref : W.ref)[at] = c0;
-          (c0 < 0 ? W.lkey : W.key)[at] = child | abit;
-        }
-        if (h1) {
-          const uint32_t at = c1 < 0 ? nl + (uint32_t)(__popc(l0) + __popc(l1 & lt))
-                                     : sp + (uint32_t)(__popc(m0) + __popc(m1 & lt));
-          (c1 < 0 ? W.lref : W.ref)[at] = c1;
-          (c1 < 0 ? W.lkey : W.key)[at] = child;
-        }
-        sp += tot;
-        nl += (uint32_t)(__popc(l0) + __popc(l1));
-        __syncwarp();
-      }
-      __syncwarp();
-      n = W.n;
-      if (n > kMaxCross) fail |= 2u;
+      n = warp_crossings(S, W.x, lane, ex, ey, ez, sx, sy, sz, ix, iy, iz, len, 0xFFFFFFFFu, fail);
     }
   }
   if (fail) {
@@ -400,19 +276,10 @@ __device__ void through_warp(const DScene& S, const DDomeLaunch& L, ThroughSmem&
     for (int b = 0; b < MAXB; b++) tp[b] = 0.0f;
     return;
   }
-  // rank sort by (t, depth-first key, primitive): every key is distinct
   for (uint32_t e = lane; e < n; e += 32u) {
-    const float te = W.t[e];
-    const unsigned long long ke = W.ckey[e];
-    const uint32_t pe = W.prim[e];
-    uint32_t r = 0;
-    for (uint32_t q = 0; q < n; q++) {
-      const float tq = W.t[q];
-      const unsigned long long kq = W.ckey[q];
-      if (tq < te || (tq == te && (kq < ke || (kq == ke && W.prim[q] < pe)))) r++;
-    }
-    W.st[r] = te;
-    W.sprim[r] = pe;
+    const uint32_t r = cross_rank(W.x, n, e);
+    W.st[r] = W.x.t[e];
+    W.sprim[r] = W.x.prim[e];
   }
   __syncwarp();
   // same-t merge (lowest surface id wins, the cluster keeps its first t),

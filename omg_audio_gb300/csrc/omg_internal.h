@@ -422,16 +422,20 @@ struct DEarly {
   uint32_t n_boxes;
   float root_lo[3], root_hi[3];  // the tree's root box (segment_hits tests it first)
   uint32_t* err;              // error bits: 1 stack, 2 crossing list, 4 walk budget, 8 hash table
+  uint32_t n_sms;
 };
 // Discovery: n_rays fan rays -> 3 candidates each (cand_key 0 = none), the
 // first occurrence of every key (hash table tkey/tidx of tcap slots, cleared
-// to 0 / 0xFFFFFFFF) compacted in candidate order into out (<= cap), *n_out.
+// to 0; tidx holds the complement of the index) compacted in candidate order into out (<= cap), *n_out.
 cudaError_t launch_early_discover(const DEarly& E, const float lis[3], uint32_t n_rays, uint32_t rot, bool use_boxes,
                                   const float* jitter, unsigned long long* cand_key, omg_chain* cand_chain,
                                   uint32_t* cand_slot, unsigned long long* tkey, uint32_t* tidx, uint32_t tcap,
                                   omg_chain* out, uint32_t cap, uint32_t* n_out, cudaStream_t s);
+// Every (source, chain) pair's record, kEarlySlice pairs per launch; live:
+// scratch of 1 + min(n_src * n_chains, kEarlySlice) words.
+constexpr uint64_t kEarlySlice = 1ull << 24;
 cudaError_t launch_early_solve(const DEarly& E, const uint16_t* ids, const float* pos, uint32_t n_src,
                                const omg_chain* chains, uint32_t n_chains, const float lis[3], const omg_aabb* extras,
-                               uint32_t n_extras, omg_mesh_record* out, cudaStream_t s);
+                               uint32_t n_extras, uint32_t* live, omg_mesh_record* out, cudaStream_t s);
 
 }  // namespace omg

@@ -373,23 +373,29 @@ int32_t upload_batch(omg_ctx* ctx, BatchRec& B) {
   return OMG_OK;
 }
 
+// The shape a batch is launched with.
+LaunchShape effective_shape(omg_ctx* ctx, const BatchRec& B) {
+  LaunchShape eff = B.shape;
+  eff.loop_guard = ctx->prm.loop_guard;
+  if (B.deep) eff.spread_warps = 32;
+  eff.box_only = B.box_only;
+  eff.solo_ok = B.solo_ok;
+  // cooperative walks need the near-tie rule and a 4-wide tree in every scene
+  if (eff.mode == 2 && !B.coop_ok) eff.mode = 0;
+  if (eff.tail_mode == 2 && !B.coop_ok) eff.tail_mode = 0;
+  return eff;
+}
+
 // The device-side work of one launch (recorded into a graph).
 // part 1: clear the scratch and trace; part 2: finalize and reverb.
 int32_t record_launch(omg_ctx* ctx, BatchRec& B, cudaStream_t s, int parts = 3) {
   if (parts & 1) {
     CK(cudaMemsetAsync(B.d_block.p, 0, B.clear_bytes, s));
-    // cooperative walks need the near-tie rule and a 4-wide tree in every scene
-    LaunchShape eff = B.shape;
-    eff.loop_guard = ctx->prm.loop_guard;
-    if (B.deep) eff.spread_warps = 32;
-    eff.box_only = B.box_only;
-    eff.solo_ok = B.solo_ok;
-    if (eff.mode == 2 && !B.coop_ok) eff.mode = 0;
-    if (eff.tail_mode == 2 && !B.coop_ok) eff.tail_mode = 0;
+    const LaunchShape eff = effective_shape(ctx, B);
     CK(launch_wavefront(B.d_jobs.p, B.n_jobs, B.total_rays, B.max_nb, ctx->d_scenes.p, B.d_job_mats.p,
                         B.d_panels.p, B.d_groups.p, B.d_acc.p, B.d_hdr.p, B.d_seg.p, B.wf, B.d_ep_q.p,
                         B.d_ep_ctl.p, eff, ctx->n_sms, ctx->prm.tie_mode != 0, s,
-                        ctx->prm.tri_test == OMG_TRI_WATERTIGHT));
+                        ctx->prm.tri_test == OMG_TRI_WATERTIGHT, B.d_tail.p));
   }
   if (parts & 2) {
     CK(launch_finalize(B.d_jobs.p, B.n_jobs, B.d_acc.p, B.d_out.p, B.n_out, s));
@@ -408,6 +414,8 @@ int32_t capture_graph(omg_ctx* ctx, BatchRec& B, cudaStream_t cs, bool io, int p
   cudaGraph_t g;
   int32_t rc = ensure_staging(ctx, B);
   if (rc) return rc;
+  const size_t tail = (size_t)kTailWords * tail_rays(effective_shape(ctx, B), B.total_rays, ctx->n_sms);
+  if (B.d_tail.n < tail) CK(B.d_tail.alloc(tail));
   cudaError_t e = cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal);
   if (e != cudaSuccess) return fail(ctx, e, "cudaStreamBeginCapture");
   if (io) {
@@ -795,10 +803,11 @@ int32_t omg_batch_kernel_count(omg_ctx* ctx, uint32_t id, uint32_t* n) {
   auto it = ctx->batches.find(id);
   if (it == ctx->batches.end()) return OMG_E_NOT_FOUND;
   // finalize, reverb; the persistent kernel once per epoch; wavefront: init,
-  // 2 per round, hand-over
+  // 2 per round, hand-over; the tail of a launch that fills the chip
   const LaunchShape& sh = it->second->shape;
   const uint32_t epochs = sh.epochs == 0 ? 1u : std::min<uint32_t>(sh.epochs, kMaxEpochs);
-  *n = 2 + epochs + (sh.wf_iters ? 2 + 2 * sh.wf_iters : 0);
+  *n = 2 + epochs + (sh.wf_iters ? 2 + 2 * sh.wf_iters : 0) +
+       (tail_rays(effective_shape(ctx, *it->second), it->second->total_rays, ctx->n_sms) ? 1 : 0);
   return OMG_OK;
 }
 

@@ -178,7 +178,10 @@ struct alignas(16) DLaunch {
   uint32_t ray_counter;   // persistent-queue head
   uint32_t error;         // kernel flags: 1 stack overflow, 2 crossing list overflow, 4 walk budget,
                           // 8 persistent-kernel loop guard
-  uint32_t pad[2];
+  // Launches with a tail (TailArgs): rays that the persistent kernel has ended,
+  // and rays that it has handed over; then total_rays - tail is where the tail
+  // launch goes on counting `ended`, its queue head.
+  uint32_t ended, tail;
 };
 
 // Histogram accumulators hold values scaled by 2^64 (exact): the float
@@ -270,6 +273,17 @@ struct EpochArgs {
   uint32_t max_loop;     // the persistent kernels' per-warp loop guard (error 8)
 };
 
+// The end of a launch that fills the chip (launch_trace): once the ray queue is
+// drained and at most `cap` rays are left, the persistent kernel saves them here
+// and solo.cu traces them to their ends, a warp each. A ray is kTailWords
+// float4: (p, distance), (d, stream bits), (segment count bits, job bits, -, -),
+// energies.
+constexpr uint32_t kTailWords = 5;
+struct TailArgs {
+  float4* rays;          // null: no tail
+  uint32_t cap;
+};
+
 // ----------------------------------------------------------- kernel launchers
 // trace.cu. `ep`: one epoch of an epoch chain (null: a single launch).
 // wt: the context's scenes carry exact vertices (watertight test)
@@ -277,16 +291,20 @@ cudaError_t launch_trace(const DJob* jobs, uint32_t n_jobs, uint32_t total_rays,
                          const DScene* scenes, const DMat* job_mats, const DPanel* panels,
                          const DPanelGroup* groups, float* acc,
                          DLaunch* hdr, uint32_t* job_segments, const LaunchShape& shape, int n_sms, bool tie,
-                         cudaStream_t s, const EpochArgs* ep = nullptr, bool wt = false);
+                         cudaStream_t s, const EpochArgs* ep = nullptr, bool wt = false, float4* tail = nullptr);
+// trace.cu: the rays that launch_trace leaves to a second launch at its end (0:
+// none): the `tail` buffer holds kTailWords float4 for each.
+uint32_t tail_rays(const LaunchShape& shape, uint32_t total_rays, int n_sms);
 // trace.cu: load the shoebox trace kernels (3 and 8 bands) now, so that a later
 // launch does not wait for the driver's lazy module loading.
 cudaError_t preload_trace_kernels();
 // solo.cu: the tracer for launches of few rays, one warp per ray (every mesh
-// scene has a 4-wide tree or is one leaf); max_loop as in EpochArgs.
+// scene has a 4-wide tree or is one leaf); max_loop as in EpochArgs. tail: the
+// rays that the persistent kernel of this launch has left, not the launch's own.
 cudaError_t launch_trace_solo(const DJob* jobs, uint32_t n_jobs, uint32_t total_rays, uint32_t max_nb,
                               const DScene* scenes, const DMat* job_mats, const DPanel* panels, float* acc,
                               DLaunch* hdr, uint32_t* job_segments, uint32_t max_loop, int n_sms, bool tie, bool wt,
-                              cudaStream_t s);
+                              cudaStream_t s, TailArgs tail = {nullptr, 0});
 // coop.cu: the mode-2 persistent kernel (same arguments as launch_trace).
 cudaError_t launch_trace_coop(const DJob* jobs, uint32_t n_jobs, uint32_t total_rays, uint32_t max_nb,
                               const DScene* scenes, const DMat* job_mats, const DPanel* panels,
@@ -299,7 +317,7 @@ cudaError_t launch_wavefront(const DJob* jobs, uint32_t n_jobs, uint32_t total_r
                              const DScene* scenes, const DMat* job_mats, const DPanel* panels,
                              const DPanelGroup* groups, float* acc, DLaunch* hdr, uint32_t* job_segments,
                              const WfState& st, uint32_t* ep_q, EpochCtl* ep_ctl, const LaunchShape& shape,
-                             int n_sms, bool tie, cudaStream_t s, bool wt = false);
+                             int n_sms, bool tie, cudaStream_t s, bool wt = false, float4* tail = nullptr);
 cudaError_t launch_finalize(const DJob* jobs, uint32_t n_jobs, const float* acc, float* out, uint64_t total_out,
                             cudaStream_t s);
 cudaError_t launch_raycast(const DScene* scene, const float* o, const float* d, uint32_t n, float* t,

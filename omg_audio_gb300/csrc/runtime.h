@@ -141,6 +141,7 @@ struct BatchRec {
   bool box_only = false;          // every job is a shoebox
   bool solo_ok = false;           // every mesh scene has a 4-wide tree or is one leaf (solo.cu)
   DevBuf<uint32_t> d_ep_q;        // epoch queues (2 x rays)
+  DevBuf<float4> d_tail;          // rays left to the tail launch (trace.cu:tail_rays), allocated once a shape has one
   LaunchShape shape;
   // recorded when first needed (batch_graph)
   cudaGraphExec_t graph = nullptr;         // device-only launch

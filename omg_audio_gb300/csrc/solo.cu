@@ -77,7 +77,7 @@ template <int NB, bool TIE, bool WT>
 __global__ void __launch_bounds__(kSoloThreads, kSoloBlocks)
     solo_kernel(const DJob* __restrict__ jobs, uint32_t n_jobs, uint32_t total_rays, const DScene* __restrict__ scenes,
                 const DMat* __restrict__ job_mats, const DPanel* __restrict__ panels, float* __restrict__ acc,
-                DLaunch* __restrict__ hdr, uint32_t* __restrict__ job_segments, uint32_t max_loop) {
+                DLaunch* __restrict__ hdr, uint32_t* __restrict__ job_segments, uint32_t max_loop, TailArgs tail) {
   constexpr unsigned FULL = 0xffffffffu;
   __shared__ SoloShare s_share[kSoloThreads / 32];
   SoloShare& sh = s_share[threadIdx.x >> 5];
@@ -85,21 +85,46 @@ __global__ void __launch_bounds__(kSoloThreads, kSoloBlocks)
   uint32_t* err = &hdr->error;
   uint32_t iters = 0;   // loop guard
   while (iters <= max_loop) {
-    uint32_t rid = 0;
-    if (lane == 0) rid = atomicAdd(&hdr->ray_counter, 1u);
-    rid = __shfl_sync(FULL, rid, 0);
-    if (rid >= total_rays) return;
-    const uint32_t ji = find_job(jobs, n_jobs, rid);
-    const DJob& J = jobs[ji];
+    uint32_t rid = 0, ji;
+    float px, py, pz, dist, dx, dy, dz, e[NB];
     Pcg rng;
-    rng.init(J.seed, rid - J.ray_base);
-    float dx, dy, dz;
-    unit_sphere(rng, dx, dy, dz);
-    float px = J.src[0], py = J.src[1], pz = J.src[2], dist = 0.0f;
-    float e[NB];
-#pragma unroll
-    for (int b = 0; b < NB; b++) e[b] = J.e0[b];
     uint32_t bounce = 0;
+    if (tail.rays == nullptr) {
+      if (lane == 0) rid = atomicAdd(&hdr->ray_counter, 1u);
+      rid = __shfl_sync(FULL, rid, 0);
+      if (rid >= total_rays) return;
+      ji = find_job(jobs, n_jobs, rid);
+      const DJob& J = jobs[ji];
+      rng.init(J.seed, rid - J.ray_base);
+      unit_sphere(rng, dx, dy, dz);
+      px = J.src[0];
+      py = J.src[1];
+      pz = J.src[2];
+      dist = 0.0f;
+#pragma unroll
+      for (int b = 0; b < NB; b++) e[b] = J.e0[b];
+    } else {
+      const uint32_t n = hdr->tail;
+      if (lane == 0) rid = atomicAdd(&hdr->ended, 1u) - (total_rays - n);
+      rid = __shfl_sync(FULL, rid, 0);
+      if (rid >= n) return;
+      const float4* T = tail.rays + (size_t)kTailWords * rid;
+      const float4 a = T[0], d = T[1], c = T[2], e0 = T[3], e1 = T[4];
+      px = a.x;
+      py = a.y;
+      pz = a.z;
+      dist = a.w;
+      dx = d.x;
+      dy = d.y;
+      dz = d.z;
+      rng.s = __float_as_uint(d.w);
+      bounce = __float_as_uint(c.x);
+      ji = __float_as_uint(c.y);
+      const float ev[8] = {e0.x, e0.y, e0.z, e0.w, e1.x, e1.y, e1.z, e1.w};
+#pragma unroll
+      for (int b = 0; b < NB; b++) e[b] = ev[b];
+    }
+    const DJob& J = jobs[ji];
     bool done = false;
     // one segment of the bounce loop (tracer.rs:103-200) a pass
     while (!done && ++iters <= max_loop) {
@@ -141,13 +166,13 @@ __global__ void __launch_bounds__(kSoloThreads, kSoloBlocks)
 cudaError_t launch_trace_solo(const DJob* jobs, uint32_t n_jobs, uint32_t total_rays, uint32_t max_nb,
                               const DScene* scenes, const DMat* job_mats, const DPanel* panels, float* acc,
                               DLaunch* hdr, uint32_t* job_segments, uint32_t max_loop, int n_sms, bool tie, bool wt,
-                              cudaStream_t s) {
+                              cudaStream_t s, TailArgs tail) {
   const uint32_t per = kSoloThreads / 32;
-  const uint32_t need = (total_rays + per - 1) / per, most = (uint32_t)n_sms * kSoloBlocks;
+  const uint32_t need = ((tail.rays ? tail.cap : total_rays) + per - 1) / per, most = (uint32_t)n_sms * kSoloBlocks;
   const uint32_t blocks = need < most ? need : most;
 #define OMG_SOLO(NB, TIE, WT)                                                                                      \
   solo_kernel<NB, TIE, WT><<<blocks, kSoloThreads, 0, s>>>(jobs, n_jobs, total_rays, scenes, job_mats, panels, acc, \
-                                                           hdr, job_segments, max_loop)
+                                                           hdr, job_segments, max_loop, tail)
   if (max_nb <= 3) {
     if (!tie) OMG_SOLO(3, false, false);
     else if (wt) OMG_SOLO(3, true, true);

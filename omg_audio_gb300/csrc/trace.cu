@@ -51,6 +51,22 @@ __device__ __noinline__ void park_ray(const WfState& rs, uint32_t rid, float px,
   rs.bounce[rid] = bounce;
 }
 
+// A ray left to the tail launch.
+template <int NB>
+__device__ __noinline__ void hand_over(float4* rays, uint32_t slot, float px, float py, float pz, float dist, float dx,
+                                       float dy, float dz, uint32_t rng_s, Bands<NB> e, uint32_t bounce,
+                                       uint32_t job) {
+  float4* T = rays + (size_t)kTailWords * slot;
+  T[0] = make_float4(px, py, pz, dist);
+  T[1] = make_float4(dx, dy, dz, __uint_as_float(rng_s));
+  T[2] = make_float4(__uint_as_float(bounce), __uint_as_float(job), 0.0f, 0.0f);
+  float v[8];
+#pragma unroll
+  for (int b = 0; b < 8; b++) v[b] = b < NB ? e.v[b] : 0.0f;
+  T[3] = make_float4(v[0], v[1], v[2], v[3]);
+  T[4] = make_float4(v[4], v[5], v[6], v[7]);
+}
+
 // An epoch's per-iteration bookkeeping, warp-aggregated (every lane calls it):
 // count the ended rays (and raise the park signal once at most `keep` remain
 // and the queue is drained), append the parked ones to the next epoch's queue.
@@ -116,7 +132,7 @@ __global__ void __launch_bounds__(256, 4) trace_kernel(const DJob* __restrict__ 
                                                        const DPanelGroup* __restrict__ groups, float* __restrict__ acc,
                                                     DLaunch* __restrict__ hdr, uint32_t* __restrict__ job_segments,
                                                     uint32_t refill_min, int walk_budget, uint32_t lane_cap,
-                                                    EpochArgs ea) {
+                                                    EpochArgs ea, TailArgs tail) {
   constexpr bool wide = TIE && WIDE;
   const unsigned FULL = 0xffffffffu;
   const uint32_t lane = threadIdx.x & 31u;
@@ -336,6 +352,26 @@ __global__ void __launch_bounds__(256, 4) trace_kernel(const DJob* __restrict__ 
       }
     }
     if (ea.cur) epoch_tally(ea, ended, parked, cold_rid(), may_park, n_rays, keep, fetch);
+    if (!BOX && tail.rays) {
+      const unsigned em = __ballot_sync(FULL, ended);
+      if (em && lane == 0) atomicAdd(&hdr->ended, (uint32_t)__popc(em));
+      if (exhausted && total_rays - *((volatile const uint32_t*)&hdr->ended) <= tail.cap) {
+        // every ray left in the launch is in some warp: no more than tail.cap are handed over
+        const unsigned am = __ballot_sync(FULL, phase != IDLE);
+        uint32_t base = 0;
+        if (lane == 0 && am) base = atomicAdd(&hdr->tail, (uint32_t)__popc(am));
+        base = __shfl_sync(FULL, base, 0);
+        if (phase != IDLE) {
+          Bands<NB> eb;
+          float dist;
+          uint32_t rng_s, bounce;
+          cold_load(eb.v, dist, rng_s, bounce);
+          hand_over<NB>(tail.rays, base + (uint32_t)__popc(am & lt_mask), px, py, pz, dist, dx, dy, dz, rng_s, eb,
+                        bounce, ji);
+        }
+        break;
+      }
+    }
   }
 }
 
@@ -553,11 +589,29 @@ __global__ void raycast_kernel(const DScene* __restrict__ scene, const float* __
 
 }  // namespace
 
+// Once the ray queue is drained, warps thin out: an iteration with 3 lanes left
+// takes 31 us where one with 32 takes 57 (64 pairs on the 40-room world: the last
+// 3 % of the rays take 1.2 of 7.5 ms), bound by the chain of one ray's segments.
+// A warp on each such ray (solo.cu) is faster from about two rays per resident
+// warp down. Calls without a tail, and with one of 28 and 56 rays a
+// multiprocessor (ms):
+//   rays            16,384  32,768  65,536  262,144  rooms 727,160  city 4,194,304
+//   none              3.31    3.73    5.14     7.92          26.72           20.58
+//   28 (4256 rays)    3.10    3.40    4.31     7.51          25.25           19.83
+//   56 (8512)         3.39    3.55    4.14     7.47          25.07           19.65
+// (84 and 112: 7.50 and 7.53 ms at 262,144). Shoeboxes, device-built trees (no
+// 4-wide form) and shapes with epochs, rounds or 4-wide walks have none.
+uint32_t tail_rays(const LaunchShape& shape, uint32_t total_rays, int n_sms) {
+  if (shape.mode != 0 || shape.wide || shape.epochs || shape.wf_iters || !shape.solo_ok || shape.box_only) return 0;
+  const uint32_t unit = 28u * (uint32_t)n_sms;
+  return total_rays < 3u * unit ? 0u : total_rays < 9u * unit ? unit : 2u * unit;
+}
+
 cudaError_t launch_trace(const DJob* jobs, uint32_t n_jobs, uint32_t total_rays, uint32_t max_nb,
                          const DScene* scenes, const DMat* job_mats, const DPanel* panels,
                          const DPanelGroup* groups, float* acc, DLaunch* hdr,
                          uint32_t* job_segments, const LaunchShape& shape, int n_sms, bool tie, cudaStream_t s,
-                         const EpochArgs* ep, bool wt) {
+                         const EpochArgs* ep, bool wt, float4* tail_buf) {
   if (n_jobs == 0 || total_rays == 0) return cudaSuccess;
   EpochArgs ea{};
   if (ep) ea = *ep;
@@ -618,10 +672,13 @@ cudaError_t launch_trace(const DJob* jobs, uint32_t n_jobs, uint32_t total_rays,
   // of 8192 rays 7.75, 7.43, 7.08, 6.95, 7.02, 7.41 ms at 1, 2, 4, 6, 8, 12 idle
   // lanes. Mesh walks are longer: there a lane is refilled at once.
   if (shape.box_only && lane_cap == 32u) refill = std::max(refill, 6u);
+  TailArgs tail{nullptr, 0};
+  if (!ep && tail_buf) tail = {tail_buf, tail_rays(shape, total_rays, n_sms)};
+  if (tail.cap == 0) tail.rays = nullptr;
 #define OMG_TRACE_LAUNCH(NB, TIE, WIDE, WT, BOX)                                                              \
   trace_kernel<NB, TIE, WIDE, WT, BOX><<<blocks, threads, 0, s>>>(jobs, n_jobs, total_rays, scenes, job_mats, \
                                                                   panels, groups, acc, hdr, job_segments,     \
-                                                                  refill, steps, lane_cap, ea)
+                                                                  refill, steps, lane_cap, ea, tail)
 #define OMG_TRACE_PICK(NB)                                                                                    \
   if (wl && tie)                                                                                              \
     trace_wl_kernel<NB, true><<<blocks, threads, 0, s>>>(jobs, n_jobs, total_rays, scenes, job_mats, panels,  \
@@ -643,7 +700,10 @@ cudaError_t launch_trace(const DJob* jobs, uint32_t n_jobs, uint32_t total_rays,
   }
 #undef OMG_TRACE_PICK
 #undef OMG_TRACE_LAUNCH
-  return cudaGetLastError();
+  const cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess || !tail.rays) return e;
+  return launch_trace_solo(jobs, n_jobs, total_rays, max_nb, scenes, job_mats, panels, acc, hdr, job_segments,
+                           ea.max_loop, n_sms, tie, wt, s, tail);
 }
 
 cudaError_t preload_trace_kernels() {

@@ -520,6 +520,7 @@ int32_t refill_batch(omg_ctx* ctx, BatchRec& B, const omg_job* jobs, uint32_t n_
                      uint32_t n_panels) {
   std::vector<DMat> old_mats = B.job_mats;
   std::vector<DPanel> old_panels = B.panels;
+  const LaunchShape old_shape = effective_shape(ctx, B);
   int32_t rc = fill_batch(ctx, B, jobs, n_jobs, panels, n_panels);
   if (rc) return rc;
   // materials and panels change rarely: re-upload only when they differ
@@ -538,8 +539,12 @@ int32_t refill_batch(omg_ctx* ctx, BatchRec& B, const omg_job* jobs, uint32_t n_
     CK(cudaMemcpyAsync(B.d_groups.p, B.groups.data(), B.groups.size() * sizeof(DPanelGroup),
                        cudaMemcpyHostToDevice, ctx->stream));
   }
-  // the context's launch shape changed since the graphs were recorded
-  if (std::memcmp(&B.shape, &ctx->shape, sizeof(LaunchShape)) != 0) {
+  // the context's launch shape changed since the graphs were recorded, or what
+  // the scenes allow (a scene's slot was given to another)
+  const LaunchShape new_shape = effective_shape(ctx, B);
+  if (std::memcmp(&B.shape, &ctx->shape, sizeof(LaunchShape)) != 0 || old_shape.solo_ok != new_shape.solo_ok ||
+      old_shape.box_only != new_shape.box_only || old_shape.spread_warps != new_shape.spread_warps ||
+      old_shape.mode != new_shape.mode || old_shape.tail_mode != new_shape.tail_mode) {
     B.shape = ctx->shape;
     if ((rc = build_graphs(ctx, B, B.graph_io != nullptr))) return rc;
   }

@@ -171,7 +171,10 @@ __device__ __forceinline__ bool solo_closest(const DScene& S, SoloShare& sh, flo
                     fabsf(oz) <= 7.0f * S.fast_m[2] && fabsf(dx) >= kTiny && fabsf(dy) >= kTiny && fabsf(dz) >= kTiny;
   uint32_t nn = 0, nl = 0, nh = 0;
   float best = FLT_MAX;          // the nearest hit so far
-  bool bail = false;             // a list is full
+  // a list is full; or the tree has no 4-wide form (a launch is chosen by the
+  // scenes it was recorded with, and a slot of the scene table may hold another
+  // scene by the time it runs)
+  bool bail = !BIN && S.root >= 0 && S.nodes4c == nullptr;
   uint32_t budget = S.walk_budget;
   if (S.root >= 0) {
     if (lane == 0) {

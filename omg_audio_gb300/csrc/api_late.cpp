@@ -155,7 +155,7 @@ int32_t omg_late_submit(omg_ctx* ctx, uint32_t field_id, const uint32_t* slots, 
       L.h_up.p[i] = DLateUpdate{slots[i], L.tick + 1, B->jobs[i].out_off, B->jobs[i].dir_off, a, 0};
       L.h_rj.p[i] = DReverbJob{(uint64_t)slots[i] * per, L.n_bins, L.nb, L.bin_dt, 0};
     }
-    std::memcpy(B->h_jobs.p, B->jobs.data(), n_jobs * sizeof(DJob));
+    stage_jobs(*B);
     CK(cudaMemcpyAsync(B->d_jobs.p, B->h_jobs.p, n_jobs * sizeof(DJob), cudaMemcpyHostToDevice, ctx->stream));
     cudaGraphExec_t g = nullptr;
     if ((rc = batch_graph(ctx, *B, &g))) return rc;

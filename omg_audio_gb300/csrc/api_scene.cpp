@@ -283,6 +283,7 @@ int32_t scene_upload_impl(omg_ctx* ctx, const float* pos, uint32_t nv, const uin
       }
     }
   }
+  ray_course(S->prim_geo, S->prim_mat, dmats, nb, S->hit_log, S->mean_path);
   uint32_t id = 1;  // lowest free slot of the fixed table
   while (id < kMaxScenes && ctx->scenes.count(id)) id++;
   if (id >= kMaxScenes) return OMG_E_INVALID;
@@ -442,7 +443,7 @@ int32_t omg_estimate_reverb(omg_ctx* ctx, const float* bins, uint32_t n_bins, ui
     rj[i].n_bins = n_bins;
     rj[i].nb = nb;
     rj[i].bin_dt = bin_dt;
-    rj[i].pad = 0;
+    rj[i].seg = 0;
   }
   cudaStream_t s = ctx->stream;
   CK(cudaMemcpyAsync(ctx->r_bins.p, bins, total * 4, cudaMemcpyHostToDevice, s));

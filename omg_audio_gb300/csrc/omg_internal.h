@@ -328,7 +328,7 @@ struct DReverbJob {
   uint32_t n_bins;
   uint32_t nb;
   float bin_dt;
-  uint32_t pad;
+  uint32_t seg;        // index of the job's segment count
 };
 cudaError_t launch_reverb(const DReverbJob* rj, uint32_t n_jobs, uint32_t max_bins, const float* bins,
                           omg_reverb* out, const uint32_t* job_segments, cudaStream_t s);

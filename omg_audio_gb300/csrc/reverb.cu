@@ -87,7 +87,7 @@ __global__ void __launch_bounds__(kReverbThreads)
     }
     if (lane == 0) {
       out[j].level[b] = fminf(sqrtf(late), 0.7f);
-      if (b == 0) out[j].segments = job_segments ? job_segments[j] : 0;
+      if (b == 0) out[j].segments = job_segments ? job_segments[rj[j].seg] : 0;
     }
     return;
   }

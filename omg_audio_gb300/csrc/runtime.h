@@ -93,6 +93,10 @@ struct SceneRec {
   std::vector<float> prim_geo;
   std::vector<uint32_t> prim_tri;
   std::vector<uint16_t> prim_mat;
+  // A ray's expected course (ray_course): per band the logarithm of what a hit
+  // leaves of its energy, and the mean distance between hits.
+  float hit_log[MAXB] = {};
+  float mean_path = 0.0f;
 };
 
 struct BatchRec {
@@ -102,6 +106,9 @@ struct BatchRec {
   uint32_t max_bins = 0;
   uint64_t n_out = 0, n_acc = 0, n_bin_floats = 0, n_dir_floats = 0;
   std::vector<DJob> jobs;
+  // Ray order of the jobs on the device (order_jobs): place[i] is job i's index
+  // in d_jobs and d_seg. Empty: the jobs' own order.
+  std::vector<uint32_t> place;
   std::vector<DMat> job_mats;
   std::vector<DPanel> panels;
   std::vector<DPanelGroup> groups;
@@ -158,6 +165,14 @@ struct BatchRec {
     if (done) cudaEventDestroy(done);
   }
 };
+
+// The batch's jobs into their pinned image, in their order on the device.
+inline void stage_jobs(BatchRec& B) {
+  if (B.place.empty())
+    std::memcpy(B.h_jobs.p, B.jobs.data(), B.n_jobs * sizeof(DJob));
+  else
+    for (uint32_t i = 0; i < B.n_jobs; i++) B.h_jobs.p[B.place[i]] = B.jobs[i];
+}
 
 struct Ticket {
   std::unique_ptr<BatchRec> batch;

@@ -77,5 +77,15 @@ float near_tie_pad(const std::vector<float>& prim_geo);
 void tri_normals(const float* pos, const uint32_t* idx, uint32_t n_tris, const uint16_t* tri_mat,
                  std::vector<float>& out);
 DMat make_dmat(const omg_material& m, uint32_t nb);
+// What a hit is expected to leave of a ray's energy (through with probability p,
+// or back), per band, added to sum[] with weight `area`.
+inline void add_hit_left(const DMat& m, uint32_t nb, float area, float sum[MAXB]) {
+  for (uint32_t b = 0; b < nb; b++) sum[b] += area * (m.p * m.wt[b] + (1.0f - m.p) * m.wr[b]);
+}
+// Its logarithm for the scene's mean over the primitives' area, per band, and the
+// mean distance between hits, 4 V / S of the bounding box's volume and the
+// primitives' area (prim_geo: 9 floats each).
+void ray_course(const std::vector<float>& prim_geo, const std::vector<uint16_t>& prim_mat,
+                const std::vector<DMat>& mats, uint32_t nb, float hit_log[MAXB], float& mean_path);
 
 }  // namespace omg

@@ -375,7 +375,7 @@ int32_t omg_mlp_train(omg_ctx* ctx, uint32_t id, const omg_mlp_train_config* tc,
       for (uint32_t i = 0; i < per_graph[k] && ce == cudaSuccess; i++) {
         ce = launch_mlp_rows(ra, E, true, cs);
         if (ce == cudaSuccess) ce = launch_mlp_dw(dw_args(M, M.train_s, B, E, 0), ctx->n_sms, cs);
-        if (ce == cudaSuccess) ce = launch_mlp_adamw(aa, ctx->n_sms, cs);
+        if (ce == cudaSuccess) ce = launch_mlp_adamw(aa, cs);
       }
       cudaGraph_t g = nullptr;
       const cudaError_t ee = cudaStreamEndCapture(cs, &g);

@@ -70,7 +70,7 @@ struct MlpAdamwArgs {
 cudaError_t mlp_net_init();
 cudaError_t launch_mlp_rows(const MlpRowsArgs& a, uint32_t members, bool train, cudaStream_t s);
 cudaError_t launch_mlp_dw(MlpDwArgs a, int n_sms, cudaStream_t s);
-cudaError_t launch_mlp_adamw(const MlpAdamwArgs& a, int n_sms, cudaStream_t s);
+cudaError_t launch_mlp_adamw(const MlpAdamwArgs& a, cudaStream_t s);
 cudaError_t launch_mlp_images(const MlpNet& net, const float* P, uint16_t* img, cudaStream_t s);
 cudaError_t launch_mlp_ensemble(const float* y, uint32_t members, uint32_t rows, uint32_t cols, const float* mean,
                                 const float* sd, float level, float* out_mean, float* out_std, float* out_spread,

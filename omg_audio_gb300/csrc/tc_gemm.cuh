@@ -66,6 +66,15 @@ __device__ __forceinline__ uint32_t tile_offset(uint32_t r, uint32_t k) {
   return (r >> 3) * kSbo + (k >> 3) * kLbo + (r & 7u) * 16u + (k & 7u) * 2u;
 }
 
+// A chain of dependent launches (launch_chained): a kernel's blocks may start
+// once every block of the one before has started, and wait here, their setup
+// done, for its end. Nothing that an earlier kernel writes is read, and nothing
+// that it reads is written, before.
+__device__ __forceinline__ void grid_wait() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 __device__ __forceinline__ void tmem_alloc(uint32_t* dst_smem, uint32_t ncols) {
   asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(dst_smem)),
                "r"(ncols)

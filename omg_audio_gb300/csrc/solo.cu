@@ -133,7 +133,7 @@ __global__ void __launch_bounds__(kSoloThreads, kSoloBlocks)
       h.m = nullptr;
       bool have;
       if (J.geom == OMG_GEOM_BOX) {
-        have = box_hit_body(J, job_mats, px, py, pz, dx, dy, dz, h);
+        have = box_hit(J, job_mats, px, py, pz, dx, dy, dz, h);
       } else {
         const DScene& S = scenes[J.scene];
         int prim = -1;

@@ -150,6 +150,73 @@ __device__ __forceinline__ bool first_of(const DScene& S, SoloShare& sh, uint32_
   return true;
 }
 
+// The near-tie rule's winner among the lanes' candidates (s, tr, t, prim; prim < 0:
+// none): the lowest surface, then triangle, then distance. Some lane has one.
+__device__ __forceinline__ void tie_winner(uint32_t s, uint32_t tr, float t, int prim, float& t_out, int& prim_out) {
+  constexpr unsigned FULL = 0xffffffffu;
+  const uint32_t s_min = __reduce_min_sync(FULL, prim >= 0 ? s : 0xFFFFFFFFu);
+  bool in = prim >= 0 && s == s_min;
+  const uint32_t tr_min = __reduce_min_sync(FULL, in ? tr : 0xFFFFFFFFu);
+  in = in && tr == tr_min;
+  const uint32_t t_bits = __reduce_min_sync(FULL, in ? __float_as_uint(t) : 0x7f800000u);
+  in = in && __float_as_uint(t) == t_bits;
+  prim_out = __shfl_sync(FULL, prim, __ffs((int)__ballot_sync(FULL, in)) - 1);
+  t_out = __uint_as_float(t_bits);
+}
+
+// Meshes of at most kSoloAll primitives (near-tie rule): every lane tests its
+// share of them all, which is the set of hits that the walk over the grown boxes
+// finds, and the rule depends on that set alone. In a 10 x 7 x 4 m room of few
+// triangles the walk's rounds, each a chain of loads, tests and votes, were 6100 of a
+// segment's 8200 cycles: 512 rays 340 -> 247 us, 4096 rays 467 -> 455 us (there
+// the shading that all lanes repeat is the larger part). 4096 rays in a room of
+// 112, 144 and 192 triangles 655, 682, 726 us by the walk; 480 us at 112 with
+// this limit, 506, 584, 658 us with 256.
+constexpr uint32_t kSoloAll = 128;
+template <bool WT>
+__device__ __noinline__ bool all_closest(const float4* __restrict__ prims, uint32_t n, float ox, float oy, float oz,
+                                            float dx, float dy, float dz, float& t_out, int& prim_out) {
+  constexpr unsigned FULL = 0xffffffffu;
+  constexpr uint32_t kEach = (kSoloAll + 31u) / 32u;
+  const uint32_t lane = threadIdx.x & 31u;
+  float t[kEach], best = FLT_MAX;
+  uint32_t s[kEach], tr[kEach];
+#pragma unroll
+  for (uint32_t r = 0; r < kEach; r++) {
+    const uint32_t i = 32u * r + lane;
+    t[r] = FLT_MAX;
+    if (32u * r < n && i < n) {
+      const float4 p0 = __ldg(prims + 3 * (size_t)i), p1 = __ldg(prims + 3 * (size_t)i + 1),
+                   p2 = __ldg(prims + 3 * (size_t)i + 2);
+      s[r] = __float_as_uint(p2.w);
+      tr[r] = __float_as_uint(p1.w);
+      float th;
+      if (WT ? ray_tri_wt_body(p0, p1, p2, ox, oy, oz, dx, dy, dz, th)
+             : ray_tri(p0, p1, p2, ox, oy, oz, dx, dy, dz, th))
+        t[r] = th;
+    }
+    best = fminf(best, t[r]);
+  }
+  __syncwarp();
+  best = __uint_as_float(__reduce_min_sync(FULL, __float_as_uint(best)));
+  if (best == FLT_MAX) return false;
+  const float win = best * (1.0f + kTieRel);
+  uint32_t bs = 0, btr = 0;
+  float bt = FLT_MAX;
+  int prim = -1;
+#pragma unroll
+  for (uint32_t r = 0; r < kEach; r++)
+    if (t[r] < FLT_MAX && t[r] <= win && (prim < 0 || tie_key_less(s[r], tr[r], t[r], bs, btr, bt))) {
+      bs = s[r];
+      btr = tr[r];
+      bt = t[r];
+      prim = (int)(32u * r + lane);
+    }
+  __syncwarp();
+  tie_winner(bs, btr, bt, prim, t_out, prim_out);
+  return true;
+}
+
 // The closest hit of one ray by the whole warp (every argument uniform). BIN:
 // over the binary tree (first-found rule only), whose boxes are the reference's
 // in every context; nodes4c is exact in first-found contexts alone. A walk that
@@ -164,6 +231,7 @@ __device__ __forceinline__ bool solo_closest(const DScene& S, SoloShare& sh, flo
   const uint32_t lane = threadIdx.x & 31u, lt = (1u << lane) - 1u, group = lane >> 2, sub = lane & 3u;
   if (S.n_prims == 0) return false;
   const float4* __restrict__ prims = WT ? S.prims_wt : S.prims;
+  if (TIE && S.n_prims <= kSoloAll) return all_closest<WT>(prims, S.n_prims, ox, oy, oz, dx, dy, dz, t_out, prim_out);
   const float ix = __frcp_rn(dx), iy = __frcp_rn(dy), iz = __frcp_rn(dz);
   // as walk_begin: the slab test by fma (near-tie rule) or minima and maxima
   const float kTiny = 8.673617379884035e-19f;   // 2^-60
@@ -324,14 +392,7 @@ __device__ __forceinline__ bool solo_closest(const DScene& S, SoloShare& sh, flo
     }
   }
   __syncwarp();
-  const uint32_t s_min = __reduce_min_sync(FULL, prim >= 0 ? s : 0xFFFFFFFFu);
-  bool in = prim >= 0 && s == s_min;
-  const uint32_t tr_min = __reduce_min_sync(FULL, in ? tr : 0xFFFFFFFFu);
-  in = in && tr == tr_min;
-  const uint32_t t_bits = __reduce_min_sync(FULL, in ? __float_as_uint(t) : kInf);
-  in = in && __float_as_uint(t) == t_bits;
-  prim_out = __shfl_sync(FULL, prim, __ffs((int)__ballot_sync(FULL, in)) - 1);
-  t_out = __uint_as_float(t_bits);
+  tie_winner(s, tr, t, prim, t_out, prim_out);
   return true;
 }
 

@@ -407,19 +407,20 @@ __global__ void __launch_bounds__(kDwThreads, 1) dw_kernel(const __grid_constant
   const MlpNet& N = g.net;
   const uint32_t L = N.n_layers;
   // this CTA's layer (widest first), member, feature block, input block, share
-  uint32_t u = blockIdx.x, l = 0, mh = 1, nh = 1;
+  uint32_t u = blockIdx.x, l = 0, mh = 1, nh = 1, splits = 1;
   for (uint32_t k = 0; k < L; k++) {
     l = k + 1 < L ? k + 1 : 0;
     mh = (N.L[l].op + 127u) / 128u;
     nh = (N.L[l].ip + kWide - 1) / kWide;
-    const uint32_t units = mh * nh * g.members * g.splits;
+    splits = l == 0 ? g.splits0 : g.splits;
+    const uint32_t units = mh * nh * g.members * splits;
     if (u < units) break;
     u -= units;
   }
   const MlpLayerDesc& D = N.L[l];
-  const uint32_t share = u % g.splits, h = (u / g.splits) % mh, nb = (u / g.splits / mh) % nh;
-  const uint32_t mi = u / (g.splits * mh * nh);                       // member of this launch
-  const uint32_t per = (g.tiles + g.splits - 1) / g.splits, tb = share * per, te = min(g.tiles, tb + per);
+  const uint32_t share = u % splits, h = (u / splits) % mh, nb = (u / splits / mh) % nh;
+  const uint32_t mi = u / (splits * mh * nh);                         // member of this launch
+  const uint32_t per = (g.tiles + splits - 1) / splits, tb = share * per, te = min(g.tiles, tb + per);
   if (tb >= te) {
     tc::grid_wait();
     return;
@@ -681,10 +682,13 @@ cudaError_t launch_mlp_dw(MlpDwArgs a, int n_sms, cudaStream_t s) {
     all += units(l);
     if (l > 0) wide += units(l);
   }
-  // shares of the row tiles: the layers beyond the first fill the chip once
-  // (the first, narrow one's CTAs are short and fill the gaps)
+  // Shares of the row tiles: the layers beyond the first fill the chip, the
+  // first, narrow one takes the multiprocessors that are left (one more block
+  // than the chip holds is a second wave).
   a.splits = std::max(1u, std::min(a.tiles, (uint32_t)n_sms / std::max(1u, wide)));
-  return launch_chained(dw_kernel, dim3(all * a.splits), kDwThreads, kDwSmem, s, a);
+  const uint32_t used = wide * a.splits, first = all - wide;
+  a.splits0 = std::max(1u, std::min(a.tiles, used < (uint32_t)n_sms ? ((uint32_t)n_sms - used) / first : 1u));
+  return launch_chained(dw_kernel, dim3(used + first * a.splits0), kDwThreads, kDwSmem, s, a);
 }
 
 cudaError_t launch_mlp_adamw(const MlpAdamwArgs& a, cudaStream_t s) {

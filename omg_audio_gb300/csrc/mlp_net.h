@@ -49,7 +49,8 @@ struct MlpRowsArgs {
 };
 struct MlpDwArgs {
   MlpNet net;
-  uint32_t tiles, members, member0, splits;   // splits: set by launch_mlp_dw
+  uint32_t tiles, members, member0;
+  uint32_t splits, splits0;              // set by launch_mlp_dw: shares of the row tiles, and for the first layer
   float* G;
   const uint16_t *xt, *at, *dzt;
   uint32_t* err;

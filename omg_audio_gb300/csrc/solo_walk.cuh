@@ -231,7 +231,9 @@ __device__ __forceinline__ bool solo_closest(const DScene& S, SoloShare& sh, flo
   const uint32_t lane = threadIdx.x & 31u, lt = (1u << lane) - 1u, group = lane >> 2, sub = lane & 3u;
   if (S.n_prims == 0) return false;
   const float4* __restrict__ prims = WT ? S.prims_wt : S.prims;
-  if (TIE && S.n_prims <= kSoloAll) return all_closest<WT>(prims, S.n_prims, ox, oy, oz, dx, dy, dz, t_out, prim_out);
+  // (a context that lowered the walk budget has its walks counted against it)
+  if (TIE && S.n_prims <= kSoloAll && S.walk_budget >= 2u * S.n_nodes + S.n_prims)
+    return all_closest<WT>(prims, S.n_prims, ox, oy, oz, dx, dy, dz, t_out, prim_out);
   const float ix = __frcp_rn(dx), iy = __frcp_rn(dy), iz = __frcp_rn(dz);
   // as walk_begin: the slab test by fma (near-tie rule) or minima and maxima
   const float kTiny = 8.673617379884035e-19f;   // 2^-60

@@ -122,8 +122,8 @@ __device__ __noinline__ void epoch_tally(const EpochArgs& ea, bool ended, bool p
 // memory, a column per thread. The 3-band near-tie kernel then has 16 bytes of
 // spill stores, against 184 with that state in registers.
 //
-// BOX: every job of the launch is a shoebox: no walk, every segment is one
-// shading pass.
+// BOX: every job of a launch without epochs is a shoebox: no walk, every segment
+// is one shading pass.
 template <int NB, bool TIE, bool WIDE, bool WT, bool BOX>
 __global__ void __launch_bounds__(256, 4) trace_kernel(const DJob* __restrict__ jobs, uint32_t n_jobs,
                                                        uint32_t total_rays, const DScene* __restrict__ scenes,
@@ -147,7 +147,7 @@ __global__ void __launch_bounds__(256, 4) trace_kernel(const DJob* __restrict__ 
   // 4 bands a column per thread in shared memory, so that it holds no
   // registers across the walk; for 8 bands in registers (there the shared
   // copy's loads and stores in every shading pass cost more than it saves)
-  constexpr bool kColdShared = NB <= 4;
+  constexpr bool kColdShared = NB <= 4 && !BOX;
   constexpr int kCols = kColdShared ? kMaxWarps * 32 : 1;
   __shared__ float s_e[kColdShared ? NB : 1][kCols];
   __shared__ float s_dist[kCols];
@@ -188,10 +188,11 @@ __global__ void __launch_bounds__(256, 4) trace_kernel(const DJob* __restrict__ 
   float walk_stack_t[STACK_DEPTH];
   uint32_t* err = &hdr->error;
   const WfState& rs = ea.st;
-  const uint32_t* rq = ea.in_q;
-  const uint32_t n_rays = ea.cur ? (rq ? ea.cur->n : total_rays) : total_rays;
-  uint32_t* fetch = ea.cur ? &ea.cur->fetch : &hdr->ray_counter;
-  const bool may_park = ea.cur && ea.out_q && n_rays > ea.park_min;
+  const bool epoch = !BOX && ea.cur;
+  const uint32_t* rq = BOX ? nullptr : ea.in_q;
+  const uint32_t n_rays = epoch ? (rq ? ea.cur->n : total_rays) : total_rays;
+  uint32_t* fetch = epoch ? &ea.cur->fetch : &hdr->ray_counter;
+  const bool may_park = epoch && ea.out_q && n_rays > ea.park_min;
   const uint32_t keep = (uint32_t)(((uint64_t)n_rays * ea.park_pct) / 100u);
   bool parking = false;
   uint32_t iters = 0;   // loop guard (warp-uniform: every lane runs every iteration)
@@ -199,7 +200,7 @@ __global__ void __launch_bounds__(256, 4) trace_kernel(const DJob* __restrict__ 
 
   // one segment from (p, d): a mesh walk, or (a shoebox) the shading pass
   // alone, which computes the box hit
-  auto begin_segment = [&](const DJob& J) { phase = BOX || J.geom == OMG_GEOM_BOX ? SHADE : WALK; };
+  auto begin_segment = [&](const DJob& J) { phase = J.geom == OMG_GEOM_BOX ? SHADE : WALK; };
 
   while (true) {
     if (++iters > ea.max_loop) {
@@ -249,37 +250,43 @@ __global__ void __launch_bounds__(256, 4) trace_kernel(const DJob* __restrict__ 
       if (exhausted) break;
       continue;
     }
-    if (BOX && exhausted && !ea.cur) {
-      // No refill, epoch or walk is left to look at: the lanes' rays to their
-      // ends. A call of few rays is one ray's chain of segments, some 1900 cycles
-      // each (1024 rays of 64 segments: 117 us a call with every segment through
-      // the loop below, 106 us here, 96 us with box_hit's quotients side by side
-      // and the wall's material loaded ahead of the receiver test).
+    if (BOX) {
+      // No walk, epoch or tail to look at: the lanes' rays on, in registers, until
+      // enough lanes wait for new ones (or to their ends, when there are none).
+      // A launch that fills the chip is bound by instructions (256 rooms of 8192
+      // rays: 6.48 ms with every segment through a loop that also served walks
+      // and epochs, 5.99 ms here), a call of few rays by one ray's chain of
+      // segments, some 1900 cycles each (1024 rays of 64 segments: 117 us a call
+      // through that loop, 106 us here, 96 us with box_hit's quotients side by
+      // side and the wall's material loaded ahead of the receiver test).
       float e[NB], dist = 0.0f;
       Pcg rng;
       uint32_t bounce = 0;
       cold_load(e, dist, rng.s, bounce);
       const DJob& J = jobs[ji];
       bool on = phase != IDLE;
-      while (__any_sync(FULL, on)) {
-        if (++iters > ea.max_loop) {
-          atomicOr(err, 8u);
-          break;
+      for (;;) {
+        if (on) {
+          Hit h;
+          h.t = FLT_MAX;
+          h.m = nullptr;
+          bool have = box_hit_body(J, job_mats, px, py, pz, dx, dy, dz, h);
+          if (J.n_groups) have = panels_hit(J, panels, groups, job_mats, px, py, pz, dx, dy, dz, have, h);
+          const float t_hit = have ? h.t : FLT_MAX;
+          const bool done = shade_segment<NB, true>(J, acc, h, have, t_hit, px, py, pz, dx, dy, dz, dist, e, rng);
+          bounce++;
+          if (done || bounce >= J.max_bounces) {
+            atomicAdd(job_segments + ji, bounce);
+            on = false;
+          }
         }
-        if (!on) continue;
-        Hit h;
-        h.t = FLT_MAX;
-        h.m = nullptr;
-        bool have = box_hit_body(J, job_mats, px, py, pz, dx, dy, dz, h);
-        if (J.n_groups) have = panels_hit(J, panels, groups, job_mats, px, py, pz, dx, dy, dz, have, h);
-        const bool done = shade_segment<NB, true>(J, acc, h, have, have ? h.t : FLT_MAX, px, py, pz, dx, dy, dz, dist, e, rng);
-        bounce++;
-        if (done || bounce >= J.max_bounces) {
-          atomicAdd(job_segments + ji, bounce);
-          on = false;
-        }
+        const uint32_t live = (uint32_t)__popc(__ballot_sync(FULL, on));
+        if (live == 0u || (!exhausted && lane_cap - live >= refill_min)) break;
+        if (++iters > ea.max_loop) break;
       }
-      break;
+      cold_save(e, dist, rng.s, bounce);
+      phase = on ? SHADE : IDLE;
+      continue;
     }
     // the epoch's park signal (sticky; raised only once its queue is drained)
     if (may_park && !parking) parking = *((volatile const uint32_t*)&ea.cur->park) != 0u;
@@ -289,48 +296,46 @@ __global__ void __launch_bounds__(256, 4) trace_kernel(const DJob* __restrict__ 
     // warp together
     int hit_prim = -1;
     float hit_t = FLT_MAX;
-    if (!BOX) {
-      Walk w;
-      w.stack_ref = walk_stack_ref;
-      w.stack_t = walk_stack_t;
-      w.cur = kDone;
-      w.leaf = 0;
-      bool walking = phase == WALK;
-      if (walking) walk_begin<TIE>(w, scenes[jobs[ji].scene], px, py, pz, dx, dy, dz, wide);
-      while (__any_sync(FULL, walking)) {
-        if (++iters > ea.max_loop) break;
-        bool over = false;
-        if (wide) {
-          if (walking)
-            over = walk_steps<TIE>(w, scenes[jobs[ji].scene], px, py, pz, dx, dy, dz, walk_budget, wide, err);
-        } else {
-          const float4* lp = nullptr;
-          if (walking) {
+    Walk w;
+    w.stack_ref = walk_stack_ref;
+    w.stack_t = walk_stack_t;
+    w.cur = kDone;
+    w.leaf = 0;
+    bool walking = phase == WALK;
+    if (walking) walk_begin<TIE>(w, scenes[jobs[ji].scene], px, py, pz, dx, dy, dz, wide);
+    while (__any_sync(FULL, walking)) {
+      if (++iters > ea.max_loop) break;
+      bool over = false;
+      if (wide) {
+        if (walking)
+          over = walk_steps<TIE>(w, scenes[jobs[ji].scene], px, py, pz, dx, dy, dz, walk_budget, wide, err);
+      } else {
+        const float4* lp = nullptr;
+        if (walking) {
+          const DScene& S = scenes[jobs[ji].scene];
+          lp = WT ? S.prims_wt : S.prims;
+          int st = walk_budget;
+          over = walk_nodes<TIE>(w, S, px, py, pz, st, err);
+        }
+        coop_leaf_rounds<TIE, WT>(w, walking && !over, lp, px, py, pz, dx, dy, dz, s_slots[threadIdx.x >> 5],
+                                  kCoopRounds, err);
+        if (walking && !over && w.cur == kDone && w.leaf == 0) {
+          over = true;
+          if (TIE) {
+            // an ambiguous near-tie window: the walk starts over in fixed mode
             const DScene& S = scenes[jobs[ji].scene];
-            lp = WT ? S.prims_wt : S.prims;
-            int st = walk_budget;
-            over = walk_nodes<TIE>(w, S, px, py, pz, st, err);
-          }
-          coop_leaf_rounds<TIE, WT>(w, walking && !over, lp, px, py, pz, dx, dy, dz, s_slots[threadIdx.x >> 5],
-                                    kCoopRounds, err);
-          if (walking && !over && w.cur == kDone && w.leaf == 0) {
-            over = true;
-            if (TIE) {
-              // an ambiguous near-tie window: the walk starts over in fixed mode
-              const DScene& S = scenes[jobs[ji].scene];
-              over = !walk_restart_fixed(w, S.root, S.walk_budget);
-            }
+            over = !walk_restart_fixed(w, S.root, S.walk_budget);
           }
         }
-        if (over) walking = false;
       }
-      if (iters > ea.max_loop) {
-        atomicOr(err, 8u);
-        break;
-      }
-      hit_prim = w.prim_best;
-      hit_t = w.t_best;
+      if (over) walking = false;
     }
+    if (iters > ea.max_loop) {
+      atomicOr(err, 8u);
+      break;
+    }
+    hit_prim = w.prim_best;
+    hit_t = w.t_best;
 
     // ---- one segment of the bounce loop (tracer.rs:103-200)
     bool ended = false, parked = false;
@@ -342,9 +347,7 @@ __global__ void __launch_bounds__(256, 4) trace_kernel(const DJob* __restrict__ 
       h.t = FLT_MAX;
       h.m = nullptr;
       bool have;
-      if (BOX) {
-        have = box_hit_body(J, job_mats, px, py, pz, dx, dy, dz, h);
-      } else if (J.geom == OMG_GEOM_BOX) {
+      if (J.geom == OMG_GEOM_BOX) {
         have = box_hit(J, job_mats, px, py, pz, dx, dy, dz, h);
       } else {
         const DScene& S = scenes[J.scene];
@@ -366,7 +369,7 @@ __global__ void __launch_bounds__(256, 4) trace_kernel(const DJob* __restrict__ 
       Pcg rng;
       uint32_t bounce;
       cold_load(e, dist, rng.s, bounce);
-      bool done = shade_segment<NB, BOX>(J, acc, h, have, t_hit, px, py, pz, dx, dy, dz, dist, e, rng);
+      bool done = shade_segment<NB>(J, acc, h, have, t_hit, px, py, pz, dx, dy, dz, dist, e, rng);
       bounce++;
       if (!done && bounce >= J.max_bounces) done = true;
       if (done) {
@@ -387,7 +390,7 @@ __global__ void __launch_bounds__(256, 4) trace_kernel(const DJob* __restrict__ 
       }
     }
     if (ea.cur) epoch_tally(ea, ended, parked, cold_rid(), may_park, n_rays, keep, fetch);
-    if (!BOX && tail.rays) {
+    if (tail.rays) {
       const unsigned em = __ballot_sync(FULL, ended);
       if (em && lane == 0) atomicAdd(&hdr->ended, (uint32_t)__popc(em));
       if (exhausted && total_rays - *((volatile const uint32_t*)&hdr->ended) <= tail.cap) {
@@ -704,8 +707,9 @@ cudaError_t launch_trace(const DJob* jobs, uint32_t n_jobs, uint32_t total_rays,
   }
   // Shoebox rays end at different lengths, a lane at a time, and a refill (job
   // lookup, sphere direction) for one lane costs as much as for many: 256 rooms
-  // of 8192 rays 7.75, 7.43, 7.08, 6.95, 7.02, 7.41 ms at 1, 2, 4, 6, 8, 12 idle
-  // lanes. Mesh walks are longer: there a lane is refilled at once.
+  // of 8192 rays 6.08, 5.99, 6.04 ms at 4, 6, 8 idle lanes (before the loop kept
+  // its rays in registers 7.75, 7.43, 7.08, 6.95, 7.02, 7.41 at 1, 2, 4, 6, 8,
+  // 12). Mesh walks are longer: there a lane is refilled at once.
   if (shape.box_only && lane_cap == 32u) refill = std::max(refill, 6u);
   TailArgs tail{nullptr, 0};
   if (!ep && tail_buf) tail = {tail_buf, tail_rays(shape, total_rays, n_sms)};
@@ -723,7 +727,7 @@ cudaError_t launch_trace(const DJob* jobs, uint32_t n_jobs, uint32_t total_rays,
     trace_wl_kernel<NB, false><<<blocks, threads, 0, s>>>(jobs, n_jobs, total_rays, scenes, job_mats, panels, \
                                                           groups, acc, hdr, job_segments, steps, wl_shade,    \
                                                           wide, ea);                                          \
-  else if (shape.box_only) OMG_TRACE_LAUNCH(NB, false, false, false, true);                                   \
+  else if (shape.box_only && !ep) OMG_TRACE_LAUNCH(NB, false, false, false, true);                            \
   else if (!tie) OMG_TRACE_LAUNCH(NB, false, false, false, false);                                            \
   else if (wide) OMG_TRACE_LAUNCH(NB, true, true, false, false);                                              \
   else if (wt) OMG_TRACE_LAUNCH(NB, true, false, true, false);                                                \

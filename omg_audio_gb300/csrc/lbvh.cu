@@ -351,7 +351,7 @@ cudaError_t lbvh_build(const float4* prims_in, uint32_t n, float4* prims_out, fl
 
 namespace {
 // Child boxes of every binary node grown by 2^-19 m[a] on each side, rounded
-// outward (DScene::nodes_f).
+// outward, axis by axis (DScene::nodes_f).
 __global__ void grow_nodes_kernel(const float4* __restrict__ in, float4* __restrict__ out, uint32_t n, float mx,
                                   float my, float mz, float pad) {
   const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
@@ -367,7 +367,8 @@ __global__ void grow_nodes_kernel(const float4* __restrict__ in, float4* __restr
       v[6 * c + a] = __fsub_rd(v[6 * c + a], g[a]);
       v[6 * c + 3 + a] = __fadd_ru(v[6 * c + 3 + a], g[a]);
     }
-  for (int i = 0; i < 4; i++) out[4 * k + i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+  for (int a = 0; a < 3; a++) out[4 * k + a] = make_float4(v[a], v[6 + a], v[3 + a], v[9 + a]);
+  out[4 * k + 3] = make_float4(v[12], v[13], v[14], v[15]);
 }
 }  // namespace
 

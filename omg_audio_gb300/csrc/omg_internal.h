@@ -69,7 +69,9 @@ struct DScene {
   // children over 4 lanes: 32 B per child, child k of node n at float4 index
   // 8 n + 2 k: (lo.x, lo.y, lo.z, hi.x), (hi.y, hi.z, ref bits, 0).
   const float4* nodes4c;
-  // `nodes` with every child box grown by 2^-19 M_a + pad on each side (M_a:
+  // `nodes`, axis by axis (n0 = (c0.lo.x, c1.lo.x, c0.hi.x, c1.hi.x), n1 the y's, n2
+  // the z's, n3 as in `nodes`: both children's faces side by side for the packed
+  // multiply-add), with every child box grown by 2^-19 M_a + pad on each side (M_a:
   // the scene's largest |coordinate| along axis a, plus 1 m; pad: 2^-17 x the
   // longest primitive edge), for the near-tie walks: the fused multiply-add
   // slab test of walks whose origin lies within |o_a| <= 7 M_a

@@ -645,15 +645,14 @@ void grow_nodes_for_fma(const std::vector<float>& dev_nodes, std::vector<float>&
         if (std::isfinite(v)) mx[j % 3] = std::max(mx[j % 3], v);
       }
   for (int a = 0; a < 3; a++) m[a] = mx[a] + 1.0f;
-  out = dev_nodes;
+  out = dev_nodes;   // the refs stay where they are
   for (size_t k = 0; k < n; k++)
     for (int c = 0; c < 2; c++)
       for (int a = 0; a < 3; a++) {
         const float grow = std::ldexp(m[a], -19) + pad;
-        float& lo = out[16 * k + 6 * c + a];
-        float& hi = out[16 * k + 6 * c + 3 + a];
-        lo = std::nextafter(lo - grow, -INFINITY);
-        hi = std::nextafter(hi + grow, INFINITY);
+        const float lo = dev_nodes[16 * k + 6 * c + a], hi = dev_nodes[16 * k + 6 * c + 3 + a];
+        out[16 * k + 4 * a + c] = std::nextafter(lo - grow, -INFINITY);
+        out[16 * k + 4 * a + 2 + c] = std::nextafter(hi + grow, INFINITY);
       }
 }
 

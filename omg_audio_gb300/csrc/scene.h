@@ -68,7 +68,7 @@ int32_t flatten_bvh4(const std::vector<float>& ref_boxes, const std::vector<uint
 // coordinate| plus 1 m). The first term covers the rounding of the fused
 // multiply-add slab test; pad (near_tie_pad) covers the hits Möller–Trumbore
 // accepts just outside a triangle, so that walks on these boxes find every
-// hit of every primitive.
+// hit of every primitive. Laid out axis by axis (DScene::nodes_f).
 void grow_nodes_for_fma(const std::vector<float>& dev_nodes, std::vector<float>& out, float m[3], float pad);
 // The same growth on reference-form boxes (6 floats each).
 void grow_ref_boxes(std::vector<float>& boxes, const float m[3], float pad);

@@ -236,12 +236,14 @@ __device__ __forceinline__ bool walk_nodes(Walk& w, const DScene& S, float ox, f
     if (w.flags & kWalkFast) {
       if (TIE) {
         const float oix = ox * w.ix, oiy = oy * w.iy, oiz = oz * w.iz;
-        h0 = ray_aabb_fma(n0.x, n0.y, n0.z, n0.w, n1.x, n1.y, oix, oiy, oiz, w.ix, w.iy, w.iz, tmax, ta);
-        h1 = ray_aabb_fma(n1.z, n1.w, n2.x, n2.y, n2.z, n2.w, oix, oiy, oiz, w.ix, w.iy, w.iz, tmax, tb);
+        ray_aabb_fma2(n0, n1, n2, oix, oiy, oiz, w.ix, w.iy, w.iz, tmax, h0, h1, ta, tb);
       } else {
         h0 = ray_aabb_minmax(n0.x, n0.y, n0.z, n0.w, n1.x, n1.y, ox, oy, oz, w.ix, w.iy, w.iz, tmax, ta);
         h1 = ray_aabb_minmax(n1.z, n1.w, n2.x, n2.y, n2.z, n2.w, ox, oy, oz, w.ix, w.iy, w.iz, tmax, tb);
       }
+    } else if (TIE) {
+      h0 = ray_aabb(n0.x, n1.x, n2.x, n0.z, n1.z, n2.z, ox, oy, oz, w.ix, w.iy, w.iz, tmax, ta);
+      h1 = ray_aabb(n0.y, n1.y, n2.y, n0.w, n1.w, n2.w, ox, oy, oz, w.ix, w.iy, w.iz, tmax, tb);
     } else {
       h0 = ray_aabb(n0.x, n0.y, n0.z, n0.w, n1.x, n1.y, ox, oy, oz, w.ix, w.iy, w.iz, tmax, ta);
       h1 = ray_aabb(n1.z, n1.w, n2.x, n2.y, n2.z, n2.w, ox, oy, oz, w.ix, w.iy, w.iz, tmax, tb);

@@ -313,7 +313,7 @@ typedef struct omg_tune_result {
     uint32_t blocks_per_sm;
     uint32_t refill_min;         /* a warp refills from the ray queue once this many lanes idle */
     uint32_t walk_steps;         /* traversal steps per lane per loop iteration (0 = whole walk) */
-    uint32_t shade_min;          /* lanes of a warp that shade together (1..32; 0 reads as 1) */
+    uint32_t shade_min;          /* 0..32, kept and returned; mode 0 shades all of a warp's rays together */
     uint32_t mode;               /* persistent kernel: 0 per-lane state machine, 1 warp-local wavefront
                                     (walks refill lane by lane; rays shade wl_shade_min at a time), 2 the same with
                                     each walk split over 4 lanes of a 4-wide tree (tie_mode 1 and

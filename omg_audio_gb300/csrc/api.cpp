@@ -1004,7 +1004,6 @@ int32_t omg_batch_autotune(omg_ctx* ctx, uint32_t id, uint32_t reps, omg_tune_re
   const uint32_t per_sm[] = {2, 4, 8};
   const uint32_t refill[] = {1, 8};
   const uint32_t walks[] = {0, 8, 32};
-  const uint32_t shade_mins[] = {1, 16, 32};
   const uint32_t wl_walks[] = {0, 4, 8, 16, 32};
   const uint32_t rounds[] = {16, 32, 48, 64, 96, 128, 192};
   const uint32_t tails[] = {0, 2048, 8192, 32768};
@@ -1034,17 +1033,15 @@ int32_t omg_batch_autotune(omg_ctx* ctx, uint32_t id, uint32_t reps, omg_tune_re
   for (uint32_t th : threads)
     for (uint32_t ps : per_sm) {
       for (uint32_t rf : refill)
-        for (uint32_t wk : walks)
-          for (uint32_t sm : shade_mins) {
-            if (rc || th * ps > 2048) continue;
-            LaunchShape sh;
-            sh.block_threads = th;
-            sh.blocks_per_sm = ps;
-            sh.refill_min = rf;
-            sh.walk_steps = wk;
-            sh.shade_min = sm;
-            rc = try_shape(sh);
-          }
+        for (uint32_t wk : walks) {
+          if (rc || th * ps > 2048) continue;
+          LaunchShape sh;
+          sh.block_threads = th;
+          sh.blocks_per_sm = ps;
+          sh.refill_min = rf;
+          sh.walk_steps = wk;
+          rc = try_shape(sh);
+        }
       for (uint32_t wk : wl_walks) {
         if (rc || th * ps > 2048) continue;
         LaunchShape sh;

@@ -202,7 +202,7 @@ struct LaunchShape {
   uint32_t blocks_per_sm = 4;
   uint32_t refill_min = 1;      // a warp refetches rays once this many lanes are idle
   uint32_t walk_steps = 0;      // traversal steps per lane per loop iteration (0 = a whole walk)
-  uint32_t shade_min = 32;      // lanes that shade together (or every waiting lane once none walks)
+  uint32_t shade_min = 32;      // kept in the interface: mode 0 shades all of a warp's rays after all of their walks
   uint32_t mode = 0;            // persistent kernel: 0 lane state machine, 1 warp-local wavefront,
                                 // 2 cooperative 4-lane walks
   uint32_t tail_mode = 0;       // the persistent kernel of epochs after the first

@@ -238,7 +238,7 @@ int32_t fill_batch(omg_ctx* ctx, BatchRec& B, const omg_job* jobs, uint32_t n_jo
   B.max_bins = 0;
   B.n_bin_floats = 0;
   B.n_dir_floats = 0;
-  bool coop_ok = P.tie_mode != 0, deep = false, box_only = true, solo_ok = true;
+  bool coop_ok = P.tie_mode != 0, deep = false, box_only = true, solo_ok = true, small = true;
   float last_time = 0.0f;
   // per-job panel materials are placed after all box wall materials
   for (uint32_t i = 0; i < n_jobs; i++) {
@@ -294,6 +294,7 @@ int32_t fill_batch(omg_ctx* ctx, BatchRec& B, const omg_job* jobs, uint32_t n_jo
       if (it->second->n_nodes4 == 0 && it->second->root >= 0) solo_ok = false;
       if (it->second->n_nodes4 == 0) coop_ok = false;
       if (it->second->n_prims > kSpreadPrims) deep = true;
+      if (it->second->n_prims > kSoloAll) small = false;
     } else {
       return OMG_E_INVALID;
     }
@@ -341,6 +342,7 @@ int32_t fill_batch(omg_ctx* ctx, BatchRec& B, const omg_job* jobs, uint32_t n_jo
   B.deep = deep;
   B.box_only = box_only;
   B.solo_ok = solo_ok;
+  B.small = small;
   B.n_acc = acc;
   B.n_out = out;
   return OMG_OK;
@@ -441,6 +443,7 @@ LaunchShape effective_shape(omg_ctx* ctx, const BatchRec& B) {
   if (B.deep) eff.spread_warps = 32;
   eff.box_only = B.box_only;
   eff.solo_ok = B.solo_ok;
+  eff.small = B.small;
   // cooperative walks need the near-tie rule and a 4-wide tree in every scene
   if (eff.mode == 2 && !B.coop_ok) eff.mode = 0;
   if (eff.tail_mode == 2 && !B.coop_ok) eff.tail_mode = 0;
@@ -608,6 +611,7 @@ int32_t refill_batch(omg_ctx* ctx, BatchRec& B, const omg_job* jobs, uint32_t n_
   // the scenes allow (a scene's slot was given to another)
   const LaunchShape new_shape = effective_shape(ctx, B);
   if (std::memcmp(&B.shape, &ctx->shape, sizeof(LaunchShape)) != 0 || old_shape.solo_ok != new_shape.solo_ok ||
+      old_shape.small != new_shape.small ||
       old_shape.box_only != new_shape.box_only || old_shape.spread_warps != new_shape.spread_warps ||
       old_shape.mode != new_shape.mode || old_shape.tail_mode != new_shape.tail_mode) {
     B.shape = ctx->shape;

@@ -219,6 +219,7 @@ struct LaunchShape {
   uint32_t spread_warps = 16;   // resident warps per multiprocessor that a launch of few rays is spread over (the
                                 // batch sets 32 when a scene's tree is beyond an L1: kSpreadPrims)
   bool solo_ok = false;         // every mesh scene can be walked by whole warps (solo.cu; set by the batch)
+  bool small = false;           // no mesh scene has more than kSoloAll primitives (set by the batch)
   bool box_only = false;        // every job of the launch is a shoebox (set by the batch)
   uint32_t loop_guard = 0;      // loop iterations of one warp of a persistent kernel before it stops
                                 // and flags error 8 (0: kDefaultLoopGuard); from omg_params.loop_guard
@@ -302,11 +303,13 @@ uint32_t tail_rays(const LaunchShape& shape, uint32_t total_rays, int n_sms);
 cudaError_t preload_trace_kernels();
 // solo.cu: the tracer for launches of few rays, one warp per ray (every mesh
 // scene has a 4-wide tree or is one leaf); max_loop as in EpochArgs. tail: the
-// rays that the persistent kernel of this launch has left, not the launch's own.
+// rays that the persistent kernel of this launch has left, not the launch's own;
+// small: no mesh scene has more than kSoloAll primitives.
+constexpr uint32_t kSoloAll = 128;
 cudaError_t launch_trace_solo(const DJob* jobs, uint32_t n_jobs, uint32_t total_rays, uint32_t max_nb,
                               const DScene* scenes, const DMat* job_mats, const DPanel* panels, float* acc,
                               DLaunch* hdr, uint32_t* job_segments, uint32_t max_loop, int n_sms, bool tie, bool wt,
-                              cudaStream_t s, TailArgs tail = {nullptr, 0});
+                              cudaStream_t s, bool small, TailArgs tail = {nullptr, 0});
 // coop.cu: the mode-2 persistent kernel (same arguments as launch_trace).
 cudaError_t launch_trace_coop(const DJob* jobs, uint32_t n_jobs, uint32_t total_rays, uint32_t max_nb,
                               const DScene* scenes, const DMat* job_mats, const DPanel* panels,

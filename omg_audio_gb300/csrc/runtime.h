@@ -147,6 +147,7 @@ struct BatchRec {
   bool deep = false;              // a scene beyond kSpreadPrims primitives
   bool box_only = false;          // every job is a shoebox
   bool solo_ok = false;           // every mesh scene has a 4-wide tree or is one leaf (solo.cu)
+  bool small = false;             // no mesh scene has more than kSoloAll primitives
   DevBuf<uint32_t> d_ep_q;        // epoch queues (2 x rays)
   DevBuf<float4> d_tail;          // rays left to the tail launch (trace.cu:tail_rays), allocated once a shape has one
   LaunchShape shape;

@@ -17,10 +17,13 @@ namespace omg {
 namespace {
 
 constexpr uint32_t kSoloThreads = 64;
-// Blocks a multiprocessor: 28 warps at 72 registers. (16: 200 bytes of spills,
-// 4096 rays on the 40-room world 845 against 811 us; 10 and 8: too few warps
-// for 4096 rays, 891 and 1066 us.)
-constexpr uint32_t kSoloBlocks = 14;
+// Blocks a multiprocessor: 24 warps at 80 registers for the walk (4096 rays on the
+// 40-room world, first-found and near-tie rule: 748 and 615 us a call, 766 and 668
+// at 14, 817 and 669 at 16, 796 and 675 at 11), 28 at 72 for launches of small
+// meshes alone (ALL), which carry no walk (4096 rays in a 12-triangle room 393 us,
+// 406 at 16, 466 at 12; 474 with the walk beside it).
+constexpr uint32_t kSoloBlocks = 12;
+constexpr uint32_t kAllBlocks = 14;
 
 // panels_hit (shade_common.cuh), one panel a lane: the reference's slab entry
 // test, the nearest entry, the lowest original index among equal ones.
@@ -73,14 +76,14 @@ __device__ __forceinline__ bool solo_panels(const DJob& J, const DPanel* __restr
   return true;
 }
 
-template <int NB, bool TIE, bool WT>
-__global__ void __launch_bounds__(kSoloThreads, kSoloBlocks)
+template <int NB, bool TIE, bool WT, bool ALL>
+__global__ void __launch_bounds__(kSoloThreads, ALL ? kAllBlocks : kSoloBlocks)
     solo_kernel(const DJob* __restrict__ jobs, uint32_t n_jobs, uint32_t total_rays, const DScene* __restrict__ scenes,
                 const DMat* __restrict__ job_mats, const DPanel* __restrict__ panels, float* __restrict__ acc,
                 DLaunch* __restrict__ hdr, uint32_t* __restrict__ job_segments, uint32_t max_loop, TailArgs tail) {
   constexpr unsigned FULL = 0xffffffffu;
-  __shared__ SoloShare s_share[kSoloThreads / 32];
-  SoloShare& sh = s_share[threadIdx.x >> 5];
+  __shared__ SoloShare s_share[ALL ? 1 : kSoloThreads / 32];
+  SoloShare& sh = s_share[ALL ? 0 : threadIdx.x >> 5];
   const uint32_t lane = threadIdx.x & 31u;
   uint32_t* err = &hdr->error;
   uint32_t iters = 0;   // loop guard
@@ -138,7 +141,8 @@ __global__ void __launch_bounds__(kSoloThreads, kSoloBlocks)
         const DScene& S = scenes[J.scene];
         int prim = -1;
         float t = FLT_MAX;
-        have = solo_closest<TIE, WT>(S, sh, px, py, pz, dx, dy, dz, t, prim, iters, max_loop, err);
+        if (ALL) have = small_closest<WT>(S, px, py, pz, dx, dy, dz, t, prim, err);
+        else have = solo_closest<TIE, WT>(S, sh, px, py, pz, dx, dy, dz, t, prim, iters, max_loop, err);
         if (have) {
           const float4 p0 = __ldg(S.prims + 3 * (size_t)prim + 0);
           const float4 p1 = __ldg(S.prims + 3 * (size_t)prim + 1);
@@ -166,22 +170,25 @@ __global__ void __launch_bounds__(kSoloThreads, kSoloBlocks)
 cudaError_t launch_trace_solo(const DJob* jobs, uint32_t n_jobs, uint32_t total_rays, uint32_t max_nb,
                               const DScene* scenes, const DMat* job_mats, const DPanel* panels, float* acc,
                               DLaunch* hdr, uint32_t* job_segments, uint32_t max_loop, int n_sms, bool tie, bool wt,
-                              cudaStream_t s, TailArgs tail) {
+                              cudaStream_t s, bool small, TailArgs tail) {
   const uint32_t per = kSoloThreads / 32;
-  const uint32_t need = ((tail.rays ? tail.cap : total_rays) + per - 1) / per, most = (uint32_t)n_sms * kSoloBlocks;
+  const uint32_t need = ((tail.rays ? tail.cap : total_rays) + per - 1) / per, most = (uint32_t)n_sms * (tie && small ? kAllBlocks : kSoloBlocks);
   const uint32_t blocks = need < most ? need : most;
-#define OMG_SOLO(NB, TIE, WT)                                                                                      \
-  solo_kernel<NB, TIE, WT><<<blocks, kSoloThreads, 0, s>>>(jobs, n_jobs, total_rays, scenes, job_mats, panels, acc, \
-                                                           hdr, job_segments, max_loop, tail)
+#define OMG_SOLO(NB, TIE, WT, ALL)                                                                              \
+  solo_kernel<NB, TIE, WT, ALL><<<blocks, kSoloThreads, 0, s>>>(jobs, n_jobs, total_rays, scenes, job_mats, panels, \
+                                                                acc, hdr, job_segments, max_loop, tail)
+#define OMG_SOLO_PICK(NB)                                      \
+  if (!tie) OMG_SOLO(NB, false, false, false);                 \
+  else if (small && wt) OMG_SOLO(NB, true, true, true);        \
+  else if (small) OMG_SOLO(NB, true, false, true);             \
+  else if (wt) OMG_SOLO(NB, true, true, false);                \
+  else OMG_SOLO(NB, true, false, false)
   if (max_nb <= 3) {
-    if (!tie) OMG_SOLO(3, false, false);
-    else if (wt) OMG_SOLO(3, true, true);
-    else OMG_SOLO(3, true, false);
+    OMG_SOLO_PICK(3);
   } else {
-    if (!tie) OMG_SOLO(8, false, false);
-    else if (wt) OMG_SOLO(8, true, true);
-    else OMG_SOLO(8, true, false);
+    OMG_SOLO_PICK(8);
   }
+#undef OMG_SOLO_PICK
 #undef OMG_SOLO
   return cudaGetLastError();
 }

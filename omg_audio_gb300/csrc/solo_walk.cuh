@@ -172,7 +172,10 @@ __device__ __forceinline__ void tie_winner(uint32_t s, uint32_t tr, float t, int
 // the shading that all lanes repeat is the larger part). 4096 rays in a room of
 // 112, 144 and 192 triangles 655, 682, 726 us by the walk; 480 us at 112 with
 // this limit, 506, 584, 658 us with 256.
-constexpr uint32_t kSoloAll = 128;
+// (A context that lowered the walk budget has its walks counted against it.)
+__device__ __forceinline__ bool small_mesh(const DScene& S) {
+  return S.n_prims <= kSoloAll && S.walk_budget >= 2u * S.n_nodes + S.n_prims;
+}
 template <bool WT>
 __device__ __noinline__ bool all_closest(const float4* __restrict__ prims, uint32_t n, float ox, float oy, float oz,
                                             float dx, float dy, float dz, float& t_out, int& prim_out) {
@@ -217,6 +220,23 @@ __device__ __noinline__ bool all_closest(const float4* __restrict__ prims, uint3
   return true;
 }
 
+// all_closest where it applies, else one lane's walk (a scene that took the slot
+// of the one this launch was recorded with).
+template <bool WT>
+__device__ __forceinline__ bool small_closest(const DScene& S, float ox, float oy, float oz, float dx, float dy,
+                                              float dz, float& t_out, int& prim_out, uint32_t* err) {
+  constexpr unsigned FULL = 0xffffffffu;
+  if (small_mesh(S)) return all_closest<WT>(WT ? S.prims_wt : S.prims, S.n_prims, ox, oy, oz, dx, dy, dz, t_out, prim_out);
+  bool have = false;
+  float t = 0.0f;
+  int prim = 0;
+  if ((threadIdx.x & 31u) == 0u) have = lane_closest<true>(S, ox, oy, oz, dx, dy, dz, t, prim, err);
+  __syncwarp();
+  t_out = __shfl_sync(FULL, t, 0);
+  prim_out = __shfl_sync(FULL, prim, 0);
+  return __shfl_sync(FULL, (int)have, 0) != 0;
+}
+
 // The closest hit of one ray by the whole warp (every argument uniform). BIN:
 // over the binary tree (first-found rule only), whose boxes are the reference's
 // in every context; nodes4c is exact in first-found contexts alone. A walk that
@@ -231,8 +251,7 @@ __device__ __forceinline__ bool solo_closest(const DScene& S, SoloShare& sh, flo
   const uint32_t lane = threadIdx.x & 31u, lt = (1u << lane) - 1u, group = lane >> 2, sub = lane & 3u;
   if (S.n_prims == 0) return false;
   const float4* __restrict__ prims = WT ? S.prims_wt : S.prims;
-  // (a context that lowered the walk budget has its walks counted against it)
-  if (TIE && S.n_prims <= kSoloAll && S.walk_budget >= 2u * S.n_nodes + S.n_prims)
+  if (TIE && small_mesh(S))
     return all_closest<WT>(prims, S.n_prims, ox, oy, oz, dx, dy, dz, t_out, prim_out);
   const float ix = __frcp_rn(dx), iy = __frcp_rn(dy), iz = __frcp_rn(dz);
   // as walk_begin: the slab test by fma (near-tie rule) or minima and maxima

@@ -667,7 +667,7 @@ cudaError_t launch_trace(const DJob* jobs, uint32_t n_jobs, uint32_t total_rays,
   if (!ep && shape.mode == 0 && !shape.wide && shape.solo_ok && !shape.box_only &&
       total_rays <= 2u * 28u * (uint32_t)n_sms)
     return launch_trace_solo(jobs, n_jobs, total_rays, max_nb, scenes, job_mats, panels, acc, hdr, job_segments,
-                             ea.max_loop, n_sms, tie, wt, s);
+                             ea.max_loop, n_sms, tie, wt, s, shape.small);
   if (shape.mode == 2 && tie && ea.st.pos)
     return launch_trace_coop(jobs, n_jobs, total_rays, max_nb, scenes, job_mats, panels, groups, acc, hdr,
                              job_segments, shape, n_sms, ea, s);
@@ -742,7 +742,7 @@ cudaError_t launch_trace(const DJob* jobs, uint32_t n_jobs, uint32_t total_rays,
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess || !tail.rays) return e;
   return launch_trace_solo(jobs, n_jobs, total_rays, max_nb, scenes, job_mats, panels, acc, hdr, job_segments,
-                           ea.max_loop, n_sms, tie, wt, s, tail);
+                           ea.max_loop, n_sms, tie, wt, s, shape.small, tail);
 }
 
 cudaError_t preload_trace_kernels() {

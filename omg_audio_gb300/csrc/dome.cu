@@ -204,7 +204,23 @@ __global__ void __launch_bounds__(kEscThreads, kEscBlocks) dome_escape_walk_kern
         }
       }
     } else if (active) {
+      // a panel whose rectangle misses the segment's box, grown by 1 cm (far more
+      // than the crossing's rounding), is not crossed on it: no division (256
+      // listeners 806 -> 791 us, 64 391 -> 385)
+      float lo[3], hi[3];
+      const float p[3] = {r.px, r.py, r.pz}, d[3] = {r.dx, r.dy, r.dz};
+#pragma unroll
+      for (int a = 0; a < 3; a++) {
+        const float q = p[a] + d[a] * t_mesh;
+        lo[a] = fminf(p[a], q) - 0.01f;
+        hi[a] = fmaxf(p[a], q) + 0.01f;
+      }
       for (uint32_t k = 0; k < L.n_panels; k++) {
+        const DDomePanel& P = L.panels[k];
+        const float alo = P.axis == 0 ? lo[0] : lo[1], ahi = P.axis == 0 ? hi[0] : hi[1];
+        const float llo = P.axis == 0 ? lo[1] : lo[0], lhi = P.axis == 0 ? hi[1] : hi[0];
+        if ((P.plane < alo) | (P.plane > ahi) | (P.lat1 < llo) | (P.lat0 > lhi) | (P.z1 < lo[2]) | (P.z0 > hi[2]))
+          continue;
         float t;
         if (panel_hit(L.panels[k], r.px, r.py, r.pz, r.dx, r.dy, r.dz, t_pan, t)) {
           t_pan = t;

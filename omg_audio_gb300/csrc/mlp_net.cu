@@ -44,52 +44,19 @@ constexpr uint32_t kWBytes = kWide * kWide * 2;
 constexpr uint32_t kRowsSmem = kTileBytes + kWBytes;
 constexpr uint32_t kPolls = 1u << 22;         // mbarrier poll limit (error 16 in the error word)
 
-// Two f32 side by side, for the packed operations: each rounds its two results as
-// the scalar ones do, in half the instructions (the epilogues are bound by them: 64
-// training steps 7.52 -> 7.46 ms).
-struct f2 {
-  unsigned long long v;
-};
-__device__ __forceinline__ f2 mk2(float a, float b) {
-  f2 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
-  return r;
-}
-__device__ __forceinline__ void un2(f2 x, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(x.v)); }
-__device__ __forceinline__ f2 mul2(f2 x, f2 y) {
-  f2 r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(x.v), "l"(y.v));
-  return r;
-}
-__device__ __forceinline__ f2 add2(f2 x, f2 y) {
-  f2 r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(x.v), "l"(y.v));
-  return r;
-}
-// 1 - x (the product by -1 is exact)
-__device__ __forceinline__ f2 one_minus2(f2 x) {
-  f2 r;
-  const f2 m = mk2(-1.0f, -1.0f), o = mk2(1.0f, 1.0f);
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(x.v), "l"(m.v), "l"(o.v));
-  return r;
+__device__ __forceinline__ float gelu_f(float z, float t) { return 0.5f * z * (1.0f + t); }
+
+// tanh form of GELU: the inner tanh, shared by the value and the derivative
+__device__ __forceinline__ float gelu_tanh(float z) {
+  const float k0 = 0.7978845608028654f, k1 = 0.044715f;
+  const float u = k0 * (z + k1 * z * z * z);
+  return tanhf(u);
 }
 
-// The tanh form of GELU and (GRAD) its derivative from one tanh, two values:
-//   u = k0 (z + k1 z^3), t = tanh u, y = z/2 (1 + t),
-//   y' = (1 + t)/2 + z/2 (1 - t^2) k0 (1 + 3 k1 z^2)
-template <bool GRAD>
-__device__ __forceinline__ void gelu2(float& z0, float& z1, float& g0, float& g1) {
+__device__ __forceinline__ float gelu_grad(float z, float t) {
   const float k0 = 0.7978845608028654f, k1 = 0.044715f;
-  const f2 z = mk2(z0, z1), kk0 = mk2(k0, k0), one = mk2(1.0f, 1.0f), half = mk2(0.5f, 0.5f);
-  const f2 u = mul2(kk0, add2(z, mul2(mul2(mul2(mk2(k1, k1), z), z), z)));
-  float u0, u1;
-  un2(u, u0, u1);
-  const f2 t = mk2(tanhf(u0), tanhf(u1)), hz = mul2(half, z), t1 = add2(one, t);
-  un2(mul2(hz, t1), z0, z1);
-  if (GRAD) {
-    const f2 du = mul2(kk0, add2(one, mul2(mul2(mk2(3.0f * k1, 3.0f * k1), z), z)));
-    un2(add2(mul2(half, t1), mul2(mul2(hz, one_minus2(mul2(t, t))), du)), g0, g1);
-  }
+  const float du = k0 * (1.0f + 3.0f * k1 * z * z);
+  return 0.5f * (1.0f + t) + 0.5f * z * (1.0f - t * t) * du;
 }
 
 __device__ __forceinline__ uint32_t pack2(float a, float b) {
@@ -169,7 +136,7 @@ __global__ void __launch_bounds__(kRowThreads, 1) rows_kernel(const __grid_const
   uint8_t* wbuf = smem + kTileBytes;           // the current layer's weights
   __shared__ __align__(8) uint64_t bar_w, bar_mma;
   __shared__ uint32_t taddr_s;
-  __shared__ __align__(8) float s_bias[kWide];
+  __shared__ float s_bias[kWide];
   const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
   const uint32_t row = (warp & 3u) * 32u + lane, cg = warp >> 2;   // TMEM lane, column group (4 of them)
   const uint32_t t0 = blockIdx.x, member = g.member0 + blockIdx.y;
@@ -294,9 +261,11 @@ __global__ void __launch_bounds__(kRowThreads, 1) rows_kernel(const __grid_const
         for_columns(my_lanes, col_lo(D.op), col_hi(D.op), [&](uint32_t c, float (&v)[16]) {
           float gp[16];
 #pragma unroll
-          for (int j = 0; j < 16; j += 2) {
-            un2(add2(mk2(v[j], v[j + 1]), *reinterpret_cast<const f2*>(s_bias + c + j)), v[j], v[j + 1]);
-            gelu2<TRAIN>(v[j], v[j + 1], gp[j], gp[j + 1]);
+          for (int j = 0; j < 16; j++) {
+            const float z = v[j] + s_bias[c + j];
+            const float t = gelu_tanh(z);
+            v[j] = gelu_f(z, t);
+            if (TRAIN) gp[j] = gelu_grad(z, t);
           }
           put16(tile, copy, row, c, v);
           if (TRAIN && l + 2 == L) {

@@ -175,7 +175,13 @@ float expected_hits(omg_ctx* ctx, const BatchRec& B, const DJob& d) {
     for (uint32_t b = 0; b < d.nb; b++) hit_log[b] = std::log(std::max(sum[b], 1e-6f));
     path = 4.0f * x * y * z / total;
   } else {
-    const SceneRec& S = *ctx->scenes.find(d.scene)->second;
+    SceneRec& S = *ctx->scenes.find(d.scene)->second;
+    if (!S.course) {
+      std::vector<DMat> mats;
+      for (const omg_material& m : S.materials) mats.push_back(make_dmat(m, S.n_bands));
+      ray_course(S.prim_geo, S.prim_mat, mats, S.n_bands, S.hit_log, S.mean_path);
+      S.course = true;
+    }
     std::memcpy(hit_log, S.hit_log, sizeof(hit_log));
     path = S.mean_path;
   }
@@ -198,7 +204,10 @@ float expected_hits(omg_ctx* ctx, const BatchRec& B, const DJob& d) {
 // ray's stream is numbered within its job, and the sums are exact.
 void order_jobs(omg_ctx* ctx, BatchRec& B, uint64_t rays) {
   B.place.clear();
-  if (B.n_jobs > 1 && rays > (uint64_t)ctx->n_sms * 1024u) {
+  bool alike = true;   // rays of one mesh live alike
+  for (const DJob& d : B.jobs)
+    alike = alike && d.geom == OMG_GEOM_MESH && d.scene == B.jobs[0].scene && d.dist_max == B.jobs[0].dist_max;
+  if (!alike && rays > (uint64_t)ctx->n_sms * 1024u) {
     std::vector<float> hits(B.n_jobs);
     std::vector<uint32_t> order(B.n_jobs);
     for (uint32_t i = 0; i < B.n_jobs; i++) {

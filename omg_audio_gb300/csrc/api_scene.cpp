@@ -283,7 +283,6 @@ int32_t scene_upload_impl(omg_ctx* ctx, const float* pos, uint32_t nv, const uin
       }
     }
   }
-  ray_course(S->prim_geo, S->prim_mat, dmats, nb, S->hit_log, S->mean_path);
   uint32_t id = 1;  // lowest free slot of the fixed table
   while (id < kMaxScenes && ctx->scenes.count(id)) id++;
   if (id >= kMaxScenes) return OMG_E_INVALID;

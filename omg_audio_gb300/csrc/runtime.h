@@ -93,8 +93,10 @@ struct SceneRec {
   std::vector<float> prim_geo;
   std::vector<uint32_t> prim_tri;
   std::vector<uint16_t> prim_mat;
-  // A ray's expected course (ray_course): per band the logarithm of what a hit
-  // leaves of its energy, and the mean distance between hits.
+  // A ray's expected course (ray_course), once a batch of several scenes asks:
+  // per band the logarithm of what a hit leaves of its energy, and the mean
+  // distance between hits.
+  bool course = false;
   float hit_log[MAXB] = {};
   float mean_path = 0.0f;
 };

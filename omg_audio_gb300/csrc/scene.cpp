@@ -720,21 +720,20 @@ DMat make_dmat(const omg_material& m, uint32_t nb) {
 
 void ray_course(const std::vector<float>& prim_geo, const std::vector<uint16_t>& prim_mat,
                 const std::vector<DMat>& mats, uint32_t nb, float hit_log[MAXB], float& mean_path) {
+  // an estimate: areas in f32, the box of the primitives' first corners
   std::vector<double> area(mats.size(), 0.0);
-  double total = 0.0;
   float lo[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, hi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
   for (size_t i = 0; i < prim_mat.size(); i++) {
     const float* g = &prim_geo[9 * i];
-    const double cx = (double)g[4] * g[8] - (double)g[5] * g[7], cy = (double)g[5] * g[6] - (double)g[3] * g[8],
-                 cz = (double)g[3] * g[7] - (double)g[4] * g[6];
-    const double a = 0.5 * std::sqrt(cx * cx + cy * cy + cz * cz);
-    area[prim_mat[i]] += a;
-    total += a;
+    const float cx = g[4] * g[8] - g[5] * g[7], cy = g[5] * g[6] - g[3] * g[8], cz = g[3] * g[7] - g[4] * g[6];
+    area[prim_mat[i]] += 0.5f * std::sqrt(cx * cx + cy * cy + cz * cz);
     for (int k = 0; k < 3; k++) {
-      lo[k] = std::min(lo[k], std::min(g[k], std::min(g[k] + g[3 + k], g[k] + g[6 + k])));
-      hi[k] = std::max(hi[k], std::max(g[k], std::max(g[k] + g[3 + k], g[k] + g[6 + k])));
+      lo[k] = g[k] < lo[k] ? g[k] : lo[k];
+      hi[k] = g[k] > hi[k] ? g[k] : hi[k];
     }
   }
+  double total = 0.0;
+  for (double a : area) total += a;
   float sum[MAXB] = {};
   for (size_t m = 0; m < mats.size(); m++)
     if (area[m] > 0.0) add_hit_left(mats[m], nb, (float)(area[m] / total), sum);

@@ -17,11 +17,12 @@ using namespace omg;
 namespace omg {
 
 // Scratch of one launch of `tiles` 128-row tiles of `members` members
-// (MlpRowsArgs): the images that the weight gradients read, GELU'(Z).
+// (MlpRowsArgs): the images that the weight gradients read, GELU'(Z), the bias
+// gradients' sums of 32 rows.
 struct MlpScratch {
   uint64_t tiles = 0;              // members x tiles
   DevBuf<uint16_t> xt, at, dzt;
-  DevBuf<float> gz;
+  DevBuf<float> gz, gb;
 };
 
 // One of the two chunks of rows in flight during inference.
@@ -108,6 +109,7 @@ int32_t ensure_scratch(omg_ctx* ctx, const MlpRec& M, MlpScratch& S, uint64_t ti
   CK(S.at.alloc(tiles * (L - 1) * 128u * M.cfg.hidden));
   CK(S.dzt.alloc(tiles * L * 128u * kMlpWide));
   CK(S.gz.alloc(tiles * (L - 1) * 128u * M.cfg.hidden));
+  CK(S.gb.alloc(tiles * 4u * L * kMlpWide));
   S.tiles = tiles;
   return OMG_OK;
 }
@@ -123,12 +125,12 @@ MlpRowsArgs rows_args(const MlpRec& M, const MlpScratch& S, const float* X, cons
   a.img = M.img.p;
   a.X = X;
   a.Y = Y;
-  a.G = M.G.p;
   a.loss = M.loss.p;
   a.xt = S.xt.p;
   a.at = S.at.p;
   a.dzt = S.dzt.p;
   a.gz = S.gz.p;
+  a.gb = S.gb.p;
   a.err = M.err.p;
   return a;
 }
@@ -143,6 +145,7 @@ MlpDwArgs dw_args(const MlpRec& M, const MlpScratch& S, uint32_t rows, uint32_t 
   a.xt = S.xt.p;
   a.at = S.at.p;
   a.dzt = S.dzt.p;
+  a.gb = S.gb.p;
   a.err = M.err.p;
   return a;
 }

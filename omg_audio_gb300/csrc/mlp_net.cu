@@ -41,7 +41,9 @@ constexpr uint32_t kWide = kMlpWide;          // widest layer, and the first lay
 constexpr uint32_t kRowThreads = 512;
 constexpr uint32_t kTileBytes = kRows * kWide * 2;
 constexpr uint32_t kWBytes = kWide * kWide * 2;
-constexpr uint32_t kRowsSmem = kTileBytes + kWBytes;
+constexpr uint32_t kSumFloats = 32u * 16u;    // column_sum16's scratch, a warp
+template <bool TRAIN>
+constexpr uint32_t kRowsSmem = kTileBytes + kWBytes + (TRAIN ? kRowThreads / 32u * kSumFloats * 4u : 0u);
 constexpr uint32_t kPolls = 1u << 22;         // mbarrier poll limit (error 16 in the error word)
 
 __device__ __forceinline__ float gelu_f(float z, float t) { return 0.5f * z * (1.0f + t); }
@@ -83,23 +85,34 @@ __device__ __forceinline__ void put16(uint8_t* tile, uint8_t* copy, uint32_t row
   }
 }
 
-// Sums of 16 columns over the warp's 32 rows, halving the columns a lane holds
-// at each step: 16 shuffles. Lane l (even) returns the sum of column
-// ((l >> 4) & 1) * 8 + ((l >> 3) & 1) * 4 + ((l >> 2) & 1) * 2 + ((l >> 1) & 1).
-__device__ __forceinline__ float column_sum16(float (&v)[16], uint32_t lane) {
+// Sums of 16 columns over the warp's 32 rows: row r, r + 8, r + 16, r + 24 one after
+// another for r = 0 .. 7, then those eight in order (a bias gradient's rounding moves
+// whole AdamW steps where the gradient is near zero, so the order stays what it was).
+// Through 2 KB of shared memory, a lane per half column: a row lies at 16 h + 4 k + i
+// (r = 8 k + 4 h + i), turned by its column, so neither the stores nor the loads
+// conflict. Lanes below 16 return their column's sum. (A halving tree of 16 shuffles
+// added in another order: rows_kernel 70.0 us for a training step of 4 x 38-256x4-192
+// at 4096 rows, 75.4 this way.)
+__device__ __forceinline__ float column_sum16(float* __restrict__ w, const float (&v)[16], uint32_t lane) {
+  const uint32_t p = ((lane & 4u) << 2) | ((lane >> 1) & 12u) | (lane & 3u);
 #pragma unroll
-  for (int h = 8; h >= 1; h >>= 1) {
-    const bool up = (lane & (2u * h)) != 0u;
+  for (uint32_t j = 0; j < 16; j++) w[32u * j + ((p + j) & 31u)] = v[j];
+  __syncwarp();
+  const uint32_t c = lane & 15u, at = (lane & 16u) + c;
+  float part[4];
 #pragma unroll
-    for (int j = 0; j < h; j++) {
-      const float keep = up ? v[j + h] : v[j], send = up ? v[j] : v[j + h];
-      v[j] = keep + __shfl_xor_sync(0xffffffffu, send, 2 * h);
-    }
+  for (uint32_t i = 0; i < 4; i++) {
+    part[i] = w[32u * c + ((at + i) & 31u)];
+#pragma unroll
+    for (uint32_t k = 1; k < 4; k++) part[i] += w[32u * c + ((at + 4u * k + i) & 31u)];
   }
-  return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
-}
-__device__ __forceinline__ uint32_t column_of(uint32_t lane) {
-  return ((lane >> 4) & 1u) * 8u + ((lane >> 3) & 1u) * 4u + ((lane >> 2) & 1u) * 2u + ((lane >> 1) & 1u);
+  __syncwarp();   // read before the next columns are stored
+  float t = part[0] + part[1];
+  t += part[2];
+  t += part[3];
+#pragma unroll
+  for (int i = 0; i < 4; i++) t += __shfl_down_sync(0xffffffffu, part[i], 16);
+  return t;
 }
 
 // The accumulator's columns [lo, hi) in chunks of 16 through f(column, values):
@@ -134,6 +147,7 @@ __global__ void __launch_bounds__(kRowThreads, 1) rows_kernel(const __grid_const
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* tile = smem;                        // the rows' activations (or gradients) of the current layer
   uint8_t* wbuf = smem + kTileBytes;           // the current layer's weights
+  float* sums = reinterpret_cast<float*>(wbuf + kWBytes) + (threadIdx.x >> 5) * kSumFloats;   // (training only)
   __shared__ __align__(8) uint64_t bar_w, bar_mma;
   __shared__ uint32_t taddr_s;
   __shared__ float s_bias[kWide];
@@ -201,6 +215,7 @@ __global__ void __launch_bounds__(kRowThreads, 1) rows_kernel(const __grid_const
 
   tc::grid_wait();
   const uint64_t mt = (uint64_t)blockIdx.y * gridDim.x + t0;       // this CTA's slot of the scratch arrays
+  float* gb = TRAIN ? g.gb + (mt * (kRows / 32u) + (warp & 3u)) * L * kWide : nullptr;   // these 32 rows' bias sums
   const uint32_t* idx = nullptr;
   uint64_t src_row = grow;
   if (TRAIN && g.perm) {
@@ -332,9 +347,8 @@ __global__ void __launch_bounds__(kRowThreads, 1) rows_kernel(const __grid_const
         }
         if (c + 16u < hi) load_y(c + 16u);
         put16(tile, copy, row, c, v);
-        const float s = column_sum16(v, lane);
-        const uint32_t col = c + column_of(lane);
-        if ((lane & 1u) == 0u && col < D.out) atomicAdd(g.G + (uint64_t)member * N.p_stride + D.b_off + col, s);
+        const float s = column_sum16(sums, v, lane);
+        if (lane < 16u) gb[l * kWide + c + lane] = s;
       });
       for (int o = 16; o > 0; o >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
       if (lane == 0) atomicAdd(g.loss + member, lsum * inv_n);
@@ -352,7 +366,7 @@ __global__ void __launch_bounds__(kRowThreads, 1) rows_kernel(const __grid_const
         if (ok) issue(D, true, D.op, false);
       }
       if (l == 0) break;
-      const MlpLayerDesc& Dl = N.L[l - 1];     // dZ of the layer below = dX * GELU'(Z)
+      // dZ of the layer below = dX * GELU'(Z)
       const uint32_t lo = col_lo(D.ip), hi = col_hi(D.ip);
       const float4* gd = reinterpret_cast<const float4*>(g.gz) + (mt * (L - 1u) + (l - 1u)) * (D.ip / 4u) * kRows + row;
       uint8_t* copy = reinterpret_cast<uint8_t*>(g.dzt + (mt * L + (l - 1u)) * (kRows * kWide));
@@ -385,8 +399,8 @@ __global__ void __launch_bounds__(kRowThreads, 1) rows_kernel(const __grid_const
           if (c + 16u < hi) load_g(c + 16u);
         }
         put16(tile, copy, row, c, v);
-        const float s = column_sum16(v, lane);
-        if ((lane & 1u) == 0u) atomicAdd(g.G + (uint64_t)member * N.p_stride + Dl.b_off + c + column_of(lane), s);
+        const float s = column_sum16(sums, v, lane);
+        if (lane < 16u) gb[(l - 1u) * kWide + c + lane] = s;
       });
     }
   }
@@ -402,17 +416,28 @@ bail:
   if (warp == 0) tc::tmem_dealloc(taddr, kRowsTmem<TRAIN>);
 }
 
-// The weight gradients: dW[out x in] = dZ^T A over the batch's row tiles, both
-// read MN-major from the tile images that rows_kernel left. A CTA takes 128
-// output features x up to 256 input features of one layer of one member over
-// one share of the row tiles, two tiles in flight (96 KB each), and adds its
-// share to the gradient. Bound by those loads: 96 KB a tile for 1024 cycles of
-// MMA. The row tiles are split so that the wide layers' CTAs of all members
-// fill the chip once (launch_mlp_dw).
+// The weight gradients: dW[out x in] = dZ^T A over the batch's rows, both read
+// MN-major from the tile images that rows_kernel left. The rows are summed in
+// shares (dw_shares), each a chain of MMAs into TMEM columns of its own. A CTA
+// takes 128 output features x up to 256 input features of one layer of one member
+// over consecutive shares, two row tiles in flight (96 KB each), adds its shares
+// up in their order and the result to the gradient; those with a layer's first share
+// also add the rows' bias sums in order (one store a feature: no atomic's arrival
+// order, so batches of up to two shares train to the same weights each time). Bound
+// by the tiles' loads: 96 KB each for 1024 cycles of MMA. 26.9 us for the training step
+// of 4 x 38-256x4-192 at 4096 rows, of 8 tiles a CTA; 25.1 us when the shares were cut
+// to fill the chip and the biases added by rows_kernel's atomics.
 constexpr uint32_t kDwThreads = 256;
 constexpr uint32_t kDwA = 16u * 16u * kRows;          // dZ: 16 feature blocks
 constexpr uint32_t kDwStage = kDwA + kTileBytes;
 constexpr uint32_t kDwSmem = 2u * kDwStage;
+constexpr uint32_t kDwTmem = 512;                     // one block a multiprocessor (its shared memory)
+// TMEM columns of one share's accumulator, nn columns wide
+__host__ __device__ __forceinline__ uint32_t dw_columns(uint32_t nn) {
+  uint32_t c = 32;
+  while (c < nn) c <<= 1;
+  return c;
+}
 
 __global__ void __launch_bounds__(kDwThreads, 1) dw_kernel(const __grid_constant__ MlpDwArgs g) {
   extern __shared__ __align__(1024) uint8_t smem[];
@@ -421,25 +446,24 @@ __global__ void __launch_bounds__(kDwThreads, 1) dw_kernel(const __grid_constant
   const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
   const MlpNet& N = g.net;
   const uint32_t L = N.n_layers;
-  // this CTA's layer (widest first), member, feature block, input block, share
-  uint32_t u = blockIdx.x, l = 0, mh = 1, nh = 1, splits = 1;
+  // this CTA's layer (widest first), member, feature block, input block, group of shares
+  uint32_t u = blockIdx.x, l = 0, mh = 1, nh = 1, per = 1, groups = 1;
   for (uint32_t k = 0; k < L; k++) {
     l = k + 1 < L ? k + 1 : 0;
     mh = (N.L[l].op + 127u) / 128u;
     nh = (N.L[l].ip + kWide - 1) / kWide;
-    splits = l == 0 ? g.splits0 : g.splits;
-    const uint32_t units = mh * nh * g.members * splits;
+    per = l == 0 ? g.group0 : g.group;
+    groups = (g.shares + per - 1) / per;
+    const uint32_t units = mh * nh * g.members * groups;
     if (u < units) break;
     u -= units;
   }
   const MlpLayerDesc& D = N.L[l];
-  const uint32_t share = u % splits, h = (u / splits) % mh, nb = (u / splits / mh) % nh;
-  const uint32_t mi = u / (splits * mh * nh);                         // member of this launch
-  const uint32_t per = (g.tiles + splits - 1) / splits, tb = share * per, te = min(g.tiles, tb + per);
-  if (tb >= te) {
-    tc::grid_wait();
-    return;
-  }
+  const uint32_t h = (u / groups) % mh, nb = (u / groups / mh) % nh;
+  const uint32_t mi = u / (groups * mh * nh);                         // member of this launch
+  const uint32_t s0 = (u % groups) * per, ns = min(per, g.shares - s0);
+  const uint32_t rb = s0 * g.share_rows, re = min(g.tiles * kRows, rb + ns * g.share_rows);   // its rows
+  const uint32_t tb = rb / kRows, te = (re + kRows - 1) / kRows;      // (a share may end in the middle of a tile)
   const uint32_t n0 = nb * kWide, nn = min(kWide, D.ip - n0);
   const uint32_t mo = min(128u, D.op - 128u * h);                     // output features here (the rest of M is unused)
   if (tid == 0) {
@@ -449,13 +473,13 @@ __global__ void __launch_bounds__(kDwThreads, 1) dw_kernel(const __grid_constant
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 0) tc::tmem_alloc(&taddr_s, 256);
+  if (warp == 0) tc::tmem_alloc(&taddr_s, kDwTmem);
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
   tc::grid_wait();
   const uint32_t taddr = taddr_s;
-  const uint32_t bz = mo * kRows * 2u, ba = nn * kRows * 2u;
+  const uint32_t bz = mo * kRows * 2u, ba = nn * kRows * 2u, cols = dw_columns(nn);
   bool ok = true;
   const uint32_t n = te - tb;
   if (tid == 0) {
@@ -473,14 +497,23 @@ __global__ void __launch_bounds__(kDwThreads, 1) dw_kernel(const __grid_constant
     load(0);
     if (n > 1) load(1);
     const uint32_t idesc = tc::idesc_bf16_f32(nn, 128u) | tc::kTransA | tc::kTransB;
+    uint32_t acc = taddr, in = 0;               // the share's columns, and its rows so far
     for (uint32_t i = 0; i < n && ok; i++) {
       const uint32_t b = i & 1u, ph = (i >> 1) & 1u;
       ok = tc::mbar_wait(&full[b], ph, kPolls);
       if (!ok) break;
       const uint32_t a0 = tc::smem_u32(smem + b * kDwStage), b0 = a0 + kDwA;
-      for (uint32_t s = 0; s < kRows / 16u; s++)
-        tc::mma_bf16(taddr, tc::smem_desc(a0 + 256u * s, 128u, 16u * kRows), tc::smem_desc(b0 + 256u * s, 128u, 16u * kRows),
-                     idesc, i > 0 || s > 0);
+      // the tile's rows of these shares, 16 a step
+      const uint32_t r0 = (tb + i) * kRows, first = (max(rb, r0) - r0) / 16u, last = (min(re, r0 + kRows) - r0) / 16u;
+      for (uint32_t s = first; s < last; s++) {
+        tc::mma_bf16(acc, tc::smem_desc(a0 + 256u * s, 128u, 16u * kRows),
+                     tc::smem_desc(b0 + 256u * s, 128u, 16u * kRows), idesc, in != 0u);
+        in += 16u;
+        if (in == g.share_rows) {
+          in = 0;
+          acc += cols;
+        }
+      }
       tc::mma_commit(&done[b]);
       // the stage is refilled once its MMAs are done, while the other stage's run
       if (i >= 1 && i + 1 < n) {
@@ -499,6 +532,23 @@ __global__ void __launch_bounds__(kDwThreads, 1) dw_kernel(const __grid_constant
       }
     }
   }
+  // the bias gradients of these features: their sums of 32 rows in order, while the products run
+  if (nb == 0 && s0 == 0 && tid >= kDwThreads - 128u) {
+    const uint32_t o = 128u * h + (tid & 127u);
+    if (o < D.out) {
+      constexpr uint32_t kAhead = 16;
+      const uint32_t groups32 = g.tiles * (kRows / 32u);          // a multiple of 4
+      const float* b = g.gb + ((uint64_t)mi * groups32 * L + l) * kWide + o;
+      float sum = 0.0f, v[kAhead];
+      for (uint32_t q = 0; q < groups32; q += kAhead) {
+#pragma unroll
+        for (uint32_t j = 0; j < kAhead; j++) v[j] = q + j < groups32 ? b[(uint64_t)(q + j) * L * kWide] : 0.0f;
+#pragma unroll
+        for (uint32_t j = 0; j < kAhead; j++) sum += v[j];
+      }
+      g.G[(uint64_t)(g.member0 + mi) * N.p_stride + D.b_off + o] = sum;
+    }
+  }
   if (!__syncthreads_or(!ok)) {
     tc::fence_after_sync();
     const uint32_t o = 128u * h + (warp & 3u) * 32u + lane;
@@ -508,6 +558,12 @@ __global__ void __launch_bounds__(kDwThreads, 1) dw_kernel(const __grid_constant
     for (uint32_t c = 16u * (warp >> 2); c < nn; c += 32u) {
       float v[16];
       tc::tmem_ld16(taddr + (((warp & 3u) * 32u) << 16) + c, v);
+      for (uint32_t q = 1; q < ns; q++) {
+        float t[16];
+        tc::tmem_ld16(taddr + (((warp & 3u) * 32u) << 16) + q * cols + c, t);
+#pragma unroll
+        for (int j = 0; j < 16; j++) v[j] += t[j];
+      }
       if (o < D.out) {
 #pragma unroll
         for (uint32_t q = 0; q < 16; q += 4) {
@@ -526,7 +582,7 @@ __global__ void __launch_bounds__(kDwThreads, 1) dw_kernel(const __grid_constant
   }
   tc::fence_before_sync();
   __syncthreads();
-  if (warp == 0) tc::tmem_dealloc(taddr, 256);
+  if (warp == 0) tc::tmem_dealloc(taddr, kDwTmem);
 }
 
 // bf16 copy of one parameter into its layer's image
@@ -674,9 +730,9 @@ static cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, uint32_t thre
 // The kernels' shared-memory limits (call it outside any stream capture,
 // before the first launch on a device; repeating it is harmless).
 cudaError_t mlp_net_init() {
-  cudaError_t e = cudaFuncSetAttribute(rows_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRowsSmem);
+  cudaError_t e = cudaFuncSetAttribute(rows_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRowsSmem<false>);
   if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(rows_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRowsSmem);
+  e = cudaFuncSetAttribute(rows_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRowsSmem<true>);
   if (e != cudaSuccess) return e;
   return cudaFuncSetAttribute(dw_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDwSmem);
 }
@@ -684,26 +740,51 @@ cudaError_t mlp_net_init() {
 cudaError_t launch_mlp_rows(const MlpRowsArgs& a, uint32_t members, bool train, cudaStream_t s) {
   if (a.rows == 0 || members == 0) return cudaSuccess;
   const dim3 grid((a.rows + kRows - 1) / kRows, members);
-  return launch_chained(train ? rows_kernel<true> : rows_kernel<false>, grid, kRowThreads, kRowsSmem, s, a);
+  return launch_chained(train ? rows_kernel<true> : rows_kernel<false>, grid, kRowThreads,
+                        train ? kRowsSmem<true> : kRowsSmem<false>, s, a);
+}
+
+// The shares of a batch's rows that a weight gradient is summed in: 512 rows each up
+// to eight of them, then an eighth, in multiples of 64. A sum's partition is part of
+// its result: AdamW makes whole steps of the roundings of near-zero gradients, so it
+// depends on the batch alone, not on the members or the chip.
+uint32_t dw_shares(uint32_t rows, uint32_t& share_rows) {
+  const uint32_t n = std::max(1u, std::min(8u, rows / 512u));
+  share_rows = ((rows + n - 1u) / n + 63u) / 64u * 64u;
+  return (rows + share_rows - 1u) / share_rows;
 }
 
 cudaError_t launch_mlp_dw(MlpDwArgs a, int n_sms, cudaStream_t s) {
   const uint32_t L = a.net.n_layers;
-  auto units = [&](uint32_t l) {
-    return ((a.net.L[l].op + 127u) / 128u) * ((a.net.L[l].ip + kWide - 1) / kWide) * a.members;
-  };
-  uint32_t wide = 0, all = 0;
+  uint32_t wide = 0, first = 0, width = 0;     // (member, feature block, input block) units; the widest input block
   for (uint32_t l = 0; l < L; l++) {
-    all += units(l);
-    if (l > 0) wide += units(l);
+    const MlpLayerDesc& D = a.net.L[l];
+    const uint32_t units = ((D.op + 127u) / 128u) * ((D.ip + kWide - 1) / kWide) * a.members;
+    (l == 0 ? first : wide) += units;
+    if (l > 0) width = std::max(width, D.ip);
   }
-  // Shares of the row tiles: the layers beyond the first fill the chip, the
-  // first, narrow one takes the multiprocessors that are left (one more block
-  // than the chip holds is a second wave).
-  a.splits = std::max(1u, std::min(a.tiles, (uint32_t)n_sms / std::max(1u, wide)));
-  const uint32_t used = wide * a.splits, first = all - wide;
-  a.splits0 = std::max(1u, std::min(a.tiles, used < (uint32_t)n_sms ? ((uint32_t)n_sms - used) / first : 1u));
-  return launch_chained(dw_kernel, dim3(used + first * a.splits0), kDwThreads, kDwSmem, s, a);
+  const uint32_t width0 = std::min(kWide, a.net.L[0].ip);
+  a.shares = dw_shares(a.tiles * kRows, a.share_rows);
+  // Shares a CTA, for the layers beyond the first and for the first, narrower one: as
+  // many as TMEM holds at most, and those whose largest CTA loads the least with all
+  // CTAs on the chip at once; where that cannot be, by the bound of a list schedule.
+  const uint32_t most = std::min(a.shares, kDwTmem / dw_columns(width)),
+                 most0 = std::min(a.shares, kDwTmem / dw_columns(width0));
+  uint64_t best = ~0ull;
+  for (uint32_t g = 1; g <= most; g++)
+    for (uint32_t g0 = 1; g0 <= most0; g0++) {
+      const uint64_t c = (uint64_t)g * (128u + width), c0 = (uint64_t)g0 * (128u + width0);
+      const uint64_t n = (uint64_t)wide * ((a.shares + g - 1) / g), n0 = (uint64_t)first * ((a.shares + g0 - 1) / g0);
+      uint64_t cost = std::max(c, c0);
+      if (n + n0 > (uint64_t)n_sms) cost += (n * c + n0 * c0) / (uint64_t)n_sms;
+      if (cost < best) {
+        best = cost;
+        a.group = g;
+        a.group0 = g0;
+      }
+    }
+  const uint32_t blocks = wide * ((a.shares + a.group - 1) / a.group) + first * ((a.shares + a.group0 - 1) / a.group0);
+  return launch_chained(dw_kernel, dim3(blocks), kDwThreads, kDwSmem, s, a);
 }
 
 cudaError_t launch_mlp_adamw(const MlpAdamwArgs& a, cudaStream_t s) {

@@ -32,14 +32,14 @@ struct MlpRowsArgs {
   const float* X;                        // [.. x in]: inference: raw, x_mean and x_sd apply; training: standardized
   const float *x_mean, *x_sd;
   float* out;                            // inference: [member][rows][out]
-  // training: targets, gradients (biases and loss are added here), scratch per
-  // (member of the launch, row tile): x image, hidden activation images, dZ
-  // images (128 x kMlpWide slots per layer), GELU'(Z) per hidden layer
+  // training: targets, the loss (added here), scratch per (member of the
+  // launch, row tile): x image, hidden activation images, dZ images (128 x
+  // kMlpWide slots per layer), GELU'(Z) per hidden layer, the bias gradients'
+  // sums of 32 rows (4 x layers x kMlpWide)
   const float* Y;
-  float* G;
   float* loss;
   uint16_t *xt, *at, *dzt;
-  float* gz;
+  float *gz, *gb;
   // rows of X and Y of this step: perm[half of the step's epoch][member][step in epoch][row]; null: row i
   const uint32_t* perm;
   uint64_t perm_half, perm_member;
@@ -50,9 +50,11 @@ struct MlpRowsArgs {
 struct MlpDwArgs {
   MlpNet net;
   uint32_t tiles, members, member0;
-  uint32_t splits, splits0;              // set by launch_mlp_dw: shares of the row tiles, and for the first layer
+  uint32_t shares, share_rows;           // set by launch_mlp_dw: the shares of the rows (dw_shares), and
+  uint32_t group, group0;                // the shares that a CTA takes, and of the first layer
   float* G;
   const uint16_t *xt, *at, *dzt;
+  const float* gb;
   uint32_t* err;
 };
 struct MlpAdamwArgs {
@@ -70,6 +72,8 @@ struct MlpAdamwArgs {
 
 cudaError_t mlp_net_init();
 cudaError_t launch_mlp_rows(const MlpRowsArgs& a, uint32_t members, bool train, cudaStream_t s);
+// The shares of `rows` rows that a weight gradient is summed in, and a share's rows (the last has what is left).
+uint32_t dw_shares(uint32_t rows, uint32_t& share_rows);
 cudaError_t launch_mlp_dw(MlpDwArgs a, int n_sms, cudaStream_t s);
 cudaError_t launch_mlp_adamw(const MlpAdamwArgs& a, cudaStream_t s);
 cudaError_t launch_mlp_images(const MlpNet& net, const float* P, uint16_t* img, cudaStream_t s);

@@ -27,8 +27,7 @@ struct MlpScratch {
 
 // One of the two chunks of rows in flight during inference.
 struct MlpChunk {
-  uint32_t cap = 0;
-  DevBuf<float> y, mean, std, spread;      // y: [member][row][out]
+  DevBuf<float> y, mean, std, spread;      // y: [member][row][out]; each grown by its own size (std by predict alone)
   cudaEvent_t done = nullptr;
   ~MlpChunk() {
     if (done) cudaEventDestroy(done);
@@ -468,13 +467,11 @@ int32_t surrogate_run(omg_ctx* ctx, uint32_t id, const float* x, uint32_t n, flo
   for (int k = 0; k < (n > chunk ? 2 : 1); k++) {
     MlpChunk& C = M.chunk[k];
     if (!C.done) CK(cudaEventCreateWithFlags(&C.done, cudaEventDisableTiming));
-    if (C.cap >= chunk && (!y_std || C.std.p)) continue;
-    C.cap = 0;
-    CK(C.y.alloc((size_t)chunk * no * E));
-    CK(C.mean.alloc((size_t)chunk * no));
-    if (y_std) CK(C.std.alloc((size_t)chunk * no));
-    CK(C.spread.alloc(chunk));
-    C.cap = chunk;
+    const size_t ny = (size_t)chunk * no;
+    if (C.y.n < ny * E) CK(C.y.alloc(ny * E));
+    if (C.mean.n < ny) CK(C.mean.alloc(ny));
+    if (y_std && C.std.n < ny) CK(C.std.alloc(ny));
+    if (C.spread.n < chunk) CK(C.spread.alloc(chunk));
   }
   auto submit = [&](uint64_t r0) -> int32_t {
     MlpChunk& C = M.chunk[(r0 / chunk) & 1u];

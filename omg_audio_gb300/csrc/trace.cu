@@ -391,9 +391,16 @@ __global__ void __launch_bounds__(256, 4) trace_kernel(const DJob* __restrict__ 
     }
     if (ea.cur) epoch_tally(ea, ended, parked, cold_rid(), may_park, n_rays, keep, fetch);
     if (tail.rays) {
+      // one lane counts and looks, and the warp goes by what it saw: other warps
+      // change the counter, and what follows needs all lanes
       const unsigned em = __ballot_sync(FULL, ended);
-      if (em && lane == 0) atomicAdd(&hdr->ended, (uint32_t)__popc(em));
-      if (exhausted && total_rays - *((volatile const uint32_t*)&hdr->ended) <= tail.cap) {
+      uint32_t left = 0;
+      if (lane == 0) {
+        if (em) atomicAdd(&hdr->ended, (uint32_t)__popc(em));
+        left = total_rays - *((volatile const uint32_t*)&hdr->ended);
+      }
+      left = __shfl_sync(FULL, left, 0);
+      if (exhausted && left <= tail.cap) {
         // every ray left in the launch is in some warp: no more than tail.cap are handed over
         const unsigned am = __ballot_sync(FULL, phase != IDLE);
         uint32_t base = 0;

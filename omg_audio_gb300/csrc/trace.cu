@@ -506,7 +506,9 @@ __global__ void __launch_bounds__(256, 4) trace_wl_kernel(const DJob* __restrict
       atomicOr(err, 8u);
       break;
     }
-    if (may_park && !parking) parking = *((volatile const uint32_t*)&ea.cur->park) != 0u;
+    // (one lane looks for the warp: another may raise the signal meanwhile, and the passes below need all lanes)
+    if (may_park && !parking)
+      parking = __shfl_sync(FULL, lane == 0 ? *((volatile const uint32_t*)&ea.cur->park) : 0u, 0) != 0u;
     if (parking && wk_cnt) {
       // rays waiting to walk are between two segments: park them as they are
       const uint32_t m = wk_cnt < 32u ? wk_cnt : 32u;

@@ -588,7 +588,9 @@ int32_t run_io(omg_ctx* ctx, BatchRec& B, float* bins, float* dirs, omg_reverb* 
 
 // New per-job values into a batch whose job layout is unchanged: the job
 // array is refilled (it travels with each launch), materials and panels are
-// re-uploaded only when they differ, graphs are rebuilt on a shape change.
+// re-uploaded only when they differ, graphs are rebuilt on a shape change. After
+// an error the batch is of no further use (its arrays hold what the device does
+// not): the caller drops it.
 int32_t refill_batch(omg_ctx* ctx, BatchRec& B, const omg_job* jobs, uint32_t n_jobs, const omg_panel* panels,
                      uint32_t n_panels) {
   std::vector<DMat> old_mats = B.job_mats;
@@ -644,7 +646,10 @@ int32_t one_shot(omg_ctx* ctx, const omg_job* jobs, uint32_t n_jobs, const omg_p
     }
   } else {
     int32_t rc = refill_batch(ctx, *ctx->cached, jobs, n_jobs, panels, n_panels);
-    if (rc) return rc;
+    if (rc) {
+      ctx->cached.reset();
+      return rc;
+    }
   }
   return run_io(ctx, *ctx->cached, bins, dirs, reverb);
 }

@@ -144,9 +144,11 @@ int32_t omg_late_submit(omg_ctx* ctx, uint32_t field_id, const uint32_t* slots, 
       if (L.cache.size() >= kLateCache) L.cache.erase(L.cache.begin());
       L.cache.emplace_back(new BatchRec());
       rc = batch_prepare(ctx, *L.cache.back(), jobs, n_jobs, panels, n_panels);
-      if (rc) L.cache.pop_back();
     }
-    if (rc) return rc;
+    if (rc) {
+      L.cache.pop_back();
+      return rc;
+    }
     B = L.cache.back().get();
     const uint64_t per = (uint64_t)L.n_bins * (L.nb + 3);
     for (uint32_t i = 0; i < n_jobs; i++) {

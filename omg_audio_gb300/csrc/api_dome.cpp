@@ -150,10 +150,8 @@ int32_t dome_submit(omg_ctx* ctx, DomeRec& D, const float* eyes, uint32_t n_eyes
   const uint64_t nr = (uint64_t)n_eyes * n_rays;
   auto pad = [](size_t bytes) { return (bytes + 15u) & ~(size_t)15u; };
   const size_t o_pan = pad(12ull * n_eyes), in_bytes = o_pan + pans.size() * sizeof(DDomePanel);
-  if (D.d_in.n < in_bytes) {
-    CK(D.d_in.alloc(in_bytes));
-    CK(D.h_in.alloc(in_bytes));
-  }
+  if (D.d_in.n < in_bytes) CK(D.d_in.alloc(in_bytes));
+  if (D.h_in.n < in_bytes) CK(D.h_in.alloc(in_bytes));
   DomeRec::Layout at;
   at.events = pad(sizeof(DLaunch));
   at.energy = at.events + pad(2 * sizeof(uint32_t));

@@ -27,7 +27,6 @@ struct EarlyRec {
   DevBuf<omg_chain> cand_chain, d_out;
   DevBuf<uint32_t> cand_slot;
   // solve scratch
-  size_t in_cap = 0, rec_cap = 0;
   DevBuf<uint8_t> d_in;            // one call's inputs: positions, blockers, chains, source ids
   std::vector<uint8_t> h_in;
   DevBuf<omg_mesh_record> d_rec;
@@ -220,6 +219,7 @@ int32_t omg_early_discover(omg_ctx* ctx, uint32_t early_id, const float listener
   const uint64_t n_cand = 3ull * n_rays;
   if (R->disc_rays < n_rays || R->disc_rays == 0) {
     const uint32_t nr = n_rays ? n_rays : 1u;
+    R->disc_rays = 0;   // (until all of them are there)
     CK(R->jitter.alloc(nr));
     CK(R->cand_key.alloc(3ull * nr));
     CK(R->cand_chain.alloc(3ull * nr));
@@ -274,15 +274,10 @@ int32_t omg_early_solve(omg_ctx* ctx, uint32_t early_id, const uint16_t* source_
   const size_t ex_off = 12ull * n_sources, ch_off = ex_off + n_extras * sizeof(omg_aabb),
                id_off = ch_off + n_chains * sizeof(omg_chain), bytes = id_off + 2ull * n_sources;
   static_assert(sizeof(omg_aabb) % 4 == 0 && sizeof(omg_chain) % 4 == 0 && alignof(omg_chain) <= 4, "packed inputs");
-  if (R->in_cap < bytes) {
-    CK(R->d_in.alloc(bytes));
-    R->in_cap = bytes;
-  }
-  if (R->rec_cap < n) {
-    CK(R->d_rec.alloc(n));
-    CK(R->d_live.alloc(1 + (n < kEarlySlice ? n : kEarlySlice)));
-    R->rec_cap = n;
-  }
+  const uint64_t n_live = 1 + (n < kEarlySlice ? n : kEarlySlice);
+  if (R->d_in.n < bytes) CK(R->d_in.alloc(bytes));
+  if (R->d_rec.n < n) CK(R->d_rec.alloc(n));
+  if (R->d_live.n < n_live) CK(R->d_live.alloc(n_live));
   R->h_in.resize(bytes);
   uint8_t* h = R->h_in.data();
   std::memcpy(h, source_pos, ex_off);

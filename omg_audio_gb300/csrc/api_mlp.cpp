@@ -289,6 +289,7 @@ int32_t omg_mlp_set_data(omg_ctx* ctx, uint32_t id, const float* x, const float*
   }
   int32_t rc = sync_norm(ctx, M);
   if (rc) return rc;
+  M.n_data = 0;   // (until both are there)
   CK(M.X.alloc(xs.size()));
   CK(M.Y.alloc(ys.size()));
   CK(cudaMemcpy(M.X.p, xs.data(), xs.size() * 4, cudaMemcpyHostToDevice));
@@ -327,10 +328,8 @@ int32_t omg_mlp_train(omg_ctx* ctx, uint32_t id, const omg_mlp_train_config* tc,
   const uint64_t half = (uint64_t)E * n, n_loss = (uint64_t)E * tc->epochs;
   CK(cudaStreamSynchronize(s));
   if (M.sched.n < sched.size()) CK(M.sched.alloc(sched.size()));
-  if (M.perm.n < 2 * half) {
-    CK(M.perm.alloc(2 * half));
-    CK(M.h_perm.alloc(2 * half));
-  }
+  if (M.perm.n < 2 * half) CK(M.perm.alloc(2 * half));
+  if (M.h_perm.n < 2 * half) CK(M.h_perm.alloc(2 * half));
   if (!M.counters.p) CK(M.counters.alloc(2));
   if (M.epoch_loss.n < n_loss) CK(M.epoch_loss.alloc(n_loss));
   int32_t rc = ensure_scratch(ctx, M, M.train_s, (uint64_t)E * (B / 128u));

@@ -397,12 +397,10 @@ int32_t omg_raycast(omg_ctx* ctx, uint32_t id, const float* o, const float* d, u
   if (!ctx || (n && (!o || !d || !t || !tri))) return OMG_E_INVALID;
   if (ctx->scenes.find(id) == ctx->scenes.end()) return OMG_E_NOT_FOUND;
   if (n == 0) return OMG_OK;
-  if (ctx->q_o.n < 3ull * n) {
-    CK(ctx->q_o.alloc(3ull * n));
-    CK(ctx->q_d.alloc(3ull * n));
-    CK(ctx->q_t.alloc(n));
-    CK(ctx->q_tri.alloc(n));
-  }
+  if (ctx->q_o.n < 3ull * n) CK(ctx->q_o.alloc(3ull * n));
+  if (ctx->q_d.n < 3ull * n) CK(ctx->q_d.alloc(3ull * n));
+  if (ctx->q_t.n < n) CK(ctx->q_t.alloc(n));
+  if (ctx->q_tri.n < n) CK(ctx->q_tri.alloc(n));
   if (!ctx->q_hdr.p) CK(ctx->q_hdr.alloc(1));
   cudaStream_t s = ctx->stream;
   CK(cudaMemsetAsync(ctx->q_hdr.p, 0, sizeof(DLaunch), s));
@@ -432,10 +430,8 @@ int32_t omg_estimate_reverb(omg_ctx* ctx, const float* bins, uint32_t n_bins, ui
     return OMG_E_INVALID;
   uint64_t per = (uint64_t)n_bins * nb, total = per * n_jobs;
   if (ctx->r_bins.n < total) CK(ctx->r_bins.alloc(total));
-  if (ctx->r_jobs.n < n_jobs) {
-    CK(ctx->r_jobs.alloc(n_jobs));
-    CK(ctx->r_out.alloc(n_jobs));
-  }
+  if (ctx->r_jobs.n < n_jobs) CK(ctx->r_jobs.alloc(n_jobs));
+  if (ctx->r_out.n < n_jobs) CK(ctx->r_out.alloc(n_jobs));
   std::vector<DReverbJob> rj(n_jobs);
   for (uint32_t i = 0; i < n_jobs; i++) {
     rj[i].bins_off = per * i;

@@ -7,6 +7,8 @@ seam, early_world.rs:36-48; mesh_record, pt_mesh.rs:186-337)."""
 from __future__ import annotations
 
 import ctypes as C
+import operator
+from array import array
 from typing import List, Sequence, Tuple
 
 import numpy as np
@@ -31,12 +33,24 @@ _RECORD = np.dtype(_lib.omg_mesh_record)
 
 
 def chains_to_c(chains: Sequence[Chain]):
-    """omg_chain records (three u16 surfaces and the u16 order each)."""
+    """omg_chain records (three u16 surfaces and the u16 order each). Integers alone;
+    one beyond 16 bits keeps its low ones, as assigned to a field."""
     arr = (_lib.omg_chain * max(1, len(chains)))()
     if len(chains):
-        flat = np.array([v for c, o in chains for v in (c[0], c[1], c[2], o)], np.int64).astype(np.uint16)
-        C.memmove(arr, _p(flat), C.sizeof(_lib.omg_chain) * len(chains))
+        flat = [v for c, o in chains for v in (c[0], c[1], c[2], o)]
+        try:
+            flat = array("H", flat)
+        except OverflowError:
+            flat = array("H", [operator.index(v) & 0xFFFF for v in flat])
+        C.memmove(arr, flat.buffer_info()[0], C.sizeof(_lib.omg_chain) * len(chains))
     return arr
+
+
+def extras_to_c(extras: Sequence):
+    """omg_aabb records of (mn, mx, transmission) triples, one of zeros for none."""
+    flat = array("f", [x for mn, mx, tr in extras
+                       for x in (mn[0], mn[1], mn[2], mx[0], mx[1], mx[2], tr[0], tr[1], tr[2])])
+    return np.frombuffer(flat, np.float32) if len(flat) else np.zeros(9, np.float32)
 
 
 class WorldEarly:
@@ -81,8 +95,7 @@ class WorldEarly:
         ns, nc = len(sources), len(chains)
         ids = np.array([s[0] for s in sources], np.uint16)
         pos = np.ascontiguousarray(np.array([s[1] for s in sources], np.float32).reshape(-1, 3))
-        ex = np.array([(mn[0], mn[1], mn[2], mx[0], mx[1], mx[2], tr[0], tr[1], tr[2]) for mn, mx, tr in extras]
-                      or [(0.0,) * 9], np.float32)                # omg_aabb records
+        ex = extras_to_c(extras)
         out = np.empty(max(1, ns * nc), _RECORD)   # every record is written by the call
         self.ctx._check(lib().omg_early_solve(self.ctx.h, self.id, _p(ids), _p(pos), ns, chains_to_c(chains), nc,
                                               _p(_f3(listener)), _p(ex), len(extras), _p(out)), "omg_early_solve")

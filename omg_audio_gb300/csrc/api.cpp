@@ -453,6 +453,7 @@ LaunchShape effective_shape(omg_ctx* ctx, const BatchRec& B) {
   eff.box_only = B.box_only;
   eff.solo_ok = B.solo_ok;
   eff.small = B.small;
+  eff.capped = ctx->prm.walk_budget != 0;
   // cooperative walks need the near-tie rule and a 4-wide tree in every scene
   if (eff.mode == 2 && !B.coop_ok) eff.mode = 0;
   if (eff.tail_mode == 2 && !B.coop_ok) eff.tail_mode = 0;
@@ -487,7 +488,10 @@ int32_t capture_graph(omg_ctx* ctx, BatchRec& B, cudaStream_t cs, bool io, int p
   cudaGraph_t g;
   int32_t rc = ensure_staging(ctx, B);
   if (rc) return rc;
-  const size_t tail = (size_t)kTailWords * tail_rays(effective_shape(ctx, B), B.total_rays, ctx->n_sms);
+  const LaunchShape eff = effective_shape(ctx, B);
+  const size_t tail = (size_t)kTailWords * tail_rays(eff, B.total_rays, ctx->n_sms);
+  B.capped = eff.capped;
+  B.loop_guard = eff.loop_guard;
   if (B.d_tail.n < tail) CK(B.d_tail.alloc(tail));
   cudaError_t e = cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal);
   if (e != cudaSuccess) return fail(ctx, e, "cudaStreamBeginCapture");
@@ -618,11 +622,11 @@ int32_t refill_batch(omg_ctx* ctx, BatchRec& B, const omg_job* jobs, uint32_t n_
   if (old_place != B.place)
     CK(cudaMemcpyAsync(B.d_rjobs.p, B.rjobs.data(), B.n_jobs * sizeof(DReverbJob), cudaMemcpyHostToDevice,
                        ctx->stream));
-  // the context's launch shape changed since the graphs were recorded, or what
-  // the scenes allow (a scene's slot was given to another)
+  // the context's launch shape or limits changed since the graphs were recorded,
+  // or what the scenes allow (a scene's slot was given to another)
   const LaunchShape new_shape = effective_shape(ctx, B);
   if (std::memcmp(&B.shape, &ctx->shape, sizeof(LaunchShape)) != 0 || old_shape.solo_ok != new_shape.solo_ok ||
-      old_shape.small != new_shape.small ||
+      old_shape.small != new_shape.small || B.capped != new_shape.capped || B.loop_guard != new_shape.loop_guard ||
       old_shape.box_only != new_shape.box_only || old_shape.spread_warps != new_shape.spread_warps ||
       old_shape.mode != new_shape.mode || old_shape.tail_mode != new_shape.tail_mode) {
     B.shape = ctx->shape;

@@ -193,6 +193,7 @@ int32_t dome_submit(omg_ctx* ctx, DomeRec& D, const float* eyes, uint32_t n_eyes
   L.events = reinterpret_cast<uint32_t*>(out + at.events);
   L.tie = ctx->prm.tie_mode;
   L.wt = ctx->prm.tri_test == OMG_TRI_WATERTIGHT ? 1u : 0u;
+  L.capped = ctx->prm.walk_budget != 0 ? 1u : 0u;
   L.n_sms = (uint32_t)ctx->n_sms;
   CK(launch_dome(L, s));
   CK(cudaMemcpyAsync(D.h_out.p, out, back, cudaMemcpyDeviceToHost, s));

@@ -521,6 +521,13 @@ __device__ __forceinline__ bool mesh_closest(const DScene& S, float ox, float oy
   return have;
 }
 
+// The same out of line: for kernels whose own walk leaves rare cases to it.
+template <bool TIE>
+__device__ __noinline__ bool lane_closest(const DScene& S, float ox, float oy, float oz, float dx, float dy, float dz,
+                                          float& t, int& prim, uint32_t* err) {
+  return mesh_closest<TIE>(S, ox, oy, oz, dx, dy, dz, t, prim, err);
+}
+
 // Closest hit with the near-tie rule (TIE = true above) over the 4-wide tree
 // (DScene::nodes4). A node step tests the 4 child boxes, tests the hit leaf
 // children at once and descends into the nearest hit internal child, pushing

@@ -125,8 +125,9 @@ __device__ __forceinline__ int escape_event(const DScene& S, const DDomeLaunch& 
 // multiprocessors, each waiting on its own loads and on its lanes' divergent
 // paths one after another; launch_dome therefore spreads the rays over the
 // warps that the chip holds.
+// SETTLE: as in trace.cu's trace_kernel.
 constexpr uint32_t kEscThreads = 128;
-template <int NB, bool TIE, bool WT>
+template <int NB, bool TIE, bool WT, bool SETTLE = false>
 __global__ void __launch_bounds__(kEscThreads, kEscBlocks) dome_escape_walk_kernel(DDomeLaunch L, uint32_t loop_guard,
                                                                                    uint32_t rays_per_warp) {
   __shared__ uint8_t s_slots[kEscThreads / 32][256];
@@ -172,10 +173,10 @@ __global__ void __launch_bounds__(kEscThreads, kEscBlocks) dome_escape_walk_kern
       bool over = false;
       if (walking) {
         int st = 1 << 30;   // the node phase runs until the warp's lanes hold leaves (bounded by the walk budget)
-        over = walk_nodes<TIE>(w, S, r.px, r.py, r.pz, st, err);
+        over = walk_nodes<TIE, SETTLE>(w, S, r.px, r.py, r.pz, st, err);
       }
-      coop_leaf_rounds<TIE, WT>(w, walking && !over, WT ? S.prims_wt : S.prims, r.px, r.py, r.pz, r.dx, r.dy, r.dz,
-                                s_slots[threadIdx.x >> 5], kCoopRounds, err);
+      coop_leaf_rounds<TIE, WT, SETTLE>(w, walking && !over, WT ? S.prims_wt : S.prims, r.px, r.py, r.pz, r.dx, r.dy,
+                                        r.dz, s_slots[threadIdx.x >> 5], kCoopRounds, err);
       if (walking && !over && w.cur == kDone && w.leaf == 0)
         over = !TIE || !walk_restart_fixed(w, S.root, S.walk_budget);
       if (over) walking = false;
@@ -184,6 +185,7 @@ __global__ void __launch_bounds__(kEscThreads, kEscBlocks) dome_escape_walk_kern
       atomicOr(err, 8u);
       break;
     }
+    if (SETTLE && active) walk_settle(w, S, r.px, r.py, r.pz, r.dx, r.dy, r.dz, err);
     // the panels: each lane its own ray against all of them, or, for few rays,
     // the whole warp on one ray at a time (80 instructions a ray against 25 a panel)
     int pan = -1;
@@ -520,14 +522,16 @@ cudaError_t launch_dome(const DDomeLaunch& L, cudaStream_t s) {
   while (rpw > 1 && total <= warps * (rpw / 2u)) rpw >>= 1;
   const uint32_t per_block = rpw * (kEscThreads / 32);
   const uint32_t blocks = (uint32_t)((total + per_block - 1) / per_block);
-#define OMG_ESCAPE(NB, TIE, WT) \
-  dome_escape_walk_kernel<NB, TIE, WT><<<blocks, kEscThreads, 0, s>>>(L, kDefaultLoopGuard, rpw)
+#define OMG_ESCAPE(NB, ...) \
+  dome_escape_walk_kernel<NB, __VA_ARGS__><<<blocks, kEscThreads, 0, s>>>(L, kDefaultLoopGuard, rpw)
   if (L.nb <= 3) {
-    if (!L.tie) OMG_ESCAPE(3, false, false);
+    if (!L.tie && L.capped) OMG_ESCAPE(3, false, false, true);
+    else if (!L.tie) OMG_ESCAPE(3, false, false);
     else if (L.wt) OMG_ESCAPE(3, true, true);
     else OMG_ESCAPE(3, true, false);
   } else {
-    if (!L.tie) OMG_ESCAPE(MAXB, false, false);
+    if (!L.tie && L.capped) OMG_ESCAPE(MAXB, false, false, true);
+    else if (!L.tie) OMG_ESCAPE(MAXB, false, false);
     else if (L.wt) OMG_ESCAPE(MAXB, true, true);
     else OMG_ESCAPE(MAXB, true, false);
   }

@@ -221,6 +221,7 @@ struct LaunchShape {
   bool solo_ok = false;         // every mesh scene can be walked by whole warps (solo.cu; set by the batch)
   bool small = false;           // no mesh scene has more than kSoloAll primitives (set by the batch)
   bool box_only = false;        // every job of the launch is a shoebox (set by the batch)
+  bool capped = false;          // the context has a walk budget of its own (set by the batch)
   uint32_t loop_guard = 0;      // loop iterations of one warp of a persistent kernel before it stops
                                 // and flags error 8 (0: kDefaultLoopGuard); from omg_params.loop_guard
 };
@@ -397,6 +398,7 @@ struct DDomeLaunch {
   uint32_t* events;           // escape events + through calls (2 counters)
   uint32_t tie;               // near-tie rule of the escape raycasts (omg_params.tie_mode)
   uint32_t wt;                // the scene carries exact vertices (watertight test)
+  uint32_t capped;            // the context has a walk budget of its own
   uint32_t n_sms;
 };
 cudaError_t launch_dome(const DDomeLaunch& L, cudaStream_t s);

@@ -153,7 +153,9 @@ struct BatchRec {
   DevBuf<uint32_t> d_ep_q;        // epoch queues (2 x rays)
   DevBuf<float4> d_tail;          // rays left to the tail launch (trace.cu:tail_rays), allocated once a shape has one
   LaunchShape shape;
-  // recorded when first needed (batch_graph)
+  // recorded when first needed (batch_graph), with these of the context's limits
+  bool capped = false;
+  uint32_t loop_guard = 0;
   cudaGraphExec_t graph = nullptr;         // device-only launch
   cudaGraphExec_t graph_io = nullptr;      // H2D jobs + launch + D2H results
   cudaGraphExec_t graph_a = nullptr;       // clear + trace

@@ -33,13 +33,6 @@ struct SoloShare {
   int hit_l[kSoloHits];
 };
 
-// The lane walk, for the cases above (called by one lane).
-template <bool TIE>
-__device__ __noinline__ bool lane_closest(const DScene& S, float ox, float oy, float oz, float dx, float dy, float dz,
-                                          float& t, int& prim, uint32_t* err) {
-  return mesh_closest<TIE>(S, ox, oy, oz, dx, dy, dz, t, prim, err);
-}
-
 // First-found rule: the hit that the reference's ordered walk ends with, from
 // the nh nearest hits of all leaves that the ray meets (nearest: `best`; kept up
 // to best * (1 + kNearRel)). That walk skips a leaf only when an earlier hit is

@@ -124,7 +124,11 @@ __device__ __noinline__ void epoch_tally(const EpochArgs& ea, bool ended, bool p
 //
 // BOX: every job of a launch without epochs is a shoebox: no walk, every segment
 // is one shading pass.
-template <int NB, bool TIE, bool WIDE, bool WT, bool BOX>
+//
+// SETTLE: first-found walks that run out of a budget which the caller lowered are
+// settled (walk_settle). A variant of its own: the call costs the others 62 bytes of
+// spills (64 pairs on the 40-room world, first-found rule, 10.07 -> 10.26 ms).
+template <int NB, bool TIE, bool WIDE, bool WT, bool BOX, bool SETTLE = false>
 __global__ void __launch_bounds__(256, 4) trace_kernel(const DJob* __restrict__ jobs, uint32_t n_jobs,
                                                        uint32_t total_rays, const DScene* __restrict__ scenes,
                                                        const DMat* __restrict__ job_mats,
@@ -315,10 +319,10 @@ __global__ void __launch_bounds__(256, 4) trace_kernel(const DJob* __restrict__ 
           const DScene& S = scenes[jobs[ji].scene];
           lp = WT ? S.prims_wt : S.prims;
           int st = walk_budget;
-          over = walk_nodes<TIE>(w, S, px, py, pz, st, err);
+          over = walk_nodes<TIE, SETTLE>(w, S, px, py, pz, st, err);
         }
-        coop_leaf_rounds<TIE, WT>(w, walking && !over, lp, px, py, pz, dx, dy, dz, s_slots[threadIdx.x >> 5],
-                                  kCoopRounds, err);
+        coop_leaf_rounds<TIE, WT, SETTLE>(w, walking && !over, lp, px, py, pz, dx, dy, dz,
+                                          s_slots[threadIdx.x >> 5], kCoopRounds, err);
         if (walking && !over && w.cur == kDone && w.leaf == 0) {
           over = true;
           if (TIE) {
@@ -334,6 +338,7 @@ __global__ void __launch_bounds__(256, 4) trace_kernel(const DJob* __restrict__ 
       atomicOr(err, 8u);
       break;
     }
+    if (SETTLE && phase == WALK) walk_settle(w, scenes[jobs[ji].scene], px, py, pz, dx, dy, dz, err);
     hit_prim = w.prim_best;
     hit_t = w.t_best;
 
@@ -723,10 +728,10 @@ cudaError_t launch_trace(const DJob* jobs, uint32_t n_jobs, uint32_t total_rays,
   TailArgs tail{nullptr, 0};
   if (!ep && tail_buf) tail = {tail_buf, tail_rays(shape, total_rays, n_sms)};
   if (tail.cap == 0) tail.rays = nullptr;
-#define OMG_TRACE_LAUNCH(NB, TIE, WIDE, WT, BOX)                                                              \
-  trace_kernel<NB, TIE, WIDE, WT, BOX><<<blocks, threads, 0, s>>>(jobs, n_jobs, total_rays, scenes, job_mats, \
-                                                                  panels, groups, acc, hdr, job_segments,     \
-                                                                  refill, steps, lane_cap, ea, tail)
+#define OMG_TRACE_LAUNCH(NB, ...)                                                                            \
+  trace_kernel<NB, __VA_ARGS__><<<blocks, threads, 0, s>>>(jobs, n_jobs, total_rays, scenes, job_mats, panels, \
+                                                           groups, acc, hdr, job_segments, refill, steps,    \
+                                                           lane_cap, ea, tail)
 #define OMG_TRACE_PICK(NB)                                                                                    \
   if (wl && tie)                                                                                              \
     trace_wl_kernel<NB, true><<<blocks, threads, 0, s>>>(jobs, n_jobs, total_rays, scenes, job_mats, panels,  \
@@ -737,6 +742,7 @@ cudaError_t launch_trace(const DJob* jobs, uint32_t n_jobs, uint32_t total_rays,
                                                           groups, acc, hdr, job_segments, steps, wl_shade,    \
                                                           wide, ea);                                          \
   else if (shape.box_only && !ep) OMG_TRACE_LAUNCH(NB, false, false, false, true);                            \
+  else if (!tie && shape.capped) OMG_TRACE_LAUNCH(NB, false, false, false, false, true);                      \
   else if (!tie) OMG_TRACE_LAUNCH(NB, false, false, false, false);                                            \
   else if (wide) OMG_TRACE_LAUNCH(NB, true, true, false, false);                                              \
   else if (wt) OMG_TRACE_LAUNCH(NB, true, false, true, false);                                                \

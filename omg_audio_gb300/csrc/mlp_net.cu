@@ -185,11 +185,13 @@ __global__ void __launch_bounds__(kRowThreads, 1) rows_kernel(const __grid_const
     loading = true;
   };
   auto wait_w = [&]() {
-    if (loading) {
-      ok = tc::mbar_wait(&bar_w, par_w, kPolls) && ok;
-      par_w ^= 1u;
-      loading = false;
+    if (!loading) return;
+    if (!tc::mbar_wait(&bar_w, par_w, kPolls)) {
+      ok = false;                              // still in flight: the block's end waits for it again
+      return;
     }
+    par_w ^= 1u;
+    loading = false;
   };
   // the tile (K features) times the weights read K-major (bwd = false: N = op)
   // or MN-major (bwd: N = ip), accumulated over K; the commit arrives on bar_mma
@@ -498,6 +500,7 @@ __global__ void __launch_bounds__(kDwThreads, 1) dw_kernel(const __grid_constant
     if (n > 1) load(1);
     const uint32_t idesc = tc::idesc_bf16_f32(nn, 128u) | tc::kTransA | tc::kTransB;
     uint32_t acc = taddr, in = 0;               // the share's columns, and its rows so far
+    uint32_t loaded = min(2u, n), issued = 0;   // tiles under way
     for (uint32_t i = 0; i < n && ok; i++) {
       const uint32_t b = i & 1u, ph = (i >> 1) & 1u;
       ok = tc::mbar_wait(&full[b], ph, kPolls);
@@ -515,21 +518,24 @@ __global__ void __launch_bounds__(kDwThreads, 1) dw_kernel(const __grid_constant
         }
       }
       tc::mma_commit(&done[b]);
+      issued = i + 1;
       // the stage is refilled once its MMAs are done, while the other stage's run
       if (i >= 1 && i + 1 < n) {
         ok = tc::mbar_wait(&done[b ^ 1u], ((i - 1) >> 1) & 1u, kPolls);
-        if (ok) load(i + 1);
+        if (ok) {
+          load(i + 1);
+          loaded = i + 2;
+        }
       }
     }
     // the last MMAs (and with them every earlier one)
     if (ok) ok = tc::mbar_wait(&done[(n - 1) & 1u], ((n - 1) >> 1) & 1u, kPolls);
     if (!ok) {
       if (g.err) atomicOr(g.err, 16u);
-      // one more bounded wait for what may be in flight
-      for (uint32_t b = 0; b < 2; b++) {
-        tc::mbar_wait(&full[b], 0, 1u << 16);
-        tc::mbar_wait(&done[b], 0, 1u << 16);
-      }
+      // one more bounded wait for what may be in flight: the last two loads, and the
+      // last MMAs issued (with them every earlier one)
+      for (uint32_t i = loaded > 2u ? loaded - 2u : 0u; i < loaded; i++) tc::mbar_wait(&full[i & 1u], (i >> 1) & 1u, kPolls);
+      if (issued) tc::mbar_wait(&done[(issued - 1u) & 1u], ((issued - 1u) >> 1) & 1u, kPolls);
     }
   }
   // the bias gradients of these features: their sums of 32 rows in order, while the products run

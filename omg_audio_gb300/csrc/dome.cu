@@ -169,7 +169,7 @@ __global__ void __launch_bounds__(kEscThreads, kEscBlocks) dome_escape_walk_kern
       walk_begin<TIE>(w, S, r.px, r.py, r.pz, r.dx, r.dy, r.dz, false);
       events++;
     }
-    while (__any_sync(FULL, walking) && ++iters <= loop_guard) {
+    while (__any_sync(FULL, walking) && (!TIE || ++iters <= loop_guard)) {
       bool over = false;
       if (walking) {
         int st = 1 << 30;   // the node phase runs until the warp's lanes hold leaves (bounded by the walk budget)

@@ -71,8 +71,7 @@ __device__ __forceinline__ bool raycast_ref(const DEarly& E, SoloShare* sh, floa
   int prim = 0;
   bool have;
   if (WARP) {
-    uint32_t iters = 0;
-    have = solo_closest<false, false, true>(E.S, *sh, ox, oy, oz, dx, dy, dz, t, prim, iters, 0xFFFFFFFFu, E.err);
+    have = solo_closest<false, false, true>(E.S, *sh, ox, oy, oz, dx, dy, dz, t, prim, E.err);
     __syncwarp();
   } else {
     have = mesh_closest<false>(E.S, ox, oy, oz, dx, dy, dz, t, prim, E.err);

@@ -303,7 +303,7 @@ uint32_t tail_rays(const LaunchShape& shape, uint32_t total_rays, int n_sms);
 // launch does not wait for the driver's lazy module loading.
 cudaError_t preload_trace_kernels();
 // solo.cu: the tracer for launches of few rays, one warp per ray (every mesh
-// scene has a 4-wide tree or is one leaf); max_loop as in EpochArgs. tail: the
+// scene has a 4-wide tree or is one leaf); max_loop as in EpochArgs, of every ray by itself. tail: the
 // rays that the persistent kernel of this launch has left, not the launch's own;
 // small: no mesh scene has more than kSoloAll primitives.
 constexpr uint32_t kSoloAll = 128;

@@ -86,8 +86,7 @@ __global__ void __launch_bounds__(kSoloThreads, ALL ? kAllBlocks : kSoloBlocks)
   SoloShare& sh = s_share[ALL ? 0 : threadIdx.x >> 5];
   const uint32_t lane = threadIdx.x & 31u;
   uint32_t* err = &hdr->error;
-  uint32_t iters = 0;   // loop guard
-  while (iters <= max_loop) {
+  for (;;) {
     uint32_t rid = 0, ji;
     float px, py, pz, dist, dx, dy, dz, e[NB];
     Pcg rng;
@@ -129,8 +128,13 @@ __global__ void __launch_bounds__(kSoloThreads, ALL ? kAllBlocks : kSoloBlocks)
     }
     const DJob& J = jobs[ji];
     bool done = false;
-    // one segment of the bounce loop (tracer.rs:103-200) a pass
-    while (!done && ++iters <= max_loop) {
+    // one segment of the bounce loop (tracer.rs:103-200) a pass; the loop guard counts
+    // two a segment, a walk and a shading pass, as a ray in a lane does (trace.cu)
+    while (!done) {
+      if (bounce >= max_loop / 2u) {
+        if (lane == 0) atomicOr(err, 8u);
+        return;
+      }
       Hit h;
       h.t = FLT_MAX;
       h.m = nullptr;
@@ -142,7 +146,7 @@ __global__ void __launch_bounds__(kSoloThreads, ALL ? kAllBlocks : kSoloBlocks)
         int prim = -1;
         float t = FLT_MAX;
         if (ALL) have = small_closest<WT>(S, px, py, pz, dx, dy, dz, t, prim, err);
-        else have = solo_closest<TIE, WT>(S, sh, px, py, pz, dx, dy, dz, t, prim, iters, max_loop, err);
+        else have = solo_closest<TIE, WT>(S, sh, px, py, pz, dx, dy, dz, t, prim, err);
         if (have) {
           const float4 p0 = __ldg(S.prims + 3 * (size_t)prim + 0);
           const float4 p1 = __ldg(S.prims + 3 * (size_t)prim + 1);
@@ -160,9 +164,8 @@ __global__ void __launch_bounds__(kSoloThreads, ALL ? kAllBlocks : kSoloBlocks)
       bounce++;
       if (bounce >= J.max_bounces) done = true;
     }
-    if (lane == 0 && done) atomicAdd(job_segments + ji, bounce);
+    if (lane == 0) atomicAdd(job_segments + ji, bounce);
   }
-  if (lane == 0) atomicOr(err, 8u);
 }
 
 }  // namespace

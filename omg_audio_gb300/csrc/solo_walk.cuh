@@ -237,8 +237,7 @@ __device__ __forceinline__ bool small_closest(const DScene& S, float ox, float o
 // lane's walk.
 template <bool TIE, bool WT, bool BIN = false>
 __device__ __forceinline__ bool solo_closest(const DScene& S, SoloShare& sh, float ox, float oy, float oz, float dx,
-                                             float dy, float dz, float& t_out, int& prim_out, uint32_t& iters,
-                                             uint32_t max_loop, uint32_t* err) {
+                                             float dy, float dz, float& t_out, int& prim_out, uint32_t* err) {
   constexpr unsigned FULL = 0xffffffffu;
   constexpr uint32_t kInf = 0x7f800000u;
   const uint32_t lane = threadIdx.x & 31u, lt = (1u << lane) - 1u, group = lane >> 2, sub = lane & 3u;
@@ -272,8 +271,7 @@ __device__ __forceinline__ bool solo_closest(const DScene& S, SoloShare& sh, flo
     nl = 1;
   }
   __syncwarp();
-  while ((nn | nl) != 0u && !bail) {
-    if (++iters > max_loop) break;
+  while ((nn | nl) != 0u && !bail) {   // (each round takes some of the budget)
     const float cull = TIE ? best * (1.0f + kTieRel) : FLT_MAX;   // (infinite before the first hit)
     if (nl >= 8u || nn == 0u || (nl != 0u && best == FLT_MAX)) {
       // ---- up to 8 leaves, four lanes each

@@ -307,8 +307,11 @@ __global__ void __launch_bounds__(256, 4) trace_kernel(const DJob* __restrict__ 
     w.leaf = 0;
     bool walking = phase == WALK;
     if (walking) walk_begin<TIE>(w, scenes[jobs[ji].scene], px, py, pz, dx, dy, dz, wide);
+    // the loop guard counts the rounds of near-tie walks, and first-found walks once,
+    // however many rounds they take: the walk's budget bounds those
+    if (!TIE && __any_sync(FULL, walking)) iters++;
     while (__any_sync(FULL, walking)) {
-      if (++iters > ea.max_loop) break;
+      if (TIE && ++iters > ea.max_loop) break;
       bool over = false;
       if (wide) {
         if (walking)

@@ -337,35 +337,38 @@ __device__ __forceinline__ bool walk_spec(Walk& w, const DScene& S, float ox, fl
   return false;
 }
 
-// The first-found walk of a lane on its own: the node phase, then its
-// postponed leaf, skipped if culled by now.
+// The first-found walk of a lane on its own, to its end or the allowance's: the
+// node phase, then its postponed leaf, skipped if culled by now, and on.
 __device__ __forceinline__ bool walk_first(Walk& w, const DScene& S, float ox, float oy, float oz, float dx, float dy,
                                            float dz, int steps, uint32_t* err) {
-  bool spent = walk_nodes<false>(w, S, ox, oy, oz, steps, err);
-  while (w.leaf < 0 && steps > 0) {
-    steps--;
-    if (w.budget == 0u) {
-      walk_spent<true>(w, err);
-      spent = true;
-      break;
-    }
-    w.budget--;
-    if (!walk_have(w) || w.leaf_t < w.t_best) {
-      const uint32_t code = ~(uint32_t)w.leaf;
-      const uint32_t start = code >> 3, end = start + (code & 7u) + 1u;
-      for (uint32_t i = start; i < end; i++) {
-        float t;
-        if (ray_tri(__ldg(S.prims + 3 * i), __ldg(S.prims + 3 * i + 1), __ldg(S.prims + 3 * i + 2), ox, oy, oz, dx, dy,
-                    dz, t) &&
-            (!walk_have(w) || t < w.t_best)) {
-          w.t_best = t;
-          w.prim_best = (int)i;
+  bool spent;
+  do {
+    spent = walk_nodes<false>(w, S, ox, oy, oz, steps, err);
+    while (w.leaf < 0 && steps > 0) {
+      steps--;
+      if (w.budget == 0u) {
+        walk_spent<true>(w, err);
+        spent = true;
+        break;
+      }
+      w.budget--;
+      if (!walk_have(w) || w.leaf_t < w.t_best) {
+        const uint32_t code = ~(uint32_t)w.leaf;
+        const uint32_t start = code >> 3, end = start + (code & 7u) + 1u;
+        for (uint32_t i = start; i < end; i++) {
+          float t;
+          if (ray_tri(__ldg(S.prims + 3 * i), __ldg(S.prims + 3 * i + 1), __ldg(S.prims + 3 * i + 2), ox, oy, oz, dx, dy,
+                      dz, t) &&
+              (!walk_have(w) || t < w.t_best)) {
+            w.t_best = t;
+            w.prim_best = (int)i;
+          }
         }
       }
+      w.leaf = 0;
+      walk_postpone<false>(w);
     }
-    w.leaf = 0;
-    walk_postpone<false>(w);
-  }
+  } while (!spent && steps > 0 && (w.cur != kDone || w.leaf < 0));
   if (spent) walk_settle(w, S, ox, oy, oz, dx, dy, dz, err);
   return w.cur == kDone && w.leaf == 0;
 }

@@ -38,3 +38,24 @@ def test_guard_counts_segments(rays):
         assert run(0) == want
         b.destroy()
         scene.release()
+
+
+@pytest.mark.parametrize("rays", [512, 20000])
+def test_guard_of_queued_walks(rays):
+    """Mode 1 with a whole walk an iteration: a walk and a shading pass a segment, and a few
+    iterations in which the queues run dry."""
+    with Context(TraceConfig(tie_mode=0, max_bounces=BOUNCES)) as ctx:
+        case = W.multiroom(seed=6)
+        scene = gpu_scene(ctx, case.recorder, _lib.BVH_SAH)
+        src, lis = case.pairs[0][:2]
+        b = ctx.batch([Job(src, lis, rays, seed=3, scene=scene)])
+        b.set_shape(mode=1, walk_steps=0, wf_rounds=0, epochs=0)
+        got = []
+        for guard in (0, 2 * BOUNCES + 8):
+            ctx.set_limits(loop_guard=guard)
+            b.launch()
+            (e, rv), = b.read()
+            got.append((rv.segments, e.bins.tobytes()))
+        assert got[0] == got[1]
+        b.destroy()
+        scene.release()

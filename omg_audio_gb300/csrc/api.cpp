@@ -556,6 +556,13 @@ int32_t check_kernel_flags(omg_ctx* ctx, const BatchRec& B) {
   return OMG_OK;
 }
 
+// While the batch runs: the pages that copy_results fills on the device's side.
+void populate_results(const BatchRec& B, float* bins, float* dirs) {
+  if (!B.direct) return;
+  populate_pages(bins, B.n_bin_floats * sizeof(float));
+  populate_pages(dirs, B.n_dir_floats * sizeof(float));
+}
+
 // The results of a finished batch into the caller's arrays: out of the pinned
 // image, or (direct) off the device on the context's stream.
 int32_t copy_results(omg_ctx* ctx, const BatchRec& B, float* bins, float* dirs, omg_reverb* reverb) {
@@ -584,6 +591,7 @@ int32_t run_io(omg_ctx* ctx, BatchRec& B, float* bins, float* dirs, omg_reverb* 
   if (rc) return rc;
   CK(cudaGraphLaunch(B.graph_io, ctx->stream));
   CK(cudaEventRecord(B.done, ctx->stream));
+  populate_results(B, bins, dirs);
   rc = wait_event(ctx, B.done, timeout_of(ctx));
   if (rc) return rc;
   if ((rc = check_kernel_flags(ctx, B))) return rc;
@@ -852,6 +860,7 @@ int32_t omg_batch_read(omg_ctx* ctx, uint32_t id, float* bins, float* dirs, omg_
   int32_t rc = record_readback(ctx, B, ctx->stream);
   if (rc) return rc;
   CK(cudaEventRecord(B.done, ctx->stream));
+  populate_results(B, bins, dirs);
   if ((rc = wait_event(ctx, B.done, timeout_of(ctx)))) return rc;
   if ((rc = check_kernel_flags(ctx, B))) return rc;
   return copy_results(ctx, B, bins, dirs, reverb);

@@ -498,6 +498,10 @@ int32_t surrogate_run(omg_ctx* ctx, uint32_t id, const float* x, uint32_t n, flo
   if ((rc = submit(0))) return rc;
   for (uint64_t r0 = 0; r0 < n; r0 += chunk) {
     if (n - r0 > chunk && (rc = submit(r0 + chunk))) return rc;
+    if (r0 == 0) {
+      populate_pages(y_mean, (size_t)n * no * 4);
+      populate_pages(y_std, (size_t)n * no * 4);
+    }
     MlpChunk& C = M.chunk[(r0 / chunk) & 1u];
     const uint64_t rows = std::min<uint64_t>(chunk, n - r0);
     if ((rc = wait_event(ctx, C.done, timeout_of(ctx)))) return rc;

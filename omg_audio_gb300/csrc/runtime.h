@@ -11,6 +11,9 @@
 #include <thread>
 #include <vector>
 
+#include <sys/mman.h>
+#include <unistd.h>
+
 #include "omg_internal.h"
 #include "scene.h"
 
@@ -55,6 +58,31 @@ struct PinBuf {
     return e;
   }
 };
+
+// Brings the pages of a caller's array in, its bytes unchanged, before the device
+// copies into them: the device faults pages that are not there yet in one by one (a
+// query of 76.8 MB into a new array 43 ms, this way 2.7, into one in use 1.1; a batch
+// of 197 MB 12.2, 5.8 and 3.3). Where the kernel does not know the request, nothing
+// happens.
+inline void populate_pages(void* p, size_t bytes) {
+#ifdef MADV_POPULATE_WRITE
+  if (!p || bytes < (256u << 10)) return;
+  const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE), lo = (uintptr_t)p & ~(page - 1u),
+                  hi = ((uintptr_t)p + bytes + page - 1u) & ~(page - 1u);
+  const size_t n = (hi - lo) / page;
+  // an array in use: nothing to do (asking for its pages all the same takes 0.3 ms for 76.8 MB)
+  std::vector<unsigned char> in(n);
+  if (mincore(reinterpret_cast<void*>(lo), hi - lo, in.data()) == 0 &&
+      std::all_of(in.begin(), in.end(), [](unsigned char c) { return (c & 1u) != 0u; }))
+    return;
+  const uintptr_t part = (n + 3u) / 4u * page;
+#pragma omp parallel for num_threads(4) schedule(static)
+  for (int i = 0; i < 4; i++) {
+    const uintptr_t at = lo + (uintptr_t)i * part, end = std::min(hi, at + part);
+    if (at < end) madvise(reinterpret_cast<void*>(at), end - at, MADV_POPULATE_WRITE);
+  }
+#endif
+}
 
 // A typed range inside a buffer that another member owns.
 template <class T>

@@ -48,6 +48,7 @@ struct MlpRec {
   // inference: a group's inputs, two chunks' outputs, the stream of the copies back
   DevBuf<float> xin;
   MlpChunk chunk[2];
+  PinBuf<float> h_small;                        // a small call's results (kSmallFloats)
   cudaStream_t back = nullptr;
   MlpScratch train_s, grad_s;
   DevBuf<float> grad_x, grad_y;                 // omg_mlp_grad's batch
@@ -70,6 +71,11 @@ struct MlpRec {
 }  // namespace omg
 
 namespace {
+
+// Results of at most this many floats come back through pinned memory, behind the
+// kernels: two copies into pageable memory, one after the other behind a wait, took 6
+// to 14 us more (a row of 1-16x1-1 57 us against 40, of 1024-64x2-8 104 against 81).
+constexpr uint64_t kSmallFloats = 1u << 14;
 
 constexpr uint32_t kGraphSteps = 8;   // training steps recorded in one graph
 
@@ -459,8 +465,11 @@ int32_t surrogate_run(omg_ctx* ctx, uint32_t id, const float* x, uint32_t n, flo
   const uint32_t wave = 128u * std::max(1u, (uint32_t)ctx->n_sms / E);
   const uint32_t parts = (n + wave - 1) / wave;
   const uint32_t chunk = std::min(n, ((n + parts - 1) / parts + 127u) / 128u * 128u);
-  const uint64_t group = (uint64_t)chunk * kGroup;
+  const uint64_t group = (uint64_t)chunk * kGroup, n_mean = (uint64_t)n * no, n_std = y_std ? n_mean : 0,
+                 n_spread = row_spread ? n : 0;
+  const bool small = n <= chunk && n_mean + n_std + n_spread <= kSmallFloats;
   cudaStream_t s = ctx->stream;
+  if (small && !M.h_small.p) CK(M.h_small.alloc(kSmallFloats));
   if (!M.back) CK(cudaStreamCreateWithFlags(&M.back, cudaStreamNonBlocking));
   if (M.xin.n < std::min<uint64_t>(n, group) * ni) CK(M.xin.alloc(std::min<uint64_t>(n, group) * ni));
   for (int k = 0; k < (n > chunk ? 2 : 1); k++) {
@@ -490,6 +499,12 @@ int32_t surrogate_run(omg_ctx* ctx, uint32_t id, const float* x, uint32_t n, flo
     CK(launch_mlp_rows(a, E, false, s));
     CK(launch_mlp_ensemble(C.y.p, E, rows, no, M.d_y_mean.p, M.d_y_std.p, level, C.mean.p, y_std ? C.std.p : nullptr,
                            row_spread ? C.spread.p : nullptr, s));
+    if (small) {
+      float* h = M.h_small.p;
+      CK(cudaMemcpyAsync(h, C.mean.p, n_mean * 4, cudaMemcpyDeviceToHost, s));
+      if (n_std) CK(cudaMemcpyAsync(h + n_mean, C.std.p, n_std * 4, cudaMemcpyDeviceToHost, s));
+      if (n_spread) CK(cudaMemcpyAsync(h + n_mean + n_std, C.spread.p, n_spread * 4, cudaMemcpyDeviceToHost, s));
+    }
     if (r0 + rows == n) CK(fetch_err(M, s));
     CK(cudaEventRecord(C.done, s));
     return OMG_OK;
@@ -505,6 +520,13 @@ int32_t surrogate_run(omg_ctx* ctx, uint32_t id, const float* x, uint32_t n, flo
     MlpChunk& C = M.chunk[(r0 / chunk) & 1u];
     const uint64_t rows = std::min<uint64_t>(chunk, n - r0);
     if ((rc = wait_event(ctx, C.done, timeout_of(ctx)))) return rc;
+    if (small) {
+      const float* h = M.h_small.p;
+      std::memcpy(y_mean, h, n_mean * 4);
+      if (n_std) std::memcpy(y_std, h + n_mean, n_std * 4);
+      if (n_spread) std::memcpy(row_spread, h + n_mean + n_std, n_spread * 4);
+      break;
+    }
     CK(cudaMemcpyAsync(y_mean + r0 * no, C.mean.p, rows * no * 4, cudaMemcpyDeviceToHost, M.back));
     if (y_std) CK(cudaMemcpyAsync(y_std + r0 * no, C.std.p, rows * no * 4, cudaMemcpyDeviceToHost, M.back));
     if (row_spread) CK(cudaMemcpyAsync(row_spread + r0, C.spread.p, rows * 4, cudaMemcpyDeviceToHost, M.back));

@@ -473,7 +473,7 @@ int32_t record_launch(omg_ctx* ctx, BatchRec& B, cudaStream_t s, int parts = 3) 
   }
   if (parts & 2) {
     CK(launch_finalize(B.d_jobs.p, B.n_jobs, B.d_acc.p, B.d_out.p, B.n_out, s));
-    CK(launch_reverb(B.d_rjobs.p, B.n_jobs, B.max_bins, B.d_out.p, B.d_reverb.p, B.d_seg.p, s));
+    CK(launch_reverb(B.d_rjobs.p, B.n_jobs, B.max_nb, B.max_bins, B.d_out.p, B.d_reverb.p, B.d_seg.p, s));
   }
   return OMG_OK;
 }

@@ -443,7 +443,7 @@ int32_t omg_estimate_reverb(omg_ctx* ctx, const float* bins, uint32_t n_bins, ui
   cudaStream_t s = ctx->stream;
   CK(cudaMemcpyAsync(ctx->r_bins.p, bins, total * 4, cudaMemcpyHostToDevice, s));
   CK(cudaMemcpyAsync(ctx->r_jobs.p, rj.data(), n_jobs * sizeof(DReverbJob), cudaMemcpyHostToDevice, s));
-  CK(launch_reverb(ctx->r_jobs.p, n_jobs, n_bins, ctx->r_bins.p, ctx->r_out.p, nullptr, s));
+  CK(launch_reverb(ctx->r_jobs.p, n_jobs, nb, n_bins, ctx->r_bins.p, ctx->r_out.p, nullptr, s));
   CK(cudaMemcpyAsync(out, ctx->r_out.p, n_jobs * sizeof(omg_reverb), cudaMemcpyDeviceToHost, s));
   cudaEvent_t ev;
   CK(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));

@@ -94,7 +94,7 @@ cudaError_t launch_late_update(const DLateUpdate* up, uint32_t n_up, const float
   const uint64_t n = (uint64_t)n_bins * (nb + 3);
   const uint32_t bx = (uint32_t)((n + 255) / 256 < 64 ? (n + 255) / 256 : 64);
   late_ema_kernel<<<dim3(bx, n_up), 256, 0, s>>>(up, n_up, fresh, avg, n_bins, nb);
-  cudaError_t e = launch_reverb(rj, n_up, n_bins, avg, rev, nullptr, s);
+  cudaError_t e = launch_reverb(rj, n_up, nb, n_bins, avg, rev, nullptr, s);
   if (e != cudaSuccess) return e;
   late_state_kernel<<<n_up, 32, 0, s>>>(up, n_up, avg, rev, version, state, n_bins, nb, from_bin, dir_band);
   return cudaGetLastError();

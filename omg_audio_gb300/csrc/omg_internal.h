@@ -336,7 +336,7 @@ struct DReverbJob {
   float bin_dt;
   uint32_t seg;        // index of the job's segment count
 };
-cudaError_t launch_reverb(const DReverbJob* rj, uint32_t n_jobs, uint32_t max_bins, const float* bins,
+cudaError_t launch_reverb(const DReverbJob* rj, uint32_t n_jobs, uint32_t nb, uint32_t max_bins, const float* bins,
                           omg_reverb* out, const uint32_t* job_segments, cudaStream_t s);
 // late.cu: blend each traced slot's fresh echogram (a batch output at
 // fresh + fresh_off) into the slot's average, then its reverb (rj: the slots'

@@ -655,9 +655,13 @@ __global__ void raycast_kernel(const DScene* __restrict__ scene, const float* __
 //   28 (4256 rays)    3.10    3.40    4.31     7.51          25.25           19.83
 //   56 (8512)         3.39    3.55    4.14     7.47          25.07           19.65
 // (84 and 112: 7.50 and 7.53 ms at 262,144). Shoeboxes, device-built trees (no
-// 4-wide form) and shapes with epochs, rounds or 4-wide walks have none.
+// 4-wide form) and shapes with epochs, rounds or 4-wide walks have none, nor has a
+// context with a walk budget of its own, which counts the lanes' visits: a whole warp
+// visits other nodes.
 uint32_t tail_rays(const LaunchShape& shape, uint32_t total_rays, int n_sms) {
-  if (shape.mode != 0 || shape.wide || shape.epochs || shape.wf_iters || !shape.solo_ok || shape.box_only) return 0;
+  if (shape.mode != 0 || shape.wide || shape.epochs || shape.wf_iters || !shape.solo_ok || shape.box_only ||
+      shape.capped)
+    return 0;
   const uint32_t unit = 28u * (uint32_t)n_sms;
   return total_rays < 3u * unit ? 0u : total_rays < 9u * unit ? unit : 2u * unit;
 }
@@ -680,8 +684,8 @@ cudaError_t launch_trace(const DJob* jobs, uint32_t n_jobs, uint32_t total_rays,
   // and 1.81 ms (near-tie rule), 0.82, 1.36, 2.18 against 1.51, 1.96, 2.38 ms
   // (first-found rule); on the 12-triangle room 0.46, 0.80, 1.40 against 0.79,
   // 0.89, 1.00 ms. Shoeboxes have no walk to share (a 4096-ray call 0.15
-  // against 0.14 ms).
-  if (!ep && shape.mode == 0 && !shape.wide && shape.solo_ok && !shape.box_only &&
+  // against 0.14 ms). A context with a walk budget of its own keeps the lanes (tail_rays).
+  if (!ep && !shape.capped && shape.mode == 0 && !shape.wide && shape.solo_ok && !shape.box_only &&
       total_rays <= 2u * 28u * (uint32_t)n_sms)
     return launch_trace_solo(jobs, n_jobs, total_rays, max_nb, scenes, job_mats, panels, acc, hdr, job_segments,
                              ea.max_loop, n_sms, tie, wt, s, shape.small);

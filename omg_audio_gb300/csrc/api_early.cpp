@@ -71,6 +71,7 @@ int32_t early_view(omg_ctx* ctx, const EarlyRec& R, DEarly& E) {
     E.root_hi[a] = R.root_hi[a];
   }
   E.err = R.words.p;
+  E.capped = ctx->prm.walk_budget != 0 ? 1u : 0u;
   E.n_sms = (uint32_t)ctx->n_sms;
   return OMG_OK;
 }

@@ -458,18 +458,20 @@ __device__ __forceinline__ void bounce_off(const DSurf& s, float hx, float hy, f
 }
 
 // After the last bounce: the source on this side of its plane, and ahead.
-__device__ __forceinline__ bool reaches_source(const DEarly& E, const omg_chain& ch, float px, float py, float pz,
-                                               float dx, float dy, float dz, float sx, float sy, float sz) {
+__device__ __forceinline__ bool same_side(const DEarly& E, const omg_chain& ch, float px, float py, float pz, float sx,
+                                          float sy, float sz) {
   if (ch.order == 0) return true;
   const DSurf& s = E.surf[ch.surf[ch.order - 1]];
-  if ((dot3(s.n, px, py, pz) - s.d) * (dot3(s.n, sx, sy, sz) - s.d) < 0.0f) return false;
+  return !((dot3(s.n, px, py, pz) - s.d) * (dot3(s.n, sx, sy, sz) - s.d) < 0.0f);
+}
+__device__ __forceinline__ bool ahead(const omg_chain& ch, float px, float py, float pz, float dx, float dy, float dz,
+                                      float sx, float sy, float sz) {
+  if (ch.order == 0) return true;
   const float qx = sx - px, qy = sy - py, qz = sz - pz;
   const float leg = len3(qx, qy, qz);
-  if (leg > 1e-4f) {
-    const float il = __frcp_rn(leg);
-    if ((qx * il) * dx + (qy * il) * dy + (qz * il) * dz < 0.995f) return false;
-  }
-  return true;
+  if (!(leg > 1e-4f)) return true;
+  const float il = __frcp_rn(leg);
+  return !((qx * il) * dx + (qy * il) * dy + (qz * il) * dz < 0.995f);
 }
 
 // What geometry alone says of a pair: false where mesh_record finds no path
@@ -485,7 +487,7 @@ __device__ __forceinline__ bool path_stands(const DEarly& E, const omg_chain& ch
     if (!plane_hit(s, px, py, pz, dx, dy, dz, t, hx, hy, hz)) return false;
     bounce_off(s, hx, hy, hz, px, py, pz, dx, dy, dz);
   }
-  return reaches_source(E, ch, px, py, pz, dx, dy, dz, sx, sy, sz);
+  return same_side(E, ch, px, py, pz, sx, sy, sz) && ahead(ch, px, py, pz, dx, dy, dz, sx, sy, sz);
 }
 
 // The leg's closest hit against the bounce at t: the bounce stands, ends the
@@ -553,8 +555,9 @@ __device__ bool mesh_record(const DEarly& E, const omg_chain& ch, uint16_t sourc
     for (int b = 0; b < 3; b++) gm[b] = gm[b] * s.refl[b];
     bounce_off(s, hx, hy, hz, px, py, pz, dx, dy, dz);
   }
-  if (!reaches_source(E, ch, px, py, pz, dx, dy, dz, sx, sy, sz)) return false;
+  if (!same_side(E, ch, px, py, pz, sx, sy, sz)) return false;
   if (!leg_transmission(E, px, py, pz, sx, sy, sz, false, 0u, 0.0f, extras, n_extras, W, gm)) return false;
+  if (!ahead(ch, px, py, pz, dx, dy, dz, sx, sy, sz)) return false;
   const float dtot = fmaxf(dist, 0.3f);
   const float kAir[3] = {1.0e-4f, 5.0e-4f, 3.0e-3f};  // AIR_ABSORPTION_PER_M, material.rs:76
   float gains[3];
@@ -610,7 +613,8 @@ __device__ __forceinline__ void no_record(omg_mesh_record& r, uint16_t source, c
 }
 
 // A thread per pair: what the pair's geometry decides without a walk. Pairs that
-// end there get their empty record; the others are listed.
+// end there get their empty record; the others are listed. (All of them where the
+// context has a walk budget of its own, which the walks of every pair count against.)
 __global__ void __launch_bounds__(kSiftThreads) early_sift_kernel(SolveArgs A) {
   const uint32_t i = blockIdx.x * kSiftThreads + threadIdx.x, lane = threadIdx.x & 31u;
   bool live = false;
@@ -618,7 +622,7 @@ __global__ void __launch_bounds__(kSiftThreads) early_sift_kernel(SolveArgs A) {
     const uint64_t k = A.first + i;
     const uint32_t s = (uint32_t)(k / A.n_chains), c = (uint32_t)(k % A.n_chains);
     const omg_chain ch = A.chains[c];
-    live = path_stands(A.E, ch, A.pos[3 * s], A.pos[3 * s + 1], A.pos[3 * s + 2], A.lx, A.ly, A.lz);
+    live = A.E.capped || path_stands(A.E, ch, A.pos[3 * s], A.pos[3 * s + 1], A.pos[3 * s + 2], A.lx, A.ly, A.lz);
     if (!live) no_record(A.out[k], A.ids[s], ch);
   }
   __syncwarp();

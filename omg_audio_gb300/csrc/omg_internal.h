@@ -447,6 +447,7 @@ struct DEarly {
   uint32_t n_boxes;
   float root_lo[3], root_hi[3];  // the tree's root box (segment_hits tests it first)
   uint32_t* err;              // error bits: 1 stack, 2 crossing list, 4 walk budget, 8 hash table
+  uint32_t capped;            // the context has a walk budget of its own
   uint32_t n_sms;
 };
 // Discovery: n_rays fan rays -> 3 candidates each (cand_key 0 = none), the

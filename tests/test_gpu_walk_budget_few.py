@@ -4,10 +4,12 @@ first-found rule refuse what the wavefront rounds do, which visit the nodes of t
 reference's walk alone. (A near-tie walk goes on while other lanes of its warp look for
 their leaves, so rays with fewer in their warp may do with less.) Early reflections count the walks of every pair, also of those that the
 pair's geometry ends after them."""
+import numpy as np
 import pytest
 
 from omg_audio_gb300 import Context, Job, TraceConfig, _lib
 from omg_audio_gb300 import workloads as W
+from omg_audio_gb300.early import WorldEarly
 
 from test_gpu_parity import gpu_scene
 
@@ -63,4 +65,54 @@ def test_trace_of_few_rays(tie, mesh, rays):
         assert accepted(few, 0) == want
         few.destroy()
         many.destroy()
+        scene.release()
+
+
+def test_early_pairs_count_their_walks():
+    with Context(TraceConfig()) as ctx:
+        case = W.multiroom(seed=6)
+        scene = gpu_scene(ctx, case.recorder)
+        early, lis = WorldEarly(ctx, scene), case.pairs[0][1]
+        chains = [c for c in early.discover(lis, 768, 1) if c[1] == 1]
+        # sources far behind every surface that the chains name: no path, after a walk each
+        sources = [(k, (lis[0] + d[0], lis[1] + d[1], lis[2] + d[2]))
+                   for k, d in enumerate(np.vstack([np.eye(3), -np.eye(3)]) * 55.0)]
+        want = early.solve(sources, chains, lis)
+
+        def accepted(budget):
+            ctx.set_limits(walk_budget=budget)
+            try:
+                return early.solve(sources, chains, lis)
+            except _lib.OmgError as err:
+                assert err.status == _lib.E_OVERFLOW
+                return None
+
+        lo = _least(lambda m: accepted(m) is not None)
+        assert np.array_equal(accepted(lo), want)
+        # the reference's walk to the first chain's surface alone visits more than this
+        assert lo > 8 and accepted(8) is None
+        ctx.set_limits(0, 0)
+        early.close()
+        scene.release()
+
+
+def test_early_pair_that_geometry_ends():
+    """A source below the floor that its chain names: the walk to the floor comes first."""
+    with Context(TraceConfig()) as ctx:
+        case = W.shoebox12(seed=1)
+        scene = gpu_scene(ctx, case.recorder)
+        early, lis = WorldEarly(ctx, scene), (4.0, 3.0, 2.0)
+        chains = [c for c in early.discover(lis, 768, 1) if c[1] == 1]
+        up = early.solve([(1, (4.5, 3.2, 1.5))], chains, lis)[0]
+        floor = [c for c, r in zip(chains, up) if r["valid"] and r["dir"][2] < -0.5]
+        assert len(floor) == 1
+        below = [(1, (4.5, 3.2, -1.5))]
+        assert not early.solve(below, floor, lis)["valid"].any()
+        ctx.set_limits(walk_budget=1)
+        with pytest.raises(_lib.OmgError) as err:
+            early.solve(below, floor, lis)
+        assert err.value.status == _lib.E_OVERFLOW
+        ctx.set_limits(0, 0)
+        assert not early.solve(below, floor, lis)["valid"].any()
+        early.close()
         scene.release()

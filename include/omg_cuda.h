@@ -586,7 +586,8 @@ int32_t omg_mlp_grad(omg_ctx* ctx, uint32_t mlp_id, uint32_t member, const float
  * out = NULL returns the count only. set_params restores the same layout. */
 int32_t omg_mlp_params(omg_ctx* ctx, uint32_t mlp_id, uint32_t what, float* out, uint64_t* count);
 int32_t omg_mlp_set_params(omg_ctx* ctx, uint32_t mlp_id, uint32_t what, const float* in, uint64_t count);
-/* The tensor-core GEMM alone (tests): C[m x n] = A[m x k] . B[n x k]^T, A and B
+/* A tensor-core GEMM of its own (not the surrogate's kernels, which run whole passes a
+ * launch; its times say nothing of theirs): C[m x n] = A[m x k] . B[n x k]^T, A and B
  * bf16 bit patterns, row-major with k contiguous; C f32. */
 int32_t omg_tc_gemm(omg_ctx* ctx, const uint16_t* a, const uint16_t* b, float* c, uint32_t m, uint32_t n,
                     uint32_t k);

@@ -1,6 +1,6 @@
 // C ABI of the GB300 tracer (include/omg_cuda.h), part 4: the learned
 // surrogate. An ensemble of MLPs (n_in -> hidden x n_hidden -> n_out, GELU)
-// trained on the GPU with the tensor-core GEMM (mlp.cu): BF16 weights and
+// trained and run by the tensor-core kernels of mlp_net.cu: BF16 weights and
 // activations, FP32 accumulation, FP32 master weights, AdamW with a cosine
 // learning-rate decay, MSE on standardized targets. Inference returns the
 // ensemble mean and spread in the caller's units.

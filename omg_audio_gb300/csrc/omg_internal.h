@@ -29,10 +29,10 @@
 namespace omg {
 
 constexpr int MAXB = OMG_MAX_BANDS;
-constexpr int STACK_DEPTH = 64;
-// Histogram bins of one echogram at most (the reverb estimate holds one band's
-// FP64 curve in a block's shared memory).
-constexpr uint32_t kMaxBins = 19370;           // mesh.rs:492 (64-entry traversal stack)
+constexpr int STACK_DEPTH = 64;                // mesh.rs:492 (64-entry traversal stack)
+// Histogram bins of one echogram at most: the ABI's limit, from a reverb estimate that
+// took 12 bytes a bin of a block's 227 KB (it takes 8 now, 155 KB).
+constexpr uint32_t kMaxBins = 19370;
 
 // tracer.rs:148-182 per material: p = clamp(max_b T_b^2, 0.02, 0.5) when
 // > 1e-5 else 0; transmitted weight T_b^2 / p; reflected weight
@@ -202,7 +202,7 @@ struct LaunchShape {
   uint32_t blocks_per_sm = 4;
   uint32_t refill_min = 1;      // a warp refetches rays once this many lanes are idle
   uint32_t walk_steps = 0;      // traversal steps per lane per loop iteration (0 = a whole walk)
-  uint32_t shade_min = 32;      // kept in the interface: mode 0 shades all of a warp's rays after all of their walks
+  uint32_t shade_min = 32;      // kept and returned, read by no kernel: mode 0 shades a warp's rays after all walks
   uint32_t mode = 0;            // persistent kernel: 0 lane state machine, 1 warp-local wavefront,
                                 // 2 cooperative 4-lane walks
   uint32_t tail_mode = 0;       // the persistent kernel of epochs after the first

@@ -10,10 +10,12 @@
 // only on the set of hits (device_common.cuh), so the walk keeps every hit that
 // may lie in the final window and takes the lowest key in it at the end.
 // First-found rule: the walk goes over the reference's own boxes with its slab
-// test, through every leaf that the ray meets (nothing is culled: in the
-// reference's order a leaf beyond the nearest hit may come before it), and
-// first_of says which hit the reference's ordered walk ends with. Where a list
-// is full, one lane walks alone.
+// test, through every leaf that the ray meets, and first_of says which hit the
+// reference's ordered walk ends with. Nothing is culled: first_of needs every hit up
+// to its bound m, which the last leaf may still move, and a hit's computed distance may
+// lie before its own leaf's computed entry, so the nearest hit so far does not say
+// which leaves are out (a wider bound would, with such hits left to the lane's walk;
+// not built). Where a list is full, one lane walks alone.
 #pragma once
 
 #include "device_common.cuh"

@@ -1,9 +1,11 @@
 // Tensor-core GEMM building blocks for sm_103a (tcgen05 + TMEM), written as
 // inline PTX: shared-memory matrix descriptors, the kind::f16 instruction
 // descriptor, TMEM allocation, MMA issue / commit, bounded mbarrier waits and
-// TMEM loads. Used by the surrogate MLP (mlp.cu).
+// TMEM loads. Used by the surrogate's network (mlp_net.cu), whose operands are images
+// without a chunked K (smem_desc with the caller's strides), and by the plain GEMM of
+// the C ABI (mlp.cu), whose operand layout is this:
 //
-// Operand layout in shared memory: K-major, no swizzle. A tile of R rows x 64
+// Shared memory, K-major, no swizzle. A tile of R rows x 64
 // K elements (bf16) is stored as 8-row x 8-element core matrices (8 rows of
 // 16 bytes, 128 B each); the 8 core matrices along K of one 8-row group are
 // contiguous (leading-dimension byte offset 128 B) and 8-row groups are
